@@ -202,6 +202,73 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     }
 }
 
+// Barriers by their shared-memory address (smem_u32): a warp-specialised pipeline touches several per
+// step, and 64-bit generic pointers cost it three to four instructions per access.
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {   // may suspend the thread for a hardware-defined time
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {   // answers at once
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t addr) {
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ ulonglong2 lds128(uint32_t addr) {
+    ulonglong2 v;
+    asm volatile("ld.shared.v2.u64 {%0,%1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
+
+// A bounded wait for the hand-offs inside a warp-specialised pipeline (see mbar_wait_bounded): no
+// sleeping, the hardware suspends a waiting thread for a while by itself.
+__device__ __forceinline__ void mbar_spin_slow(uint32_t bar, uint32_t parity, uint32_t abort, uint64_t limit_ns);
+__device__ __forceinline__ void mbar_spin(uint32_t bar, uint32_t parity, uint32_t abort, uint64_t limit_ns) {
+    if (!mbar_try_wait(bar, parity)) mbar_spin_slow(bar, parity, abort, limit_ns);
+}
+__device__ __forceinline__ void mbar_spin_slow(uint32_t bar, uint32_t parity, uint32_t abort, uint64_t limit_ns) {
+    uint64_t t0 = 0;
+    for (uint32_t polls = 1;; ++polls) {
+        if (mbar_try_wait(bar, parity)) return;
+        if (polls & 63u) continue;
+        if (lds32(abort)) return;
+        const uint64_t now = global_ns();
+        if (t0 == 0) {
+            t0 = now;
+        } else if (now - t0 > limit_ns) {
+            sts32(abort, 1u);
+            return;
+        }
+    }
+}
+
 // Touches the line at p without using it: the address translation (and the line in the L2) is there
 // by the time a dependent access needs it. Used before griddepcontrol.wait, on buffers whose
 // first access would otherwise pay a translation miss in the middle of a latency chain.
@@ -239,11 +306,10 @@ __device__ __forceinline__ uint64_t l2_policy_evict_normal() {   // the default 
     asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(policy));
     return policy;
 }
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
+__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {   // shared-memory addresses
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
+__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) { bulk_g2s(smem_u32(dst), src, bytes, smem_u32(bar)); }
 
 // Non-blocking arrival at a hardware barrier that other threads bar.sync on.
 __device__ __forceinline__ void named_bar_arrive(int id, int threads) {

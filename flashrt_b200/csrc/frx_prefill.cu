@@ -4,25 +4,27 @@
 // Numerics are the decode path's, i.e. the reference CPU path's: int8 activation codes per 32
 // values, exact integer dot products per 32-block, then scale and accumulate in the reference's
 // order and roundings. The tensor core does only the exact part. Operands are small integers held
-// in fp16 -- the weight codes q - 1 in {-1, 0, 1, 2} and the activation codes in [-127, 127] -- so
-// every product and every partial sum of one 32-block (|sum| <= 8128) is exact in the fp32
-// accumulator. Each 64-weight block therefore yields two accumulators S0, S1 per (row, token) in
-// tensor memory, which the epilogue warps turn into d * (a0 * S0 + a1 * S1) and add to running
-// sums held in registers, block after block.
+// in e4m3: the weight codes q - 1 in {-1, 0, 1, 2}, and every activation code as the sum of two
+// e4m3 values, a multiple of 16 in [-128, 128] and a rest in [-8, 7]. The two products of a
+// 32-block go into one accumulator, so it holds the block's integer sum (|sum| <= 8128), exact.
+// Each 64-weight block yields two accumulators S0, S1 per (row, token) in tensor memory, which the
+// epilogue warps turn into d * (a0 * S0 + a1 * S1) and add to running sums held in registers, block
+// after block.
 //
-// Per CTA (one per SM), warp roles: 0 = TMA producer, 1 = MMA issuer and tensor-memory owner,
-// 2-3 = dequant (2-bit codes of 128 rows x 64 weights -> fp16 core-matrix layout in shared
-// memory), 4-19 = epilogue (tensor memory -> registers, scaling, stores of the (gate, up) sums or
-// the output rows): each epilogue warp owns 32 rows (its quarter of the tensor-memory lanes) x 32
-// token columns. 640 threads leave 96 registers per thread, which lets an epilogue thread fetch
-// 16 columns of both sums per round trip to tensor memory (a round trip costs several hundred
-// cycles whatever its size). Hand-offs are shared-memory barriers; a barrier operation has about a
-// hundred cycles of latency and a thread's steps are serial, so each role tests the next step's
-// barriers while it still works on the current one.
-// All waits are bounded; a wait that runs out sets the workspace status word and the block drains.
+// One block per SM works on tiles of 256 matrix rows x up to 48 tokens of one expert, in units of 128
+// weights of K. Warps: packed weights (bulk copies), activations and scales (bulk copies), two MMA
+// issuers (one per row tile of 128), eight dequant warps (2-bit codes -> e4m3, written to tensor memory,
+// which spares shared memory the A operand's traffic: 48 KB per unit), sixteen epilogue warps. Tensor
+// memory: 384 columns of sums (two 64-blocks), 128 of weights. What bounds it: the fp32 pipe in
+// principle (four packed operations per two sums, 770 cycles per unit), in practice the issue slots
+// (5,400 warp instructions per unit, a packed operation taking two slots) and the hand-off of the two
+// sets of sums between the MMAs and the epilogue (about 600 cycles round trip). A unit takes 1,900
+// cycles. 16,384 tokens, 512 experts top-10, hidden 2048, width 512: gate/up 1,585 us, down 1,060 us; before, with
+// fp16 operands in shared memory, tiles of 128 x 128 and a hand-off per 64 weights: 2,520 and 1,620.
 #include "frx_umma.cuh"
 
 #include <cuda_bf16.h>
+#include <cuda_fp8.h>
 
 #include <mutex>
 
@@ -32,27 +34,34 @@ namespace {
 #include "frx_group.cuh"
 
 constexpr int kTileRows = 128;     // M of the MMA: 8 groups of 16 matrix rows
-constexpr int kTileTok = 128;      // most tokens of one tile (N of the MMA), a multiple of 16
+constexpr int kRowTiles = 2;       // row tiles of a block's tile: 256 matrix rows share the activations
+constexpr int kTileTok = 48;       // most tokens of one tile (N of the MMA), a multiple of 16
 constexpr int kTokPad = 16;        // every expert's token count is padded to this
-// fp16 A tile of one 64-block: 16 groups of 8 rows, each 8 core matrices (8 rows x 16 bytes) 192
-// bytes apart rather than 128, so that the dequant warps' 8-byte stores to two neighbouring
-// chunks fall into different banks
-constexpr int kALbo = 192, kASbo = 8 * kALbo;
-constexpr int kStepBytesA = (kTileRows / 8) * kASbo;   // 24 KB
-constexpr int kStepBytesB = kTileTok * 64 * 2;    // fp16 B tile of one 64-block: 16 KB
-constexpr int kStepBytesS = kTileTok * 8;         // activation scales of one 64-block: 1 KB
-constexpr int kUnitTileBytes = 8 * kUnitBytes;    // packed weights of 8 groups x one unit: 4608 B
-constexpr int kStagesW = 8, kStagesA = 4, kStagesB = 4, kStagesD = 2;
-static_assert(kStagesA == kStagesB, "one barrier frees an A and a B stage together");
-constexpr int kStageColsD = 2 * kTileTok;   // tensor-memory columns of one step: the two 32-value sums of every token
-static_assert(kStagesD * kStageColsD <= 512, "tensor memory has 512 columns");
-constexpr int kWarpsDequant = 2, kWarpsEpilogue = 16;
-constexpr int kThreads = (2 + kWarpsDequant + kWarpsEpilogue) * 32;   // 640: 96 registers per thread
-constexpr int kGroupsPerDequantWarp = 8 / kWarpsDequant;             // 16-row groups of the tile per dequant warp
+constexpr int kBlockBytesB = kTileTok * 128;       // one 64-block: 64 values x 2 e4m3 pieces per token
+constexpr int kUnitBytesB = 2 * kBlockBytesB;      // one unit (128 weights of K): 12 KB
+constexpr int kBlockBytesS = kTileTok * 8;         // activation scales of one 64-block
+constexpr int kUnitBytesS = 2 * kBlockBytesS + kRowTiles * kTileRows * 4;   // and the two block scales of every row
+constexpr int kTileBytesW = 8 * kUnitBytes;        // packed weights of one row tile x one unit: 4608 B
+constexpr int kUnitBytesW = kRowTiles * kTileBytesW;
+constexpr int kStagesW = 8, kStagesB = 8, kStagesS = 16, kStagesA = 2;   // units in flight: packed weights, activations, scales, e4m3 weights
+// Scale slots are not handed back by a barrier: activations of unit g are fetched once the MMAs of
+// unit g - kStagesB have completed, which waited for the epilogue to read the accumulators of the unit
+// before, so every unit up to g - kStagesB - 2 is finished.
+static_assert(kStagesS >= kStagesB + 2, "a scale slot may still be in use");
+// Tensor memory: the sums of the two 64-blocks of a unit (per row tile two 32-value sums of every
+// token), then the e4m3 weights (32 columns of four bytes per row tile and unit).
+constexpr int kColsRow = 2 * kTileTok, kColsBlock = kRowTiles * kColsRow, kColsA = kRowTiles * 32, kColA0 = 2 * kColsBlock;
+constexpr int kTmemCols = 512;
+static_assert(kColA0 + kStagesA * kColsA <= kTmemCols, "tensor memory has 512 columns");
+constexpr int kWarpsDequant = 8, kWarpsAux = 4 + kWarpsDequant, kWarpsEpilogue = 16;
+constexpr int kThreads = (kWarpsAux + kWarpsEpilogue) * 32;
+// registers: 896 threads are launched with 72 each; the auxiliary warps give up 32 of theirs, the
+// epilogue warps take 24 more: 384 * 40 + 512 * 96 = 896 * 72
+constexpr int kRegsAux = 40, kRegsEpilogue = 96;
 
 // meta words: [0] padded positions in use, [1] token blocks
 struct PfuLayout {
-    size_t status, chunk_cnt, bounds, item_off, perm, pb, tbo, meta, tb_e, tb_p0, tb_n, pslot, xq, xd, xg, xa, hf, hg, ha, total;
+    size_t status, chunk_cnt, bounds, item_off, perm, pb, tbo, meta, tb_e, tb_p0, tb_n, pslot, xe, xd, xg, xa, hf, hg, ha, total;
     int n_chunks, max_tb;
     size_t pmax;
 };
@@ -81,7 +90,7 @@ PfuLayout pfu_layout(int T, int K, int n, int ff, int E) {
     L.tb_p0 = take(size_t(L.max_tb) * 4);
     L.tb_n = take(size_t(L.max_tb) * 4);
     L.pslot = take(L.pmax * 4);
-    L.xq = take(size_t(T) * n);
+    L.xe = take(size_t(T) * n * 2);
     L.xd = take(size_t(T) * (n / kQ8) * 4);
     L.xg = take(L.pmax * n * 2);
     L.xa = take(L.pmax * (n / kQK) * 8);
@@ -94,7 +103,8 @@ PfuLayout pfu_layout(int T, int K, int n, int ff, int E) {
 
 // ---------------------------------------------------------------------------------------------
 // Plan: pad every expert's slot count to 16 (padded position space p), cut it into token blocks of
-// at most 128. One block of 1024 threads.
+// at most kTileTok, as equal as multiples of 16 allow (a tile costs its fixed steps whatever its
+// width). One block of 1024 threads.
 __global__ void __launch_bounds__(1024) k_pfu_plan(const int* __restrict__ bounds, int E, int* __restrict__ pb, int* __restrict__ tbo,
                                                    int* __restrict__ meta, int* __restrict__ tb_e, int* __restrict__ tb_p0,
                                                    int* __restrict__ tb_n, int max_tb, int* __restrict__ status) {
@@ -131,10 +141,12 @@ __global__ void __launch_bounds__(1024) k_pfu_plan(const int* __restrict__ bound
         const int c = bounds[e + 1] - bounds[e], pc = (c + kTokPad - 1) / kTokPad * kTokPad;
         pb[e] = at_p;
         tbo[e] = at_t;
-        for (int j = 0; j * kTileTok < c; ++j) {
+        const int nblk = (c + kTileTok - 1) / kTileTok, n16 = pc / kTokPad;
+        for (int j = 0; j < nblk; ++j) {
+            const int lo = n16 * j / nblk, hi = n16 * (j + 1) / nblk;
             tb_e[at_t] = e;
-            tb_p0[at_t] = at_p + j * kTileTok;
-            tb_n[at_t] = min(kTileTok, pc - j * kTileTok);
+            tb_p0[at_t] = at_p + lo * kTokPad;
+            tb_n[at_t] = (hi - lo) * kTokPad;
             ++at_t;
         }
         at_p += pc;
@@ -147,9 +159,31 @@ __global__ void __launch_bounds__(1024) k_pfu_plan(const int* __restrict__ bound
     }
 }
 
-// Offset, in bytes, of the 16-byte chunk `c` (8 fp16 values of K) of padded position p in the
-// grouped fp16 operand: [64-block][p / 8][chunk 0..7][p % 8][16 bytes] -- the MMA's K-major
-// core-matrix order, so a token block's tile for one 64-block is one contiguous range.
+// The e4m3 pieces of activation codes. A 64-block of one token is 128 bytes, eight 16-byte chunks
+// [half s][piece: 0 the multiple of 16, 1 the rest][c]; inside a half, element 16 q + 4 t + i sits in
+// chunk c = t >> 1 at byte (t & 1) * 8 + q * 4 + i: the order in which a lane of the dequant warps
+// writes the weights' bytes. This is the place of the four codes of element group (s, q, t).
+__device__ __forceinline__ int piece_chunk(int s, int piece, int t) { return s * 4 + piece * 2 + (t >> 1); }
+__device__ __forceinline__ int piece_byte(int q, int t) { return (t & 1) * 8 + q * 4; }
+
+// Four int8 codes (as ints in [-127, 127]) -> their multiples of 16 and their rests as e4m3 bytes (exact:
+// four significant bits are enough for either).
+__device__ __forceinline__ void split_codes(const int (&c)[4], uint32_t& hi, uint32_t& lo) {
+    float h[4], l[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int rest = ((c[i] + 8) & 15) - 8;
+        l[i] = float(rest);
+        h[i] = float(c[i] - rest);
+    }
+    auto two = [](float a, float b) { return uint32_t(__nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3)); };
+    hi = two(h[0], h[1]) | (two(h[2], h[3]) << 16);
+    lo = two(l[0], l[1]) | (two(l[2], l[3]) << 16);
+}
+
+// Offset, in bytes, of 16-byte chunk `chunk` of 64-block b64 of padded position p in the grouped
+// operand: [64-block][p / 8][chunk 0..7][p % 8][16 bytes] -- the MMA's K-major core-matrix order, so
+// a token block's tile for one 64-block is one contiguous range.
 __device__ __forceinline__ size_t grouped_chunk_off(size_t pmax, int b64, int p, int chunk) {
     return (((size_t(b64) * (pmax / 8) + size_t(p >> 3)) * 8 + size_t(chunk)) * 8 + size_t(p & 7)) * 16;
 }
@@ -158,11 +192,50 @@ __device__ __forceinline__ size_t grouped_scale_idx(size_t pmax, int b64, int p,
     return (size_t(b64) * pmax + size_t(p & ~1)) * 2 + size_t(half) * 2 + size_t(p & 1);
 }
 
-// Gather: for every padded position, its slot (or -1), the int8 codes of the slot's token as fp16
-// in the grouped operand layout, and the token's block scales. Block = 8 positions x 32 chunks.
+// Q8 of x rows (q2_0::quantize_q8, quant/q2_0/q2_0.cpp:101-113) straight into e4m3 pieces, token-major
+// [T][n / 64][128 bytes], and the block scales d [T][n / 32]. A thread owns four consecutive values,
+// eight neighbouring lanes one 32-block. n_quads is a multiple of 32: warps are live as a whole.
+__global__ void __launch_bounds__(256) k_pfu_quant_x(const float* __restrict__ x, size_t n_quads, uint8_t* __restrict__ xe,
+                                                     float* __restrict__ d, int block64) {
+    const size_t quad = size_t(blockIdx.x) * 256 + threadIdx.x;
+    if (quad >= n_quads) return;
+    const float4 v = reinterpret_cast<const float4*>(x)[quad];
+    float am = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
+    if (block64) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 8));
+    const float dd = __fdiv_rn(am, 127.0f);
+    const float id = dd != 0.0f ? __fdiv_rn(1.0f, dd) : 0.0f;
+    const int c[4] = {int(round_half_away(__fmul_rn(v.x, id))), int(round_half_away(__fmul_rn(v.y, id))), int(round_half_away(__fmul_rn(v.z, id))),
+                      int(round_half_away(__fmul_rn(v.w, id)))};
+    uint32_t hi, lo;
+    split_codes(c, hi, lo);
+    const int j = int(quad & 7), s = int(quad >> 3) & 1, q = j >> 2, t = j & 3;
+    uint8_t* blk = xe + (quad >> 4) * 128;
+    *reinterpret_cast<uint32_t*>(blk + piece_chunk(s, 0, t) * 16 + piece_byte(q, t)) = hi;
+    *reinterpret_cast<uint32_t*>(blk + piece_chunk(s, 1, t) * 16 + piece_byte(q, t)) = lo;
+    if (j == 0) d[quad >> 3] = __half2float(__float2half_rn(dd));
+}
+
+// The same pieces from codes that arrive already quantized (natural order, as frx_quantize_q8 writes them).
+__global__ void __launch_bounds__(256) k_pfu_expand_q8(const int8_t* __restrict__ xq, size_t n_quads, uint8_t* __restrict__ xe) {
+    const size_t quad = size_t(blockIdx.x) * 256 + threadIdx.x;
+    if (quad >= n_quads) return;
+    const char4 v = reinterpret_cast<const char4*>(xq)[quad];
+    const int c[4] = {v.x, v.y, v.z, v.w};
+    uint32_t hi, lo;
+    split_codes(c, hi, lo);
+    const int j = int(quad & 7), s = int(quad >> 3) & 1, q = j >> 2, t = j & 3;
+    uint8_t* blk = xe + (quad >> 4) * 128;
+    *reinterpret_cast<uint32_t*>(blk + piece_chunk(s, 0, t) * 16 + piece_byte(q, t)) = hi;
+    *reinterpret_cast<uint32_t*>(blk + piece_chunk(s, 1, t) * 16 + piece_byte(q, t)) = lo;
+}
+
+// Gather: for every padded position, its slot (or -1), the e4m3 pieces of the slot's token in the
+// grouped operand layout, and the token's block scales. Block = 8 positions x 32 chunks.
 __global__ void __launch_bounds__(256) k_pfu_gather(const int* __restrict__ bounds, const int* __restrict__ pb, int E,
                                                     const int32_t* __restrict__ perm, const int* __restrict__ meta, int K, int n,
-                                                    size_t pmax, const int8_t* __restrict__ xq, const float* __restrict__ xd,
+                                                    size_t pmax, const uint8_t* __restrict__ xe, const float* __restrict__ xd,
                                                     uint8_t* __restrict__ xg, float* __restrict__ xa, int32_t* __restrict__ pslot) {
     const int r = threadIdx.x & 7, cl = threadIdx.x >> 3;
     const int p = blockIdx.x * 8 + r;
@@ -179,14 +252,7 @@ __global__ void __launch_bounds__(256) k_pfu_gather(const int* __restrict__ boun
     const int chunks = n / 8, nb = n / kQK;
     for (int ch = cl; ch < chunks; ch += 32) {
         uint4 out = make_uint4(0u, 0u, 0u, 0u);
-        if (slot >= 0) {
-            const uint2 q = *reinterpret_cast<const uint2*>(xq + size_t(t) * n + size_t(ch) * 8);
-            const int8_t* b = reinterpret_cast<const int8_t*>(&q);
-            __half2 h[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) h[i] = __halves2half2(__int2half_rn(int(b[2 * i])), __int2half_rn(int(b[2 * i + 1])));
-            out = *reinterpret_cast<const uint4*>(h);
-        }
+        if (slot >= 0) out = *reinterpret_cast<const uint4*>(xe + size_t(t) * n * 2 + size_t(ch) * 16);
         *reinterpret_cast<uint4*>(xg + grouped_chunk_off(pmax, ch >> 3, p, ch & 7)) = out;
     }
     for (int b = cl; b < nb; b += 32) {
@@ -197,41 +263,18 @@ __global__ void __launch_bounds__(256) k_pfu_gather(const int* __restrict__ boun
     }
 }
 
-// Natural-order Q8 of x rows (q2_0::quantize_q8): warp per 32-block.
-__device__ __forceinline__ int q8_block_pf(float v, float& d_out, float partner) {
-    float am = fmaxf(fabsf(v), fabsf(partner));   // partner: the other half of a 64-value scale block (block64), else 0
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
-    const float d = __fdiv_rn(am, 127.0f);
-    const float id = d != 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
-    d_out = __half2float(__float2half_rn(d));
-    return int(round_half_away(__fmul_rn(v, id)));
-}
-
-__global__ void __launch_bounds__(256) k_pfu_quant_x(const float* __restrict__ x, size_t n_blocks, int8_t* __restrict__ q,
-                                                     float* __restrict__ d, int block64) {
-    const size_t blk = size_t(blockIdx.x) * 8 + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (blk >= n_blocks) return;
-    float dd;
-    const int c = q8_block_pf(x[blk * kQ8 + lane], dd, block64 ? x[(blk ^ 1) * kQ8 + lane] : 0.0f);
-    q[blk * kQ8 + lane] = int8_t(c);
-    if (lane == 0) d[blk] = dd;
-}
-
-// Q8 of the hidden rows (one row of ff per padded position) straight into the grouped fp16
-// operand layout and scale table of the down product. A thread owns 8 consecutive hidden values
-// (one 16-byte chunk of the operand), four neighbouring lanes one 32-block: silu(gate x) * up x is
-// formed here (eight independent exponentials per thread hide their latency), the block maximum
-// comes from two shuffles, and each thread stores its chunk whole.
+// Q8 of the hidden rows (one row of ff per padded position) straight into the grouped operand
+// layout and scale table of the down product. A thread owns 8 consecutive hidden values, four
+// neighbouring lanes one 32-block: silu(gate x) * up x is formed here (eight independent
+// exponentials per thread hide their latency) and the block maximum comes from two shuffles.
 __global__ void __launch_bounds__(256) k_pfu_quant_h(const float2* __restrict__ hf, int ff, size_t pmax, const int* __restrict__ meta,
                                                      const int32_t* __restrict__ pslot, uint8_t* __restrict__ hg, float* __restrict__ ha,
                                                      int block64) {
-    const int cpr = ff / 8;   // chunks per row
+    const int cpr = ff / 8;   // threads per row
     const size_t chunk = size_t(blockIdx.x) * 256 + threadIdx.x;
     const size_t p = chunk / cpr;
     const bool in_range = p < size_t(meta[0]);   // no early exit: the shuffles below need the whole warp
-    const int c = int(chunk % cpr);              // chunk of the row: values 8 c .. 8 c + 7
+    const int c = int(chunk % cpr);              // values 8 c .. 8 c + 7 of the row
     const bool live = in_range && pslot[p] >= 0;
     float hv[8];
     float am = 0.0f;
@@ -255,15 +298,23 @@ __global__ void __launch_bounds__(256) k_pfu_quant_h(const float2* __restrict__ 
     // quant/q2_0/q2_0.cpp:101-113: d = amax / 127, id = 1 / d, q = roundf(v * id), d through fp16
     const float d = __fdiv_rn(am, 127.0f);
     const float id = d != 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
-    __half2 h[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-        h[i] = __halves2half2(__int2half_rn(int(round_half_away(__fmul_rn(hv[2 * i], id)))),
-                              __int2half_rn(int(round_half_away(__fmul_rn(hv[2 * i + 1], id)))));
-    const int b64 = c >> 3, k8 = c & 7;   // the 64-block and the chunk inside it
     if (!in_range) return;
-    *reinterpret_cast<uint4*>(hg + grouped_chunk_off(pmax, b64, int(p), k8)) = *reinterpret_cast<const uint4*>(h);
-    if ((c & 3) == 0) ha[grouped_scale_idx(pmax, b64, int(p), k8 >> 2)] = __half2float(__float2half_rn(d));
+    const int b64 = c >> 3, s = (c >> 2) & 1, q = (c >> 1) & 1;   // values 32 s + 16 q + 8 (c & 1) .. of the 64-block: groups t = 2 (c & 1), + 1
+    uint32_t hi[2], lo[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        int code[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) code[i] = int(round_half_away(__fmul_rn(hv[4 * u + i], id)));
+        split_codes(code, hi[u], lo[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int t = 2 * (c & 1) + u;
+        *reinterpret_cast<uint32_t*>(hg + grouped_chunk_off(pmax, b64, int(p), piece_chunk(s, 0, t)) + piece_byte(q, t)) = hi[u];
+        *reinterpret_cast<uint32_t*>(hg + grouped_chunk_off(pmax, b64, int(p), piece_chunk(s, 1, t)) + piece_byte(q, t)) = lo[u];
+    }
+    if ((c & 3) == 0) ha[grouped_scale_idx(pmax, b64, int(p), s)] = __half2float(__float2half_rn(d));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -274,7 +325,7 @@ struct UmmaParams {
     const int* tb_e;
     const int* tb_p0;
     const int* tb_n;
-    const uint8_t* act;       // grouped fp16 codes (xg or hg)
+    const uint8_t* act;       // grouped e4m3 codes (xg or hg)
     const float* act_scale;   // grouped block scales (xa or ha)
     const int32_t* pslot;
     float2* hf;               // gate/up: (gate x, up x) of every hidden element [pmax][ff]
@@ -282,29 +333,25 @@ struct UmmaParams {
     int* status;
     size_t pmax;
     unsigned long long wait_ns;   // the longest a wait on a shared-memory barrier may last
+    float neg0;               // -0.0f, an addend the compiler does not know (see scale_add)
     int n, ff;
     int y_bf16;               // down: yd holds bf16 rows
 };
 
 struct PfSmem {
-    uint32_t w, a, b, s, sw, bars, tmem, abort, total;
+    uint32_t w, b, s, bars, tmem, abort, total;
 };
 __host__ __device__ constexpr PfSmem pf_smem() {
     PfSmem m{};
     uint32_t off = 0;
-    m.w = off;
-    off += kStagesW * kUnitTileBytes;
-    off = (off + 1023u) & ~1023u;
-    m.a = off;
-    off += kStagesA * kStepBytesA;
     m.b = off;
-    off += kStagesB * kStepBytesB;
+    off += kStagesB * kUnitBytesB;
+    m.w = off;
+    off += kStagesW * kUnitBytesW;
     m.s = off;
-    off += kStagesB * kStepBytesS;
-    m.sw = off;
-    off += kStagesA * kTileRows * 4;
+    off += kStagesS * kUnitBytesS;
     m.bars = off;
-    off += 48 * 8;
+    off += 64 * 8;
     m.tmem = off;
     off += 16;
     m.abort = off;
@@ -313,291 +360,375 @@ __host__ __device__ constexpr PfSmem pf_smem() {
     return m;
 }
 
-// Barrier indices
+// Barrier indices (a unit is 128 weights of K; its uses of a barrier are numbered by the unit)
 enum : int {
-    kBarWFull = 0,                      // + stage: packed weights of a unit have landed
-    kBarWFree = kBarWFull + kStagesW,   // dequant warps are done with them
-    kBarAFull = kBarWFree + kStagesW,   // fp16 A tile written
-    kBarAFree = kBarAFull + kStagesA,   // the epilogue is done with a step's row and activation scales (and so the MMAs that
-                                        // read its A and B tiles have completed): frees the A stage and the B stage of the step
-    kBarBFull = kBarAFree + kStagesA,   // fp16 B tile and activation scales have landed
-    kBarDFull = kBarBFull + kStagesB,   // accumulators of a step are complete in tensor memory
-    kBarDFree = kBarDFull + kStagesD,   // epilogue warps have read them
-    kBarCount = kBarDFree + kStagesD
+    kBarWFull = 0,                                 // + stage: packed weights have landed
+    kBarWFree = kBarWFull + kStagesW,              // the dequant warps are done with them
+    kBarBFull = kBarWFree + kStagesW,              // B tiles have landed
+    kBarBFree = kBarBFull + kStagesB,              // the MMAs that read them have completed
+    kBarSFull = kBarBFree + kStagesB,              // activation scales have landed, row scales are written
+    kBarAFull = kBarSFull + kStagesS,              // + row tile * kStagesA + stage: e4m3 weights are in tensor memory
+    kBarAFree = kBarAFull + kRowTiles * kStagesA,  // the MMAs that read them have completed
+    kBarDFull = kBarAFree + kRowTiles * kStagesA,  // + 64-block of the unit: its sums are complete in tensor memory
+    kBarDFree = kBarDFull + 2,                     // the epilogue warps have read them
+    kBarCount = kBarDFree + 2
 };
-static_assert(kBarCount <= 48, "barrier block too small");
+static_assert(kBarCount <= 64, "barrier block too small");
 
-// 8 fp32 columns of tensor memory for this thread's lane, packed in pairs.
-__device__ __forceinline__ void tmem_ld8_pairs(uint32_t taddr, uint64_t (&v)[4]) {
+// The tiles of a block: tile = token block * row_blocks + row block, blocks take them round robin, so
+// that the row blocks of a token block (which share its B tiles) are in flight together.
+struct TileWalk {
+    int tile, rb, e, p0, ntok;
+    __device__ __forceinline__ void load(const UmmaParams& p, int row_blocks, int n_tiles) {
+        if (tile >= n_tiles) return;
+        const int tb = tile / row_blocks;
+        rb = tile - tb * row_blocks;
+        // (the shuffles tell the compiler that the values are the same in all lanes)
+        e = __shfl_sync(0xffffffffu, p.tb_e[tb], 0);
+        p0 = __shfl_sync(0xffffffffu, p.tb_p0[tb], 0);
+        ntok = __shfl_sync(0xffffffffu, p.tb_n[tb], 0);
+    }
+};
+
+// 16 code words of 2 bits (the four bytes 4t .. 4t + 3 of a block of one row: field f of byte i is
+// element 16 f + 4 t + i) -> the e4m3 bytes of q - 1 in the order of piece_byte: lo = fields 0, 1, hi =
+// fields 2, 3. A byte permute looks four codes up at once in a table of four bytes.
+__device__ __forceinline__ void codes_to_e4m3(uint32_t w, uint32_t* lo, uint32_t* hi) {
+    constexpr uint32_t kTable = 0x403800B8u;   // -1, 0, 1, 2
+    const uint32_t y = w & 0x33333333u, z = (w >> 2) & 0x33333333u;
+    const uint32_t r0 = __byte_perm(kTable, 0u, y), r1 = __byte_perm(kTable, 0u, y >> 16);   // fields 0 and 2, interleaved
+    const uint32_t q0 = __byte_perm(kTable, 0u, z), q1 = __byte_perm(kTable, 0u, z >> 16);   // fields 1 and 3
+    lo[0] = __byte_perm(r0, r1, 0x6420);
+    lo[1] = __byte_perm(q0, q1, 0x6420);
+    hi[0] = __byte_perm(r0, r1, 0x7531);
+    hi[1] = __byte_perm(q0, q1, 0x7531);
+}
+
+// The sums S0, S1 of NCH * 4 tokens for this thread's row of both row tiles: v[(r * 2 + s) * NCH * 4 + token].
+// The loads and the wait for them are one statement, so that nothing that reads the registers can
+// move in front of the wait and none of them is copied.
+template <int NCH>
+__device__ __forceinline__ void tmem_ld_sums(uint32_t t0, uint32_t (&v)[16 * NCH]);
+template <>
+__device__ __forceinline__ void tmem_ld_sums<1>(uint32_t t0, uint32_t (&v)[16]) {
     asm volatile(
-        "{\n\t.reg .b32 r<8>;\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {r0,r1,r2,r3,r4,r5,r6,r7}, [%4];\n\t"
-        "mov.b64 %0, {r0,r1};\n\tmov.b64 %1, {r2,r3};\n\tmov.b64 %2, {r4,r5};\n\tmov.b64 %3, {r6,r7};\n\t}"
-        : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3])
-        : "r"(taddr));
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%16];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%4,%5,%6,%7}, [%17];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%8,%9,%10,%11}, [%18];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%12,%13,%14,%15}, [%19];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(t0), "r"(t0 + kTileTok), "r"(t0 + kColsRow), "r"(t0 + kColsRow + kTileTok)
+        : "memory");
+}
+template <>
+__device__ __forceinline__ void tmem_ld_sums<2>(uint32_t t0, uint32_t (&v)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%32];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%33];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16,%17,%18,%19,%20,%21,%22,%23}, [%34];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%24,%25,%26,%27,%28,%29,%30,%31}, [%35];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(t0), "r"(t0 + kTileTok), "r"(t0 + kColsRow), "r"(t0 + kColsRow + kTileTok)
+        : "memory");
+}
+template <>
+__device__ __forceinline__ void tmem_ld_sums<3>(uint32_t t0, uint32_t (&v)[48]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%48];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%8,%9,%10,%11}, [%49];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%12,%13,%14,%15,%16,%17,%18,%19}, [%50];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%20,%21,%22,%23}, [%51];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%24,%25,%26,%27,%28,%29,%30,%31}, [%52];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%32,%33,%34,%35}, [%53];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%36,%37,%38,%39,%40,%41,%42,%43}, [%54];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%44,%45,%46,%47}, [%55];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31]), "=r"(v[32]), "=r"(v[33]), "=r"(v[34]), "=r"(v[35]), "=r"(v[36]), "=r"(v[37]), "=r"(v[38]), "=r"(v[39]), "=r"(v[40]), "=r"(v[41]), "=r"(v[42]), "=r"(v[43]), "=r"(v[44]), "=r"(v[45]), "=r"(v[46]), "=r"(v[47])
+        : "r"(t0), "r"(t0 + 8), "r"(t0 + kTileTok), "r"(t0 + kTileTok + 8), "r"(t0 + kColsRow), "r"(t0 + kColsRow + 8), "r"(t0 + kColsRow + kTileTok), "r"(t0 + kColsRow + kTileTok + 8)
+        : "memory");
+}
+
+// acc += d * (a0 * S0 + a1 * S1) for two tokens, with the reference's roundings: a0 * S0 is exact, so the
+// fused multiply-add rounds once; the multiply by d and the addition round separately. The multiply
+// is written as a fused multiply-add of -0.0, which changes no value and which the assembler, not
+// knowing the addend, cannot merge with the addition that follows.
+__device__ __forceinline__ uint64_t scale_add(uint64_t acc, const ulonglong2& a, const uint32_t* s0, const uint32_t* s1, uint64_t dd, uint64_t neg0) {
+    const uint64_t p0 = pack2(__uint_as_float(s0[0]), __uint_as_float(s0[1])), p1 = pack2(__uint_as_float(s1[0]), __uint_as_float(s1[1]));
+    return add2(acc, fma2(dd, fma2(a.y, p1, mul2(a.x, p0)), neg0));
+}
+
+// What an epilogue warp does with the units of one tile; NCH chunks of 4 tokens per thread and block,
+// for the thread's row of both row tiles (they share the tokens' scales).
+struct EpiArgs {
+    uint32_t bars, abort, smem_s;   // shared-memory addresses
+    unsigned long long wait_ns;
+    uint32_t taddr;                 // tensor memory: this warp's lanes, its first token column
+    uint32_t tok_off, row_off;      // of the thread's first token pair and of its row inside a unit's scales
+    int units;
+    bool leader;                    // lane 0
+    uint64_t neg0;
+};
+template <int NCH>
+__device__ __forceinline__ void epilogue_tile(const EpiArgs& q, uint32_t& gu, uint64_t (&acc)[12]) {
+#pragma unroll
+    for (int i = 0; i < 4 * NCH; ++i) acc[i] = 0ull;
+#pragma unroll 1
+    for (int u = 0; u < q.units; ++u, ++gu) {
+        const uint32_t ss = q.smem_s + (gu % kStagesS) * kUnitBytesS, bar_s = q.bars + (kBarSFull + gu % kStagesS) * 8;
+        // the scales are complete long ago (the MMAs needed what arrives with them): tested so that this
+        // thread acquires them; the test of the first block's sums goes out with it
+        const bool ok_s = mbar_test_wait(bar_s, (gu / kStagesS) & 1u), ok_d = mbar_test_wait(q.bars + kBarDFull * 8, gu & 1u);
+        if (!ok_s) mbar_spin(bar_s, (gu / kStagesS) & 1u, q.abort, q.wait_ns);
+        const uint32_t e0 = lds32(ss + q.row_off), e1 = lds32(ss + q.row_off + kTileRows * 4);
+        const __half2 dh0 = *reinterpret_cast<const __half2*>(&e0), dh1 = *reinterpret_cast<const __half2*>(&e1);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            uint32_t v[16 * NCH];
+            if (j == 1 || !ok_d) mbar_spin(q.bars + (kBarDFull + j) * 8, gu & 1u, q.abort, q.wait_ns);
+            tc_fence_after_sync();
+            tmem_ld_sums<NCH>(q.taddr + j * kColsBlock, v);
+            tc_fence_before_sync();
+            if (q.leader) mbar_arrive(q.bars + (kBarDFree + j) * 8);   // the sums are all in registers: the accumulators go back
+            const float d0 = j ? __high2float(dh0) : __low2float(dh0), d1 = j ? __high2float(dh1) : __low2float(dh1);
+            const uint64_t dd0 = pack2(d0, d0), dd1 = pack2(d1, d1);
+#pragma unroll
+            for (int i = 0; i < 2 * NCH; ++i) {
+                const ulonglong2 a = lds128(ss + q.tok_off + j * kBlockBytesS + i * 16);
+                acc[i] = scale_add(acc[i], a, v + 2 * i, v + 4 * NCH + 2 * i, dd0, q.neg0);
+                acc[2 * NCH + i] = scale_add(acc[2 * NCH + i], a, v + 8 * NCH + 2 * i, v + 12 * NCH + 2 * i, dd1, q.neg0);
+            }
+        }
+    }
 }
 
 template <bool GATE_UP>
 __global__ void __launch_bounds__(kThreads, 1) k_pf_umma(const UmmaParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr PfSmem sm = pf_smem();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + sm.bars);
+    // (the shuffle tells the compiler that the value is the same in all lanes)
+    const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + sm.tmem);
-    volatile int* abort = reinterpret_cast<volatile int*>(smem + sm.abort);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + sm.abort);
+    const uint32_t s0 = smem_u32(smem), bars = s0 + sm.bars, abort = s0 + sm.abort;
+    const unsigned long long wait_ns = p.wait_ns;
 
     const int kdim = GATE_UP ? p.n : p.ff;
-    const int steps = kdim / kQK;                       // 64-blocks of K
-    const int row_blocks = GATE_UP ? (2 * p.ff) / kTileRows : p.n / kTileRows;
-    const uint32_t group_bytes = uint32_t(kdim / kUnitK) * kUnitBytes;
+    const int units = kdim / kUnitK;
+    const int row_tiles = GATE_UP ? (2 * p.ff) / kTileRows : p.n / kTileRows;
+    const int row_blocks = (row_tiles + kRowTiles - 1) / kRowTiles;
+    const uint32_t group_bytes = uint32_t(units) * kUnitBytes;
     const size_t section = GATE_UP ? 0 : size_t(p.ff / 8) * (size_t(p.n / kUnitK) * kUnitBytes);
     const int n_tiles = p.meta[1] * row_blocks;
 
     if (threadIdx.x == 0) {
+        uint64_t* b = reinterpret_cast<uint64_t*>(smem + sm.bars);
         for (int i = 0; i < kStagesW; ++i) {
-            mbar_init(bars + kBarWFull + i, 1);
-            mbar_init(bars + kBarWFree + i, kWarpsDequant);
-        }
-        for (int i = 0; i < kStagesA; ++i) {
-            mbar_init(bars + kBarAFull + i, kWarpsDequant);
-            mbar_init(bars + kBarAFree + i, kWarpsEpilogue);
+            mbar_init(b + kBarWFull + i, 1);
+            mbar_init(b + kBarWFree + i, kWarpsDequant);
         }
         for (int i = 0; i < kStagesB; ++i) {
-            mbar_init(bars + kBarBFull + i, 1);
+            mbar_init(b + kBarBFull + i, 1);
+            mbar_init(b + kBarBFree + i, kRowTiles);
         }
-        for (int i = 0; i < kStagesD; ++i) {
-            mbar_init(bars + kBarDFull + i, 1);
-            mbar_init(bars + kBarDFree + i, kWarpsEpilogue);
+        for (int i = 0; i < kStagesS; ++i) mbar_init(b + kBarSFull + i, 1 + kWarpsDequant);
+        for (int i = 0; i < kRowTiles * kStagesA; ++i) {
+            mbar_init(b + kBarAFull + i, kWarpsDequant / kRowTiles);
+            mbar_init(b + kBarAFree + i, 1);
         }
-        *abort = 0;
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(b + kBarDFull + i, kRowTiles);
+            mbar_init(b + kBarDFree + i, kWarpsEpilogue);
+        }
+        *abort_flag = 0;
         mbar_fence_init();
     }
-    if (warp == 1) tmem_alloc(tmem_slot, 512);
+    if (warp == 2) tmem_alloc(tmem_slot, kTmemCols);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    TileWalk t;
+    t.tile = blockIdx.x;
 
     // "free" barriers are waited on with the parity of the phase before the one about to be used,
     // which a fresh barrier reports as complete
-    auto wait_full = [&](int bar, uint32_t use) { return mbar_wait_bounded<false>(bars + bar, use & 1u, abort, p.wait_ns); };
-    auto wait_free = [&](int bar, uint32_t use) { return mbar_wait_bounded<false>(bars + bar, (use & 1u) ^ 1u, abort, p.wait_ns); };
-
-    if (warp == 0) {
-        // ---------------- producer
-        if (lane == 0) {
-            uint32_t g = 0, gu = 0;   // steps and units issued so far
-            for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-                const int tb = tile / row_blocks, rb = tile % row_blocks;
-                const int e = p.tb_e[tb], p0 = p.tb_p0[tb], ntok = p.tb_n[tb];
-                const uint8_t* wsrc = p.experts + size_t(e) * p.stride + section + size_t(rb) * 8 * group_bytes;
-                for (int b = 0; b < steps; ++b, ++g) {
-                    if ((b & 1) == 0) {
-                        const uint32_t ws = gu % kStagesW;
-                        wait_free(kBarWFree + ws, gu / kStagesW);
-                        mbar_expect_tx(bars + kBarWFull + ws, kUnitTileBytes);
-                        for (int gi = 0; gi < 8; ++gi)
-                            bulk_g2s(smem + sm.w + ws * kUnitTileBytes + gi * kUnitBytes, wsrc + size_t(gi) * group_bytes + size_t(b >> 1) * kUnitBytes,
-                                     kUnitBytes, bars + kBarWFull + ws);
-                        ++gu;
-                    }
-                    const uint32_t bs = g % kStagesB;
-                    wait_free(kBarAFree + bs, g / kStagesB);
-                    const uint32_t bbytes = uint32_t(ntok) * 128u, sbytes = uint32_t(ntok) * 8u;
-                    mbar_expect_tx(bars + kBarBFull + bs, bbytes + sbytes);
-                    bulk_g2s(smem + sm.b + bs * kStepBytesB, p.act + (size_t(b) * (p.pmax / 8) + size_t(p0 >> 3)) * 1024, bbytes, bars + kBarBFull + bs);
-                    bulk_g2s(smem + sm.s + bs * kStepBytesS, p.act_scale + (size_t(b) * p.pmax + size_t(p0)) * 2, sbytes, bars + kBarBFull + bs);
-                }
-            }
-        }
-    } else if (warp == 1) {
-        // ---------------- MMA issuer
-        if (lane == 0) {
+    if (warp < kWarpsAux) {
+        regs_dec<kRegsAux>();
+        if (warp == 0) {
+            // ---------------- packed weights: one lane per row group. A last row tile that does not exist
+            // (n an odd multiple of 128) is computed as a copy of the one before and not stored.
             uint32_t g = 0;
-            bool a_ok = false, b_ok = false, d_ok = false;
-            for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-                const int ntok = p.tb_n[tile / row_blocks];
-                const uint32_t idesc = umma_idesc_f16(kTileRows, ntok);
-                for (int b = 0; b < steps; ++b, ++g) {
-                    const uint32_t as = g % kStagesA, bs = g % kStagesB, ds = g % kStagesD;
-                    if (!a_ok) wait_full(kBarAFull + as, g / kStagesA);
-                    if (!b_ok) wait_full(kBarBFull + bs, g / kStagesB);
-                    if (!d_ok) wait_free(kBarDFree + ds, g / kStagesD);
-                    // the next step's tests, answered while this step's MMAs are being issued
-                    a_ok = mbar_try_wait(bars + kBarAFull + (g + 1) % kStagesA, ((g + 1) / kStagesA) & 1u);
-                    b_ok = mbar_try_wait(bars + kBarBFull + (g + 1) % kStagesB, ((g + 1) / kStagesB) & 1u);
-                    d_ok = mbar_try_wait(bars + kBarDFree + (g + 1) % kStagesD, (((g + 1) / kStagesD) & 1u) ^ 1u);
-                    tc_fence_after_sync();
-                    const uint32_t a_addr = smem_u32(smem + sm.a + as * kStepBytesA), b_addr = smem_u32(smem + sm.b + bs * kStepBytesB);
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {   // four K = 16 instructions: two per 32-block
-                        const uint64_t da = umma_desc(a_addr + kk * 2 * kALbo, kALbo, kASbo), db = umma_desc(b_addr + kk * 256, 128, 1024);
-                        umma_f16(tmem + ds * kStageColsD + (kk >> 1) * kTileTok, da, db, idesc, kk & 1);
-                    }
-                    // one commit per step: the epilogue warps release the A and B stages after they
-                    // have seen it, which also tells that the MMAs are done reading those stages
-                    umma_commit(bars + kBarDFull + ds);
+            for (; t.tile < n_tiles; t.tile += gridDim.x) {
+                t.load(p, row_blocks, n_tiles);
+                const int rt = min(t.rb * kRowTiles + ((lane >> 3) & 1), row_tiles - 1);
+                const uint8_t* src = p.experts + size_t(t.e) * p.stride + section + size_t(rt * 8 + (lane & 7)) * group_bytes;
+                for (int u = 0; u < units; ++u, ++g) {
+                    const uint32_t ws = g % kStagesW, full = bars + (kBarWFull + ws) * 8;
+                    mbar_spin(bars + (kBarWFree + ws) * 8, ((g / kStagesW) & 1u) ^ 1u, abort, wait_ns);
+                    if (lane == 0) mbar_expect_tx(full, kUnitBytesW);
+                    __syncwarp();
+                    if (lane < 8 * kRowTiles) bulk_g2s(s0 + sm.w + ws * kUnitBytesW + lane * kUnitBytes, src + size_t(u) * kUnitBytes, kUnitBytes, full);
                 }
             }
-        }
-    } else if (warp < 2 + kWarpsDequant) {
-        // ---------------- dequant: packed 2-bit codes -> fp16 (q - 1) in the A tile
-        const int dw = warp - 2;   // the group (16 rows) of the tile this warp unpacks
-        const int g8 = lane >> 2, t4 = lane & 3;
-        const __half2 k1025 = __floats2half2_rn(1025.0f, 1025.0f);
-        uint32_t g = 0, gu = 0;
-        bool a_free = false, w_ready = false;   // the next step's A stage / weights were already seen free / landed
-        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-            for (int b = 0; b < steps; ++b, ++g) {
-                const int j = b & 1;
-                const uint32_t ws = gu % kStagesW, as = g % kStagesA;
-                // (the tests were issued during the previous step's work, see the epilogue)
-                if (j == 0 && !w_ready) wait_full(kBarWFull + ws, gu / kStagesW);
-                // an A stage (the fp16 tile and its row scales) is free once the MMAs that read the
-                // tile have completed and the epilogue warps have used the scales
-                if (!a_free) wait_free(kBarAFree + as, g / kStagesA);
-                uint8_t* at = smem + sm.a + as * kStepBytesA;
-                uint4 wvs[kGroupsPerDequantWarp];
+        } else if (warp == 1) {
+            // ---------------- activations: B tiles and scales of a unit's two blocks
+            uint32_t g = 0;
+            for (; t.tile < n_tiles; t.tile += gridDim.x) {
+                t.load(p, row_blocks, n_tiles);
+                const uint32_t bbytes = uint32_t(t.ntok) * 128u, sbytes = uint32_t(t.ntok) * 8u;
+                for (int u = 0; u < units; ++u, ++g) {
+                    const uint32_t bs = g % kStagesB, ss = g % kStagesS, full_b = bars + (kBarBFull + bs) * 8, full_s = bars + (kBarSFull + ss) * 8;
+                    mbar_spin(bars + (kBarBFree + bs) * 8, ((g / kStagesB) & 1u) ^ 1u, abort, wait_ns);
+                    if (lane == 0) mbar_expect_tx(full_b, 2 * bbytes);
+                    if (lane == 1) mbar_expect_tx(full_s, 2 * sbytes);
+                    __syncwarp();
+                    const size_t b = size_t(2 * u + (lane & 1));
+                    if (lane < 2)
+                        bulk_g2s(s0 + sm.b + bs * kUnitBytesB + lane * kBlockBytesB, p.act + (b * (p.pmax / 8) + size_t(t.p0 >> 3)) * 1024, bbytes, full_b);
+                    else if (lane < 4)
+                        bulk_g2s(s0 + sm.s + ss * kUnitBytesS + (lane & 1) * kBlockBytesS, p.act_scale + (b * p.pmax + size_t(t.p0)) * 2, sbytes, full_s);
+                }
+            }
+        } else if (warp < 4) {
+            // ---------------- MMA issuers, one warp per row tile; one elected lane issues, the warp stays together
+            // (so that what it computes is known to be uniform)
+            const int r = warp - 2;
+            const uint64_t b_desc0 = umma_desc(s0 + sm.b, 128, 1024);
+            uint32_t g = 0;
+            for (; t.tile < n_tiles; t.tile += gridDim.x) {
+                t.load(p, row_blocks, n_tiles);
+                const uint32_t idesc = umma_idesc_e4m3(kTileRows, t.ntok);
+                for (int u = 0; u < units; ++u, ++g) {
+                    const uint32_t bs = g % kStagesB, as = g % kStagesA;
+                    const uint32_t bar_b = bars + (kBarBFull + bs) * 8, bar_a = bars + (kBarAFull + r * kStagesA + as) * 8, bar_d = bars + kBarDFree * 8;
+                    const uint32_t pb = (g / kStagesB) & 1u, pa = (g / kStagesA) & 1u, pd = (g & 1u) ^ 1u;
+                    // (a barrier test has a latency of tens of cycles and this warp is on the critical path:
+                    // the three tests go out together, and the second block's in front of the first's MMAs)
+                    const bool ok_b = mbar_test_wait(bar_b, pb), ok_a = mbar_test_wait(bar_a, pa), ok_d = mbar_test_wait(bar_d, pd);
+                    if (!ok_b) mbar_spin(bar_b, pb, abort, wait_ns);
+                    if (!ok_a) mbar_spin(bar_a, pa, abort, wait_ns);
+                    if (!ok_d) mbar_spin(bar_d, pd, abort, wait_ns);
+                    const bool ok_d1 = mbar_test_wait(bar_d + 8, pd);
+                    const uint32_t a0 = tmem + kColA0 + as * kColsA + r * 32;
+                    const uint64_t b0 = b_desc0 + uint64_t(bs * (kUnitBytesB >> 4));
 #pragma unroll
-                for (int gi = 0; gi < kGroupsPerDequantWarp; ++gi)   // words [h][j] of this lane, per group
-                    wvs[gi] = *reinterpret_cast<const uint4*>(smem + sm.w + ws * kUnitTileBytes + (dw * kGroupsPerDequantWarp + gi) * kUnitBytes + lane * 16);
-                a_free = mbar_try_wait(bars + kBarAFree + (g + 1) % kStagesA, (((g + 1) / kStagesA) & 1u) ^ 1u);
-                if (j == 1) w_ready = mbar_try_wait(bars + kBarWFull + (gu + 1) % kStagesW, ((gu + 1) / kStagesW) & 1u);
+                    for (int j = 0; j < 2; ++j) {
+                        if (j == 1 && !ok_d1) mbar_spin(bar_d + 8, pd, abort, wait_ns);
+                        tc_fence_after_sync();
+                        if (elect_one()) {
 #pragma unroll
-                for (int gh = 0; gh < 2 * kGroupsPerDequantWarp; ++gh) {
-                    const int gi = gh >> 1, h = gh & 1;
-                    const uint4 wv = wvs[gi];
-                    const uint32_t w = h ? (j ? wv.w : wv.z) : (j ? wv.y : wv.x);
-                    const int row = (dw * kGroupsPerDequantWarp + gi) * 16 + g8 + 8 * h;
-                    uint8_t* dst = at + (row >> 3) * kASbo + (row & 7) * 16 + (t4 & 1) * 8;
+                            for (int s = 0; s < 2; ++s)
 #pragma unroll
-                    for (int f = 0; f < 4; ++f) {   // field f: elements 16 f + 4 t4 .. + 3 of the block
-                        const uint32_t x = (w >> (2 * f)) & 0x03030303u;
-                        uint32_t lo = __byte_perm(x, 0x64646464u, 0x5140), hi = __byte_perm(x, 0x64646464u, 0x7362);   // fp16 1024 + q
-                        const __half2 l2 = __hsub2(*reinterpret_cast<__half2*>(&lo), k1025), h2 = __hsub2(*reinterpret_cast<__half2*>(&hi), k1025);
-                        uint2 out;
-                        out.x = *reinterpret_cast<const uint32_t*>(&l2);
-                        out.y = *reinterpret_cast<const uint32_t*>(&h2);
-                        *reinterpret_cast<uint2*>(dst + (2 * f + (t4 >> 1)) * kALbo) = out;
+                                for (int piece = 0; piece < 2; ++piece)   // a 32-block: its multiples of 16, then its rests, into the same sums
+                                    umma_f8_ta(tmem + j * kColsBlock + r * kColsRow + s * kTileTok, a0 + j * 16 + s * 8,
+                                               b0 + uint64_t((j * kBlockBytesB + (s * 4 + piece * 2) * 128) >> 4), idesc, piece);
+                            umma_commit(bars + (kBarDFull + j) * 8);
+                            if (j == 1) {
+                                umma_commit(bar_a + (kBarAFree - kBarAFull) * 8);
+                                umma_commit(bar_b + (kBarBFree - kBarBFull) * 8);
+                            }
+                        }
+                        __syncwarp();
                     }
                 }
+            }
+        } else {
+            // ---------------- dequant: packed 2-bit codes -> e4m3 (q - 1) in tensor memory, a thread per row
+            const int r = (warp - 4) >> 2, row = (warp & 3) * 32 + lane;
+            // of this row inside a stage of packed weights: code words [t] at 16 t, of block j at + 4 j; the two scales
+            const uint32_t code_off = uint32_t(r) * kTileBytesW + uint32_t(row >> 4) * kUnitBytes + uint32_t(row & 7) * 64 + uint32_t((row >> 3) & 1) * 8;
+            const uint32_t scale_off = uint32_t(r) * kTileBytesW + uint32_t(row >> 4) * kUnitBytes + kUnitCodeBytes + uint32_t(row & 7) * 8 + uint32_t((row >> 3) & 1) * 4;
+            const uint32_t a_addr = tmem + (uint32_t((warp & 3) * 32) << 16) + kColA0 + r * 32;
+            uint32_t g = 0;
+            for (; t.tile < n_tiles; t.tile += gridDim.x) {
+#pragma unroll 1
+                for (int u = 0; u < units; ++u, ++g) {
+                    const uint32_t ws = g % kStagesW, as = g % kStagesA, ss = g % kStagesS;
+                    const uint32_t bar_w = bars + (kBarWFull + ws) * 8, bar_a = bars + (kBarAFull + r * kStagesA + as) * 8;
+                    mbar_spin(bar_w, (g / kStagesW) & 1u, abort, wait_ns);
+                    const bool ok_a = mbar_test_wait(bar_a + (kBarAFree - kBarAFull) * 8, ((g / kStagesA) & 1u) ^ 1u);
+                    const uint32_t wsrc = s0 + sm.w + ws * kUnitBytesW;
+                    uint2 wv[4];   // words of blocks 0, 1
 #pragma unroll
-                for (int r = lane; r < 16 * kGroupsPerDequantWarp; r += 32) {   // this step's weight scales of the warp's rows
-                    const int gi = r >> 4, l16 = r & 15;
-                    const uint8_t* wt = smem + sm.w + ws * kUnitTileBytes + (dw * kGroupsPerDequantWarp + gi) * kUnitBytes;
-                    const __half sc = *reinterpret_cast<const __half*>(wt + kUnitCodeBytes + (l16 & 7) * 8 + ((l16 >> 3) * 2 + j) * 2);
-                    reinterpret_cast<float*>(smem + sm.sw)[as * kTileRows + (dw * kGroupsPerDequantWarp + gi) * 16 + l16] = __half2float(sc);
+                    for (int q = 0; q < 4; ++q) wv[q] = lds64(wsrc + code_off + q * 16);
+                    sts32(s0 + sm.s + ss * kUnitBytesS + 2 * kBlockBytesS + (r * kTileRows + row) * 4, lds32(wsrc + scale_off));
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(bars + (kBarSFull + ss) * 8);
+                        mbar_arrive(bar_w + (kBarWFree - kBarWFull) * 8);
+                    }
+                    if (!ok_a) mbar_spin(bar_a + (kBarAFree - kBarAFull) * 8, ((g / kStagesA) & 1u) ^ 1u, abort, wait_ns);
+                    tc_fence_after_sync();
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        uint32_t o[16];   // the two halves of the block, eight columns each
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) codes_to_e4m3(j ? wv[q].y : wv[q].x, o + 2 * q, o + 8 + 2 * q);
+                        tmem_st16(a_addr + as * kColsA + j * 16, o);
+                    }
+                    tmem_st_wait();
+                    tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_a);
                 }
-                fence_async_smem();
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(bars + kBarAFull + as);
-                    if (j == 1) mbar_arrive(bars + kBarWFree + ws);
-                }
-                if (j == 1) ++gu;
             }
         }
     } else {
         // ---------------- epilogue
-        const int ew = warp - (2 + kWarpsDequant);
+        regs_inc<kRegsEpilogue>();
+        const int ew = warp - kWarpsAux;
         const int quarter = warp & 3;             // the tensor-memory lanes this warp may read
-        const int cq = ew >> 2;                   // which 32 token columns
-        const int row = quarter * 32 + lane;      // M row of the tile
-        const uint32_t lane_addr = uint32_t(quarter * 32) << 16;
+        const int row = quarter * 32 + lane;      // M row of the row tiles
+        EpiArgs q;
+        q.bars = bars;
+        q.abort = abort;
+        q.smem_s = s0 + sm.s;
+        q.wait_ns = wait_ns;
+        q.units = units;
+        q.leader = lane == 0;
+        q.row_off = 2 * kBlockBytesS + row * 4;
+        q.neg0 = pack2(p.neg0, p.neg0);
         uint32_t g = 0;
-        bool d_ready = false;   // this step's accumulators were already seen complete
-        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-            const int tb = tile / row_blocks, rb = tile % row_blocks;
-            const int p0 = p.tb_p0[tb], ntok = p.tb_n[tb];
-            const int ncols = max(0, min(32, ntok - 32 * cq));
-            const int last_chunk = ncols > 0 ? (ncols - 1) >> 4 : 0;   // the last 16-column chunk this thread reads
-            float acc[32];
-#pragma unroll
-            for (int i = 0; i < 32; ++i) acc[i] = 0.0f;
-            for (int b = 0; b < steps; ++b, ++g) {
-                const uint32_t as = g % kStagesA, bs = g % kStagesB, ds = g % kStagesD;
-                // Every barrier operation costs on the order of a hundred cycles of latency, and a
-                // thread's steps are serial (its sums are added block after block), so the tests
-                // are issued ahead of where their answer is needed: the one for this step's
-                // accumulators was issued during the previous step's arithmetic.
-                if (!d_ready) wait_full(kBarDFull + ds, g / kStagesD);
-                tc_fence_after_sync();
-                // complete long ago (the MMAs needed them); tested so that what the dequant warps
-                // (row scales) and the TMA (activation scales) wrote is acquired by this thread
-                bool a_ready = mbar_try_wait(bars + kBarAFull + as, (g / kStagesA) & 1u);
-                bool b_ready = mbar_try_wait(bars + kBarBFull + bs, (g / kStagesB) & 1u);
-                const uint32_t t0 = tmem + lane_addr + ds * kStageColsD + cq * 32;
-                const ulonglong2* sc = reinterpret_cast<const ulonglong2*>(smem + sm.s + bs * kStepBytesS) + cq * 16;
-                uint64_t dd = 0ull;
-                // two chunks of 16 columns: a round trip to tensor memory costs several hundred cycles
-                // whatever its size, so few, large loads (as large as the registers allow)
-#pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    uint32_t v0[16], v1[16];
-                    if (c * 16 < ncols) {
-                        tmem_ld16(t0 + c * 16, v0);
-                        tmem_ld16(t0 + kTileTok + c * 16, v1);
-                        tmem_ld_wait();
-                    }
-                    if (c == last_chunk) {
-                        // all of this thread's sums are in registers: the tensor-memory stage goes back
-                        // before the arithmetic on the last chunk; the stages limit the MMAs in flight
-                        tc_fence_before_sync();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(bars + kBarDFree + ds);
-                        d_ready = mbar_try_wait(bars + kBarDFull + (g + 1) % kStagesD, ((g + 1) / kStagesD) & 1u);
-                    }
-                    if (c == 0) {
-                        if (!a_ready) a_ready = wait_full(kBarAFull + as, g / kStagesA);
-                        if (!b_ready) b_ready = wait_full(kBarBFull + bs, g / kStagesB);
-                        const float d = reinterpret_cast<const float*>(smem + sm.sw)[as * kTileRows + row];
-                        dd = pack2(d, d);
-                    }
-                    if (c * 16 < ncols) {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            const ulonglong2 a = sc[c * 8 + i];   // {a0 of the two tokens}, {a1 of the two tokens}
-                            const uint64_t s0 = pack2(__uint_as_float(v0[2 * i]), __uint_as_float(v0[2 * i + 1]));
-                            const uint64_t s1 = pack2(__uint_as_float(v1[2 * i]), __uint_as_float(v1[2 * i + 1]));
-                            // packed multiply by the row scale, then *scalar* adds: a packed add (or a
-                            // packed t * 1 + acc) would be contracted with the multiply into one rounding
-                            float u0, u1;
-                            unpack2(mul2(dd, fma2(a.y, s1, mul2(a.x, s0))), u0, u1);
-                            acc[c * 16 + 2 * i] = __fadd_rn(acc[c * 16 + 2 * i], u0);
-                            acc[c * 16 + 2 * i + 1] = __fadd_rn(acc[c * 16 + 2 * i + 1], u1);
-                        }
-                    }
-                }
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(bars + kBarAFree + as);
-                }
+        for (; t.tile < n_tiles; t.tile += gridDim.x) {
+            t.load(p, row_blocks, n_tiles);
+            const int share = t.ntok >> 2, nch = share >> 2;   // four warps share a row's tokens evenly
+            const int tok0 = (ew >> 2) * share;
+            q.tok_off = tok0 * 8;
+            q.taddr = tmem + (uint32_t(quarter * 32) << 16) + uint32_t(tok0);
+            uint64_t acc[12];
+            switch (nch) {
+                case 1: epilogue_tile<1>(q, g, acc); break;
+                case 2: epilogue_tile<2>(q, g, acc); break;
+                default: epilogue_tile<3>(q, g, acc); break;
             }
-            // ---- tile done: acc[i] holds this row's sum for token 32 cq + i
-            if (GATE_UP) {
-                // rows m < 8 of a group are gate rows, m >= 8 the up rows of the same ff rows: a
-                // warp's 32 rows are 16 (gate, up) pairs, 128 contiguous bytes per token
-                const int m = row & 15, ffrow = rb * 64 + (row >> 4) * 8 + (m & 7);
-                float* dst = reinterpret_cast<float*>(p.hf) + size_t(ffrow) * 2 + (m >> 3);
+            // ---- tile done: acc[r * 2 nch + i] holds the sums of row tile r for tokens tok0 + 2 i, + 1
+            const int pos0 = t.p0 + tok0;
 #pragma unroll
-                for (int i = 0; i < 32; ++i)
-                    if (i < ncols) dst[size_t(p0 + 32 * cq + i) * p.ff * 2] = acc[i];
-            } else {
-                const int orow = rb * kTileRows + row;
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    if (2 * i < ncols) {
-                        const float v0 = acc[2 * i], v1 = acc[2 * i + 1];
-                        const int pos = p0 + 32 * cq + 2 * i;
-                        const int sl0 = p.pslot[pos], sl1 = p.pslot[pos + 1];
-                        if (p.y_bf16) {
-                            __nv_bfloat16* yb = reinterpret_cast<__nv_bfloat16*>(p.yd);
-                            if (sl0 >= 0) yb[size_t(sl0) * p.n + orow] = __float2bfloat16_rn(v0);
-                            if (sl1 >= 0) yb[size_t(sl1) * p.n + orow] = __float2bfloat16_rn(v1);
-                        } else {
-                            if (sl0 >= 0) p.yd[size_t(sl0) * p.n + orow] = v0;
-                            if (sl1 >= 0) p.yd[size_t(sl1) * p.n + orow] = v1;
-                        }
+            for (int k = 0; k < 12; ++k) {
+                if (k >= 4 * nch) break;
+                const int r = k >= 2 * nch ? 1 : 0, i = k - r * 2 * nch, rt = t.rb * kRowTiles + r, pos = pos0 + 2 * i;
+                if (rt >= row_tiles) break;
+                float v0, v1;
+                unpack2(acc[k], v0, v1);
+                if (GATE_UP) {
+                    // rows m < 8 of a group are gate rows, m >= 8 the up rows of the same ff rows: a
+                    // warp's 32 rows are 16 (gate, up) pairs, 128 contiguous bytes per token
+                    const int m = row & 15, ffrow = rt * 64 + (row >> 4) * 8 + (m & 7);
+                    float* dst = reinterpret_cast<float*>(p.hf) + (size_t(pos) * p.ff + ffrow) * 2 + (m >> 3);
+                    dst[0] = v0;
+                    dst[size_t(p.ff) * 2] = v1;
+                } else {
+                    const int orow = rt * kTileRows + row;
+                    const int sl0 = p.pslot[pos], sl1 = p.pslot[pos + 1];
+                    if (p.y_bf16) {
+                        __nv_bfloat16* yb = reinterpret_cast<__nv_bfloat16*>(p.yd);
+                        if (sl0 >= 0) yb[size_t(sl0) * p.n + orow] = __float2bfloat16_rn(v0);
+                        if (sl1 >= 0) yb[size_t(sl1) * p.n + orow] = __float2bfloat16_rn(v1);
+                    } else {
+                        if (sl0 >= 0) p.yd[size_t(sl0) * p.n + orow] = v0;
+                        if (sl1 >= 0) p.yd[size_t(sl1) * p.n + orow] = v1;
                     }
                 }
             }
@@ -605,7 +736,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pf_umma(const UmmaParams p) {
     }
     tc_fence_before_sync();
     __syncthreads();
-    if (*abort) {
+    if (*abort_flag) {
         // A wait ran out: bulk copies and MMAs may still be in flight. Give them time to land
         // before tensor memory and the block's shared memory are released.
         const uint64_t t0 = global_ns();
@@ -613,8 +744,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_pf_umma(const UmmaParams p) {
         }
         __syncthreads();
     }
-    if (warp == 1) tmem_free(tmem, 512);
-    if (threadIdx.x == 0 && *abort) p.status[0] = kDevWaitTimeout;
+    if (warp == 2) tmem_free(tmem, kTmemCols);
+    if (threadIdx.x == 0 && *abort_flag) p.status[0] = kDevWaitTimeout;
 }
 
 
@@ -636,9 +767,12 @@ int set_pf_attr() {
 
 using namespace frx;
 
-// The tensor-memory form pays per 128-row x 64-weight step whatever the number of tokens in the tile,
-// so it is taken only when experts get many tokens on average.
-constexpr int kUmmaMinTokensPerExpert = 256;
+// Which form: the tensor-memory form pays per unit of 256 rows x 128 weights whatever the number of tokens
+// in the tile, the streaming form reads an expert again for every eight tokens. Measured on B200
+// (us, uniform routing; hidden / width, experts; streaming against tensor memory): 2048 / 512, 512:
+// 16 tokens per expert 346 against 410, 24: 469 against 440, 32: 592 against 484, 128: 2098 against
+// 1419; 384 / 640, 128: 24: 87 against 92, 32: 101 against 97. With skewed routing they meet at 32.
+constexpr int kUmmaMinTokensPerExpert = 32;
 
 extern "C" {
 
@@ -670,6 +804,7 @@ static int prefill_umma_impl(const void* experts, size_t stride, int E, const in
         return fail(FRX_ERR_SHAPE, "frx_moe_prefill: unsupported T %d, K %d, E %d", T, K, E);
     if ((uintptr_t(experts) | stride) % 16 || uintptr_t(ws) % kAlign)
         return fail(FRX_ERR_ARG, "frx_moe_prefill: experts and stride must be 16-byte aligned, ws 256-byte aligned");
+    if (uintptr_t(x) % 16 || uintptr_t(xq_in) % 4) return fail(FRX_ERR_ARG, "frx_moe_prefill: x must be 16-byte aligned, xq 4-byte aligned");
     if (stride < frx_q2_expert_bytes(n, ff)) return fail(FRX_ERR_ARG, "frx_moe_prefill: stride %zu < blob %zu", stride, frx_q2_expert_bytes(n, ff));
     if (T == 0) return FRX_OK;
     const PfuLayout L = pfu_layout(T, K, n, ff, E);
@@ -688,18 +823,20 @@ static int prefill_umma_impl(const void* experts, size_t stride, int E, const in
     int* tb_p0 = reinterpret_cast<int*>(base + L.tb_p0);
     int* tb_n = reinterpret_cast<int*>(base + L.tb_n);
     int32_t* pslot = reinterpret_cast<int32_t*>(base + L.pslot);
-    const int8_t* xq = xq_in ? xq_in : reinterpret_cast<const int8_t*>(base + L.xq);
-    const float* xd = xd_in ? xd_in : reinterpret_cast<const float*>(base + L.xd);
     const int S = T * K;
-    const size_t nblk = size_t(T) * (n / kQ8);
-    if (!xq_in)   // else the activations arrived already quantized
-        FRX_LAUNCH(kKQuant, stream, k_pfu_quant_x<<<unsigned((nblk + 7) / 8), 256, 0, stream>>>(x, nblk, reinterpret_cast<int8_t*>(base + L.xq),
-                                                                                   reinterpret_cast<float*>(base + L.xd), block64));
+    uint8_t* xe = base + L.xe;
+    float* xd = reinterpret_cast<float*>(base + L.xd);
+    const size_t nquads = size_t(T) * (n / 4);
+    const unsigned qgrid = unsigned((nquads + 255) / 256);
+    if (xq_in)   // the activations arrived already quantized
+        FRX_LAUNCH(kKQuant, stream, k_pfu_expand_q8<<<qgrid, 256, 0, stream>>>(xq_in, nquads, xe));
+    else
+        FRX_LAUNCH(kKQuant, stream, k_pfu_quant_x<<<qgrid, 256, 0, stream>>>(x, nquads, xe, xd, block64));
     FRX_LAUNCH(kKGroup, stream, k_pf_hist<<<L.n_chunks, 256, size_t(E) * 4, stream>>>(ids, S, E, chunk_cnt, status, e_map, E_all));
     FRX_LAUNCH(kKGroup, stream, k_pf_scan<<<1, 1024, 0, stream>>>(chunk_cnt, L.n_chunks, E, bounds, item_off, status, 1 << 30));
     FRX_LAUNCH(kKGroup, stream, k_pf_place<<<L.n_chunks, 32, size_t(E) * 4, stream>>>(ids, S, E, chunk_cnt, bounds, perm, e_map, E_all));
     FRX_LAUNCH(kKGroup, stream, k_pfu_plan<<<1, 1024, 0, stream>>>(bounds, E, pb, tbo, meta, tb_e, tb_p0, tb_n, L.max_tb, status));
-    FRX_LAUNCH(kKGroup, stream, k_pfu_gather<<<unsigned(L.pmax / 8), 256, 0, stream>>>(bounds, pb, E, perm, meta, K, n, L.pmax, xq, xd, base + L.xg,
+    FRX_LAUNCH(kKGroup, stream, k_pfu_gather<<<unsigned(L.pmax / 8), 256, 0, stream>>>(bounds, pb, E, perm, meta, K, n, L.pmax, xe, xq_in ? xd_in : xd, base + L.xg,
                                                                                    reinterpret_cast<float*>(base + L.xa), pslot));
     UmmaParams p{};
     p.experts = static_cast<const uint8_t*>(experts);
@@ -715,18 +852,19 @@ static int prefill_umma_impl(const void* experts, size_t stride, int E, const in
     p.status = status;
     p.pmax = L.pmax;
     p.wait_ns = wait_limit_ns();
+    p.neg0 = -0.0f;
     p.n = n;
     p.ff = ff;
-    const int sms = sm_count();
+    const int blocks = sm_count();
     p.act = base + L.xg;
     p.act_scale = reinterpret_cast<const float*>(base + L.xa);
-    FRX_LAUNCH(kKGateUp, stream, k_pf_umma<true><<<sms, kThreads, pf_smem().total, stream>>>(p));
+    FRX_LAUNCH(kKGateUp, stream, k_pf_umma<true><<<blocks, kThreads, pf_smem().total, stream>>>(p));
     const size_t hchunks = L.pmax * size_t(ff / 8);
     FRX_LAUNCH(kKQuant, stream, k_pfu_quant_h<<<unsigned((hchunks + 255) / 256), 256, 0, stream>>>((const float2*)p.hf, ff, L.pmax, meta, pslot, base + L.hg,
                                                                                     reinterpret_cast<float*>(base + L.ha), block64));
     p.act = base + L.hg;
     p.act_scale = reinterpret_cast<const float*>(base + L.ha);
-    FRX_LAUNCH(kKDown, stream, k_pf_umma<false><<<sms, kThreads, pf_smem().total, stream>>>(p));
+    FRX_LAUNCH(kKDown, stream, k_pf_umma<false><<<blocks, kThreads, pf_smem().total, stream>>>(p));
     FRX_CUDA(cudaGetLastError());
     return FRX_OK;
 }
@@ -750,10 +888,7 @@ int frx_moe_prefill_q8_ep(const void* experts_local, size_t stride, int E_local,
     return frx_moe_prefill_stream_q8_ep(experts_local, stride, E_local, e_map, E_all, n, ff, xq, xd, ids, T, K, yd, ws, ws_bytes, stream);
 }
 
-// ---- the public entry. Both forms compute the same bits; the choice is by measured speed: the
-// tensor-memory form pays per 128-row x 64-weight step whatever the number of tokens in the tile,
-// so it is taken only when experts get many tokens on average (256 or more, where it is on a par
-// with or ahead of the streaming form on B200), and the streaming form otherwise.
+// ---- the public entry: both forms compute the same bits, see kUmmaMinTokensPerExpert
 
 size_t frx_moe_prefill_workspace_bytes(int T, int K, int n, int ff, int E) {
     const size_t a = frx_moe_prefill_stream_workspace_bytes(T, K, n, ff, E), b = frx_moe_prefill_umma_workspace_bytes(T, K, n, ff, E);
