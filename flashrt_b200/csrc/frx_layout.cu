@@ -3,6 +3,8 @@
 // the tests check them against the CPU oracle byte for byte.
 #include "frx_common.cuh"
 
+#include <algorithm>
+
 namespace frx {
 namespace {
 
@@ -38,62 +40,64 @@ struct Geo {
     __host__ __device__ size_t total_units() const { return size_t(gu_groups) * gu_units + size_t(dn_groups) * dn_units; }
 };
 
-// For unit `unit` of an expert and M row m: the planar matrix offset, its row count, blocks per
-// row, and the matrix row that M row m is.
-__device__ __forceinline__ void unit_source(const Geo& G, size_t unit, int m, size_t& mat_off, int& rows, int& nb, int& row,
-                                            int& u) {
-    const size_t gu_total = size_t(G.gu_groups) * G.gu_units;
-    if (unit < gu_total) {
-        const int grp = int(unit / G.gu_units);
-        u = int(unit % G.gu_units);
-        mat_off = m < 8 ? 0 : G.gu_mat;   // gate, then up
-        rows = G.ff;
-        nb = G.n / kQK;
-        row = grp * 8 + (m & 7);
-    } else {
-        const size_t k = unit - gu_total;
-        const int grp = int(k / G.dn_units);
-        u = int(k % G.dn_units);
-        mat_off = 2 * G.gu_mat;
-        rows = G.n;
-        nb = G.ff / kQK;
-        row = grp * 16 + m;
-    }
-}
-
-// One thread per 32-bit word of a unit: 128 code words, then 16 scale words (two fp16 each).
-// TO_TILED: planar -> tiled; otherwise tiled -> planar.
+// A warp per unit: lane L moves the 16 bytes of codes of lane L, lanes 0..15 a scale word each (two fp16).
+// Neighbouring warps of a block take neighbouring units, i.e. the same matrix rows further along K, so
+// the 32 bytes a row gives to a unit share their lines in the L1. TO_TILED: planar -> tiled;
+// otherwise tiled -> planar. Bound: HBM, two passes over the weights. (A thread per word, each with its own
+// 64-bit divisions to find its place, took twice as long.)
 template <bool TO_TILED>
-__global__ void k_tile(const uint8_t* __restrict__ src, size_t src_stride, uint8_t* __restrict__ dst, size_t dst_stride, int n,
-                       int ff, size_t units_per_expert, size_t total_words) {
-    const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= total_words) return;
+__global__ void __launch_bounds__(256) k_tile(const uint8_t* __restrict__ src, size_t src_stride, uint8_t* __restrict__ dst, size_t dst_stride, int n, int ff,
+                                              int units_per_expert, int n_experts) {
+    const int unit = blockIdx.x * 8 + int(threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (unit >= units_per_expert) return;
     const Geo G(n, ff);
-    constexpr int kWordsPerUnit = kUnitBytes / 4;   // 144
-    const size_t unit_global = i / kWordsPerUnit;
-    const int w = int(i % kWordsPerUnit);
-    const size_t e = unit_global / units_per_expert, unit = unit_global % units_per_expert;
-    const uint8_t* planar = (TO_TILED ? src + e * src_stride : nullptr);
-    uint8_t* planar_out = (TO_TILED ? nullptr : dst + e * dst_stride);
-    const size_t tiled_off = unit * kUnitBytes + size_t(w) * 4;
-    size_t mat_off;
-    int rows, nb, row, u;
-    if (w < 128) {   // codes: lane L = w / 4, word (h, j) = w % 4
-        const int L = w >> 2, h = (w >> 1) & 1, j = w & 1, g = L >> 2, t = L & 3;
-        unit_source(G, unit, g + 8 * h, mat_off, rows, nb, row, u);
-        const size_t p_off = mat_off + (size_t(row) * nb + (2 * u + j)) * 16 + size_t(t) * 4;
-        if (TO_TILED)
-            *reinterpret_cast<uint32_t*>(dst + e * dst_stride + tiled_off) = *reinterpret_cast<const uint32_t*>(planar + p_off);
-        else
-            *reinterpret_cast<uint32_t*>(planar_out + p_off) = *reinterpret_cast<const uint32_t*>(src + e * src_stride + tiled_off);
-    } else {         // scales: word s = w - 128 holds [g][h][j = 0, 1], g = s / 2, h = s % 2
-        const int s = w - 128, g = s >> 1, h = s & 1;
-        unit_source(G, unit, g + 8 * h, mat_off, rows, nb, row, u);
-        const size_t p_off = mat_off + size_t(rows) * nb * 16 + (size_t(row) * nb + 2 * u) * 2;   // two adjacent blocks
-        if (TO_TILED)
-            *reinterpret_cast<uint32_t*>(dst + e * dst_stride + tiled_off) = *reinterpret_cast<const uint32_t*>(planar + p_off);
-        else
-            *reinterpret_cast<uint32_t*>(planar_out + p_off) = *reinterpret_cast<const uint32_t*>(src + e * src_stride + tiled_off);
+    const int gu_total = G.gu_groups * G.gu_units;
+    const bool gu = unit < gu_total;
+    const int k = gu ? unit : unit - gu_total, per = gu ? G.gu_units : G.dn_units, grp = k / per, u = k - grp * per;
+    const int nb = (gu ? n : ff) / kQK, rows = gu ? ff : n;
+    // M row m of the unit: gate rows, then up rows (m >= 8), or 16 down rows
+    auto mat_row = [&](int m, size_t& mat) {
+        mat = gu ? (m < 8 ? 0 : G.gu_mat) : 2 * G.gu_mat;
+        return gu ? grp * 8 + (m & 7) : grp * 16 + m;
+    };
+    const int g = lane >> 2, t = lane & 3;
+    size_t code_off[2], scale_off = 0;   // of the planar blob: block 2u of rows g, g + 8 (this lane's word); its scale word
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        size_t mat;
+        const int row = mat_row(g + 8 * h, mat);
+        code_off[h] = mat + (size_t(row) * nb + 2 * u) * 16 + size_t(t) * 4;
+    }
+    if (lane < 16) {   // scale word s holds [g = s / 2][h = s % 2][j = 0, 1]
+        size_t mat;
+        const int row = mat_row((lane >> 1) + 8 * (lane & 1), mat);
+        scale_off = mat + size_t(rows) * nb * 16 + (size_t(row) * nb + 2 * u) * 2;
+    }
+    const size_t tiled_off = size_t(unit) * kUnitBytes;
+    for (int e = blockIdx.y; e < n_experts; e += gridDim.y) {
+        const uint8_t* s = src + size_t(e) * src_stride;
+        uint8_t* d = dst + size_t(e) * dst_stride;
+        if (TO_TILED) {
+            uint4 v;
+            v.x = *reinterpret_cast<const uint32_t*>(s + code_off[0]);
+            v.y = *reinterpret_cast<const uint32_t*>(s + code_off[0] + 16);
+            v.z = *reinterpret_cast<const uint32_t*>(s + code_off[1]);
+            v.w = *reinterpret_cast<const uint32_t*>(s + code_off[1] + 16);
+            uint32_t* o = reinterpret_cast<uint32_t*>(d + tiled_off);
+            if (uintptr_t(o) % 16 == 0) {
+                reinterpret_cast<uint4*>(o)[lane] = v;
+            } else {
+                o[lane * 4] = v.x, o[lane * 4 + 1] = v.y, o[lane * 4 + 2] = v.z, o[lane * 4 + 3] = v.w;
+            }
+            if (lane < 16) o[128 + lane] = *reinterpret_cast<const uint32_t*>(s + scale_off);
+        } else {
+            const uint32_t* i = reinterpret_cast<const uint32_t*>(s + tiled_off);
+            *reinterpret_cast<uint32_t*>(d + code_off[0]) = i[lane * 4];
+            *reinterpret_cast<uint32_t*>(d + code_off[0] + 16) = i[lane * 4 + 1];
+            *reinterpret_cast<uint32_t*>(d + code_off[1]) = i[lane * 4 + 2];
+            *reinterpret_cast<uint32_t*>(d + code_off[1] + 16) = i[lane * 4 + 3];
+            if (lane < 16) *reinterpret_cast<uint32_t*>(d + scale_off) = i[128 + lane];
+        }
     }
 }
 
@@ -150,10 +154,9 @@ int tile_launch(const char* who, const void* src, size_t src_stride, void* dst, 
                     dst_stride, blob);
     if (n_experts == 0) return FRX_OK;
     const Geo G(n, ff);
-    const size_t words = size_t(n_experts) * G.total_units() * (kUnitBytes / 4);
-    const unsigned grid = unsigned((words + 255) / 256);
-    k_tile<TO_TILED><<<grid, 256, 0, stream>>>(static_cast<const uint8_t*>(src), src_stride, static_cast<uint8_t*>(dst), dst_stride,
-                                               n, ff, G.total_units(), words);
+    const int units = int(G.total_units());
+    k_tile<TO_TILED><<<dim3(unsigned((units + 7) / 8), unsigned(std::min(n_experts, 65535))), 256, 0, stream>>>(
+        static_cast<const uint8_t*>(src), src_stride, static_cast<uint8_t*>(dst), dst_stride, n, ff, units, n_experts);
     FRX_CUDA(cudaGetLastError());
     return FRX_OK;
 }
