@@ -70,15 +70,9 @@ struct DotArgs {
     int rows_per_tile;         // weight rows staged per step
     int tma;                   // 1: tiles are fetched by bulk copies (alignment checked on the host)
     unsigned long long wait_ns;
-    // direct jobs (gemv): job j has expert ids[j] (0 without ids), activation row j / act_div, output row j
+    // job j has expert ids[j] (0 without ids), activation row j / act_div, output row j
     const int32_t* ids;
     int n_jobs, act_div;
-    // grouped jobs (gemm): item i = up to NT slots of one expert from the grouped order
-    const int* bounds;
-    const int* item_off;
-    const int32_t* perm;
-    int* status;               // [1] = number of items
-    int E, K, x_per_slot;
 };
 
 struct DotSmem {
@@ -153,24 +147,7 @@ __global__ void __launch_bounds__(kDotThreads) k_ggml_dot(const DotArgs a) {
     __shared__ int s_act_rows[NT];
     int e = 0, m = 1;
     int act_rows[NT], dst_rows[NT];
-    if (a.perm) {
-        const int i = blockIdx.x;
-        if (i >= a.status[1]) return;
-        int lo = 0, hi = a.E;   // the expert with item_off[e] <= i < item_off[e + 1]
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (a.item_off[mid] <= i) lo = mid; else hi = mid;
-        }
-        e = lo;
-        const int base = a.bounds[e] + (i - a.item_off[e]) * kTokPerItem;
-        m = min(min(kTokPerItem, NT), a.bounds[e + 1] - base);
-#pragma unroll
-        for (int j = 0; j < NT; ++j) {
-            const int slot = j < m ? a.perm[base + j] : 0;
-            dst_rows[j] = slot;
-            act_rows[j] = a.x_per_slot ? slot : slot / a.K;
-        }
-    } else {
+    {
         const int j = blockIdx.x;
         e = a.ids ? a.ids[j] : 0;
 #pragma unroll
@@ -296,7 +273,6 @@ __global__ void __launch_bounds__(kDotThreads) k_ggml_dot(const DotArgs a) {
             }
         }
     }
-    if (*abort && tid == 0 && a.status) a.status[0] = kDevWaitTimeout;
 }
 
 int dot_tile_rows(int ncols) {
@@ -343,65 +319,318 @@ int check_dot_shape(const char* who, uint32_t type, int64_t ncols, int64_t nrows
     return FRX_OK;
 }
 
-// ---- Q8_0 -> Q2_0 (arch/qwen4exp/mtp.cu:129-201): one warp per 64 values. Lane l holds values l
-// and 32 + l; lanes 0..23 each try one candidate scale, adding the squared errors in index order.
-__device__ __forceinline__ int q2_code_dev(float v) { return int(v >= 0.5f) + int(v >= 1.5f) - int(v <= -0.5f); }
-__global__ void __launch_bounds__(256) k_q8_0_to_q2_0(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, size_t nblocks64) {
-    const size_t b = size_t(blockIdx.x) * 8 + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (b >= nblocks64) return;
-    const uint8_t* s = src + b * 68;
-    const float d_lo = __half2float(__ushort_as_half(uint16_t(s[0] | (s[1] << 8))));
-    const float d_hi = __half2float(__ushort_as_half(uint16_t(s[34] | (s[35] << 8))));
-    const float x_lo = __fmul_rn(d_lo, float(int8_t(s[2 + lane]))), x_hi = __fmul_rn(d_hi, float(int8_t(s[36 + lane])));
-    float amax = fmaxf(fabsf(x_lo), fabsf(x_hi));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    // candidate `lane`: d = amax / (2.5f - 1.5f * float(c) / 23.0f), through fp16
-    const float div = __fsub_rn(2.5f, __fdiv_rn(__fmul_rn(1.5f, float(lane)), 23.0f));
-    const float dq = __half2float(__float2half_rn(__fdiv_rn(amax, div)));
-    const bool usable = dq > 0.0f && dq < INFINITY;   // else every code is 0 (see the oracle's note on lround)
-    float e = 0.0f;
-    for (int j = 0; j < 64; ++j) {
-        const float xj = __shfl_sync(0xffffffffu, j < 32 ? x_lo : x_hi, j & 31);
-        const int q = usable ? q2_code_dev(__fdiv_rn(xj, dq)) : 0;
-        const float r = __fsub_rn(xj, __fmul_rn(float(q), dq));
-        e = __fadd_rn(e, __fmul_rn(r, r));
+// ---- Q8_0 -> Q2_0 (arch/qwen4exp/mtp.cu:129-201): a thread per 64 values, kept in registers; the 24 candidate
+// scales one after the other, the squared errors added in index order. A block's input (68 bytes per 64
+// values) and output (18 bytes) pass through shared memory in whole vectors.
+//
+// The inner loop has no division and no comparison. The values are d8 * q8 (exact, at most 18 significant
+// bits), a candidate d is an fp16 value (11 bits): if x / d is not exactly on a rounding boundary (-0.5, 0.5,
+// 1.5) it is at least 2^-18 of itself away from it, so a quotient good to 2^-22 gives the reference's code; on a
+// boundary either neighbour leaves the same |x - q d|, and only its square is used. The quotient is taken
+// as sat((x / d + 1) / 3) * 3, which clamps it to [-1, 2] in the same instruction, rounded by a magic
+// addition; x - q d rounds once in a fused multiply-add because q d is exact. The codes of the chosen scale
+// are decided by exact comparisons with 0.5 d and 1.5 d.
+// Bound: fp32 issue, six instructions per value and candidate. 48 experts of 2560 x 640 (236 M values): 8.1 ms
+// before (a warp per 64 values, one candidate per lane, a shuffle and an IEEE division per value), 1.2 ms now.
+constexpr int kRqThreads = 128;
+__global__ void __launch_bounds__(kRqThreads) k_q8_0_to_q2_0(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, size_t nblocks64) {
+    __shared__ __align__(16) uint8_t in[kRqThreads * 68];
+    __shared__ __align__(16) uint8_t out[kRqThreads * 18];
+    const size_t b0 = size_t(blockIdx.x) * kRqThreads;
+    const int tid = threadIdx.x, nb = int(min(size_t(kRqThreads), nblocks64 - b0));
+    const uint8_t* s = src + b0 * 68;
+    if (nb == kRqThreads && uintptr_t(s) % 16 == 0) {
+        for (int i = tid; i < kRqThreads * 68 / 16; i += kRqThreads) reinterpret_cast<uint4*>(in)[i] = reinterpret_cast<const uint4*>(s)[i];
+    } else {
+        for (int i = tid; i < nb * 68; i += kRqThreads) in[i] = s[i];
     }
-    // the first candidate with the smallest error wins; a NaN or infinite error never does
-    bool ok = lane < 24 && amax > 0.0f && e < INFINITY;
-    float be = ok ? e : INFINITY, bd = ok ? dq : 0.0f;
-    int bc = ok ? lane : 64;
+    __syncthreads();
+    if (tid < nb) {
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(in) + tid * 17;   // {d, 32 codes}, {d, 32 codes}
+        float x[64];
+        float amax = 0.0f;
+        const float d_lo = __half2float(__ushort_as_half(uint16_t(w[0] & 0xffffu))), d_hi = __half2float(__ushort_as_half(uint16_t(w[8] >> 16)));
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float oe = __shfl_xor_sync(0xffffffffu, be, o), od = __shfl_xor_sync(0xffffffffu, bd, o);
-        const int oc = __shfl_xor_sync(0xffffffffu, bc, o);
-        if (oc < 64 && (bc == 64 || oe < be || (oe == be && oc < bc))) {
-            be = oe;
-            bd = od;
-            bc = oc;
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t lo = __funnelshift_r(w[i], w[i + 1], 16), hi = w[9 + i];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                x[4 * i + k] = __fmul_rn(d_lo, float(int8_t(lo >> (8 * k))));
+                x[32 + 4 * i + k] = __fmul_rn(d_hi, float(int8_t(hi >> (8 * k))));
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 64; ++i) amax = fmaxf(amax, fabsf(x[i]));
+        float best_e = INFINITY, best_d = 0.0f;
+#pragma unroll 1
+        for (int c = 0; c < 24; ++c) {
+            // d = amax / (2.5f - 1.5f * float(c) / 23.0f), through fp16
+            const float div = __fsub_rn(2.5f, __fdiv_rn(__fmul_rn(1.5f, float(c)), 23.0f));
+            const float dq = __half2float(__float2half_rn(__fdiv_rn(amax, div)));
+            const bool usable = dq > 0.0f && dq < INFINITY;   // else every code is 0 (see the oracle's note on lround)
+            const float d = usable ? dq : 0.0f, inv3 = usable ? __fdiv_rn(1.0f, 3.0f * d) : 0.0f;
+            float e = 0.0f;
+#pragma unroll
+            for (int j = 0; j < 64; ++j) {
+                const float t = __fmaf_rn(__saturatef(__fmaf_rn(x[j], inv3, 1.0f / 3.0f)), 3.0f, kMagic);   // kMagic + q + 1
+                const float q = __fsub_rn(t, kMagic + 1.0f);
+                const float r = __fmaf_rn(-q, d, x[j]);
+                e = __fadd_rn(e, __fmul_rn(r, r));
+            }
+            // the first candidate with the smallest error wins; a NaN or infinite error never does
+            if (amax > 0.0f && dq < INFINITY && e < best_e) {
+                best_e = e;
+                best_d = dq;
+            }
+        }
+        const bool fin = best_d > 0.0f && best_d < INFINITY;
+        const float h1 = 0.5f * best_d, h3 = 1.5f * best_d;
+        uint16_t* o = reinterpret_cast<uint16_t*>(out + tid * 18);
+        o[0] = __half_as_ushort(__float2half_rn(best_d));
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {   // two bytes of four elements each
+            uint32_t v = 0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float xv = x[8 * k + i];
+                const int code = fin ? 1 + int(xv >= h1) + int(xv >= h3) - int(xv <= -h1) : 1;
+                v |= uint32_t(code) << (2 * i);
+            }
+            o[1 + k] = uint16_t(v);
         }
     }
-    const float best_d = bc < 64 ? bd : 0.0f;
-    const bool fin = best_d > 0.0f && best_d < INFINITY;
-    const int c_lo = best_d > 0.0f ? (fin ? q2_code_dev(__fdiv_rn(x_lo, best_d)) : 0) + 1 : 1;
-    const int c_hi = best_d > 0.0f ? (fin ? q2_code_dev(__fdiv_rn(x_hi, best_d)) : 0) + 1 : 1;
-    // byte L (L < 16) holds elements 4 L .. 4 L + 3
-    uint32_t byte = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int srcl = (4 * lane + k) & 31;
-        const int v_lo = __shfl_sync(0xffffffffu, c_lo, srcl), v_hi = __shfl_sync(0xffffffffu, c_hi, srcl);
-        byte |= uint32_t(lane < 8 ? v_lo : v_hi) << (2 * k);
+    __syncthreads();
+    uint8_t* d = dst + b0 * 18;
+    if (nb == kRqThreads && uintptr_t(d) % 16 == 0) {
+        for (int i = tid; i < kRqThreads * 18 / 16; i += kRqThreads) reinterpret_cast<uint4*>(d)[i] = reinterpret_cast<const uint4*>(out)[i];
+    } else {
+        for (int i = tid; i < nb * 18; i += kRqThreads) d[i] = out[i];
     }
-    uint8_t* o = dst + b * 18;
-    if (lane < 16) o[2 + lane] = uint8_t(byte);
-    if (lane == 0) *reinterpret_cast<__half*>(o) = __float2half_rn(best_d);   // blocks are 18 bytes: the scale is 2-byte aligned
+}
+
+// ---- the grouped product (gemm::moe_run): int8 tensor cores
+// A block takes 128 weight rows and up to 64 of the slots of one expert and walks K in chunks of 128 (two
+// blocks of weights, 36 bytes per row) through a ring of shared-memory stages filled with cp.async: the
+// rows as they are in the file, the activations in the MMA's fragment order, their scales and the
+// accumulators' initial values per pair of slots. 8 warps, 32 rows x 32 slots each: a lane reads a
+// row's 36 bytes (at a stride of 48: conflict-free 16-byte loads shared by the four lanes of a quad),
+// shifts lane t's crumbs into place and masks them, which gives the A operand for a K order of
+// {t, 4 + t, 8 + t, 12 + t}; the quantizer writes the activation codes in that order.
+// Per 32 values the MMA starts at kMagicBits - sum(codes) and so ends at kMagicBits + sum((q - 1) * a), which
+// read as a float is kMagic plus the chunk's exact integer sum.
+// What bounds it: issue slots and the int8 MMA together (a 16 x 8 x 64 tile costs two MMAs and eight packed
+// fp32 operations). 1,000 tokens x 8 of 128 experts of 2560 x 640, three products: 11.8 ms before (the dp4a kernel below,
+// eight slots per pass over the weights), 0.5 ms now.
+constexpr int kGmRows = 128, kGmTok = 64, kGmK = 128, kGmStages = 4, kGmThreads = 256;
+constexpr int kGmWStride = 48;                               // bytes per row of a chunk: 36 used
+constexpr int kGmBytesW = kGmRows * kGmWStride;              // 6 KB
+constexpr int kGmBytesB = kGmTok * kGmK;                     // [block][8 slots][lane] 16 bytes
+constexpr int kGmBytesA = 2 * (kGmTok / 2) * 16;             // [block][pair of slots] {a0, a0', a1, a1'}
+constexpr int kGmBytesC = 2 * (kGmTok / 2) * 32;             // [block][pair][half] {c, c', c, c'}
+constexpr int kGmStage = kGmBytesW + kGmBytesB + kGmBytesA + kGmBytesC;
+constexpr int kGmSmem = kGmStages * kGmStage;
+
+// Workspace form of the activations: per row int8 codes in fragment order (word (t * 4 + 2 s + h) of a 64-block
+// holds elements 32 s + 16 h + {t, 4 + t, 8 + t, 12 + t}), the chunk scales d (through fp16, as Q8_1 stores them),
+// and kMagicBits - sum(codes). Quantization is quantize.cu's: d = amax / 127, q = roundf(x / d).
+struct GmAct {
+    int8_t* q;     // [rows][ncols]
+    float* d;      // [rows][ncols / 32]
+    int32_t* c;    // [rows][ncols / 32]
+};
+__global__ void __launch_bounds__(256) k_gm_quant(const float* __restrict__ x, int ncols, size_t n_quads, GmAct a) {
+    const size_t quad = size_t(blockIdx.x) * 256 + threadIdx.x;   // four consecutive values; eight lanes one chunk of 32
+    if (quad >= n_quads) return;                                  // (a multiple of 32: warps are live as a whole)
+    float hv[4];
+    if (uintptr_t(x) % 16 == 0) {
+        const float4 v = reinterpret_cast<const float4*>(x)[quad];
+        hv[0] = v.x, hv[1] = v.y, hv[2] = v.z, hv[3] = v.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) hv[i] = x[quad * 4 + i];
+    }
+    float am = fmaxf(fmaxf(fabsf(hv[0]), fabsf(hv[1])), fmaxf(fabsf(hv[2]), fabsf(hv[3])));
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
+    const float d = __fdiv_rn(am, 127.0f);
+    int sum = 0;
+    const int j = int(quad & 7), h = j >> 2, i = j & 3;           // elements 16 h + 4 i + t of the chunk, t = 0 .. 3
+    const size_t chunk = quad >> 3;
+    int8_t* blk = a.q + (chunk >> 1) * 64 + (chunk & 1) * 8 + h * 4 + i;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        const int code = am == 0.0f ? 0 : int(round_half_away(__fdiv_rn(hv[t], d)));
+        sum += code;
+        blk[t * 16] = int8_t(code);
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (j == 0) {
+        a.d[chunk] = __half2float(__float2half_rn(d));
+        a.c[chunk] = kMagicBits - sum;
+    }
+}
+
+struct GmArgs {
+    const uint8_t* w;        // expert e's matrix at w + e * expert_stride
+    size_t expert_stride;
+    GmAct act;
+    float* dst;              // [slots][nrows]
+    int ncols, nrows;
+    const int* bounds;       // [E + 1] of the grouped order
+    const int* item_off;     // [E + 1] items of kGmTok slots in front of an expert
+    const int32_t* perm;
+    const int* status;       // [1] = number of items
+    int E, K, x_per_slot;
+};
+
+__device__ __forceinline__ void gm_cp4(uint32_t dst, const void* src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ void gm_cp16(uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
+
+__global__ void __launch_bounds__(kGmThreads, 2) k_gm_mma(const GmArgs a) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ int s_slot[kGmTok], s_act[kGmTok];
+    const int item = blockIdx.x;
+    if (item >= a.status[1]) return;
+    int lo = 0, hi = a.E;   // the expert with item_off[e] <= item < item_off[e + 1]
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (a.item_off[mid] <= item) lo = mid; else hi = mid;
+    }
+    const int e = lo, base = a.bounds[e] + (item - a.item_off[e]) * kGmTok, m = min(kGmTok, a.bounds[e + 1] - base);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+    if (tid < kGmTok) {   // columns beyond m repeat the last slot and are not stored
+        const int slot = a.perm[base + min(tid, m - 1)];
+        s_slot[tid] = slot;
+        s_act[tid] = a.x_per_slot ? slot : slot / a.K;
+    }
+    __syncthreads();
+    const int r0 = blockIdx.y * kGmRows, rows = min(kGmRows, a.nrows - r0);
+    const uint32_t row_bytes = uint32_t(a.ncols / kQK) * kBlockBytes;
+    const uint8_t* wsrc = a.w + size_t(e) * a.expert_stride + size_t(r0) * row_bytes;
+    const uint32_t s0 = smem_u32(smem);
+    const int m8 = (m + 7) & ~7;   // slots whose activations are fetched
+
+    // this thread's copies of a chunk. Weights: 128 rows x 9 words, 4.5 per thread; codes: m8 x 8 vectors of 16 bytes
+    const int nch = a.ncols / kQ8;
+    auto fetch = [&](int kc) {
+        const uint32_t st = s0 + uint32_t(kc % kGmStages) * kGmStage;
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+            const int idx = tid + i * kGmThreads;
+            if (idx < kGmRows * 9) {
+                const int row = idx / 9, w = idx - row * 9;
+                gm_cp4(st + row * kGmWStride + w * 4, wsrc + size_t(min(row, rows - 1)) * row_bytes + size_t(kc) * 36 + w * 4);
+            }
+        }
+        const uint32_t sb = st + kGmBytesW;
+        for (int idx = tid; idx < m8 * 8; idx += kGmThreads) {
+            const int tok = idx >> 3, v = idx & 7;   // vector v: block v >> 2, lane t = v & 3
+            gm_cp16(sb + (v >> 2) * (kGmTok * 64) + (tok >> 3) * 512 + ((tok & 7) * 4 + (v & 3)) * 16, a.act.q + size_t(s_act[tok]) * a.ncols + size_t(kc) * kGmK + v * 16);
+        }
+        const uint32_t sa = sb + kGmBytesB, sc = sa + kGmBytesA;
+        for (int idx = tid; idx < m8 * 4; idx += kGmThreads) {
+            const int tok = idx >> 2, ch = idx & 3, b = ch >> 1, h = ch & 1;   // chunk ch of the four of 128 values
+            const size_t at = size_t(s_act[tok]) * nch + size_t(kc) * 4 + ch;
+            const uint32_t pair = uint32_t(b * (kGmTok / 2) + (tok >> 1));
+            gm_cp4(sa + pair * 16 + h * 8 + (tok & 1) * 4, a.act.d + at);
+            gm_cp4(sc + pair * 32 + h * 16 + (tok & 1) * 4, a.act.c + at);
+            gm_cp4(sc + pair * 32 + h * 16 + 8 + (tok & 1) * 4, a.act.c + at);
+        }
+    };
+    const int chunks = a.ncols / kGmK;
+#pragma unroll
+    for (int i = 0; i < kGmStages - 1; ++i) {
+        if (i < chunks) fetch(i);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    const int wr = (warp & 3) * 32, wt = (warp >> 2) * 32;   // this warp's rows and slots of the tile
+    const int nt = min(4, (m - wt + 7) >> 3);                // live columns of eight slots
+    uint64_t acc[2][4][2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int n = 0; n < 4; ++n) acc[r][n][0] = acc[r][n][1] = 0ull;
+    const uint64_t magic = pack2(kMagic, kMagic);
+    for (int kc = 0; kc < chunks; ++kc) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kGmStages - 2) : "memory");
+        __syncthreads();   // everyone's share of this chunk has landed, and everyone is done with the chunk before
+        if (kc + kGmStages - 1 < chunks) fetch(kc + kGmStages - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (nt <= 0) continue;
+        const uint8_t* st = smem + (kc % kGmStages) * kGmStage;
+        const uint8_t* sw = st + (wr + g) * kGmWStride;
+        uint32_t w[2][2][8];      // [group of 16 rows][row g / g + 8][word]: this lane's crumbs, lowest two bits of every byte
+        uint64_t dw[2][2][2];     // [group][row][block]: the weight scale, twice
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint8_t* p = sw + (r * 16 + h * 8) * kGmWStride;
+                const uint4 v0 = *reinterpret_cast<const uint4*>(p), v1 = *reinterpret_cast<const uint4*>(p + 16);
+                const uint32_t v2 = *reinterpret_cast<const uint32_t*>(p + 32);
+                const float d0 = __half2float(__ushort_as_half(uint16_t(v0.x & 0xffffu))), d1 = __half2float(__ushort_as_half(uint16_t(v1.x >> 16)));
+                dw[r][h][0] = pack2(d0, d0);
+                dw[r][h][1] = pack2(d1, d1);
+                w[r][h][0] = __funnelshift_r(v0.x, v0.y, 16);
+                w[r][h][1] = __funnelshift_r(v0.y, v0.z, 16);
+                w[r][h][2] = __funnelshift_r(v0.z, v0.w, 16);
+                w[r][h][3] = __funnelshift_r(v0.w, v1.x, 16);
+                w[r][h][4] = v1.y;
+                w[r][h][5] = v1.z;
+                w[r][h][6] = v1.w;
+                w[r][h][7] = v2;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) w[r][h][i] = (w[r][h][i] >> (2 * t4)) & 0x03030303u;
+            }
+        const uint8_t* sb = st + kGmBytesW + (wt >> 3) * 512 + lane * 16;
+        const uint8_t* sa = st + kGmBytesW + kGmBytesB + ((wt >> 1) + t4) * 16;
+        const uint8_t* sc = st + kGmBytesW + kGmBytesB + kGmBytesA + ((wt >> 1) + t4) * 32;
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+            for (int n = 0; n < 4; ++n) {
+                if (n >= nt) break;
+                const uint4 bf = *reinterpret_cast<const uint4*>(sb + b * (kGmTok * 64) + n * 512);
+                const ulonglong2 d8 = *reinterpret_cast<const ulonglong2*>(sa + b * (kGmTok / 2 * 16) + n * 64);
+                const int4 c0 = *reinterpret_cast<const int4*>(sc + b * (kGmTok / 2 * 32) + n * 128), c1 = *reinterpret_cast<const int4*>(sc + b * (kGmTok / 2 * 32) + n * 128 + 16);
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    uint64_t lo0, hi0, lo1, hi1;
+                    mma_u8s8_c4(lo0, hi0, w[r][0][4 * b], w[r][1][4 * b], w[r][0][4 * b + 1], w[r][1][4 * b + 1], bf.x, bf.y, c0);
+                    mma_u8s8_c4(lo1, hi1, w[r][0][4 * b + 2], w[r][1][4 * b + 2], w[r][0][4 * b + 3], w[r][1][4 * b + 3], bf.z, bf.w, c1);
+                    // acc += d2 * (d8[0] * sum0 + d8[1] * sum1)
+                    const uint64_t u_lo = fma2(d8.y, sub2(lo1, magic), mul2(d8.x, sub2(lo0, magic)));
+                    const uint64_t u_hi = fma2(d8.y, sub2(hi1, magic), mul2(d8.x, sub2(hi0, magic)));
+                    acc[r][n][0] = fma2(dw[r][0][b], u_lo, acc[r][n][0]);
+                    acc[r][n][1] = fma2(dw[r][1][b], u_hi, acc[r][n][1]);
+                }
+            }
+    }
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+        if (n >= nt) break;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int tok = wt + n * 8 + 2 * t4 + k;
+            if (tok >= m) continue;
+            float* o = a.dst + size_t(s_slot[tok]) * a.nrows + r0;
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float v0, v1;
+                    unpack2(acc[r][n][h], v0, v1);
+                    const int row = wr + r * 16 + h * 8 + g;
+                    if (row < rows) o[row] = k ? v1 : v0;
+                }
+        }
+    }
 }
 
 // ---- grouped plan in a workspace
 struct PlanLayout {
-    size_t status, chunk_cnt, bounds, item_off, perm, act, total;
+    size_t status, chunk_cnt, bounds, item_off, perm, act_q, act_d, act_c, total;
     int n_chunks, max_items;
 };
 PlanLayout plan_layout(int64_t ncols, int64_t rows, int E) {
@@ -413,17 +642,22 @@ PlanLayout plan_layout(int64_t ncols, int64_t rows, int E) {
         return o;
     };
     L.n_chunks = int((rows + kChunkSlots - 1) / kChunkSlots);
-    L.max_items = int(rows / kTokPerItem) + E;
+    L.max_items = int(rows / kGmTok) + E;
     L.status = take(64);
     L.chunk_cnt = take(size_t(L.n_chunks) * E * 4);
     L.bounds = take(size_t(E + 1) * 4);
     L.item_off = take(size_t(E + 1) * 4);
     L.perm = take(size_t(rows) * 4);
-    L.act = take(size_t(rows) * act_row_bytes(ncols));
+    L.act_q = take(size_t(rows) * ncols);
+    L.act_d = take(size_t(rows) * (ncols / kQ8) * 4);
+    L.act_c = take(size_t(rows) * (ncols / kQ8) * 4);
     L.total = off;
     return L;
 }
 constexpr int kPlanMaxExperts = 4096;
+GmAct plan_act(uint8_t* base, const PlanLayout& L) {
+    return GmAct{reinterpret_cast<int8_t*>(base + L.act_q), reinterpret_cast<float*>(base + L.act_d), reinterpret_cast<int32_t*>(base + L.act_c)};
+}
 
 }  // namespace
 }  // namespace frx
@@ -572,10 +806,11 @@ int frx_gemm_moe_prepare(frx_gemm_moe_plan* plan, uint32_t ggml_type, int n_expe
     int* item_off = reinterpret_cast<int*>(base + L.item_off);
     int32_t* perm = reinterpret_cast<int32_t*>(base + L.perm);
     const int S = int(rows), E = n_experts;
-    // one Q8_1 row per token, or per (token, expert) slot when every slot has its own activations
-    if (int rc = frx_gemv_quantize_q8_1(x, ncols, int(x_per_slot ? rows : T), base + L.act, stream)) return rc;
+    // one row of codes per token, or per (token, expert) slot when every slot has its own activations
+    const size_t n_quads = size_t(x_per_slot ? rows : T) * size_t(ncols / 4);
+    FRX_LAUNCH(kKQuant, stream, k_gm_quant<<<unsigned((n_quads + 255) / 256), 256, 0, stream>>>(x, int(ncols), n_quads, plan_act(base, L)));
     FRX_LAUNCH(kKGroup, stream, k_pf_hist<<<L.n_chunks, 256, size_t(E) * 4, stream>>>(ids, S, E, chunk_cnt, status));
-    FRX_LAUNCH(kKGroup, stream, k_pf_scan<<<1, 1024, 0, stream>>>(chunk_cnt, L.n_chunks, E, bounds, item_off, status, L.max_items));
+    FRX_LAUNCH(kKGroup, stream, k_pf_scan<<<1, 1024, 0, stream>>>(chunk_cnt, L.n_chunks, E, bounds, item_off, status, L.max_items, kGmTok));
     FRX_LAUNCH(kKGroup, stream, k_pf_place<<<L.n_chunks, 32, size_t(E) * 4, stream>>>(ids, S, E, chunk_cnt, bounds, perm));
     FRX_CUDA(cudaGetLastError());
     return FRX_OK;
@@ -590,22 +825,29 @@ int frx_gemm_moe_run(const frx_gemm_moe_plan* plan, const void* W, int64_t exper
     if (plan->T == 0) return FRX_OK;
     const PlanLayout L = plan_layout(plan->ncols, plan->rows, plan->n_experts);
     auto* base = static_cast<uint8_t*>(plan->ws);
-    DotArgs a{};
+    static std::once_flag once[64];
+    int dev = 0;
+    FRX_CUDA(cudaGetDevice(&dev));
+    cudaError_t attr = cudaSuccess;
+    if (dev >= 0 && dev < 64) std::call_once(once[dev], [&] { attr = cudaFuncSetAttribute(k_gm_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, kGmSmem); });
+    if (attr != cudaSuccess) return cuda_fail(attr, "gemm::moe_run: cudaFuncSetAttribute");
+    GmArgs a{};
     a.w = static_cast<const uint8_t*>(W);
     a.expert_stride = size_t(expert_stride_bytes);
-    a.xq = base + L.act;
-    a.act_row = act_row_bytes(plan->ncols);
+    a.act = plan_act(base, L);
     a.dst = y;
     a.ncols = int(plan->ncols);
     a.nrows = int(nrows);
     a.bounds = reinterpret_cast<const int*>(base + L.bounds);
     a.item_off = reinterpret_cast<const int*>(base + L.item_off);
     a.perm = reinterpret_cast<const int32_t*>(base + L.perm);
-    a.status = reinterpret_cast<int*>(base + L.status);
+    a.status = reinterpret_cast<const int*>(base + L.status);
     a.E = plan->n_experts;
     a.K = plan->K;
     a.x_per_slot = plan->x_per_slot;
-    FRX_LAUNCH(kKDown, stream, { if (int rc = launch_dot<kTokPerItem, false>(a, L.max_items, stream)) return rc; });
+    const dim3 grid(unsigned(L.max_items), unsigned((nrows + kGmRows - 1) / kGmRows));
+    FRX_LAUNCH(kKDown, stream, k_gm_mma<<<grid, kGmThreads, kGmSmem, stream>>>(a));
+    FRX_CUDA(cudaGetLastError());
     return FRX_OK;
 }
 
@@ -620,7 +862,7 @@ int frx_convert_q8_0_to_q2_0(const void* src_q8_0, void* dst_q2_0, size_t nblock
     if (nblocks64 == 0) return FRX_OK;
     if (!src_q8_0 || !dst_q2_0) return fail(FRX_ERR_ARG, "convert_q8_0_to_q2_0: null pointer");
     if (nblocks64 > (size_t(1) << 34)) return fail(FRX_ERR_SHAPE, "convert_q8_0_to_q2_0: too many blocks");
-    FRX_LAUNCH(kKLayout, stream, k_q8_0_to_q2_0<<<unsigned((nblocks64 + 7) / 8), 256, 0, stream>>>(static_cast<const uint8_t*>(src_q8_0), static_cast<uint8_t*>(dst_q2_0), nblocks64));
+    FRX_LAUNCH(kKLayout, stream, k_q8_0_to_q2_0<<<unsigned((nblocks64 + kRqThreads - 1) / kRqThreads), kRqThreads, 0, stream>>>(static_cast<const uint8_t*>(src_q8_0), static_cast<uint8_t*>(dst_q2_0), nblocks64));
     FRX_CUDA(cudaGetLastError());
     return FRX_OK;
 }

@@ -48,9 +48,9 @@ __global__ void __launch_bounds__(256) k_pf_hist(const int32_t* __restrict__ ids
 }
 
 // per expert: exclusive offsets of its slots over the chunks (written back into chunk_cnt), its
-// bounds in the grouped order, and the range of its items. bounds, item_off: [E + 1].
+// bounds in the grouped order, and the range of its items of per_item slots. bounds, item_off: [E + 1].
 __global__ void __launch_bounds__(1024) k_pf_scan(int* __restrict__ chunk_cnt, int n_chunks, int E, int* __restrict__ bounds,
-                                                  int* __restrict__ item_off, int* __restrict__ status, int max_items) {
+                                                  int* __restrict__ item_off, int* __restrict__ status, int max_items, int per_item = kTokPerItem) {
     __shared__ int scan_s[1024], scan_i[1024];
     const int tid = threadIdx.x;
     const int per = (E + 1023) / 1024, e0 = tid * per, e1 = min(E, e0 + per);
@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(1024) k_pf_scan(int* __restrict__ chunk_cnt, i
         }
         bounds[e] = run;   // the count for now
         slots += run;
-        items += (run + kTokPerItem - 1) / kTokPerItem;
+        items += (run + per_item - 1) / per_item;
     }
     scan_s[tid] = slots;
     scan_i[tid] = items;
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(1024) k_pf_scan(int* __restrict__ chunk_cnt, i
         bounds[e] = at_s;
         item_off[e] = at_i;
         at_s += c;
-        at_i += (c + kTokPerItem - 1) / kTokPerItem;
+        at_i += (c + per_item - 1) / per_item;
     }
     if (tid == 0) {
         bounds[E] = scan_s[1023];

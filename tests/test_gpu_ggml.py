@@ -137,3 +137,23 @@ def test_unsupported_type_and_shapes_are_rejected():
         moe.gemv.moe_q(8, z, None, z, ids, 512, 4, 144 * 4, False)
     with pytest.raises(moe.FrxError, match="multiple of 128"):
         moe.gemv.moe_q(Q2_0, z, None, z, ids, 192, 4, 54 * 4, False)
+
+
+@pytest.mark.parametrize("ncols,nrows,T,K,E", [(128, 1, 1, 1, 1), (256, 129, 65, 1, 1), (384, 127, 64, 2, 2), (640, 130, 9, 3, 5), (2560, 96, 33, 2, 1)])
+def test_grouped_products_at_tile_edges(port, ncols, nrows, T, K, E):
+    # tiles of 128 rows x 64 slots x 128 of K: one value of each, one less, one more, and fewer chunks than ring stages
+    rng = np.random.default_rng(ncols + nrows)
+    w = np.stack([synth.ggml_blocks(rng, nrows, ncols) for _ in range(E)]).reshape(E, -1)
+    stride = (w.shape[1] + 35) // 36 * 36                  # a whole number of blocks and of 4-byte words
+    wp = np.zeros((E, stride), np.uint8)
+    wp[:, :w.shape[1]] = w
+    ids = rng.integers(0, E, size=(T, K)).astype(np.int32)
+    x = rng.standard_normal((T, ncols)).astype(np.float32)
+    ws = moe.workspace(moe.gemm.workspace_bytes(ncols, T * K))
+    plan = moe.gemm.moe_prepare(Q2_0, E, cuda(x), False, cuda(ids), ncols, ws)
+    y = moe.gemm.moe_run(plan, cuda(wp.reshape(-1)), stride, nrows).cpu().numpy()
+    xq = port.quantize_q8_1(x)
+    for t0 in range(0, T, 8):
+        want = port.moe_q2_0(wp.reshape(-1), None, xq[t0:t0 + 8].reshape(-1), ids[t0:t0 + 8], ncols, nrows, stride, False)
+        # another order of at most 80 fp32 additions per row: 80 * 2^-24 of the terms' magnitude
+        assert rel_l2(y[t0:t0 + 8], want) < 1e-5
