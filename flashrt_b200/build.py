@@ -1,4 +1,5 @@
-"""Compiles libfrx.so (every CUDA source under csrc/) for sm_100a, in tree.
+"""Compiles libfrx.so (every CUDA source under csrc/) for sm_100a, in tree, and _frxpy.so, the Python
+binding of its frequently called entry points.
 
     python -m flashrt_b200.build
 
@@ -10,10 +11,12 @@ import glob
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 LIB = os.path.join(HERE, "libfrx.so")
+BINDING = os.path.join(HERE, "_frxpy.so")
 
 
 def sources() -> list[str]:
@@ -21,10 +24,10 @@ def sources() -> list[str]:
 
 
 def needs_build() -> bool:
-    if not os.path.exists(LIB):
+    if not os.path.exists(LIB) or not os.path.exists(BINDING):
         return True
-    t = os.path.getmtime(LIB)
-    deps = sources() + glob.glob(os.path.join(HERE, "csrc", "*.cuh")) + glob.glob(os.path.join(ROOT, "include", "*.h"))
+    t = min(os.path.getmtime(LIB), os.path.getmtime(BINDING))
+    deps = sources() + glob.glob(os.path.join(HERE, "csrc", "*.c")) + glob.glob(os.path.join(HERE, "csrc", "*.cuh")) + glob.glob(os.path.join(ROOT, "include", "*.h"))
     return any(os.path.getmtime(d) > t for d in deps)
 
 
@@ -43,7 +46,17 @@ def build(force: bool = False, verbose: bool = False) -> str:
         raise RuntimeError("nvcc failed:\n" + r.stdout + r.stderr)
     if verbose:
         print(r.stderr)
+    build_binding()
     return LIB
+
+
+def build_binding() -> str:
+    cmd = [os.environ.get("CC", "gcc"), "-O2", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"], "-I" + os.path.join(ROOT, "include"),
+           "-o", BINDING, os.path.join(HERE, "csrc", "py_frx.c"), "-L" + HERE, "-l:libfrx.so", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("the Python binding does not compile:\n" + r.stdout + r.stderr)
+    return BINDING
 
 
 if __name__ == "__main__":

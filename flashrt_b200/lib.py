@@ -28,6 +28,8 @@ if not os.path.exists(LIB_PATH):
 
 lib = C.CDLL(LIB_PATH)
 
+from . import _frxpy as fast  # noqa: E402  (the frequently called entry points without ctypes; built with the library)
+
 _vp, _sz, _i, _i64 = C.c_void_p, C.c_size_t, C.c_int, C.c_int64
 
 # name -> (restype, argtypes); every symbol include/frx.h declares

@@ -13,7 +13,7 @@ import ctypes as C
 import torch
 
 from . import lib as _l
-from .lib import FrxError, check, lib  # noqa: F401
+from .lib import FrxError, check, fast, lib  # noqa: F401
 
 Q2_0_TYPE = 42          # ggml type id (core/formats.hpp:11-18)
 BLOCK, BLOCK_BYTES, Q8_BLOCK = 64, 18, 32
@@ -23,9 +23,20 @@ def _ptr(t: torch.Tensor | None):
     return None if t is None else C.c_void_p(t.data_ptr())
 
 
+_current_raw_stream, _current_device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+
+
+def _raw_stream(stream=None) -> int:
+    """The handle of `stream`, or of the current one (without making a Stream object of it)."""
+    return _current_raw_stream(_current_device()) if stream is None else stream.cuda_stream
+
+
 def _stream(stream=None):
-    s = torch.cuda.current_stream() if stream is None else stream
-    return C.c_void_p(s.cuda_stream)
+    return C.c_void_p(_raw_stream(stream))
+
+
+def _addr(t: torch.Tensor | None):
+    return None if t is None else t.data_ptr()
 
 
 def _dev(*ts):
@@ -187,10 +198,9 @@ def moe_route_topk(logits: torch.Tensor, k: int, counts: torch.Tensor | None = N
     index) and weights float [T][k]."""
     _dev(logits, counts, tail_counts)
     T, E = logits.shape
-    ids = torch.empty(T, k, dtype=torch.int32, device=logits.device)
-    wts = torch.empty(T, k, dtype=torch.float32, device=logits.device)
-    check(lib.frx_route_topk(_stream(stream), _ptr(logits), T, E, k, _ptr(ids), _ptr(wts), _ptr(counts), _ptr(tail_counts),
-                             tail_from))
+    ids = logits.new_empty((T, k), dtype=torch.int32)
+    wts = logits.new_empty((T, k), dtype=torch.float32)
+    check(fast.route_topk(_raw_stream(stream), logits.data_ptr(), T, E, k, ids.data_ptr(), wts.data_ptr(), _addr(counts), _addr(tail_counts), tail_from))
     return ids, wts
 
 
@@ -202,9 +212,9 @@ def router_logits(w_router: torch.Tensor, w_gate: torch.Tensor | None, x: torch.
         raise FrxError(_l.ERR_ARG, "router_logits: bf16 weights and fp32 activations")
     T, n = x.shape
     E = w_router.shape[0]
-    logits = torch.empty(T, E, dtype=torch.float32, device=x.device)
-    gate = torch.empty(T, dtype=torch.float32, device=x.device) if w_gate is not None else None
-    check(lib.frx_router_logits(_stream(stream), _ptr(w_router), _ptr(w_gate), _ptr(x), T, E, n, _ptr(logits), _ptr(gate)))
+    logits = x.new_empty((T, E))
+    gate = x.new_empty((T,)) if w_gate is not None else None
+    check(fast.router_logits(_raw_stream(stream), w_router.data_ptr(), _addr(w_gate), x.data_ptr(), T, E, n, logits.data_ptr(), _addr(gate)))
     return logits, gate
 
 
@@ -212,9 +222,9 @@ def quantize_q8(x: torch.Tensor, stream=None):
     """q2_0::quantize_q8 for every row of x [T][n]: codes int8 [T][n], scales float [T][n/32]."""
     _dev(x)
     T, n = x.shape
-    q = torch.empty(T, n, dtype=torch.int8, device=x.device)
-    d = torch.empty(T, n // Q8_BLOCK, dtype=torch.float32, device=x.device)
-    check(lib.frx_quantize_q8(_stream(stream), _ptr(x), T, n, _ptr(q), _ptr(d)))
+    q = x.new_empty((T, n), dtype=torch.int8)
+    d = x.new_empty((T, n // Q8_BLOCK), dtype=torch.float32)
+    check(fast.quantize_q8(_raw_stream(stream), x.data_ptr(), T, n, q.data_ptr(), d.data_ptr()))
     return q, d
 
 
@@ -233,10 +243,15 @@ def workspace(nbytes: int, device="cuda") -> torch.Tensor:
     return torch.zeros(nbytes + 256, dtype=torch.uint8, device=device)
 
 
-def _ws_ptr(ws: torch.Tensor):
+def _ws_span(ws: torch.Tensor):
     p = ws.data_ptr()
-    a = (p + 255) // 256 * 256
-    return C.c_void_p(a), ws.numel() - (a - p)
+    a = (p + 255) & ~255
+    return a, ws.numel() - (a - p)
+
+
+def _ws_ptr(ws: torch.Tensor):
+    a, n = _ws_span(ws)
+    return C.c_void_p(a), n
 
 
 def workspace_status(ws: torch.Tensor, stream=None) -> None:
@@ -256,9 +271,9 @@ def moe_decode(experts: int, stride: int, E: int, shared: int | None, n: int, ff
         out = torch.empty(T, n, dtype=torch.float32, device=x.device)
     if ws is None:
         ws = workspace(moe_decode_workspace_bytes(T, K, n, ff), x.device)
-    wp, wb = _ws_ptr(ws)
-    check(lib.frx_moe_decode(C.c_void_p(experts), stride, E, C.c_void_p(shared) if shared else None, n, ff, _ptr(x), _ptr(ids),
-                             _ptr(wts), _ptr(gate_logit), T, K, _ptr(out), _ptr(yslot), wp, wb, _stream(stream)))
+    wp, wb = _ws_span(ws)
+    check(fast.moe_decode(experts, stride, E, shared, n, ff, x.data_ptr(), ids.data_ptr(), wts.data_ptr(), _addr(gate_logit), T, K, out.data_ptr(),
+                          _addr(yslot), wp, wb, _raw_stream(stream)))
     return out
 
 
@@ -268,8 +283,8 @@ def moe_decode_static(experts: int, stride: int, E: int, shared: int | None, n: 
     4 MiB scratch is used (frx_moe_decode_static). Calls on one device must not overlap."""
     _dev(x, ids, wts, gate_logit, out)
     T, K = ids.shape
-    check(lib.frx_moe_decode_static(C.c_void_p(experts), stride, E, C.c_void_p(shared) if shared else None, n, ff, _ptr(x), _ptr(ids),
-                                    _ptr(wts), _ptr(gate_logit), T, K, _ptr(out), _stream(stream)))
+    check(fast.moe_decode_static(experts, stride, E, shared, n, ff, x.data_ptr(), ids.data_ptr(), wts.data_ptr(), _addr(gate_logit), T, K, out.data_ptr(),
+                                 _raw_stream(stream)))
     return out
 
 
@@ -283,9 +298,9 @@ def moe_layer(experts: int, stride: int, E: int, shared: int | None, n: int, ff:
         out = torch.empty(T, n, dtype=torch.float32, device=x.device)
     if ws is None:
         ws = workspace(moe_layer_workspace_bytes(T, K, n, ff), x.device)
-    wp, wb = _ws_ptr(ws)
-    check(lib.frx_moe_layer(C.c_void_p(experts), stride, E, C.c_void_p(shared) if shared else None, n, ff, _ptr(x), _ptr(logits),
-                            _ptr(gate_logit), T, K, _ptr(out), _ptr(ids_out), _ptr(wts_out), wp, wb, _stream(stream)))
+    wp, wb = _ws_span(ws)
+    check(fast.moe_layer(experts, stride, E, shared, n, ff, x.data_ptr(), logits.data_ptr(), _addr(gate_logit), T, K, out.data_ptr(), _addr(ids_out),
+                         _addr(wts_out), wp, wb, _raw_stream(stream)))
     return out
 
 
@@ -390,8 +405,8 @@ def moe_hits(hit_ptr: torch.Tensor, hit_n: torch.Tensor, K: int, x: torch.Tensor
     _dev(hit_ptr, hit_n, x, yh, scratch)
     if scratch is None:
         scratch = workspace(moe_hits_scratch_bytes(K, n, ff, T), x.device)
-    sp, sb = _ws_ptr(scratch)
-    check(lib.frx_moe_hits(_ptr(hit_ptr), _ptr(hit_n), K, _ptr(x), n, ff, sp, sb, _ptr(yh), _stream(stream), T))
+    sp, sb = _ws_span(scratch)
+    check(fast.moe_hits(hit_ptr.data_ptr(), hit_n.data_ptr(), K, x.data_ptr(), n, ff, sp, sb, yh.data_ptr(), _raw_stream(stream), T))
     return yh
 
 
@@ -401,8 +416,8 @@ def moe_combine(yh: torch.Tensor, w: torch.Tensor, hit_n: torch.Tensor | None, s
     _dev(yh, w, hit_n, shexp, gate, out)
     T, K, n = yh.shape
     if out is None:
-        out = torch.empty(T, n, dtype=torch.float32, device=yh.device)
-    check(lib.frx_moe_combine(_ptr(out), _ptr(yh), _ptr(w), _ptr(hit_n), _ptr(shexp), _ptr(gate), n, K, T, _stream(stream)))
+        out = yh.new_empty((T, n), dtype=torch.float32)
+    check(fast.moe_combine(out.data_ptr(), yh.data_ptr(), w.data_ptr(), _addr(hit_n), _addr(shexp), _addr(gate), n, K, T, _raw_stream(stream)))
     return out
 
 
@@ -452,6 +467,11 @@ class gemv:
         return int(lib.frx_gemv_q8_1_bytes(ncols, n_tok))
 
     @staticmethod
+    def _q8_1_bytes(ncols: int, n_tok: int) -> int:
+        """q8_1_bytes for sizes that the call it is for checks: rows padded to 512 values, 36 bytes per 32."""
+        return max(n_tok, 0) * ((ncols + 511) // 512 * 576)
+
+    @staticmethod
     def row_bytes(ggml_type: int, ncols: int) -> int:
         return int(lib.frx_gemv_row_bytes(ggml_type, ncols))
 
@@ -459,16 +479,16 @@ class gemv:
     def quantize_q8_1(x: torch.Tensor, stream=None) -> torch.Tensor:
         _dev(x)
         n_tok, ncols = x.shape
-        xq = torch.empty(gemv.q8_1_bytes(ncols, n_tok), dtype=torch.uint8, device=x.device)
-        check(lib.frx_gemv_quantize_q8_1(_ptr(x), ncols, n_tok, _ptr(xq), _stream(stream)))
+        xq = x.new_empty((gemv._q8_1_bytes(ncols, n_tok),), dtype=torch.uint8)
+        check(fast.gemv_quantize_q8_1(x.data_ptr(), ncols, n_tok, xq.data_ptr(), _raw_stream(stream)))
         return xq
 
     @staticmethod
     def swiglu_q8_1(g: torch.Tensor, u: torch.Tensor, stream=None) -> torch.Tensor:
         _dev(g, u)
         n_tok, ncols = g.shape
-        xq = torch.empty(gemv.q8_1_bytes(ncols, n_tok), dtype=torch.uint8, device=g.device)
-        check(lib.frx_gemv_swiglu_q8_1(_ptr(g), _ptr(u), ncols, n_tok, _ptr(xq), _stream(stream)))
+        xq = g.new_empty((gemv._q8_1_bytes(ncols, n_tok),), dtype=torch.uint8)
+        check(fast.gemv_swiglu_q8_1(g.data_ptr(), u.data_ptr(), ncols, n_tok, xq.data_ptr(), _raw_stream(stream)))
         return xq
 
     @staticmethod
@@ -477,9 +497,9 @@ class gemv:
         """dst [n_tok][k][nrows] = W_{ids[t][j]} x (silu(G x) * (W x) with gate)."""
         _dev(w, gate, xq, ids)
         n_tok, k = ids.shape
-        dst = torch.empty(n_tok, k, nrows, dtype=torch.float32, device=w.device)
-        check(lib.frx_gemv_moe_q(ggml_type, _ptr(w), _ptr(gate), _ptr(xq), _ptr(ids), _ptr(dst), n_tok, k, ncols, nrows, expert_stride_bytes,
-                                 int(act_per_expert), _stream(stream)))
+        dst = w.new_empty((n_tok, k, nrows), dtype=torch.float32)
+        check(fast.gemv_moe_q(ggml_type, w.data_ptr(), _addr(gate), xq.data_ptr(), ids.data_ptr(), dst.data_ptr(), n_tok, k, ncols, nrows,
+                              expert_stride_bytes, int(act_per_expert), _raw_stream(stream)))
         return dst
 
     @staticmethod
@@ -487,18 +507,18 @@ class gemv:
                  slot_stride_bytes: int, per_channel_act: bool, stream=None) -> torch.Tensor:
         _dev(w, gate, xq, ids)
         n_ids = ids.numel()
-        dst = torch.empty(n_ids, nrows, dtype=torch.float32, device=w.device)
-        check(lib.frx_gemv_moe_q2_0(_ptr(w), _ptr(gate), _ptr(xq), _ptr(ids), _ptr(dst), n_ids, ncols, nrows, slot_stride_bytes,
-                                    int(per_channel_act), _stream(stream)))
+        dst = w.new_empty((n_ids, nrows), dtype=torch.float32)
+        check(fast.gemv_moe_q2_0(w.data_ptr(), _addr(gate), xq.data_ptr(), ids.data_ptr(), dst.data_ptr(), n_ids, ncols, nrows, slot_stride_bytes,
+                                 int(per_channel_act), _raw_stream(stream)))
         return dst
 
     @staticmethod
     def matvec(ggml_type: int, W: torch.Tensor, x: torch.Tensor, nrows: int, stream=None) -> torch.Tensor:
         _dev(W, x)
         n_tok, ncols = x.shape
-        y = torch.empty(n_tok, nrows, dtype=torch.float32, device=x.device)
-        scratch = torch.empty(gemv.q8_1_bytes(ncols, n_tok), dtype=torch.uint8, device=x.device)
-        check(lib.frx_gemv_matvec(ggml_type, _ptr(W), _ptr(x), _ptr(y), ncols, nrows, n_tok, _ptr(scratch), _stream(stream)))
+        y = x.new_empty((n_tok, nrows), dtype=torch.float32)
+        scratch = x.new_empty((gemv._q8_1_bytes(ncols, n_tok),), dtype=torch.uint8)
+        check(fast.gemv_matvec(ggml_type, W.data_ptr(), x.data_ptr(), y.data_ptr(), ncols, nrows, n_tok, scratch.data_ptr(), _raw_stream(stream)))
         return y
 
 
@@ -520,16 +540,16 @@ class gemm:
         _dev(x, ids)
         T, K = ids.shape
         plan = _GemmPlan()
-        wp, wb = _ws_ptr(ws)
-        check(lib.frx_gemm_moe_prepare(C.byref(plan), ggml_type, n_experts, _ptr(x), int(x_per_slot), _ptr(ids), T, K, ncols, wp, wb,
-                                       _stream(stream)))
+        wp, wb = _ws_span(ws)
+        check(fast.gemm_moe_prepare(C.addressof(plan), ggml_type, n_experts, x.data_ptr(), int(x_per_slot), ids.data_ptr(), T, K, ncols, wp, wb,
+                                    _raw_stream(stream)))
         return plan
 
     @staticmethod
     def moe_run(plan: _GemmPlan, W: torch.Tensor, expert_stride_bytes: int, nrows: int, stream=None) -> torch.Tensor:
         _dev(W)
-        y = torch.empty(plan.T, plan.K, nrows, dtype=torch.float32, device=W.device)
-        check(lib.frx_gemm_moe_run(C.byref(plan), _ptr(W), expert_stride_bytes, _ptr(y), nrows, _stream(stream)))
+        y = W.new_empty((plan.T, plan.K, nrows), dtype=torch.float32)
+        check(fast.gemm_moe_run(C.addressof(plan), W.data_ptr(), expert_stride_bytes, y.data_ptr(), nrows, _raw_stream(stream)))
         return y
 
 
@@ -548,5 +568,5 @@ def chain_rmsnorm_unit(x: torch.Tensor, y: torch.Tensor, out: torch.Tensor | Non
     T, n = x.shape
     if out is None:
         out = torch.empty_like(x)
-    check(lib.frx_chain_rmsnorm_unit(_ptr(x), _ptr(y), _ptr(out), T, n, _stream(stream)))
+    check(fast.chain_rmsnorm_unit(x.data_ptr(), y.data_ptr(), out.data_ptr(), T, n, _raw_stream(stream)))
     return out
