@@ -833,6 +833,8 @@ __global__ void __launch_bounds__(NW * 32, 1) k_stream(const StreamParams p) {
 
 #include "frx_ffn.cuh"
 
+#include "frx_small.cuh"
+
 #include "frx_combine.cuh"
 
 // ---------------------------------------------------------------------------------------------
@@ -1157,6 +1159,81 @@ void launch_ffn(StreamParams p, const ActBufs& xb, const ActBufs& hb, size_t h_r
         FRX_LAUNCH(kKDown, stream, launch_stream<false>(p, cfg.nw_dn, p.ff / kUnitK, cfg.smem_dn, stream));
 }
 
+// Which calls take the two-kernel form (frx_small.cuh): at most this many tokens, and at most five rounds of its first
+// kernel's tasks over the SMs. Measured on B200 (148 SMs, 512 experts top-10 + shared, us per layer, the other form -> this one):
+// hidden 2048, width 512: 1 / 2 / 3 / 4 / 5 tokens 27.6 / 31.0 / 32.9 / 33.8 / 35.5 -> 15.0 / 19.4 / 23.2 / 29.5 / 34.9;
+// 2560 / 640: 30.2 / 34.2 / 42.1 / 41.6 -> 18.0 / 25.5 / 33.9 / 45.9; 512 / 256 (128 experts top-8), 1 / 4 / 6 / 8:
+// 23.5 / 22.4 / 23.6 / 24.3 -> 9.0 / 17.2 / 21.6 / 27.0.
+int g_small_tokens = 6;
+constexpr int kSmallRounds = 5;
+constexpr int kUpRing = 2;
+
+// The shared memory of the two-kernel form for one call. Blocks of both kernels of a layer (and so the second one's
+// routing, grouping and first weights) run side by side where they fit into an SM together: the ring of the second is cut
+// to what the first leaves, and the first gives up one of its buffers of terms if that leaves less than three quads.
+struct SmallCfg {
+    int tbufs, ring;
+    size_t up, down;
+};
+bool small_cfg(int T, int K, int n, int ff, bool shared, SmallCfg& c) {
+    if (T < 1 || T > g_small_tokens || T > kSmallMaxT || T * K > kSmallMaxSlots || !g_fold_quant || !g_narrow || g_fused || g_stream_stamps) return false;
+    const int slots = T * K + (shared ? T : 0), items = T * K + (shared ? (T + kSmallTok - 1) / kSmallTok : 0), quads = (items + 3) / 4;
+    if (items * (ff / kQ8) > kSmallRounds * sm_count()) return false;
+    const size_t budget = size_t(std::max(max_smem_optin() - 1024, 0)), both = budget;   // an SM holds 1 KB more than a block may ask for, and takes 1 KB per block
+    for (c.tbufs = 2; c.tbufs >= 1; --c.tbufs) {
+        c.up = small_up_smem(T, n, kUpRing, c.tbufs).total;
+        for (c.ring = quads; c.ring >= std::min(quads, c.tbufs == 2 ? 3 : 2); --c.ring) {
+            c.down = small_down_smem(slots, ff, c.ring).total;
+            if (c.up + c.down <= both) return true;
+        }
+    }
+    c.tbufs = 2;
+    c.up = small_up_smem(T, n, kUpRing, c.tbufs).total;
+    c.ring = quads;
+    c.down = small_down_smem(slots, ff, c.ring).total;
+    return c.up <= budget && c.down <= budget;
+}
+
+int launch_small(SmallParams p, const SmallCfg& c, cudaStream_t stream) {
+    static std::mutex mu;
+    static bool done[64] = {};
+    int dev = 0;
+    FRX_CUDA(cudaGetDevice(&dev));
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        if (dev < 0 || dev >= 64 || !done[dev]) {
+            const void* fns[] = {reinterpret_cast<const void*>(k_small_up<0>),   reinterpret_cast<const void*>(k_small_up<1>),
+                                 reinterpret_cast<const void*>(k_small_up<4>),   reinterpret_cast<const void*>(k_small_up<8>),
+                                 reinterpret_cast<const void*>(k_small_down<0>), reinterpret_cast<const void*>(k_small_down<1>),
+                                 reinterpret_cast<const void*>(k_small_down<4>), reinterpret_cast<const void*>(k_small_down<8>)};
+            for (const void* f : fns) {
+                FRX_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin() - 1024));
+                // the two kernels of a layer are to be resident side by side
+                FRX_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+            }
+            if (dev >= 0 && dev < 64) done[dev] = true;
+        }
+    }
+    p.wait_ns = wait_limit_ns();
+    auto go = [&](auto k_up, auto k_down) {
+        p.ring = kUpRing;
+        p.tbufs = c.tbufs;
+        FRX_LAUNCH(kKGateUp, stream, launch_pdl(k_up, dim3(unsigned(sm_count())), dim3(kUpThreads), c.up, stream, p));
+        p.ring = c.ring;
+        FRX_LAUNCH(kKDown, stream, launch_pdl(k_down, dim3(unsigned(p.n / 16)), dim3(kDnThreads), c.down, stream, p));
+    };
+    if (!p.logits)
+        go(k_small_up<0>, k_small_down<0>);
+    else if (p.E <= 128)
+        go(k_small_up<1>, k_small_down<1>);
+    else if (p.E <= 512)
+        go(k_small_up<4>, k_small_down<4>);
+    else
+        go(k_small_up<8>, k_small_down<8>);
+    FRX_CUDA(cudaGetLastError());
+    return FRX_OK;
+}
+
 template <class LayoutT>
 ActBufs act_x(uint8_t* base, const LayoutT& L) {
     return ActBufs{reinterpret_cast<int8_t*>(base + L.xq), reinterpret_cast<float*>(base + L.xa), reinterpret_cast<float*>(base + L.xc)};
@@ -1191,6 +1268,35 @@ int decode_steps(const void* experts, size_t stride, int E, int e_lo, int e_hi, 
     if (T == 0) return FRX_OK;
     const Layout L = make_layout(T, K, n, ff);
     if (ws_bytes < L.total) return fail(FRX_ERR_WORKSPACE, "frx_moe_decode: workspace %zu < %zu", ws_bytes, L.total);
+    SmallCfg scfg;
+    if (!ep && e_lo == 0 && e_hi == E && (!shared || (shared_t0 <= 0 && shared_t1 >= T)) && small_cfg(T, K, n, ff, shared != nullptr, scfg)) {
+        auto* b = static_cast<uint8_t*>(ws);
+        SmallParams p{};
+        p.logits = logits;
+        p.ids = logits ? nullptr : ids;
+        p.wts = wts;
+        p.ids_out = ids;
+        p.wts_out = wts;
+        p.experts = static_cast<const uint8_t*>(experts);
+        p.stride = stride;
+        p.shared = static_cast<const uint8_t*>(shared);
+        p.x = x;
+        p.gate_logit = gate_logit;
+        p.xq = reinterpret_cast<int8_t*>(b + L.xq);
+        p.xa = reinterpret_cast<float*>(b + L.xa);
+        p.xc = reinterpret_cast<float*>(b + L.xc);
+        p.hq = reinterpret_cast<int8_t*>(b + L.hq);
+        p.hs = reinterpret_cast<float4*>(b + L.ha);   // 16 bytes per block: the two scale buffers, which lie back to back
+        p.out = out;
+        p.y = yslot;
+        p.status = reinterpret_cast<int*>(b + L.status);
+        p.T = T;
+        p.K = K;
+        p.E = E;
+        p.n = n;
+        p.ff = ff;
+        return launch_small(p, scfg, stream);
+    }
     // with items cut at four tokens either streaming kernel may take tasks of four row groups
     const bool task4_gu = g_narrow && (g_task4 & 1), task4_dn = g_narrow && (g_task4 & 2);
     StreamCfg cfg;
@@ -1624,6 +1730,11 @@ int frx_debug_set_down_item_weight(int sixteenths) {
     g_down_per_item = sixteenths;
     return FRX_OK;
 }
+int frx_debug_set_small_tokens(int tokens) {
+    if (tokens < 0 || tokens > kSmallMaxT) return fail(FRX_ERR_ARG, "frx_debug_set_small_tokens: 0 .. %d", kSmallMaxT);
+    g_small_tokens = tokens;
+    return FRX_OK;
+}
 int frx_debug_set_evict_first(int on) {
     g_evict_first = on ? 1 : 0;
     return FRX_OK;
@@ -1724,6 +1835,23 @@ int frx_moe_hits(const uint8_t* const* hit_ptr, const int32_t* hit_n, int K, con
     if (uintptr_t(scratch) % kAlign || uintptr_t(x) % 16) return fail(FRX_ERR_ARG, "frx_moe_hits: scratch must be 256-byte aligned, x 16-byte aligned");
     const HitsLayout L = hits_layout(K, n, ff, T);
     if (scratch_bytes < L.total) return fail(FRX_ERR_WORKSPACE, "frx_moe_hits: scratch %zu < %zu", scratch_bytes, L.total);
+    SmallCfg scfg;
+    if (small_cfg(T, K, n, ff, false, scfg)) {
+        auto* b = static_cast<uint8_t*>(scratch);
+        SmallParams p{};
+        p.hit_ptr = hit_ptr;
+        p.hit_n = hit_n;
+        p.x = x;
+        p.hq = reinterpret_cast<int8_t*>(b + L.hq);
+        p.hs = reinterpret_cast<float4*>(b + L.ha);
+        p.y = yh;
+        p.status = reinterpret_cast<int*>(b + L.status);
+        p.T = T;
+        p.K = K;
+        p.n = n;
+        p.ff = ff;
+        return launch_small(p, scfg, stream);
+    }
     StreamCfg cfg;
     if (int rc = stream_cfg(n, ff, cfg)) return rc;
     if (int rc = set_smem_attr()) return rc;

@@ -91,6 +91,7 @@ SIGNATURES = {
     "frx_debug_set_down_item_weight": (_i, [_i]),
     "frx_debug_set_stream_stamps": (_i, [_vp]),
     "frx_debug_set_ffn_buffers": (_i, [_i, _i]),
+    "frx_debug_set_small_tokens": (_i, [_i]),
     "frx_debug_set_wait_limit_ns": (_i, [C.c_ulonglong]),
     "frx_moe_decode_static_status": (_i, [_vp]),
     "frx_moe_layer_ep_allreduce": (_i, [_vp, _sz, _i, _i, _i, _vp, _i, _i, _vp, _vp, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),

@@ -105,6 +105,9 @@ int frx_debug_set_down_item_weight(int sixteenths);
  * finished; and block 0 of the layer's first kernel four more behind them: [0] the kernels in front have ended,
  * [1] its own tokens routed, [2] all tokens routed, [3] work items written. NULL (default) switches it off. */
 int frx_debug_set_stream_stamps(void* device_buffer);
+/* Calls of at most `tokens` tokens (0 .. 8, default 6; 0: never) may take the two-kernel form of the decode layer
+ * and of frx_moe_hits, where it is the faster one. Same bits either way. */
+int frx_debug_set_small_tokens(int tokens);
 int frx_debug_set_ffn_buffers(int gate_up, int down);
 int frx_debug_set_wait_limit_ns(unsigned long long ns);
 

@@ -378,3 +378,60 @@ def test_stream_stamps_are_written_and_ordered(port):
     assert busy.any() and (np.diff(dn[busy], axis=1) >= 0).all()
     assert (np.diff(head) >= 0).all() and head[0] > 0
     assert head[3] <= gu[gu[:, 1] > 0, 1].min()           # gate/up's wait returns after the head has written the items
+
+
+@pytest.mark.parametrize("n,ff,E,K,T,shared", [(128, 128, 1, 1, 1, True), (2048, 512, 48, 10, 4, True), (2560, 640, 40, 10, 3, False),
+                                               (384, 640, 130, 32, 1, True), (512, 256, 600, 12, 6, True), (256, 128, 33, 16, 2, False)])
+def test_two_kernel_form_gives_the_same_bits(port, n, ff, E, K, T, shared):
+    # few tokens: routing, grouping and sums by every block; against the other form, which the oracle pins, at one and two
+    # warps' worth of slots, one to eight logits per thread, ties in the router, and every unit count of the shapes in use
+    from flashrt_b200.lib import check, lib
+    rng = np.random.default_rng(n + E)
+    planar = synth.planar_experts_random(rng, min(E, 48) + 1, n, ff)
+    stride = moe.expert_stride(n, ff)
+    some = moe.tile_experts(cuda(planar.reshape(-1)), n, ff, len(planar)).view(len(planar), stride)
+    tiled = some[torch.arange(E + 1, device="cuda") % len(planar)].contiguous()        # the experts repeat: ids are what matters
+    x, gate = cuda(synth.activations(T, n)), cuda(np.linspace(-2, 2, T).astype(np.float32))
+    for lg in (synth.router_logits(T, E), synth.tie_heavy_logits(T, E), np.zeros((T, E), np.float32)):
+        got = []
+        for tokens in (0, 6):
+            try:
+                check(lib.frx_debug_set_small_tokens(tokens))
+                ids, wts = torch.empty(T, K, dtype=torch.int32, device="cuda"), torch.empty(T, K, device="cuda")
+                ws = moe.workspace(moe.moe_layer_workspace_bytes(T, K, n, ff))
+                args = (tiled.data_ptr(), stride, E, tiled[E].data_ptr() if shared else None, n, ff, x)
+                out = moe.moe_layer(*args, cuda(lg), gate, K, ids_out=ids, wts_out=wts, ws=ws)
+                yslot = torch.full((T * K, n), float("nan"), device="cuda")
+                out2 = moe.moe_decode(*args, ids, wts, gate, yslot=yslot, ws=ws)      # the given routing
+                moe.workspace_status(ws)
+                got.append((out, out2, ids, wts, yslot))
+            finally:
+                check(lib.frx_debug_set_small_tokens(6))
+        assert torch.equal(got[0][2], got[1][2]), "ids"
+        # the softmax sum is added in another order in double: at most one ulp of the weights
+        assert torch.allclose(got[0][3], got[1][3], rtol=2 ** -23, atol=0)
+        assert torch.equal(got[0][4], got[1][4]), "per-slot rows"
+        for a, b in zip(got[0][:2], got[1][:2]):
+            assert torch.allclose(a, b, rtol=1e-5, atol=1e-5 * float(a.abs().max()))
+
+
+@pytest.mark.parametrize("T,K", [(1, 3), (2, 10), (4, 10), (5, 9)])
+def test_two_kernel_hits_give_the_same_bits(port, T, K):
+    from flashrt_b200.lib import check, lib
+    n, ff = 512, 256
+    ex = Experts(port, n, ff, 16, shared=False)
+    rng = np.random.default_rng(T * K)
+    ptrs = torch.tensor((ex.base + rng.integers(0, 16, size=T * K).astype(np.int64) * ex.stride), dtype=torch.int64, device="cuda")
+    hit_n = cuda(rng.integers(0, K + 1, size=T).astype(np.int32))
+    x, got = cuda(synth.activations(T, n)), []
+    for tokens in (0, 6):
+        try:
+            check(lib.frx_debug_set_small_tokens(tokens))
+            yh = torch.full((T, K, n), 7.0, device="cuda")
+            scratch = moe.workspace(moe.moe_hits_scratch_bytes(K, n, ff, T))
+            moe.moe_hits(ptrs, hit_n, K, x, n, ff, yh, scratch=scratch, T=T)
+            moe.workspace_status(scratch)
+            got.append(yh)
+        finally:
+            check(lib.frx_debug_set_small_tokens(6))
+    assert torch.equal(got[0], got[1])
