@@ -890,24 +890,25 @@ __global__ void __launch_bounds__(1024) k_group_ptr(const uint8_t* const* __rest
     }
 }
 
-// one thread per item: its expert (binary search over item_off) and its slots
-__global__ void __launch_bounds__(256) k_pf_items(const int* __restrict__ bounds, const int* __restrict__ item_off, int E,
-                                                  const int32_t* __restrict__ perm, const uint8_t* __restrict__ experts, size_t stride,
-                                                  const int* __restrict__ status, Item* __restrict__ items) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= status[1]) return;
-    int lo = 0, hi = E;   // the e with item_off[e] <= i < item_off[e + 1]
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (item_off[mid] <= i) lo = mid; else hi = mid;
-    }
-    const int e = lo, base = bounds[e] + (i - item_off[e]) * kTokPerItem, m = min(kTokPerItem, bounds[e + 1] - base);
-    Item it;
-    it.blob = experts + size_t(e) * stride;
-    it.expert = e;
-    it.n_tok = m;
-    for (int j = 0; j < kTokPerItem; ++j) it.slot[j] = j < m ? perm[base + j] : 0;
-    items[i] = it;
+// Grouping of the streaming form: a slot's place in the grouped order is also its place in a work item.
+__global__ void __launch_bounds__(kChunkSlots) k_pf_place_items(const int32_t* __restrict__ ids, int S, int E, const int* __restrict__ chunk_off,
+                                                                const int* __restrict__ bounds, int32_t* __restrict__ perm, const int32_t* __restrict__ e_map,
+                                                                int E_all, const int* __restrict__ item_off, const uint8_t* __restrict__ experts, size_t stride,
+                                                                Item* __restrict__ items) {
+    pdl_wait();
+    pdl_trigger();
+    pf_place(ids, S, E, chunk_off, bounds, perm, e_map, E_all, [&](int s, int e, int idx) {
+        Item& it = items[item_off[e] + idx / kTokPerItem];
+        const int at = idx % kTokPerItem;
+        it.slot[at] = s;
+        if (at == 0) {
+            const int m = min(kTokPerItem, bounds[e + 1] - bounds[e] - idx);
+            it.blob = experts + size_t(e) * stride;
+            it.expert = e;
+            it.n_tok = m;
+            for (int j = m; j < kTokPerItem; ++j) it.slot[j] = 0;
+        }
+    });
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1943,11 +1944,10 @@ int prefill_stream_impl(const void* experts, size_t stride, int E, const int32_t
     } else {
         launch_quant_x(x, T, n, xb, stream, block64);
     }
-    FRX_LAUNCH(kKGroup, stream, k_pf_hist<<<L.n_chunks, 256, size_t(E) * 4, stream>>>(ids, S, E, chunk_cnt, status, e_map, E_all));
-    FRX_LAUNCH(kKGroup, stream, k_pf_scan<<<1, 1024, 0, stream>>>(chunk_cnt, L.n_chunks, E, bounds, item_off, status, L.max_items));
-    FRX_LAUNCH(kKGroup, stream, k_pf_place<<<L.n_chunks, 32, size_t(E) * 4, stream>>>(ids, S, E, chunk_cnt, bounds, perm, e_map, E_all));
-    FRX_LAUNCH(kKGroup, stream, k_pf_items<<<(L.max_items + 255) / 256, 256, 0, stream>>>(bounds, item_off, E, perm, static_cast<const uint8_t*>(experts), stride,
-                                                             status, items));
+    FRX_LAUNCH(kKGroup, stream, launch_pdl(k_pf_hist, dim3(L.n_chunks), dim3(256), size_t(E) * 4, stream, ids, S, E, chunk_cnt, status, e_map, E_all));
+    FRX_LAUNCH(kKGroup, stream, launch_pdl(k_pf_scan, dim3(1), dim3(1024), 0, stream, chunk_cnt, L.n_chunks, E, bounds, item_off, status, L.max_items, kTokPerItem, TokenBlocks{}));
+    FRX_LAUNCH(kKGroup, stream, launch_pdl(k_pf_place_items, dim3(L.n_chunks), dim3(kChunkSlots), pf_place_smem(E), stream, ids, S, E, (const int*)chunk_cnt, (const int*)bounds, perm,
+                                           e_map, E_all, (const int*)item_off, static_cast<const uint8_t*>(experts), stride, items));
     StreamParams p{};
     p.items = items;
     p.status = status;

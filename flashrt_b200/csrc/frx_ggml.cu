@@ -809,9 +809,10 @@ int frx_gemm_moe_prepare(frx_gemm_moe_plan* plan, uint32_t ggml_type, int n_expe
     // one row of codes per token, or per (token, expert) slot when every slot has its own activations
     const size_t n_quads = size_t(x_per_slot ? rows : T) * size_t(ncols / 4);
     FRX_LAUNCH(kKQuant, stream, k_gm_quant<<<unsigned((n_quads + 255) / 256), 256, 0, stream>>>(x, int(ncols), n_quads, plan_act(base, L)));
-    FRX_LAUNCH(kKGroup, stream, k_pf_hist<<<L.n_chunks, 256, size_t(E) * 4, stream>>>(ids, S, E, chunk_cnt, status));
-    FRX_LAUNCH(kKGroup, stream, k_pf_scan<<<1, 1024, 0, stream>>>(chunk_cnt, L.n_chunks, E, bounds, item_off, status, L.max_items, kGmTok));
-    FRX_LAUNCH(kKGroup, stream, k_pf_place<<<L.n_chunks, 32, size_t(E) * 4, stream>>>(ids, S, E, chunk_cnt, bounds, perm));
+    FRX_LAUNCH(kKGroup, stream, launch_pdl(k_pf_hist, dim3(L.n_chunks), dim3(256), size_t(E) * 4, stream, ids, S, E, chunk_cnt, status, (const int32_t*)nullptr, 0));
+    FRX_LAUNCH(kKGroup, stream, launch_pdl(k_pf_scan, dim3(1), dim3(1024), 0, stream, chunk_cnt, L.n_chunks, E, bounds, item_off, status, L.max_items, kGmTok, TokenBlocks{}));
+    FRX_LAUNCH(kKGroup, stream, launch_pdl(k_pf_place, dim3(L.n_chunks), dim3(kChunkSlots), pf_place_smem(E), stream, ids, S, E, (const int*)chunk_cnt, (const int*)bounds, perm,
+                                           (const int32_t*)nullptr, 0));
     FRX_CUDA(cudaGetLastError());
     return FRX_OK;
 }

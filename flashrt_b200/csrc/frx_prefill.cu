@@ -59,11 +59,10 @@ constexpr int kThreads = (kWarpsAux + kWarpsEpilogue) * 32;
 // epilogue warps take 24 more: 384 * 40 + 512 * 96 = 896 * 72
 constexpr int kRegsAux = 40, kRegsEpilogue = 96;
 
-// meta words: [0] padded positions in use, [1] token blocks
+// meta words: [1] token blocks
 struct PfuLayout {
-    size_t status, chunk_cnt, bounds, item_off, perm, pb, tbo, meta, tb_e, tb_p0, tb_n, pslot, xe, xd, xg, xa, hf, hg, ha, total;
+    size_t status, chunk_cnt, bounds, item_off, perm, meta, tb, xe, xd, hf, he, hd, total;
     int n_chunks, max_tb;
-    size_t pmax;
 };
 
 PfuLayout pfu_layout(int T, int K, int n, int ff, int E) {
@@ -76,87 +75,21 @@ PfuLayout pfu_layout(int T, int K, int n, int ff, int E) {
     };
     const size_t S = size_t(T) * K;
     L.n_chunks = int((S + kChunkSlots - 1) / kChunkSlots);
-    L.pmax = align_up(S + size_t(kTokPad) * size_t(E < int(S) ? E : int(S)), 128);
     L.max_tb = int(S / kTileTok) + E + 1;
     L.status = take(64);
     L.chunk_cnt = take(size_t(L.n_chunks) * E * 4);
     L.bounds = take(size_t(E + 1) * 4);
     L.item_off = take(size_t(E + 1) * 4);
     L.perm = take(S * 4);
-    L.pb = take(size_t(E + 1) * 4);
-    L.tbo = take(size_t(E + 1) * 4);
     L.meta = take(64);
-    L.tb_e = take(size_t(L.max_tb) * 4);
-    L.tb_p0 = take(size_t(L.max_tb) * 4);
-    L.tb_n = take(size_t(L.max_tb) * 4);
-    L.pslot = take(L.pmax * 4);
+    L.tb = take(size_t(L.max_tb) * sizeof(int4));
     L.xe = take(size_t(T) * n * 2);
     L.xd = take(size_t(T) * (n / kQ8) * 4);
-    L.xg = take(L.pmax * n * 2);
-    L.xa = take(L.pmax * (n / kQK) * 8);
-    L.hf = take(L.pmax * ff * 8);   // (gate x, up x) pairs
-    L.hg = take(L.pmax * ff * 2);
-    L.ha = take(L.pmax * (ff / kQK) * 8);
+    L.hf = take(S * ff * 8);   // (gate x, up x) pairs
+    L.he = take(S * ff * 2);
+    L.hd = take(S * (ff / kQ8) * 4);
     L.total = off;
     return L;
-}
-
-// ---------------------------------------------------------------------------------------------
-// Plan: pad every expert's slot count to 16 (padded position space p), cut it into token blocks of
-// at most kTileTok, as equal as multiples of 16 allow (a tile costs its fixed steps whatever its
-// width). One block of 1024 threads.
-__global__ void __launch_bounds__(1024) k_pfu_plan(const int* __restrict__ bounds, int E, int* __restrict__ pb, int* __restrict__ tbo,
-                                                   int* __restrict__ meta, int* __restrict__ tb_e, int* __restrict__ tb_p0,
-                                                   int* __restrict__ tb_n, int max_tb, int* __restrict__ status) {
-    __shared__ int scan_p[1024], scan_t[1024];
-    const int tid = threadIdx.x;
-    const int per = (E + 1023) / 1024, e0 = tid * per, e1 = min(E, e0 + per);
-    int pp = 0, tt = 0;
-    for (int e = e0; e < e1; ++e) {
-        const int c = bounds[e + 1] - bounds[e];
-        pp += (c + kTokPad - 1) / kTokPad * kTokPad;
-        tt += (c + kTileTok - 1) / kTileTok;
-    }
-    scan_p[tid] = pp;
-    scan_t[tid] = tt;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {
-        const int a = tid >= o ? scan_p[tid - o] : 0, b = tid >= o ? scan_t[tid - o] : 0;
-        __syncthreads();
-        scan_p[tid] += a;
-        scan_t[tid] += b;
-        __syncthreads();
-    }
-    const int n_tb = scan_t[1023];
-    if (n_tb > max_tb) {
-        if (tid == 0) {
-            status[0] = kDevTooManyItems;
-            meta[0] = 0;
-            meta[1] = 0;
-        }
-        return;
-    }
-    int at_p = scan_p[tid] - pp, at_t = scan_t[tid] - tt;
-    for (int e = e0; e < e1; ++e) {
-        const int c = bounds[e + 1] - bounds[e], pc = (c + kTokPad - 1) / kTokPad * kTokPad;
-        pb[e] = at_p;
-        tbo[e] = at_t;
-        const int nblk = (c + kTileTok - 1) / kTileTok, n16 = pc / kTokPad;
-        for (int j = 0; j < nblk; ++j) {
-            const int lo = n16 * j / nblk, hi = n16 * (j + 1) / nblk;
-            tb_e[at_t] = e;
-            tb_p0[at_t] = at_p + lo * kTokPad;
-            tb_n[at_t] = (hi - lo) * kTokPad;
-            ++at_t;
-        }
-        at_p += pc;
-    }
-    if (tid == 0) {
-        pb[E] = scan_p[1023];
-        tbo[E] = n_tb;
-        meta[0] = scan_p[1023];
-        meta[1] = n_tb;
-    }
 }
 
 // The e4m3 pieces of activation codes. A 64-block of one token is 128 bytes, eight 16-byte chunks
@@ -181,22 +114,13 @@ __device__ __forceinline__ void split_codes(const int (&c)[4], uint32_t& hi, uin
     lo = two(l[0], l[1]) | (two(l[2], l[3]) << 16);
 }
 
-// Offset, in bytes, of 16-byte chunk `chunk` of 64-block b64 of padded position p in the grouped
-// operand: [64-block][p / 8][chunk 0..7][p % 8][16 bytes] -- the MMA's K-major core-matrix order, so
-// a token block's tile for one 64-block is one contiguous range.
-__device__ __forceinline__ size_t grouped_chunk_off(size_t pmax, int b64, int p, int chunk) {
-    return (((size_t(b64) * (pmax / 8) + size_t(p >> 3)) * 8 + size_t(chunk)) * 8 + size_t(p & 7)) * 16;
-}
-// Activation scales: [64-block][p / 2][a0 of p even, a0 of p odd, a1 of p even, a1 of p odd].
-__device__ __forceinline__ size_t grouped_scale_idx(size_t pmax, int b64, int p, int half) {
-    return (size_t(b64) * pmax + size_t(p & ~1)) * 2 + size_t(half) * 2 + size_t(p & 1);
-}
-
 // Q8 of x rows (q2_0::quantize_q8, quant/q2_0/q2_0.cpp:101-113) straight into e4m3 pieces, token-major
 // [T][n / 64][128 bytes], and the block scales d [T][n / 32]. A thread owns four consecutive values,
 // eight neighbouring lanes one 32-block. n_quads is a multiple of 32: warps are live as a whole.
 __global__ void __launch_bounds__(256) k_pfu_quant_x(const float* __restrict__ x, size_t n_quads, uint8_t* __restrict__ xe,
                                                      float* __restrict__ d, int block64) {
+    pdl_wait();
+    pdl_trigger();
     const size_t quad = size_t(blockIdx.x) * 256 + threadIdx.x;
     if (quad >= n_quads) return;
     const float4 v = reinterpret_cast<const float4*>(x)[quad];
@@ -219,6 +143,8 @@ __global__ void __launch_bounds__(256) k_pfu_quant_x(const float* __restrict__ x
 
 // The same pieces from codes that arrive already quantized (natural order, as frx_quantize_q8 writes them).
 __global__ void __launch_bounds__(256) k_pfu_expand_q8(const int8_t* __restrict__ xq, size_t n_quads, uint8_t* __restrict__ xe) {
+    pdl_wait();
+    pdl_trigger();
     const size_t quad = size_t(blockIdx.x) * 256 + threadIdx.x;
     if (quad >= n_quads) return;
     const char4 v = reinterpret_cast<const char4*>(xq)[quad];
@@ -231,90 +157,48 @@ __global__ void __launch_bounds__(256) k_pfu_expand_q8(const int8_t* __restrict_
     *reinterpret_cast<uint32_t*>(blk + piece_chunk(s, 1, t) * 16 + piece_byte(q, t)) = lo;
 }
 
-// Gather: for every padded position, its slot (or -1), the e4m3 pieces of the slot's token in the
-// grouped operand layout, and the token's block scales. Block = 8 positions x 32 chunks.
-__global__ void __launch_bounds__(256) k_pfu_gather(const int* __restrict__ bounds, const int* __restrict__ pb, int E,
-                                                    const int32_t* __restrict__ perm, const int* __restrict__ meta, int K, int n,
-                                                    size_t pmax, const uint8_t* __restrict__ xe, const float* __restrict__ xd,
-                                                    uint8_t* __restrict__ xg, float* __restrict__ xa, int32_t* __restrict__ pslot) {
-    const int r = threadIdx.x & 7, cl = threadIdx.x >> 3;
-    const int p = blockIdx.x * 8 + r;
-    if (blockIdx.x * 8 >= meta[0]) return;
-    int lo = 0, hi = E;   // the expert whose padded range holds p
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (pb[mid] <= p) lo = mid; else hi = mid;
-    }
-    const int e = lo, k = p - pb[e], c = bounds[e + 1] - bounds[e];
-    const int slot = (p < meta[0] && k < c) ? perm[bounds[e] + k] : -1;
-    if (cl == 0) pslot[p] = slot;
-    const int t = slot >= 0 ? slot / K : 0;
-    const int chunks = n / 8, nb = n / kQK;
-    for (int ch = cl; ch < chunks; ch += 32) {
-        uint4 out = make_uint4(0u, 0u, 0u, 0u);
-        if (slot >= 0) out = *reinterpret_cast<const uint4*>(xe + size_t(t) * n * 2 + size_t(ch) * 16);
-        *reinterpret_cast<uint4*>(xg + grouped_chunk_off(pmax, ch >> 3, p, ch & 7)) = out;
-    }
-    for (int b = cl; b < nb; b += 32) {
-        const float a0 = slot >= 0 ? xd[size_t(t) * (n / kQ8) + 2 * b] : 0.0f;
-        const float a1 = slot >= 0 ? xd[size_t(t) * (n / kQ8) + 2 * b + 1] : 0.0f;
-        xa[grouped_scale_idx(pmax, b, p, 0)] = a0;
-        xa[grouped_scale_idx(pmax, b, p, 1)] = a1;
-    }
-}
-
-// Q8 of the hidden rows (one row of ff per padded position) straight into the grouped operand
-// layout and scale table of the down product. A thread owns 8 consecutive hidden values, four
-// neighbouring lanes one 32-block: silu(gate x) * up x is formed here (eight independent
-// exponentials per thread hide their latency) and the block maximum comes from two shuffles.
-__global__ void __launch_bounds__(256) k_pfu_quant_h(const float2* __restrict__ hf, int ff, size_t pmax, const int* __restrict__ meta,
-                                                     const int32_t* __restrict__ pslot, uint8_t* __restrict__ hg, float* __restrict__ ha,
-                                                     int block64) {
-    const int cpr = ff / 8;   // threads per row
-    const size_t chunk = size_t(blockIdx.x) * 256 + threadIdx.x;
-    const size_t p = chunk / cpr;
-    const bool in_range = p < size_t(meta[0]);   // no early exit: the shuffles below need the whole warp
-    const int c = int(chunk % cpr);              // values 8 c .. 8 c + 7 of the row
-    const bool live = in_range && pslot[p] >= 0;
+// Q8 of the hidden rows (in the grouped order, the first *n_rows of them) into e4m3 pieces and block scales, like
+// k_pfu_quant_x. A thread owns the eight values of element group t of a 32-block (4 t .. + 3 and 16 + 4 t .. + 3), four
+// neighbouring lanes one 32-block: silu(gate x) * up x is formed here (eight independent exponentials
+// per thread hide their latency), the block maximum comes from two shuffles, each piece is one 8-byte store.
+__global__ void __launch_bounds__(256) k_pfu_quant_h(const float2* __restrict__ hf, int ff, const int* __restrict__ n_rows, uint8_t* __restrict__ he,
+                                                     float* __restrict__ hd, int block64) {
+    pdl_wait();
+    pdl_trigger();
+    const size_t g = size_t(blockIdx.x) * 256 + threadIdx.x, blk = g >> 2;   // blk: the 32-block, over all rows
+    if (blk >= size_t(*n_rows) * (ff / kQ8)) return;                          // (ff is a multiple of 128: warps of 8 blocks are live as a whole)
+    const int t = int(g & 3), s = int(blk & 1);
+    const float4* src = reinterpret_cast<const float4*>(hf + blk * kQ8);
     float hv[8];
     float am = 0.0f;
-    if (live) {
-        const float4* src = reinterpret_cast<const float4*>(hf + p * ff + size_t(c) * 8);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float4 gu = src[i];   // (gate, up) of two hidden values
-            hv[2 * i] = swiglu_ref(gu.x, gu.y);
-            hv[2 * i + 1] = swiglu_ref(gu.z, gu.w);
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float4 gu = src[q * 8 + t * 2 + i];   // (gate, up) of two hidden values
+            hv[q * 4 + 2 * i] = swiglu_ref(gu.x, gu.y);
+            hv[q * 4 + 2 * i + 1] = swiglu_ref(gu.z, gu.w);
         }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) am = fmaxf(am, fabsf(hv[i]));
-    } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) hv[i] = 0.0f;
-    }
+    for (int i = 0; i < 8; ++i) am = fmaxf(am, fabsf(hv[i]));
     am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 1));
     am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 2));
     if (block64) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 4));   // eight lanes hold one 64-value scale block
     // quant/q2_0/q2_0.cpp:101-113: d = amax / 127, id = 1 / d, q = roundf(v * id), d through fp16
     const float d = __fdiv_rn(am, 127.0f);
     const float id = d != 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
-    if (!in_range) return;
-    const int b64 = c >> 3, s = (c >> 2) & 1, q = (c >> 1) & 1;   // values 32 s + 16 q + 8 (c & 1) .. of the 64-block: groups t = 2 (c & 1), + 1
     uint32_t hi[2], lo[2];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
+    for (int q = 0; q < 2; ++q) {
         int code[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) code[i] = int(round_half_away(__fmul_rn(hv[4 * u + i], id)));
-        split_codes(code, hi[u], lo[u]);
+        for (int i = 0; i < 4; ++i) code[i] = int(round_half_away(__fmul_rn(hv[4 * q + i], id)));
+        split_codes(code, hi[q], lo[q]);
     }
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-        const int t = 2 * (c & 1) + u;
-        *reinterpret_cast<uint32_t*>(hg + grouped_chunk_off(pmax, b64, int(p), piece_chunk(s, 0, t)) + piece_byte(q, t)) = hi[u];
-        *reinterpret_cast<uint32_t*>(hg + grouped_chunk_off(pmax, b64, int(p), piece_chunk(s, 1, t)) + piece_byte(q, t)) = lo[u];
-    }
-    if ((c & 3) == 0) ha[grouped_scale_idx(pmax, b64, int(p), s)] = __half2float(__float2half_rn(d));
+    uint8_t* o = he + (blk >> 1) * 128 + piece_byte(0, t);
+    *reinterpret_cast<uint2*>(o + piece_chunk(s, 0, t) * 16) = make_uint2(hi[0], hi[1]);
+    *reinterpret_cast<uint2*>(o + piece_chunk(s, 1, t) * 16) = make_uint2(lo[0], lo[1]);
+    if (t == 0) hd[blk] = __half2float(__float2half_rn(d));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -322,24 +206,27 @@ struct UmmaParams {
     const uint8_t* experts;   // tiled blobs
     size_t stride;
     const int* meta;          // [1] = token blocks
-    const int* tb_e;
-    const int* tb_p0;
-    const int* tb_n;
-    const uint8_t* act;       // grouped e4m3 codes (xg or hg)
-    const float* act_scale;   // grouped block scales (xa or ha)
-    const int32_t* pslot;
-    float2* hf;               // gate/up: (gate x, up x) of every hidden element [pmax][ff]
+    const int4* tb;           // {expert, first position in the grouped order, slots, slots rounded up to kTokPad}
+    const int32_t* perm;      // the slot at every position
+    const uint8_t* act;       // e4m3 pieces, a row per token (xe) or per position (he)
+    const float* act_scale;   // block scales, likewise
+    float2* hf;               // gate/up: (gate x, up x) of every hidden element [positions][ff]
     float* yd;                // down: [slots][n]
     int* status;
-    size_t pmax;
     unsigned long long wait_ns;   // the longest a wait on a shared-memory barrier may last
     float neg0;               // -0.0f, an addend the compiler does not know (see scale_add)
-    int n, ff;
+    int n, ff, K;
     int y_bf16;               // down: yd holds bf16 rows
 };
 
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
 struct PfSmem {
-    uint32_t w, b, s, bars, tmem, abort, total;
+    uint32_t w, b, s, slots, bars, tmem, abort, total;
 };
 __host__ __device__ constexpr PfSmem pf_smem() {
     PfSmem m{};
@@ -350,6 +237,8 @@ __host__ __device__ constexpr PfSmem pf_smem() {
     off += kStagesW * kUnitBytesW;
     m.s = off;
     off += kStagesS * kUnitBytesS;
+    m.slots = off;
+    off += kStagesS * kTileTok * 4;   // of the last kStagesS tiles (a tile has at least one unit)
     m.bars = off;
     off += 64 * 8;
     m.tmem = off;
@@ -364,7 +253,7 @@ __host__ __device__ constexpr PfSmem pf_smem() {
 enum : int {
     kBarWFull = 0,                                 // + stage: packed weights have landed
     kBarWFree = kBarWFull + kStagesW,              // the dequant warps are done with them
-    kBarBFull = kBarWFree + kStagesW,              // B tiles have landed
+    kBarBFull = kBarWFree + kStagesW,              // B tiles have landed (and been made visible to the tensor core)
     kBarBFree = kBarBFull + kStagesB,              // the MMAs that read them have completed
     kBarSFull = kBarBFree + kStagesB,              // activation scales have landed, row scales are written
     kBarAFull = kBarSFull + kStagesS,              // + row tile * kStagesA + stage: e4m3 weights are in tensor memory
@@ -376,17 +265,31 @@ enum : int {
 static_assert(kBarCount <= 64, "barrier block too small");
 
 // The tiles of a block: tile = token block * row_blocks + row block, blocks take them round robin, so
-// that the row blocks of a token block (which share its B tiles) are in flight together.
+// that the row blocks of a token block (which share its B tiles) are in flight together. The entry of
+// the tile after the current one is fetched ahead: a role would otherwise start every tile with a round
+// trip to memory (of a down tile's 10,400 cycles, with its four units of 1,950, most of the rest was this).
 struct TileWalk {
-    int tile, rb, e, p0, ntok;
-    __device__ __forceinline__ void load(const UmmaParams& p, int row_blocks, int n_tiles) {
-        if (tile >= n_tiles) return;
-        const int tb = tile / row_blocks;
-        rb = tile - tb * row_blocks;
+    int tile, rb, e, p0, live, ntok;
+    int4 nxt;
+    __device__ __forceinline__ void begin(const UmmaParams& p, int row_blocks, int n_tiles) {
+        tile = int(blockIdx.x) - int(gridDim.x);
+        fetch(p, row_blocks, n_tiles);
+    }
+    __device__ __forceinline__ void fetch(const UmmaParams& p, int row_blocks, int n_tiles) {
+        const int t = tile + int(gridDim.x);
+        nxt = t < n_tiles ? __ldg(p.tb + t / row_blocks) : make_int4(0, 0, 0, 0);
+    }
+    __device__ __forceinline__ bool next(const UmmaParams& p, int row_blocks, int n_tiles) {
+        tile += gridDim.x;
+        if (tile >= n_tiles) return false;
+        rb = tile % row_blocks;
         // (the shuffles tell the compiler that the values are the same in all lanes)
-        e = __shfl_sync(0xffffffffu, p.tb_e[tb], 0);
-        p0 = __shfl_sync(0xffffffffu, p.tb_p0[tb], 0);
-        ntok = __shfl_sync(0xffffffffu, p.tb_n[tb], 0);
+        e = __shfl_sync(0xffffffffu, nxt.x, 0);
+        p0 = __shfl_sync(0xffffffffu, nxt.y, 0);
+        live = __shfl_sync(0xffffffffu, nxt.z, 0);
+        ntok = __shfl_sync(0xffffffffu, nxt.w, 0);
+        fetch(p, row_blocks, n_tiles);
+        return true;
     }
 };
 
@@ -520,7 +423,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_pf_umma(const UmmaParams p) {
     const int row_blocks = (row_tiles + kRowTiles - 1) / kRowTiles;
     const uint32_t group_bytes = uint32_t(units) * kUnitBytes;
     const size_t section = GATE_UP ? 0 : size_t(p.ff / 8) * (size_t(p.n / kUnitK) * kUnitBytes);
-    const int n_tiles = p.meta[1] * row_blocks;
 
     if (threadIdx.x == 0) {
         uint64_t* b = reinterpret_cast<uint64_t*>(smem + sm.bars);
@@ -532,7 +434,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pf_umma(const UmmaParams p) {
             mbar_init(b + kBarBFull + i, 1);
             mbar_init(b + kBarBFree + i, kRowTiles);
         }
-        for (int i = 0; i < kStagesS; ++i) mbar_init(b + kBarSFull + i, 1 + kWarpsDequant);
+        for (int i = 0; i < kStagesS; ++i) mbar_init(b + kBarSFull + i, 1 + kWarpsDequant);   // the activation warp, the dequant warps
         for (int i = 0; i < kRowTiles * kStagesA; ++i) {
             mbar_init(b + kBarAFull + i, kWarpsDequant / kRowTiles);
             mbar_init(b + kBarAFree + i, 1);
@@ -544,13 +446,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_pf_umma(const UmmaParams p) {
         *abort_flag = 0;
         mbar_fence_init();
     }
+    pdl_wait();
+    pdl_trigger();
+    const int n_tiles = p.meta[1] * row_blocks;
     if (warp == 2) tmem_alloc(tmem_slot, kTmemCols);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     TileWalk t;
-    t.tile = blockIdx.x;
+    t.begin(p, row_blocks, n_tiles);
 
     // "free" barriers are waited on with the parity of the phase before the one about to be used,
     // which a fresh barrier reports as complete
@@ -560,8 +465,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pf_umma(const UmmaParams p) {
             // ---------------- packed weights: one lane per row group. A last row tile that does not exist
             // (n an odd multiple of 128) is computed as a copy of the one before and not stored.
             uint32_t g = 0;
-            for (; t.tile < n_tiles; t.tile += gridDim.x) {
-                t.load(p, row_blocks, n_tiles);
+            while (t.next(p, row_blocks, n_tiles)) {
                 const int rt = min(t.rb * kRowTiles + ((lane >> 3) & 1), row_tiles - 1);
                 const uint8_t* src = p.experts + size_t(t.e) * p.stride + section + size_t(rt * 8 + (lane & 7)) * group_bytes;
                 for (int u = 0; u < units; ++u, ++g) {
@@ -573,32 +477,66 @@ __global__ void __launch_bounds__(kThreads, 1) k_pf_umma(const UmmaParams p) {
                 }
             }
         } else if (warp == 1) {
-            // ---------------- activations: B tiles and scales of a unit's two blocks
-            uint32_t g = 0;
-            for (; t.tile < n_tiles; t.tile += gridDim.x) {
-                t.load(p, row_blocks, n_tiles);
-                const uint32_t bbytes = uint32_t(t.ntok) * 128u, sbytes = uint32_t(t.ntok) * 8u;
+            // ---------------- activations: the rows of the tile's tokens, gathered 16 bytes at a time (cp.async) into the MMA's
+            // core-matrix order, their scales, and the tile's slots. A unit is handed on kLag units after its copies
+            // were issued: they are generic-proxy writes, so each lane waits for its own and makes them visible to the
+            // tensor core before the arrival. (A kernel that gathered the rows into this order in memory first took
+            // 237 us at 163,840 slots of 2048 and made the products read 671 MB from HBM instead of the L2.)
+            constexpr uint32_t kLag = 4;
+            static_assert(kLag < kStagesB, "a unit must be handed on before its stage is needed again");
+            const uint32_t dst_l = uint32_t(lane >> 3) * 128 + uint32_t(lane & 7) * 16;   // chunk lane / 8 of token lane % 8
+            const size_t row_bytes = size_t(kdim) * 2, srow = size_t(kdim / kQ8);
+            uint32_t g = 0, tile_no = 0;
+            auto hand_on = [&](uint32_t u) {
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(bars + (kBarBFull + u % kStagesB) * 8);
+                    mbar_arrive(bars + (kBarSFull + u % kStagesS) * 8);
+                }
+            };
+            while (t.next(p, row_blocks, n_tiles)) {
+                const int groups = t.ntok >> 3;
+                int row[kTileTok / 8];   // of token group i: the row of token lane % 8 (tokens beyond the live ones repeat the last)
+#pragma unroll
+                for (int i = 0; i < kTileTok / 8; ++i) {
+                    const int pos = t.p0 + min(i * 8 + (lane & 7), t.live - 1);
+                    row[i] = GATE_UP ? (i < groups ? p.perm[pos] / p.K : 0) : pos;
+                    if (!GATE_UP && i < groups && lane < 8) sts32(s0 + sm.slots + ((tile_no % kStagesS) * kTileTok + i * 8 + lane) * 4, uint32_t(p.perm[pos]));
+                }
+                ++tile_no;
                 for (int u = 0; u < units; ++u, ++g) {
-                    const uint32_t bs = g % kStagesB, ss = g % kStagesS, full_b = bars + (kBarBFull + bs) * 8, full_s = bars + (kBarSFull + ss) * 8;
+                    const uint32_t bs = g % kStagesB, ss = g % kStagesS;
                     mbar_spin(bars + (kBarBFree + bs) * 8, ((g / kStagesB) & 1u) ^ 1u, abort, wait_ns);
-                    if (lane == 0) mbar_expect_tx(full_b, 2 * bbytes);
-                    if (lane == 1) mbar_expect_tx(full_s, 2 * sbytes);
-                    __syncwarp();
-                    const size_t b = size_t(2 * u + (lane & 1));
-                    if (lane < 2)
-                        bulk_g2s(s0 + sm.b + bs * kUnitBytesB + lane * kBlockBytesB, p.act + (b * (p.pmax / 8) + size_t(t.p0 >> 3)) * 1024, bbytes, full_b);
-                    else if (lane < 4)
-                        bulk_g2s(s0 + sm.s + ss * kUnitBytesS + (lane & 1) * kBlockBytesS, p.act_scale + (b * p.pmax + size_t(t.p0)) * 2, sbytes, full_s);
+                    const uint32_t db = s0 + sm.b + bs * kUnitBytesB + dst_l, ds = s0 + sm.s + ss * kUnitBytesS;
+                    const uint8_t* src = p.act + size_t(u) * 256 + (lane >> 3) * 16;
+                    const float* ssrc = p.act_scale + size_t(u) * 4 + (lane & 3);
+#pragma unroll
+                    for (int i = 0; i < kTileTok / 8; ++i) {
+                        const int srow_i = __shfl_sync(0xffffffffu, row[i], lane >> 2);
+                        if (i < groups) {
+                            const uint8_t* r = src + size_t(row[i]) * row_bytes;
+#pragma unroll
+                            for (int c = 0; c < 4; ++c) cp_async16(db + (c >> 1) * kBlockBytesB + i * 1024 + (c & 1) * 512, r + c * 64);
+                            // the scale of 32-block lane % 4 of the unit, of token lane / 4 of the group
+                            cp_async4(ds + ((lane >> 1) & 1) * kBlockBytesS + (i * 4 + (lane >> 3)) * 16 + (lane & 1) * 8 + ((lane >> 2) & 1) * 4,
+                                      ssrc + size_t(srow_i) * srow);
+                        }
+                    }
+                    cp_async_commit();
+                    cp_async_wait<kLag>();
+                    if (g >= kLag) hand_on(g - kLag);
                 }
             }
+            cp_async_wait<0>();
+            for (uint32_t u = g > kLag ? g - kLag : 0; u < g; ++u) hand_on(u);
         } else if (warp < 4) {
             // ---------------- MMA issuers, one warp per row tile; one elected lane issues, the warp stays together
             // (so that what it computes is known to be uniform)
             const int r = warp - 2;
             const uint64_t b_desc0 = umma_desc(s0 + sm.b, 128, 1024);
             uint32_t g = 0;
-            for (; t.tile < n_tiles; t.tile += gridDim.x) {
-                t.load(p, row_blocks, n_tiles);
+            while (t.next(p, row_blocks, n_tiles)) {
                 const uint32_t idesc = umma_idesc_e4m3(kTileRows, t.ntok);
                 for (int u = 0; u < units; ++u, ++g) {
                     const uint32_t bs = g % kStagesB, as = g % kStagesA;
@@ -642,7 +580,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pf_umma(const UmmaParams p) {
             const uint32_t scale_off = uint32_t(r) * kTileBytesW + uint32_t(row >> 4) * kUnitBytes + kUnitCodeBytes + uint32_t(row & 7) * 8 + uint32_t((row >> 3) & 1) * 4;
             const uint32_t a_addr = tmem + (uint32_t((warp & 3) * 32) << 16) + kColA0 + r * 32;
             uint32_t g = 0;
-            for (; t.tile < n_tiles; t.tile += gridDim.x) {
+            for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
 #pragma unroll 1
                 for (int u = 0; u < units; ++u, ++g) {
                     const uint32_t ws = g % kStagesW, as = g % kStagesA, ss = g % kStagesS;
@@ -690,9 +628,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_pf_umma(const UmmaParams p) {
         q.leader = lane == 0;
         q.row_off = 2 * kBlockBytesS + row * 4;
         q.neg0 = pack2(p.neg0, p.neg0);
-        uint32_t g = 0;
-        for (; t.tile < n_tiles; t.tile += gridDim.x) {
-            t.load(p, row_blocks, n_tiles);
+        uint32_t g = 0, tile_no = 0;
+        for (; t.next(p, row_blocks, n_tiles); ++tile_no) {
             const int share = t.ntok >> 2, nch = share >> 2;   // four warps share a row's tokens evenly
             const int tok0 = (ew >> 2) * share;
             q.tok_off = tok0 * 8;
@@ -704,31 +641,32 @@ __global__ void __launch_bounds__(kThreads, 1) k_pf_umma(const UmmaParams p) {
                 default: epilogue_tile<3>(q, g, acc); break;
             }
             // ---- tile done: acc[r * 2 nch + i] holds the sums of row tile r for tokens tok0 + 2 i, + 1
-            const int pos0 = t.p0 + tok0;
+            const uint32_t slots = s0 + sm.slots + (tile_no % kStagesS) * kTileTok * 4;
 #pragma unroll
             for (int k = 0; k < 12; ++k) {
                 if (k >= 4 * nch) break;
-                const int r = k >= 2 * nch ? 1 : 0, i = k - r * 2 * nch, rt = t.rb * kRowTiles + r, pos = pos0 + 2 * i;
+                const int r = k >= 2 * nch ? 1 : 0, i = k - r * 2 * nch, rt = t.rb * kRowTiles + r, tok = tok0 + 2 * i;
                 if (rt >= row_tiles) break;
                 float v0, v1;
                 unpack2(acc[k], v0, v1);
+                const bool on0 = tok < t.live, on1 = tok + 1 < t.live;
                 if (GATE_UP) {
                     // rows m < 8 of a group are gate rows, m >= 8 the up rows of the same ff rows: a
                     // warp's 32 rows are 16 (gate, up) pairs, 128 contiguous bytes per token
                     const int m = row & 15, ffrow = rt * 64 + (row >> 4) * 8 + (m & 7);
-                    float* dst = reinterpret_cast<float*>(p.hf) + (size_t(pos) * p.ff + ffrow) * 2 + (m >> 3);
-                    dst[0] = v0;
-                    dst[size_t(p.ff) * 2] = v1;
+                    float* dst = reinterpret_cast<float*>(p.hf) + (size_t(t.p0 + tok) * p.ff + ffrow) * 2 + (m >> 3);
+                    if (on0) dst[0] = v0;
+                    if (on1) dst[size_t(p.ff) * 2] = v1;
                 } else {
-                    const int orow = rt * kTileRows + row;
-                    const int sl0 = p.pslot[pos], sl1 = p.pslot[pos + 1];
+                    const uint2 sl = lds64(slots + tok * 4);
+                    const size_t o0 = size_t(sl.x) * p.n + rt * kTileRows + row, o1 = size_t(sl.y) * p.n + rt * kTileRows + row;
                     if (p.y_bf16) {
                         __nv_bfloat16* yb = reinterpret_cast<__nv_bfloat16*>(p.yd);
-                        if (sl0 >= 0) yb[size_t(sl0) * p.n + orow] = __float2bfloat16_rn(v0);
-                        if (sl1 >= 0) yb[size_t(sl1) * p.n + orow] = __float2bfloat16_rn(v1);
+                        if (on0) yb[o0] = __float2bfloat16_rn(v0);
+                        if (on1) yb[o1] = __float2bfloat16_rn(v1);
                     } else {
-                        if (sl0 >= 0) p.yd[size_t(sl0) * p.n + orow] = v0;
-                        if (sl1 >= 0) p.yd[size_t(sl1) * p.n + orow] = v1;
+                        if (on0) p.yd[o0] = v0;
+                        if (on1) p.yd[o1] = v1;
                     }
                 }
             }
@@ -816,55 +754,46 @@ static int prefill_umma_impl(const void* experts, size_t stride, int E, const in
     int* bounds = reinterpret_cast<int*>(base + L.bounds);
     int* item_off = reinterpret_cast<int*>(base + L.item_off);
     int32_t* perm = reinterpret_cast<int32_t*>(base + L.perm);
-    int* pb = reinterpret_cast<int*>(base + L.pb);
-    int* tbo = reinterpret_cast<int*>(base + L.tbo);
     int* meta = reinterpret_cast<int*>(base + L.meta);
-    int* tb_e = reinterpret_cast<int*>(base + L.tb_e);
-    int* tb_p0 = reinterpret_cast<int*>(base + L.tb_p0);
-    int* tb_n = reinterpret_cast<int*>(base + L.tb_n);
-    int32_t* pslot = reinterpret_cast<int32_t*>(base + L.pslot);
+    int4* tb = reinterpret_cast<int4*>(base + L.tb);
     const int S = T * K;
     uint8_t* xe = base + L.xe;
     float* xd = reinterpret_cast<float*>(base + L.xd);
     const size_t nquads = size_t(T) * (n / 4);
     const unsigned qgrid = unsigned((nquads + 255) / 256);
     if (xq_in)   // the activations arrived already quantized
-        FRX_LAUNCH(kKQuant, stream, k_pfu_expand_q8<<<qgrid, 256, 0, stream>>>(xq_in, nquads, xe));
+        FRX_LAUNCH(kKQuant, stream, launch_pdl(k_pfu_expand_q8, dim3(qgrid), dim3(256), 0, stream, xq_in, nquads, xe));
     else
-        FRX_LAUNCH(kKQuant, stream, k_pfu_quant_x<<<qgrid, 256, 0, stream>>>(x, nquads, xe, xd, block64));
-    FRX_LAUNCH(kKGroup, stream, k_pf_hist<<<L.n_chunks, 256, size_t(E) * 4, stream>>>(ids, S, E, chunk_cnt, status, e_map, E_all));
-    FRX_LAUNCH(kKGroup, stream, k_pf_scan<<<1, 1024, 0, stream>>>(chunk_cnt, L.n_chunks, E, bounds, item_off, status, 1 << 30));
-    FRX_LAUNCH(kKGroup, stream, k_pf_place<<<L.n_chunks, 32, size_t(E) * 4, stream>>>(ids, S, E, chunk_cnt, bounds, perm, e_map, E_all));
-    FRX_LAUNCH(kKGroup, stream, k_pfu_plan<<<1, 1024, 0, stream>>>(bounds, E, pb, tbo, meta, tb_e, tb_p0, tb_n, L.max_tb, status));
-    FRX_LAUNCH(kKGroup, stream, k_pfu_gather<<<unsigned(L.pmax / 8), 256, 0, stream>>>(bounds, pb, E, perm, meta, K, n, L.pmax, xe, xq_in ? xd_in : xd, base + L.xg,
-                                                                                   reinterpret_cast<float*>(base + L.xa), pslot));
+        FRX_LAUNCH(kKQuant, stream, launch_pdl(k_pfu_quant_x, dim3(qgrid), dim3(256), 0, stream, x, nquads, xe, xd, block64));
+    FRX_LAUNCH(kKGroup, stream, launch_pdl(k_pf_hist, dim3(L.n_chunks), dim3(256), size_t(E) * 4, stream, ids, S, E, chunk_cnt, status, e_map, E_all));
+    FRX_LAUNCH(kKGroup, stream, launch_pdl(k_pf_scan, dim3(1), dim3(1024), 0, stream, chunk_cnt, L.n_chunks, E, bounds, item_off, status, 1 << 30, kTokPerItem,
+                                           TokenBlocks{kTileTok, kTokPad, meta, tb, L.max_tb}));
+    FRX_LAUNCH(kKGroup, stream, launch_pdl(k_pf_place, dim3(L.n_chunks), dim3(kChunkSlots), pf_place_smem(E), stream, ids, S, E, (const int*)chunk_cnt, (const int*)bounds, perm, e_map, E_all));
     UmmaParams p{};
     p.experts = static_cast<const uint8_t*>(experts);
     p.stride = stride;
     p.meta = meta;
-    p.tb_e = tb_e;
-    p.tb_p0 = tb_p0;
-    p.tb_n = tb_n;
-    p.pslot = pslot;
+    p.tb = tb;
+    p.perm = perm;
     p.hf = reinterpret_cast<float2*>(base + L.hf);
     p.yd = static_cast<float*>(yd);
     p.y_bf16 = yd_bf16 ? 1 : 0;
     p.status = status;
-    p.pmax = L.pmax;
     p.wait_ns = wait_limit_ns();
     p.neg0 = -0.0f;
     p.n = n;
     p.ff = ff;
-    const int blocks = sm_count();
-    p.act = base + L.xg;
-    p.act_scale = reinterpret_cast<const float*>(base + L.xa);
-    FRX_LAUNCH(kKGateUp, stream, k_pf_umma<true><<<blocks, kThreads, pf_smem().total, stream>>>(p));
-    const size_t hchunks = L.pmax * size_t(ff / 8);
-    FRX_LAUNCH(kKQuant, stream, k_pfu_quant_h<<<unsigned((hchunks + 255) / 256), 256, 0, stream>>>((const float2*)p.hf, ff, L.pmax, meta, pslot, base + L.hg,
-                                                                                    reinterpret_cast<float*>(base + L.ha), block64));
-    p.act = base + L.hg;
-    p.act_scale = reinterpret_cast<const float*>(base + L.ha);
-    FRX_LAUNCH(kKDown, stream, k_pf_umma<false><<<blocks, kThreads, pf_smem().total, stream>>>(p));
+    p.K = K;
+    const dim3 blocks{unsigned(sm_count())};
+    p.act = xe;
+    p.act_scale = xq_in ? xd_in : xd;
+    FRX_LAUNCH(kKGateUp, stream, launch_pdl(k_pf_umma<true>, blocks, dim3(kThreads), pf_smem().total, stream, p));
+    const size_t groups = size_t(S) * size_t(ff / 8);
+    FRX_LAUNCH(kKQuant, stream, launch_pdl(k_pfu_quant_h, dim3(unsigned((groups + 255) / 256)), dim3(256), 0, stream, (const float2*)p.hf, ff, (const int*)(bounds + E), base + L.he,
+                                           reinterpret_cast<float*>(base + L.hd), block64));
+    p.act = base + L.he;
+    p.act_scale = reinterpret_cast<const float*>(base + L.hd);
+    FRX_LAUNCH(kKDown, stream, launch_pdl(k_pf_umma<false>, blocks, dim3(kThreads), pf_smem().total, stream, p));
     FRX_CUDA(cudaGetLastError());
     return FRX_OK;
 }
