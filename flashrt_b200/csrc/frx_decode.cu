@@ -1715,7 +1715,10 @@ int frx_moe_combine(float* out, const float* yh, const float* w, const int32_t* 
     if (!out || !yh || !w) return fail(FRX_ERR_ARG, "frx_moe_combine: null pointer");
     if (n < 1 || K < 1 || T < 0) return fail(FRX_ERR_ARG, "frx_moe_combine: n %d, K %d, T %d", n, K, T);
     if (T == 0) return FRX_OK;
-    FRX_LAUNCH(kKCombine, stream, k_combine_hits<<<dim3((n + 255) / 256, T), 256, 0, stream>>>(out, yh, w, hit_n, shexp, gate, n, K));
+    const bool vec = n % 4 == 0 && (uintptr_t(out) | uintptr_t(yh) | uintptr_t(shexp)) % 16 == 0;
+    const int per = vec ? 4 : 1, threads = n / per >= 256 ? 256 : 128;
+    const dim3 grid((n + threads * per - 1) / (threads * per), T);
+    FRX_LAUNCH(kKCombine, stream, launch_pdl(vec ? k_combine_hits<4> : k_combine_hits<1>, grid, dim3(threads), 0, stream, out, yh, w, hit_n, shexp, gate, n, K));
     FRX_CUDA(cudaGetLastError());
     return FRX_OK;
 }

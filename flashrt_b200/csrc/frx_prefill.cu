@@ -238,7 +238,7 @@ __host__ __device__ constexpr PfSmem pf_smem() {
     m.s = off;
     off += kStagesS * kUnitBytesS;
     m.slots = off;
-    off += kStagesS * kTileTok * 4;   // of the last kStagesS tiles (a tile has at least one unit)
+    off += kStagesS * kTileTok * 4;   // of the last kStagesS token blocks (each has at least one unit)
     m.bars = off;
     off += 64 * 8;
     m.tmem = off;
@@ -264,32 +264,63 @@ enum : int {
 };
 static_assert(kBarCount <= 64, "barrier block too small");
 
-// The tiles of a block: tile = token block * row_blocks + row block, blocks take them round robin, so
-// that the row blocks of a token block (which share its B tiles) are in flight together. The entry of
-// the tile after the current one is fetched ahead: a role would otherwise start every tile with a round
-// trip to memory (of a down tile's 10,400 cycles, with its four units of 1,950, most of the rest was this).
+// The tiles of a block. A block takes whole token blocks, gridDim.x apart, and walks the row blocks of each (so the
+// blocks work on neighbouring token blocks, whose experts' weights and rows are shared in the L2, and nothing has
+// to be looked up when only the row block changes); the token blocks that are left over are dealt out tile by tile.
+// The entry of the token block after the current one is fetched ahead.
 struct TileWalk {
-    int tile, rb, e, p0, live, ntok;
+    int tb, rb, tail, e, p0, live, ntok;   // tail: the tile among the left-over ones, or -1
+    bool fresh;                            // the token block is another one than in the tile before
+    int row_blocks, full, tail_tiles;      // full: token blocks taken whole
     int4 nxt;
-    __device__ __forceinline__ void begin(const UmmaParams& p, int row_blocks, int n_tiles) {
-        tile = int(blockIdx.x) - int(gridDim.x);
-        fetch(p, row_blocks, n_tiles);
+    const int4* list;
+    __device__ __forceinline__ void begin(const UmmaParams& p, int rows, int n_tb) {
+        list = p.tb;
+        row_blocks = rows;
+        full = n_tb / int(gridDim.x) * int(gridDim.x);
+        tail_tiles = (n_tb - full) * rows;
+        tb = int(blockIdx.x) - int(gridDim.x);
+        rb = rows - 1;
+        tail = -1;
+        fetch();
     }
-    __device__ __forceinline__ void fetch(const UmmaParams& p, int row_blocks, int n_tiles) {
-        const int t = tile + int(gridDim.x);
-        nxt = t < n_tiles ? __ldg(p.tb + t / row_blocks) : make_int4(0, 0, 0, 0);
+    // the token block behind the current one, or -1
+    __device__ __forceinline__ int following(int& t) const {
+        t = tail;
+        if (t < 0) {
+            if (tb + int(gridDim.x) < full) return tb + int(gridDim.x);
+            t = int(blockIdx.x);
+        } else {
+            t += int(gridDim.x);
+        }
+        return t < tail_tiles ? full + t / row_blocks : -1;
     }
-    __device__ __forceinline__ bool next(const UmmaParams& p, int row_blocks, int n_tiles) {
-        tile += gridDim.x;
-        if (tile >= n_tiles) return false;
-        rb = tile % row_blocks;
+    __device__ __forceinline__ void fetch() {
+        int t;
+        const int n = following(t);
+        nxt = n >= 0 ? __ldg(list + n) : make_int4(0, 0, 0, 0);
+    }
+    __device__ __forceinline__ bool next() {
+        fresh = false;
+        if (tail < 0 && ++rb < row_blocks) return true;
+        int t;
+        const int n = following(t);
+        if (n < 0) return false;
+        tail = n >= full ? t : -1;
+        tb = n;
+        rb = tail >= 0 ? t % row_blocks : 0;
+        fresh = true;
         // (the shuffles tell the compiler that the values are the same in all lanes)
         e = __shfl_sync(0xffffffffu, nxt.x, 0);
         p0 = __shfl_sync(0xffffffffu, nxt.y, 0);
         live = __shfl_sync(0xffffffffu, nxt.z, 0);
         ntok = __shfl_sync(0xffffffffu, nxt.w, 0);
-        fetch(p, row_blocks, n_tiles);
+        fetch();
         return true;
+    }
+    __device__ __forceinline__ int count() const {   // tiles of this block
+        const int left = tail_tiles - int(blockIdx.x);
+        return full / int(gridDim.x) * row_blocks + (left > 0 ? (left + int(gridDim.x) - 1) / int(gridDim.x) : 0);
     }
 };
 
@@ -372,9 +403,19 @@ struct EpiArgs {
     int units;
     bool leader;                    // lane 0
     uint64_t neg0;
+    // the tile's results: live tokens of this thread, whether the second row tile exists, where the first token's
+    // value goes (gate/up) or its row of every slot starts and the slots are (down), bytes per token or slot
+    int live;
+    bool second;
+    uint8_t* dst;
+    uint32_t slots, step;
 };
-template <int NCH>
-__device__ __forceinline__ void epilogue_tile(const EpiArgs& q, uint32_t& gu, uint64_t (&acc)[12]) {
+// (The stores are part of it: with the number of tokens known at compile time they are four to five instructions per
+// token and row tile. Written once for any number they were thirty, and with all epilogue warps there at the same
+// time a tile's end took some 2,000 cycles: a down tile's four units take 8,000.)
+template <bool GATE_UP, int NCH>
+__device__ __forceinline__ void epilogue_tile(const EpiArgs& q, uint32_t& gu, bool y_bf16) {
+    uint64_t acc[4 * NCH];
 #pragma unroll
     for (int i = 0; i < 4 * NCH; ++i) acc[i] = 0ull;
 #pragma unroll 1
@@ -402,6 +443,31 @@ __device__ __forceinline__ void epilogue_tile(const EpiArgs& q, uint32_t& gu, ui
                 acc[i] = scale_add(acc[i], a, v + 2 * i, v + 4 * NCH + 2 * i, dd0, q.neg0);
                 acc[2 * NCH + i] = scale_add(acc[2 * NCH + i], a, v + 8 * NCH + 2 * i, v + 12 * NCH + 2 * i, dd1, q.neg0);
             }
+        }
+    }
+    // acc[r * 2 NCH + i]: the sums of row tile r for the thread's tokens 2 i, 2 i + 1
+    constexpr uint32_t kNextF = GATE_UP ? 64 * 8 : kTileRows * 4, kNextH = kTileRows * 2;   // bytes from a row tile to the next: float (pairs), bf16
+    uint8_t* d = q.dst;
+#pragma unroll
+    for (int i = 0; i < 2 * NCH; ++i) {
+        float v[2][2];
+        unpack2(acc[i], v[0][0], v[0][1]);
+        unpack2(acc[2 * NCH + i], v[1][0], v[1][1]);
+        uint2 sl;
+        if (!GATE_UP) sl = lds64(q.slots + i * 8);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            if (!GATE_UP) d = q.dst + size_t(k ? sl.y : sl.x) * q.step;
+            if (2 * i + k < q.live) {
+                if (!GATE_UP && y_bf16) {
+                    *reinterpret_cast<__nv_bfloat16*>(d) = __float2bfloat16_rn(v[0][k]);
+                    if (q.second) *reinterpret_cast<__nv_bfloat16*>(d + kNextH) = __float2bfloat16_rn(v[1][k]);
+                } else {
+                    *reinterpret_cast<float*>(d) = v[0][k];
+                    if (q.second) *reinterpret_cast<float*>(d + kNextF) = v[1][k];
+                }
+            }
+            if (GATE_UP) d += q.step;
         }
     }
 }
@@ -448,14 +514,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_pf_umma(const UmmaParams p) {
     }
     pdl_wait();
     pdl_trigger();
-    const int n_tiles = p.meta[1] * row_blocks;
     if (warp == 2) tmem_alloc(tmem_slot, kTmemCols);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     TileWalk t;
-    t.begin(p, row_blocks, n_tiles);
+    t.begin(p, row_blocks, p.meta[1]);
 
     // "free" barriers are waited on with the parity of the phase before the one about to be used,
     // which a fresh barrier reports as complete
@@ -465,7 +530,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pf_umma(const UmmaParams p) {
             // ---------------- packed weights: one lane per row group. A last row tile that does not exist
             // (n an odd multiple of 128) is computed as a copy of the one before and not stored.
             uint32_t g = 0;
-            while (t.next(p, row_blocks, n_tiles)) {
+            while (t.next()) {
                 const int rt = min(t.rb * kRowTiles + ((lane >> 3) & 1), row_tiles - 1);
                 const uint8_t* src = p.experts + size_t(t.e) * p.stride + section + size_t(rt * 8 + (lane & 7)) * group_bytes;
                 for (int u = 0; u < units; ++u, ++g) {
@@ -486,7 +551,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pf_umma(const UmmaParams p) {
             static_assert(kLag < kStagesB, "a unit must be handed on before its stage is needed again");
             const uint32_t dst_l = uint32_t(lane >> 3) * 128 + uint32_t(lane & 7) * 16;   // chunk lane / 8 of token lane % 8
             const size_t row_bytes = size_t(kdim) * 2, srow = size_t(kdim / kQ8);
-            uint32_t g = 0, tile_no = 0;
+            uint32_t g = 0, tb_no = 0;
             auto hand_on = [&](uint32_t u) {
                 fence_async_smem();
                 __syncwarp();
@@ -495,16 +560,22 @@ __global__ void __launch_bounds__(kThreads, 1) k_pf_umma(const UmmaParams p) {
                     mbar_arrive(bars + (kBarSFull + u % kStagesS) * 8);
                 }
             };
-            while (t.next(p, row_blocks, n_tiles)) {
-                const int groups = t.ntok >> 3;
-                int row[kTileTok / 8];   // of token group i: the row of token lane % 8 (tokens beyond the live ones repeat the last)
+            int row[kTileTok / 8];   // of token group i: the row of token lane % 8 (tokens beyond the live ones repeat the last)
 #pragma unroll
-                for (int i = 0; i < kTileTok / 8; ++i) {
-                    const int pos = t.p0 + min(i * 8 + (lane & 7), t.live - 1);
-                    row[i] = GATE_UP ? (i < groups ? p.perm[pos] / p.K : 0) : pos;
-                    if (!GATE_UP && i < groups && lane < 8) sts32(s0 + sm.slots + ((tile_no % kStagesS) * kTileTok + i * 8 + lane) * 4, uint32_t(p.perm[pos]));
+            for (int i = 0; i < kTileTok / 8; ++i) row[i] = 0;
+            while (t.next()) {
+                const int groups = t.ntok >> 3;
+                if (t.fresh) {
+                    const uint32_t slots = s0 + sm.slots + (tb_no % kStagesS) * kTileTok * 4;
+                    ++tb_no;
+#pragma unroll
+                    for (int i = 0; i < kTileTok / 8; ++i) {
+                        const int pos = t.p0 + min(i * 8 + (lane & 7), t.live - 1);
+                        const int slot = i < groups ? p.perm[pos] : 0;
+                        row[i] = GATE_UP ? slot / p.K : pos;
+                        if (!GATE_UP && i < groups && lane < 8) sts32(slots + (i * 8 + lane) * 4, uint32_t(slot));
+                    }
                 }
-                ++tile_no;
                 for (int u = 0; u < units; ++u, ++g) {
                     const uint32_t bs = g % kStagesB, ss = g % kStagesS;
                     mbar_spin(bars + (kBarBFree + bs) * 8, ((g / kStagesB) & 1u) ^ 1u, abort, wait_ns);
@@ -536,7 +607,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pf_umma(const UmmaParams p) {
             const int r = warp - 2;
             const uint64_t b_desc0 = umma_desc(s0 + sm.b, 128, 1024);
             uint32_t g = 0;
-            while (t.next(p, row_blocks, n_tiles)) {
+            while (t.next()) {
                 const uint32_t idesc = umma_idesc_e4m3(kTileRows, t.ntok);
                 for (int u = 0; u < units; ++u, ++g) {
                     const uint32_t bs = g % kStagesB, as = g % kStagesA;
@@ -579,10 +650,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_pf_umma(const UmmaParams p) {
             const uint32_t code_off = uint32_t(r) * kTileBytesW + uint32_t(row >> 4) * kUnitBytes + uint32_t(row & 7) * 64 + uint32_t((row >> 3) & 1) * 8;
             const uint32_t scale_off = uint32_t(r) * kTileBytesW + uint32_t(row >> 4) * kUnitBytes + kUnitCodeBytes + uint32_t(row & 7) * 8 + uint32_t((row >> 3) & 1) * 4;
             const uint32_t a_addr = tmem + (uint32_t((warp & 3) * 32) << 16) + kColA0 + r * 32;
-            uint32_t g = 0;
-            for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+            const uint32_t n_units = uint32_t(t.count()) * uint32_t(units);
+            {
 #pragma unroll 1
-                for (int u = 0; u < units; ++u, ++g) {
+                for (uint32_t g = 0; g < n_units; ++g) {
                     const uint32_t ws = g % kStagesW, as = g % kStagesA, ss = g % kStagesS;
                     const uint32_t bar_w = bars + (kBarWFull + ws) * 8, bar_a = bars + (kBarAFull + r * kStagesA + as) * 8;
                     mbar_spin(bar_w, (g / kStagesW) & 1u, abort, wait_ns);
@@ -628,47 +699,32 @@ __global__ void __launch_bounds__(kThreads, 1) k_pf_umma(const UmmaParams p) {
         q.leader = lane == 0;
         q.row_off = 2 * kBlockBytesS + row * 4;
         q.neg0 = pack2(p.neg0, p.neg0);
-        uint32_t g = 0, tile_no = 0;
-        for (; t.next(p, row_blocks, n_tiles); ++tile_no) {
+        uint32_t g = 0, tb_no = 0;
+        while (t.next()) {
+            tb_no += t.fresh;   // (of the token blocks so far)
             const int share = t.ntok >> 2, nch = share >> 2;   // four warps share a row's tokens evenly
             const int tok0 = (ew >> 2) * share;
             q.tok_off = tok0 * 8;
             q.taddr = tmem + (uint32_t(quarter * 32) << 16) + uint32_t(tok0);
-            uint64_t acc[12];
-            switch (nch) {
-                case 1: epilogue_tile<1>(q, g, acc); break;
-                case 2: epilogue_tile<2>(q, g, acc); break;
-                default: epilogue_tile<3>(q, g, acc); break;
+            q.live = t.live - tok0;
+            const int rt = t.rb * kRowTiles;
+            q.second = rt + 1 < row_tiles;
+            if (GATE_UP) {
+                // rows m < 8 of a group are gate rows, m >= 8 the up rows of the same ff rows: a
+                // warp's 32 rows are 16 (gate, up) pairs, 128 contiguous bytes per token
+                const int m = row & 15, ffrow = rt * 64 + (row >> 4) * 8 + (m & 7);
+                q.dst = reinterpret_cast<uint8_t*>(p.hf) + (size_t(t.p0 + tok0) * p.ff + ffrow) * 8 + (m >> 3) * 4;
+                q.step = uint32_t(p.ff) * 8;
+            } else {
+                const uint32_t size = p.y_bf16 ? 2 : 4;
+                q.dst = reinterpret_cast<uint8_t*>(p.yd) + size_t(rt * kTileRows + row) * size;
+                q.step = uint32_t(p.n) * size;
+                q.slots = s0 + sm.slots + (((tb_no - 1) % kStagesS) * kTileTok + tok0) * 4;
             }
-            // ---- tile done: acc[r * 2 nch + i] holds the sums of row tile r for tokens tok0 + 2 i, + 1
-            const uint32_t slots = s0 + sm.slots + (tile_no % kStagesS) * kTileTok * 4;
-#pragma unroll
-            for (int k = 0; k < 12; ++k) {
-                if (k >= 4 * nch) break;
-                const int r = k >= 2 * nch ? 1 : 0, i = k - r * 2 * nch, rt = t.rb * kRowTiles + r, tok = tok0 + 2 * i;
-                if (rt >= row_tiles) break;
-                float v0, v1;
-                unpack2(acc[k], v0, v1);
-                const bool on0 = tok < t.live, on1 = tok + 1 < t.live;
-                if (GATE_UP) {
-                    // rows m < 8 of a group are gate rows, m >= 8 the up rows of the same ff rows: a
-                    // warp's 32 rows are 16 (gate, up) pairs, 128 contiguous bytes per token
-                    const int m = row & 15, ffrow = rt * 64 + (row >> 4) * 8 + (m & 7);
-                    float* dst = reinterpret_cast<float*>(p.hf) + (size_t(t.p0 + tok) * p.ff + ffrow) * 2 + (m >> 3);
-                    if (on0) dst[0] = v0;
-                    if (on1) dst[size_t(p.ff) * 2] = v1;
-                } else {
-                    const uint2 sl = lds64(slots + tok * 4);
-                    const size_t o0 = size_t(sl.x) * p.n + rt * kTileRows + row, o1 = size_t(sl.y) * p.n + rt * kTileRows + row;
-                    if (p.y_bf16) {
-                        __nv_bfloat16* yb = reinterpret_cast<__nv_bfloat16*>(p.yd);
-                        if (on0) yb[o0] = __float2bfloat16_rn(v0);
-                        if (on1) yb[o1] = __float2bfloat16_rn(v1);
-                    } else {
-                        if (on0) p.yd[o0] = v0;
-                        if (on1) p.yd[o1] = v1;
-                    }
-                }
+            switch (nch) {
+                case 1: epilogue_tile<GATE_UP, 1>(q, g, p.y_bf16 != 0); break;
+                case 2: epilogue_tile<GATE_UP, 2>(q, g, p.y_bf16 != 0); break;
+                default: epilogue_tile<GATE_UP, 3>(q, g, p.y_bf16 != 0); break;
             }
         }
     }

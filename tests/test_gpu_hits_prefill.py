@@ -83,3 +83,29 @@ def test_prefill_config_shape_sample(port):
     for s in range(0, T * K, 97):
         t, k = divmod(s, K)
         assert rel_max(yd[s], port.expert_ffn(ex.planar[ids[t, k]], n, ff, xq[t], xd[t])) < 1e-5
+
+
+@pytest.mark.parametrize("T,E,K", [(1, 3, 1), (127, 5, 3), (129, 4096, 2), (1024, 2, 1), (1025, 300, 3), (2500, 48, 4)])
+def test_grouping_edges(port, T, E, K):
+    # chunks of 1024 slots in parts of 128, items of 8, token blocks of 48: one more, one less, all slots on one expert; both
+    # forms group for themselves, and every slot's row must be its own expert's
+    n, ff = 128, 128
+    planar = synth.planar_experts_random(np.random.default_rng(E), min(E, 24), n, ff)
+    stride = moe.expert_stride(n, ff)
+    some = moe.tile_experts(cuda(planar.reshape(-1)), n, ff, len(planar)).view(len(planar), stride)
+    tiled = some[torch.arange(E, device="cuda") % len(planar)].contiguous()
+    rng = np.random.default_rng(T)
+    ids = rng.integers(0, E, size=(T, K)).astype(np.int32)
+    ids[: T // 2] = E - 1                                                # half the slots on one expert
+    x = synth.activations(T, n)
+    ws = moe.workspace(moe.moe_q2.workspace_bytes(T, K, n, ff, E))
+    yd = {}
+    for form in ("stream", "umma"):
+        yd[form] = moe.moe_q2.run(tiled.data_ptr(), stride, E, n, ff, cuda(x), cuda(ids), ws=ws, form=form)
+        moe.workspace_status(ws)
+    assert torch.equal(yd["stream"], yd["umma"])
+    xq, xd = port.quantize_q8(x)
+    got = yd["stream"].cpu().numpy()
+    for s in sorted({0, T * K - 1, *rng.integers(0, T * K, size=24).tolist()}):
+        t, k = divmod(s, K)
+        assert rel_max(got[s], port.expert_ffn(planar[ids[t, k] % len(planar)], n, ff, xq[t], xd[t])) < 1e-5
