@@ -109,3 +109,34 @@ def test_router_projection(T, E, n, gate):
     ids, _ = moe.moe_route_topk(logits, min(8, E))
     top = np.argsort(-logits.cpu().numpy(), axis=1, kind="stable")[:, :min(8, E)]
     assert np.array_equal(ids.cpu().numpy(), top)
+
+
+@pytest.mark.parametrize("T,E", [(15, 512), (16, 40), (17, 512), (33, 512), (40, 15), (41, 512), (64, 512), (137, 511), (293, 512), (321, 16)])
+def test_router_projection_same_bits_for_any_tile(T, E):
+    # every tile adds in the same order (eight slices of n one after the other), so a token's logits do not
+    # depend on how many tokens the call has; tails of rows and tokens included
+    n = 768
+    g = torch.Generator(device="cuda").manual_seed(T)
+    w = torch.randn(E, n, generator=g, device="cuda").to(torch.bfloat16)
+    wg = torch.randn(n, generator=g, device="cuda").to(torch.bfloat16)
+    x = torch.randn(T, n, generator=g, device="cuda")
+    logits, gate = moe.router_logits(w, wg, x)
+    for t in {0, T // 2, T - 2, T - 1}:
+        one, g1 = moe.router_logits(w, wg, x[t:t + 1].contiguous())
+        assert torch.equal(one[0], logits[t]) and torch.equal(g1[0], gate[t])
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 512, 2048, 4095, 4096, 4097, 9000])
+def test_chain_rmsnorm_order_of_additions(n):
+    rng = np.random.default_rng(n)
+    x, y = rng.standard_normal((3, n), dtype=np.float32), rng.standard_normal((3, n), dtype=np.float32)
+    r = x + y
+    sq = np.zeros((3, -(-n // 32) * 32))
+    sq[:, :n] = r.astype(np.float64) ** 2
+    lanes = np.zeros((3, 32))
+    for row in sq.reshape(3, -1, 32).transpose(1, 0, 2):
+        lanes = lanes + row
+    for o in (16, 8, 4, 2, 1):
+        lanes = lanes + lanes[:, np.arange(32) ^ o]
+    inv = (1.0 / np.sqrt(lanes[:, :1] / n + 1e-6)).astype(np.float32)
+    assert np.array_equal(moe.chain_rmsnorm_unit(cuda(x), cuda(y)).cpu().numpy(), r * inv)
