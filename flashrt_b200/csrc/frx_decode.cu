@@ -1023,9 +1023,12 @@ bool ffn_cfg(int n, int ff, long long max_items, FfnCfg& c) {
 template <bool GATE_UP, int NW>
 void launch_stream_nw(const StreamParams& p, int upc, uint32_t smem, cudaStream_t stream) {
     const int sms = sm_count();
-    constexpr int kFixed = 4;   // the benchmark shapes: n = 2048 in four chunks, ff = 512
-    if (upc == kFixed)
-        launch_pdl(k_stream<GATE_UP, NW, kFixed>, dim3(sms), dim3(NW * 32), smem, stream, p);
+    // A loop of known length is unrolled and its address arithmetic folded: 4 units for n = 2048 in four chunks and ff = 512,
+    // 5 for n = 2560 in four chunks and ff = 640.
+    if (upc == 4)
+        launch_pdl(k_stream<GATE_UP, NW, 4>, dim3(sms), dim3(NW * 32), smem, stream, p);
+    else if (upc == 5)
+        launch_pdl(k_stream<GATE_UP, NW, 5>, dim3(sms), dim3(NW * 32), smem, stream, p);
     else
         launch_pdl(k_stream<GATE_UP, NW, 0>, dim3(sms), dim3(NW * 32), smem, stream, p);   // any other split of K
 }
@@ -1039,6 +1042,12 @@ void launch_stream4(const StreamParams& p, int nw, int upc, uint32_t smem, cudaS
             case 4: go(k_stream<GATE_UP, 4, 2, true>, 128); break;
             case 8: go(k_stream<GATE_UP, 8, 2, true>, 256); break;
             default: go(k_stream<GATE_UP, 16, 2, true>, 512); break;
+        }
+    } else if (upc == 1) {   // an odd number of units
+        switch (nw) {
+            case 4: go(k_stream<GATE_UP, 4, 1, true>, 128); break;
+            case 8: go(k_stream<GATE_UP, 8, 1, true>, 256); break;
+            default: go(k_stream<GATE_UP, 16, 1, true>, 512); break;
         }
     } else {
         switch (nw) {
@@ -1071,22 +1080,22 @@ int set_smem_attr() {
     if (dev >= 0 && dev < 64 && done[dev]) return FRX_OK;
     const int lim = max_smem_optin() - 2048;   // dynamic part only: the kernels also hold a little static shared memory
     const void* fns[] = {
-        reinterpret_cast<const void*>(k_stream<true, 4, 4>),   reinterpret_cast<const void*>(k_stream<true, 4, 0>),
-        reinterpret_cast<const void*>(k_stream<false, 4, 4>),  reinterpret_cast<const void*>(k_stream<false, 4, 0>),
-        reinterpret_cast<const void*>(k_stream<true, 8, 4>),   reinterpret_cast<const void*>(k_stream<true, 8, 0>),
-        reinterpret_cast<const void*>(k_stream<false, 8, 4>),  reinterpret_cast<const void*>(k_stream<false, 8, 0>),
-        reinterpret_cast<const void*>(k_stream<true, 12, 4>),  reinterpret_cast<const void*>(k_stream<true, 12, 0>),
-        reinterpret_cast<const void*>(k_stream<false, 12, 4>), reinterpret_cast<const void*>(k_stream<false, 12, 0>),
-        reinterpret_cast<const void*>(k_stream<true, 16, 4>),  reinterpret_cast<const void*>(k_stream<true, 16, 0>),
-        reinterpret_cast<const void*>(k_stream<false, 16, 4>), reinterpret_cast<const void*>(k_stream<false, 16, 0>),
-        reinterpret_cast<const void*>(k_stream<true, 20, 4>),  reinterpret_cast<const void*>(k_stream<true, 20, 0>),
-        reinterpret_cast<const void*>(k_stream<false, 20, 4>), reinterpret_cast<const void*>(k_stream<false, 20, 0>),
-        reinterpret_cast<const void*>(k_stream<true, 4, 2, true>),   reinterpret_cast<const void*>(k_stream<true, 4, 0, true>),
-        reinterpret_cast<const void*>(k_stream<false, 4, 2, true>),  reinterpret_cast<const void*>(k_stream<false, 4, 0, true>),
-        reinterpret_cast<const void*>(k_stream<true, 8, 2, true>),   reinterpret_cast<const void*>(k_stream<true, 8, 0, true>),
-        reinterpret_cast<const void*>(k_stream<false, 8, 2, true>),  reinterpret_cast<const void*>(k_stream<false, 8, 0, true>),
-        reinterpret_cast<const void*>(k_stream<true, 16, 2, true>),  reinterpret_cast<const void*>(k_stream<true, 16, 0, true>),
-        reinterpret_cast<const void*>(k_stream<false, 16, 2, true>), reinterpret_cast<const void*>(k_stream<false, 16, 0, true>),
+        reinterpret_cast<const void*>(k_stream<true, 4, 4>), reinterpret_cast<const void*>(k_stream<true, 4, 5>),   reinterpret_cast<const void*>(k_stream<true, 4, 0>),
+        reinterpret_cast<const void*>(k_stream<false, 4, 4>), reinterpret_cast<const void*>(k_stream<false, 4, 5>),  reinterpret_cast<const void*>(k_stream<false, 4, 0>),
+        reinterpret_cast<const void*>(k_stream<true, 8, 4>), reinterpret_cast<const void*>(k_stream<true, 8, 5>),   reinterpret_cast<const void*>(k_stream<true, 8, 0>),
+        reinterpret_cast<const void*>(k_stream<false, 8, 4>), reinterpret_cast<const void*>(k_stream<false, 8, 5>),  reinterpret_cast<const void*>(k_stream<false, 8, 0>),
+        reinterpret_cast<const void*>(k_stream<true, 12, 4>), reinterpret_cast<const void*>(k_stream<true, 12, 5>),  reinterpret_cast<const void*>(k_stream<true, 12, 0>),
+        reinterpret_cast<const void*>(k_stream<false, 12, 4>), reinterpret_cast<const void*>(k_stream<false, 12, 5>), reinterpret_cast<const void*>(k_stream<false, 12, 0>),
+        reinterpret_cast<const void*>(k_stream<true, 16, 4>), reinterpret_cast<const void*>(k_stream<true, 16, 5>),  reinterpret_cast<const void*>(k_stream<true, 16, 0>),
+        reinterpret_cast<const void*>(k_stream<false, 16, 4>), reinterpret_cast<const void*>(k_stream<false, 16, 5>), reinterpret_cast<const void*>(k_stream<false, 16, 0>),
+        reinterpret_cast<const void*>(k_stream<true, 20, 4>), reinterpret_cast<const void*>(k_stream<true, 20, 5>),  reinterpret_cast<const void*>(k_stream<true, 20, 0>),
+        reinterpret_cast<const void*>(k_stream<false, 20, 4>), reinterpret_cast<const void*>(k_stream<false, 20, 5>), reinterpret_cast<const void*>(k_stream<false, 20, 0>),
+        reinterpret_cast<const void*>(k_stream<true, 4, 2, true>), reinterpret_cast<const void*>(k_stream<true, 4, 1, true>),   reinterpret_cast<const void*>(k_stream<true, 4, 0, true>),
+        reinterpret_cast<const void*>(k_stream<false, 4, 2, true>), reinterpret_cast<const void*>(k_stream<false, 4, 1, true>),  reinterpret_cast<const void*>(k_stream<false, 4, 0, true>),
+        reinterpret_cast<const void*>(k_stream<true, 8, 2, true>), reinterpret_cast<const void*>(k_stream<true, 8, 1, true>),   reinterpret_cast<const void*>(k_stream<true, 8, 0, true>),
+        reinterpret_cast<const void*>(k_stream<false, 8, 2, true>), reinterpret_cast<const void*>(k_stream<false, 8, 1, true>),  reinterpret_cast<const void*>(k_stream<false, 8, 0, true>),
+        reinterpret_cast<const void*>(k_stream<true, 16, 2, true>), reinterpret_cast<const void*>(k_stream<true, 16, 1, true>),  reinterpret_cast<const void*>(k_stream<true, 16, 0, true>),
+        reinterpret_cast<const void*>(k_stream<false, 16, 2, true>), reinterpret_cast<const void*>(k_stream<false, 16, 1, true>), reinterpret_cast<const void*>(k_stream<false, 16, 0, true>),
         reinterpret_cast<const void*>(k_ffn<4>), reinterpret_cast<const void*>(k_ffn<8>), reinterpret_cast<const void*>(k_ffn<16>)};
     for (const void* f : fns) FRX_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
     // the head kernel's grouping tables: 12 bytes per expert, 4 per slot, 52 per item (at most 4096 experts, 64 x 32 slots, 2064 items)
