@@ -319,23 +319,70 @@ int check_dot_shape(const char* who, uint32_t type, int64_t ncols, int64_t nrows
     return FRX_OK;
 }
 
-// ---- Q8_0 -> Q2_0 (arch/qwen4exp/mtp.cu:129-201): a thread per 64 values, kept in registers; the 24 candidate
-// scales one after the other, the squared errors added in index order. A block's input (68 bytes per 64
-// values) and output (18 bytes) pass through shared memory in whole vectors.
+// ---- Q8_0 -> Q2_0 (arch/qwen4exp/mtp.cu:129-201): a thread per 64 values. Of 24 candidate scales d the reference takes the
+// first with the smallest sum of (x - q d)^2, added in fp32 in index order, q = x / d rounded and clamped to [-1, 2].
 //
-// The inner loop has no division and no comparison. The values are d8 * q8 (exact, at most 18 significant
-// bits), a candidate d is an fp16 value (11 bits): if x / d is not exactly on a rounding boundary (-0.5, 0.5,
-// 1.5) it is at least 2^-18 of itself away from it, so a quotient good to 2^-22 gives the reference's code; on a
-// boundary either neighbour leaves the same |x - q d|, and only its square is used. The quotient is taken
-// as sat((x / d + 1) / 3) * 3, which clamps it to [-1, 2] in the same instruction, rounded by a magic
-// addition; x - q d rounds once in a fused multiply-add because q d is exact. The codes of the chosen scale
-// are decided by exact comparisons with 0.5 d and 1.5 d.
-// Bound: fp32 issue, six instructions per value and candidate. 48 experts of 2560 x 640 (236 M values): 8.1 ms
-// before (a warp per 64 values, one candidate per lane, a shuffle and an IEEE division per value), 1.2 ms now.
-constexpr int kRqThreads = 128;
-__global__ void __launch_bounds__(kRqThreads) k_q8_0_to_q2_0(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, size_t nblocks64) {
+// The sums are not formed candidate by candidate. With S1 = sum(q x) and S2 = sum(q^2) a sum is X2 - d (2 S1 - d S2), and
+// q changes only where |x| passes 0.5 d or x passes 1.5 d: a value adds |x| to S1 and 1 to S2 for every candidate with
+// 0.5 d <= |x|, and again |x| and 3 for every one with 1.5 d <= x. The candidates grow with their index, so each
+// value goes into at most two of 25 bins (how many candidates it has passed) of the thread's own column in shared
+// memory, and 24 suffix sums give S1 and S2 of all candidates, exactly: a bin is a float that counts passes in
+// units of 16384 above a sum of 8-bit magnitudes (both below 2^24 together), one half of the block at a time.
+// The bin follows from amax / |x|, good to 0.02 of a bin (the candidates are rounded to fp16: 2^-11 of 2.5 * 46 / 3 bins) and
+// settled by one exact comparison with the candidate it may just have missed.
+// What rounding remains (1.2e-6 X2 here, 66 * 2^-24 of the sum in the reference's order) decides nothing: candidates closer
+// to the best than that are summed again in the reference's order and compared as it does, about one block in a hundred.
+// Blocks whose candidates are not all normal fp16 numbers are summed so for all 24.
+//
+// In that sum a division is not needed: the values are d8 * q8 (exact, at most 18 significant bits), a candidate is an
+// fp16 value (11 bits): if x / d is not exactly on a rounding boundary (-0.5, 0.5, 1.5) it is at least 2^-18 of itself
+// away from it, so a quotient good to 2^-22 gives the reference's code; on a boundary either neighbour leaves the same
+// |x - q d|, and only its square is used. The quotient is taken as sat((x / d + 1) / 3) * 3, which clamps it to
+// [-1, 2] in the same instruction, rounded by a magic addition; x - q d rounds once in a fused multiply-add because q d
+// is exact. The codes of the chosen scale come from the same quotient enlarged by 2^-20, which takes it past a boundary
+// it lies on and past none that it does not.
+// Bound: issue slots, about 40 per value (six per value and candidate when each candidate was summed). 48 experts of
+// 2560 x 640 (236 M values): 1.35 ms with a sum per candidate, 0.65 ms so.
+constexpr int kRqThreads = 128, kRqCand = 24;
+constexpr float kRqCount = 16384.0f;   // a pass in a bin; the magnitudes of 32 values, twice each, stay below 8192
+constexpr uint32_t kRqRow = kRqThreads * 4;
+
+// the thread's own column of shared memory, by address (volatile: in program order)
+__device__ __forceinline__ float rq_load(uint32_t a) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void rq_store(uint32_t a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
+// word i (four values) of a block's half h: the 68 bytes are {d, 32 codes}, {d, 32 codes}
+__device__ __forceinline__ uint32_t rq_word(const uint32_t* w, int h, int i) { return h ? w[9 + i] : __funnelshift_r(w[i], w[i + 1], 16); }
+// value k of such a word as a float
+__device__ __forceinline__ float rq_value(uint32_t biased, int k) { return __uint_as_float(__byte_perm(biased, 0x4B000000u, 0x7440u + k)) - 8388736.0f; }
+
+// the reference's sum for one candidate, in its order
+__device__ __forceinline__ float rq_error(const uint32_t* w, float d_lo, float d_hi, float dq) {
+    const bool usable = dq > 0.0f && dq < INFINITY;   // else every code is 0 (see the oracle's note on lround)
+    const float d = usable ? dq : 0.0f, inv3 = usable ? __fdiv_rn(1.0f, 3.0f * d) : 0.0f;
+    float e = 0.0f;
+#pragma unroll 1
+    for (int i = 0; i < 16; ++i) {
+        const uint32_t v = rq_word(w, i >> 3, i & 7) ^ 0x80808080u;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float x = __fmul_rn(i < 8 ? d_lo : d_hi, rq_value(v, k));
+            const float t = __fmaf_rn(__saturatef(__fmaf_rn(x, inv3, 1.0f / 3.0f)), 3.0f, kMagic);   // kMagic + q + 1
+            const float r = __fmaf_rn(-__fsub_rn(t, kMagic + 1.0f), d, x);
+            e = __fadd_rn(e, __fmul_rn(r, r));
+        }
+    }
+    return e;
+}
+
+__global__ void __launch_bounds__(kRqThreads, 6) k_q8_0_to_q2_0(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, size_t nblocks64) {
     __shared__ __align__(16) uint8_t in[kRqThreads * 68];
     __shared__ __align__(16) uint8_t out[kRqThreads * 18];
+    __shared__ float half_d[kRqCand * kRqThreads];        // [candidate][thread]: 0.5 d
+    __shared__ float bins[(kRqCand + 1) * kRqThreads];    // [candidates passed][thread]
     const size_t b0 = size_t(blockIdx.x) * kRqThreads;
     const int tid = threadIdx.x, nb = int(min(size_t(kRqThreads), nblocks64 - b0));
     const uint8_t* s = src + b0 * 68;
@@ -346,57 +393,138 @@ __global__ void __launch_bounds__(kRqThreads) k_q8_0_to_q2_0(const uint8_t* __re
     }
     __syncthreads();
     if (tid < nb) {
-        const uint32_t* w = reinterpret_cast<const uint32_t*>(in) + tid * 17;   // {d, 32 codes}, {d, 32 codes}
-        float x[64];
-        float amax = 0.0f;
-        const float d_lo = __half2float(__ushort_as_half(uint16_t(w[0] & 0xffffu))), d_hi = __half2float(__ushort_as_half(uint16_t(w[8] >> 16)));
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(in) + tid * 17;
+        const float d8[2] = {__half2float(__ushort_as_half(uint16_t(w[0] & 0xffffu))), __half2float(__ushort_as_half(uint16_t(w[8] >> 16)))};
+        // the largest magnitude and the sum of squares of each half. A signed 16-bit maximum of {byte, byte below it}
+        // pairs is decided by the upper byte.
+        float mag[2];
+        int sq[2];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const uint32_t lo = __funnelshift_r(w[i], w[i + 1], 16), hi = w[9 + i];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                x[4 * i + k] = __fmul_rn(d_lo, float(int8_t(lo >> (8 * k))));
-                x[32 + 4 * i + k] = __fmul_rn(d_hi, float(int8_t(hi >> (8 * k))));
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 64; ++i) amax = fmaxf(amax, fabsf(x[i]));
-        float best_e = INFINITY, best_d = 0.0f;
-#pragma unroll 1
-        for (int c = 0; c < 24; ++c) {
-            // d = amax / (2.5f - 1.5f * float(c) / 23.0f), through fp16
-            const float div = __fsub_rn(2.5f, __fdiv_rn(__fmul_rn(1.5f, float(c)), 23.0f));
-            const float dq = __half2float(__float2half_rn(__fdiv_rn(amax, div)));
-            const bool usable = dq > 0.0f && dq < INFINITY;   // else every code is 0 (see the oracle's note on lround)
-            const float d = usable ? dq : 0.0f, inv3 = usable ? __fdiv_rn(1.0f, 3.0f * d) : 0.0f;
-            float e = 0.0f;
-#pragma unroll
-            for (int j = 0; j < 64; ++j) {
-                const float t = __fmaf_rn(__saturatef(__fmaf_rn(x[j], inv3, 1.0f / 3.0f)), 3.0f, kMagic);   // kMagic + q + 1
-                const float q = __fsub_rn(t, kMagic + 1.0f);
-                const float r = __fmaf_rn(-q, d, x[j]);
-                e = __fadd_rn(e, __fmul_rn(r, r));
-            }
-            // the first candidate with the smallest error wins; a NaN or infinite error never does
-            if (amax > 0.0f && dq < INFINITY && e < best_e) {
-                best_e = e;
-                best_d = dq;
-            }
-        }
-        const bool fin = best_d > 0.0f && best_d < INFINITY;
-        const float h1 = 0.5f * best_d, h3 = 1.5f * best_d;
-        uint16_t* o = reinterpret_cast<uint16_t*>(out + tid * 18);
-        o[0] = __half_as_ushort(__float2half_rn(best_d));
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {   // two bytes of four elements each
-            uint32_t v = 0;
+        for (int h = 0; h < 2; ++h) {
+            uint32_t hi = 0x80008000u, lo = 0x7fff7fffu;
+            int q = 0;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                const float xv = x[8 * k + i];
-                const int code = fin ? 1 + int(xv >= h1) + int(xv >= h3) - int(xv <= -h1) : 1;
-                v |= uint32_t(code) << (2 * i);
+                const uint32_t v = rq_word(w, h, i), u = v << 8;
+                hi = __vmaxs2(__vmaxs2(hi, v), u);
+                lo = __vmins2(__vmins2(lo, v), u);
+                q = __dp4a(int(v), int(v), q);
             }
-            o[1 + k] = uint16_t(v);
+            const int top = max(int(hi) >> 24, int(int16_t(hi & 0xffffu)) >> 8), bot = min(int(lo) >> 24, int(int16_t(lo & 0xffffu)) >> 8);
+            mag[h] = float(max(top, -bot));
+            sq[h] = q;
+        }
+        const float amax = fmaxf(fmaxf(0.0f, __fmul_rn(fabsf(d8[0]), mag[0])), __fmul_rn(fabsf(d8[1]), mag[1]));
+#pragma unroll
+        for (int c = 0; c < kRqCand; ++c) {
+            // d = amax / (2.5f - 1.5f * float(c) / 23.0f), through fp16
+            const float div = __fsub_rn(2.5f, __fdiv_rn(__fmul_rn(1.5f, float(c)), 23.0f));
+            half_d[c * kRqThreads + tid] = 0.5f * __half2float(__float2half_rn(__fdiv_rn(amax, div)));
+        }
+        uint32_t near_best = (1u << kRqCand) - 1;   // candidates that may have the smallest sum
+        if (amax >= 0x1p-12f && amax < 32768.0f && fabsf(d8[0]) < INFINITY && fabsf(d8[1]) < INFINITY) {
+            float first[kRqCand];   // suffix sums of the first half
+            const uint32_t cand0 = smem_u32(half_d) + tid * 4, bin0 = smem_u32(bins) + tid * 4;
+            const uint32_t base = cand0 - (0x4B000000u * kRqRow), to_bin = bin0 - cand0;
+            float best = 0.0f, x2 = 0.0f;
+            float gain[kRqCand];    // d (2 S1 - d S2)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+#pragma unroll
+                for (int c = 0; c <= kRqCand; ++c) rq_store(bin0 + c * kRqRow, 0.0f);
+                // candidates passed: floor((2.5 - amax / (2 |x|)) * 46 / 3 + 1); 0.03 less, so that the candidate to compare
+                // with is the next one, and rounded to nearest, so 0.5 less; in units of 23 for the clamp
+                const float c1 = __fdiv_rn(amax, -3.0f * fabsf(d8[h])), off = (2.5f * 46.0f / 3.0f + 0.47f) / 23.0f;
+#pragma unroll 1
+                for (int i = 0; i < 8; i += 2) {
+                    float x[8], one[8];
+                    uint32_t a1[8], a3[8];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        const float xf = rq_value(rq_word(w, h, i + k / 4) ^ 0x80808080u, k % 4);
+                        float r;
+                        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fabsf(xf)));
+                        x[k] = __fmul_rn(d8[h], xf);
+                        one[k] = fabsf(xf) + kRqCount;
+                        a1[k] = __float_as_uint(__fmaf_rn(__saturatef(__fmaf_rn(r, c1, off)), 23.0f, 8388608.0f)) * kRqRow + base;
+                        a3[k] = __float_as_uint(__fmaf_rn(__saturatef(__fmaf_rn(r, 3.0f * c1, off)), 23.0f, 8388608.0f)) * kRqRow + base;
+                    }
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        if (fabsf(x[k]) >= rq_load(a1[k])) a1[k] += kRqRow;
+                        if (x[k] >= 3.0f * rq_load(a3[k])) a3[k] += kRqRow;
+                    }
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        rq_store(a1[k] + to_bin, rq_load(a1[k] + to_bin) + one[k]);
+                        if (x[k] > 0.0f) rq_store(a3[k] + to_bin, rq_load(a3[k] + to_bin) + (one[k] + 2.0f * kRqCount));
+                    }
+                }
+                float sum = 0.0f;
+#pragma unroll
+                for (int c = kRqCand - 1; c >= 0; --c) {
+                    sum += rq_load(bin0 + (c + 1) * kRqRow);   // exact: an integer below 2^24
+                    if (h == 0) {
+                        first[c] = sum;
+                    } else {
+                        const float n0 = __fmaf_rn(first[c], 1.0f / kRqCount, kMagic) - kMagic, n1 = __fmaf_rn(sum, 1.0f / kRqCount, kMagic) - kMagic;
+                        const float s1 = __fmaf_rn(fabsf(d8[0]), __fmaf_rn(n0, -kRqCount, first[c]), fabsf(d8[1]) * __fmaf_rn(n1, -kRqCount, sum));
+                        const float d = 2.0f * rq_load(cand0 + c * kRqRow);
+                        gain[c] = d * __fmaf_rn(-d, n0 + n1, 2.0f * s1);
+                        best = fmaxf(best, gain[c]);
+                    }
+                }
+                x2 = __fmaf_rn(d8[h] * d8[h], float(sq[h]), x2);
+            }
+            const float least = best - (3e-6f * x2 + 1e-5f * fmaxf(x2 - best, 0.0f));
+            near_best = 0;
+#pragma unroll
+            for (int c = 0; c < kRqCand; ++c) near_best |= uint32_t(gain[c] >= least) << c;
+        }
+        float best_d = 0.0f;
+        if ((near_best & (near_best - 1)) == 0) {
+            best_d = 2.0f * half_d[(31 - __clz(near_best)) * kRqThreads + tid];
+        } else if (amax > 0.0f) {
+            // the first candidate with the smallest error wins; a NaN or infinite error never does
+            float best_e = INFINITY;
+#pragma unroll 1
+            for (uint32_t m = near_best; m; m &= m - 1) {
+                const float dq = 2.0f * half_d[(__ffs(m) - 1) * kRqThreads + tid];
+                const float e = dq < INFINITY ? rq_error(w, d8[0], d8[1], dq) : INFINITY;
+                if (e < best_e) {
+                    best_e = e;
+                    best_d = dq;
+                }
+            }
+        }
+        uint16_t* o = reinterpret_cast<uint16_t*>(out + tid * 18);
+        o[0] = __half_as_ushort(__float2half_rn(best_d));
+        if (best_d >= 0x1p-14f && best_d < INFINITY) {
+            const float inv3 = __fdiv_rn(1.0f + 0x1p-20f, 3.0f * best_d);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {   // two bytes of four elements each
+                const float f = d8[k / 4] * inv3;
+                uint32_t v = 0;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float xf = rq_value(rq_word(w, k / 4, (k % 4) * 2 + i / 4) ^ 0x80808080u, i % 4);
+                    v += __float_as_uint(__fmaf_rn(__saturatef(__fmaf_rn(xf, f, 1.0f / 3.0f)), 3.0f, kMagic)) << (2 * i);   // (kMagic's own bits leave the low 16)
+                }
+                o[1 + k] = uint16_t(v);
+            }
+        } else {
+            const bool fin = best_d > 0.0f && best_d < INFINITY;
+            const float h1 = 0.5f * best_d, h3 = 1.5f * best_d;
+#pragma unroll 1
+            for (int k = 0; k < 8; ++k) {
+                uint32_t v = 0;
+                for (int i = 0; i < 8; ++i) {
+                    const float xv = __fmul_rn(d8[k / 4], rq_value(rq_word(w, k / 4, (k % 4) * 2 + i / 4) ^ 0x80808080u, i % 4));
+                    const int code = fin ? 1 + int(xv >= h1) + int(xv >= h3) - int(xv <= -h1) : 1;
+                    v |= uint32_t(code) << (2 * i);
+                }
+                o[1 + k] = uint16_t(v);
+            }
         }
     }
     __syncthreads();
