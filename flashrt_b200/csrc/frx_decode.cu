@@ -335,6 +335,14 @@ __global__ void __launch_bounds__(1024) k_prologue(const float* __restrict__ log
 // While a warp computes on one chunk, its next rpw - 1 chunks are in flight.
 constexpr int kDownGroups = 4;
 
+// The large block has 12 warps that multiply and 4 that only build item buffers, three and one to each scheduler. When every
+// warp also built, the stream stopped for a trip to memory (and, in down, the exponentials) at every item; 16 multiplying
+// warps beside them leave 96 registers each, which is not enough. us per layer, 16 warps that did both -> 12 + 4: 64 tokens
+// 105.6 -> 103.2 (2048 / 512), 51.5 -> 47.3 (512 / 256); 8 tokens 48.4 -> 46.3; 120 tokens of prefill 148 -> 143, 900
+// tokens 549 -> 529. The smaller blocks (launches with few tasks per SM) have hardly a second item: their warps do both.
+constexpr int kStreamWarps = 12;
+__host__ __device__ constexpr int stream_builders(int nw) { return nw == kStreamWarps ? 4 : 0; }
+
 struct StreamParams {
     const Item* items;
     int* status;
@@ -406,7 +414,8 @@ __host__ __device__ inline SmemPlan smem_plan(int kdim, uint32_t chunk_bytes, in
 // K, a chunk the same K range of all four (four bulk copies on one barrier); items of one or two
 // tokens take units_mma_n2, items of three or four units_mma_n4x2.
 template <bool GATE_UP, int NW, int UPC, bool TASK4 = false>
-__global__ void __launch_bounds__(NW * 32, 1) k_stream(const StreamParams p) {
+__global__ void __launch_bounds__((NW + stream_builders(NW)) * 32, 1) k_stream(const StreamParams p) {
+    constexpr int NB = stream_builders(NW), NT = NW + NB;   // warps that only build, and all of them
     extern __shared__ __align__(128) uint8_t smem[];
     // Gate/up follows the kernel that makes the work items, so it waits for it at once. Down follows
     // the hidden-row quantizer, which itself started only after gate/up and therefore after the
@@ -453,7 +462,7 @@ __global__ void __launch_bounds__(NW * 32, 1) k_stream(const StreamParams p) {
     if (threadIdx.x == 0) {   // (before the wait: this needs nothing from the kernels in front)
         for (int s = 0; s < slots; ++s) mbar_init(reinterpret_cast<uint64_t*>(smem + sp.bars) + s, 1);
         for (int b = 0; b < kMaxItemBufs; ++b) {
-            mbar_init(ready + b, NW);
+            mbar_init(ready + b, NT);
             mbar_init(done + b, NW);
         }
         *abort = 0;
@@ -493,7 +502,7 @@ __global__ void __launch_bounds__(NW * 32, 1) k_stream(const StreamParams p) {
     const int first_item = int(lo / tasks_per_expert), last_item = int((hi - 1) / tasks_per_expert);
     int is_item = 0, is_task = 0, is_i = warp, is_c = 0, is_slot = 0;   // the next chunk to issue
     const uint8_t* is_blob = nullptr;
-    if (lane == 0) {
+    if (lane == 0 && warp < NW) {
         const long long tau = lo + warp;
         is_item = int(tau / tasks_per_expert);
         is_task = int(tau % tasks_per_expert);
@@ -531,7 +540,7 @@ __global__ void __launch_bounds__(NW * 32, 1) k_stream(const StreamParams p) {
             }
         }
     };
-    if (lane == 0)
+    if (lane == 0 && warp < NW)
         for (int k = 0; k < rpw; ++k) issue_next();
     int cs_slot = 0;
     uint32_t cs_phase = 0;   // the chunk being consumed: its slot and that slot's barrier phase
@@ -564,18 +573,17 @@ __global__ void __launch_bounds__(NW * 32, 1) k_stream(const StreamParams p) {
         if (btid < kItemWords) reinterpret_cast<uint32_t*>(smem + sp.item + buf * 64)[btid] = reinterpret_cast<const uint32_t*>(it)[btid];
         const int m = it->n_tok;
         const bool narrow = m <= kNarrowTok && p.narrow;   // see units_mma_narrow
-        const int NT = bthreads;
         if (!GATE_UP && p.from_gu) {   // the hidden rows are made here (every item is narrow then)
-            build_hidden_narrow<32>(p.gu, p.ff, it, bw, daw, ciw, btid, NT);
+            build_hidden_narrow<32>(p.gu, p.ff, it, bw, daw, ciw, btid, bthreads);
             return;
         }
         // column g of the B fragments, scales and biases <- activation row of the item's g-th slot
         const int vpr = nb * 4;   // 16-byte vectors per row
-        for (int base = btid; base < m * vpr; base += 4 * NT) {
+        for (int base = btid; base < m * vpr; base += 4 * bthreads) {
             uint4 v[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const int idx = base + k * NT;
+                const int idx = base + k * bthreads;
                 if (idx < m * vpr) {
                     const int g = idx / vpr, r = idx % vpr;
                     const int slot = it->slot[g];
@@ -585,14 +593,14 @@ __global__ void __launch_bounds__(NW * 32, 1) k_stream(const StreamParams p) {
             }
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const int idx = base + k * NT;
+                const int idx = base + k * bthreads;
                 if (idx < m * vpr) {
                     const int g = idx / vpr, r = idx % vpr;
                     reinterpret_cast<uint4*>(bw)[(r >> 2) * 32 + g * 4 + (r & 3)] = v[k];
                 }
             }
         }
-        for (int idx = btid; idx < m * nb * 2; idx += NT) {
+        for (int idx = btid; idx < m * nb * 2; idx += bthreads) {
             const int g = idx / (nb * 2), r = idx % (nb * 2), b = r >> 1, s = r & 1;
             const int slot = it->slot[g];
             const size_t row = GATE_UP ? size_t(slot_token(slot, p.K, p.TK)) : size_t(slot);
@@ -623,6 +631,8 @@ __global__ void __launch_bounds__(NW * 32, 1) k_stream(const StreamParams p) {
     // its tasks of item q builds its share of item q + nbuf - 1 (into the buffer item q - 1 used, once
     // every warp has left that item) and goes on to item q + 1 as soon as all shares of it are in.
     // With three buffers a warp can run one item ahead of the slowest warp.
+    // With warps that only build (see stream_builders) the others never stop for it: those build item q as soon as item
+    // q - nbuf has left its buffer.
     // down: the output row of a slot (routed slots in y, float or bf16 rows; shared-expert slots in ysh,
     // always float), and the store of rows `row` and `row + 8` of it
     auto out_row = [&](int sl) -> float* {
@@ -642,8 +652,8 @@ __global__ void __launch_bounds__(NW * 32, 1) k_stream(const StreamParams p) {
     if (!GATE_UP) pdl_wait();   // the first weight chunks are already in flight
     stamp_now(1);   // the kernels in front have ended, the first copies are issued
     if (ahead == 2 && nseg >= 2) {   // the first two items side by side: one half of the warps each
-        constexpr int H = NW / 2;
-        build(warp < H ? 0 : 1, warp < H ? ctid : ctid - H * 32, warp < H ? H * 32 : (NW - H) * 32);
+        constexpr int H = NT / 2;
+        build(warp < H ? 0 : 1, warp < H ? ctid : ctid - H * 32, warp < H ? H * 32 : (NT - H) * 32);
         __syncwarp();
         if (lane == 0) {   // every warp arrives at both barriers; they complete when the builders have
             mbar_arrive(ready + 0);
@@ -651,12 +661,21 @@ __global__ void __launch_bounds__(NW * 32, 1) k_stream(const StreamParams p) {
         }
     } else {
         for (int q = 0; q < ahead && q < nseg; ++q) {
-            build(q, ctid, NW * 32);
+            build(q, ctid, NT * 32);
             __syncwarp();
             if (lane == 0) mbar_arrive(ready + q % nbuf);
         }
     }
-    for (int q = 0; q < nseg; ++q) {
+    if (NB > 0 && warp >= NW) {
+        for (int q = ahead; q < nseg; ++q) {
+            const int buf = q % nbuf;
+            if (q >= nbuf) mbar_wait_bounded(done + buf, uint32_t((q - nbuf) / nbuf) & 1u, abort, p.wait_ns);
+            build(q, ctid - NW * 32, NB * 32);
+            __syncwarp();
+            if (lane == 0) mbar_arrive_n(ready + buf, NT / (NB > 0 ? NB : 1));
+        }
+    }
+    for (int q = 0; q < (warp < NW ? nseg : 0); ++q) {
         const int item = first_item + q, buf = q % nbuf;
         mbar_wait_bounded(ready + buf, uint32_t(q / nbuf) & 1u, abort, p.wait_ns);
         if (q == 0) stamp_now(2);   // the first item buffer is built
@@ -811,7 +830,7 @@ __global__ void __launch_bounds__(NW * 32, 1) k_stream(const StreamParams p) {
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(done + buf);
-        if (q + ahead < nseg) {
+        if (NB == 0 && q + ahead < nseg) {
             const int nxt = (q + ahead) % nbuf;   // the buffer of item q - 1
             if (q >= 1) mbar_wait_bounded(done + nxt, uint32_t((q - 1) / nbuf) & 1u, abort, p.wait_ns);
             build(q + ahead, ctid, NW * 32);
@@ -913,7 +932,7 @@ __global__ void __launch_bounds__(kChunkSlots) k_pf_place_items(const int32_t* _
 
 // ---------------------------------------------------------------------------------------------
 
-int g_nw = 16;   // consumer warps of k_stream (8, 12 or 16)
+int g_nw = kStreamWarps;   // warps of k_stream that multiply (8 or kStreamWarps)
 int g_small4 = 0, g_small8 = 8;   // launches of at most this many tasks per SM take blocks of 4 / 8 warps with deeper rings (measured at 1 to 3 tokens: 8 warps 26.9 us per layer, 4 warps 27.7, 16 warps 28.9)
 int g_narrow = 1; // items of at most kNarrowTok tokens take the narrow form of the inner product
 int g_gu_chunks = 0;   // chunks per gate/up task (0: by shape)
@@ -932,7 +951,10 @@ struct StreamCfg {
 // blocks of 4 or 8 warps with deeper rings serve small batches better.
 // decode, when every item has at most four tokens: bit 0 = gate/up, bit 1 = down take tasks of four row groups
 // (k_stream's TASK4 form). Measured at batch 64: down gains from it, gate/up does not.
+// With an odd number of units (one to a chunk) down gains up to 16 tokens only (kTask4OddTokens): ff = 640 at 64 tokens 147.1
+// us per layer with it and 143.6 without, 384 / 640 at 16 tokens 41.7 and 43.8.
 int g_task4 = 2;
+constexpr int kTask4OddTokens = 16;
 int g_evict_first = 1;  // decode: the weight copies carry an evict-first L2 policy (see l2_policy_evict_first)
 int g_down_per_item = 256;   // weight of an item's buffer in down's split, in 1/16 of a task (measured best near 16 tasks: 102.4 us per layer against 103.5 with 0 and 106.5 with 1024)
 int g_down_heavy = 22;  // decode: weight of a down task of an item of three or four tokens when the tasks are shared out (16 = as one of a smaller item, 0 = even split by count)
@@ -955,11 +977,11 @@ int stream_cfg(int n, int ff, StreamCfg& c, long long max_items = 0, bool task4 
     auto fit = [&](int kdim, uint32_t task_bytes, int chunks, long long max_tasks, int& nw, int& cpt, int& rpw, int& nbuf, uint32_t& bytes) {
         cpt = chunks;
         const uint32_t chunk = task_bytes / uint32_t(cpt);
-        int first = task4 ? (g_nw >= 12 ? 16 : 8) : g_nw;
+        int first = g_nw;
         if (max_tasks > 0 && max_tasks <= (long long)g_small4 * sms) first = 4;
         else if (max_tasks > 0 && max_tasks <= (long long)g_small8 * sms) first = 8;
-        const int prefs[3] = {first, first > 16 ? 16 : first > 12 ? 12 : 8, 8};
-        for (int k = 0; k < 3; ++k) {
+        const int prefs[2] = {first, 8};
+        for (int k = 0; k < 2; ++k) {
             nw = prefs[k];
             for (nbuf = kMaxItemBufs; nbuf >= 2; --nbuf)
                 for (rpw = nw <= 4 ? 8 : 4; rpw >= 2; --rpw) {
@@ -976,8 +998,6 @@ int stream_cfg(int n, int ff, StreamCfg& c, long long max_items = 0, bool task4 
         if (!fit(n, uint32_t(gu_units) * kUnitBytes * 4, gu_c, max_items * (ff / 32), c.nw_gu, c.cpt_gu, c.rpw_gu, c.nbuf_gu, c.smem_gu) ||
             !fit(ff, uint32_t(dn_units) * kUnitBytes * 4, dn_c, max_items * (n / 64), c.nw_dn, c.cpt_dn, c.rpw_dn, c.nbuf_dn, c.smem_dn))
             return fail(FRX_ERR_SHAPE, "n %d / ff %d: tiles do not fit in shared memory", n, ff);
-        auto round_nw = [](int nw) { return nw >= 12 ? 16 : nw >= 8 ? 8 : 4; };   // the forms that are built
-        if (round_nw(c.nw_gu) != c.nw_gu || round_nw(c.nw_dn) != c.nw_dn) return fail(FRX_ERR_SHAPE, "unsupported warp count for four-group tasks");
         return FRX_OK;
     }
     // gate/up: a task is two groups, fetched in K slices; down: kDownGroups groups in two chunks of whole groups
@@ -1004,7 +1024,7 @@ bool ffn_cfg(int n, int ff, long long max_items, FfnCfg& c) {
     if (ug % kFfnUnitsGu || ud % kFfnUnitsDn) return false;
     const int budget = max_smem_optin() - 2048, sms = sm_count();
     const long long max_tasks = max_items * (ff / 16);
-    int first = g_nw >= 12 ? 16 : 8;
+    int first = g_nw == 8 ? 8 : 16;
     if (max_tasks > 0 && max_tasks <= 4LL * sms) first = 4;
     else if (max_tasks > 0 && max_tasks <= 8LL * sms) first = 8;
     const int prefs[3] = {first, first > 8 ? 8 : first, 4};
@@ -1020,57 +1040,41 @@ bool ffn_cfg(int n, int ff, long long max_items, FfnCfg& c) {
     return false;
 }
 
-template <bool GATE_UP, int NW>
+template <bool GATE_UP, bool TASK4, int NW>
 void launch_stream_nw(const StreamParams& p, int upc, uint32_t smem, cudaStream_t stream) {
-    const int sms = sm_count();
-    // A loop of known length is unrolled and its address arithmetic folded: 4 units for n = 2048 in four chunks and ff = 512,
-    // 5 for n = 2560 in four chunks and ff = 640.
-    if (upc == 4)
-        launch_pdl(k_stream<GATE_UP, NW, 4>, dim3(sms), dim3(NW * 32), smem, stream, p);
-    else if (upc == 5)
-        launch_pdl(k_stream<GATE_UP, NW, 5>, dim3(sms), dim3(NW * 32), smem, stream, p);
-    else
-        launch_pdl(k_stream<GATE_UP, NW, 0>, dim3(sms), dim3(NW * 32), smem, stream, p);   // any other split of K
-}
-
-template <bool GATE_UP>
-void launch_stream4(const StreamParams& p, int nw, int upc, uint32_t smem, cudaStream_t stream) {
-    const int sms = sm_count();
-    auto go = [&](auto kernel, int threads) { launch_pdl(kernel, dim3(sms), dim3(threads), smem, stream, p); };
-    if (upc == 2) {
-        switch (nw) {
-            case 4: go(k_stream<GATE_UP, 4, 2, true>, 128); break;
-            case 8: go(k_stream<GATE_UP, 8, 2, true>, 256); break;
-            default: go(k_stream<GATE_UP, 16, 2, true>, 512); break;
-        }
-    } else if (upc == 1) {   // an odd number of units
-        switch (nw) {
-            case 4: go(k_stream<GATE_UP, 4, 1, true>, 128); break;
-            case 8: go(k_stream<GATE_UP, 8, 1, true>, 256); break;
-            default: go(k_stream<GATE_UP, 16, 1, true>, 512); break;
-        }
+    auto go = [&](auto kernel) { launch_pdl(kernel, dim3(sm_count()), dim3((NW + stream_builders(NW)) * 32), smem, stream, p); };
+    // A loop of known length is unrolled and its address arithmetic folded. Pairs of groups: 4 units for n = 2048 in four
+    // chunks and ff = 512, 5 for n = 2560 in four chunks and ff = 640; four groups: two units a chunk, or one if odd.
+    if constexpr (TASK4) {
+        if (upc == 2) go(k_stream<GATE_UP, NW, 2, true>);
+        else go(k_stream<GATE_UP, NW, 1, true>);
     } else {
-        switch (nw) {
-            case 4: go(k_stream<GATE_UP, 4, 0, true>, 128); break;
-            case 8: go(k_stream<GATE_UP, 8, 0, true>, 256); break;
-            default: go(k_stream<GATE_UP, 16, 0, true>, 512); break;
-        }
+        if (upc == 4) go(k_stream<GATE_UP, NW, 4>);
+        else if (upc == 5) go(k_stream<GATE_UP, NW, 5>);
+        else go(k_stream<GATE_UP, NW, 0>);   // any other split of K
     }
 }
-
-template <bool GATE_UP>
+template <bool GATE_UP, bool TASK4>
 void launch_stream(const StreamParams& p, int nw, int upc, uint32_t smem, cudaStream_t stream) {
     switch (nw) {
-        case 4: launch_stream_nw<GATE_UP, 4>(p, upc, smem, stream); break;
-        case 8: launch_stream_nw<GATE_UP, 8>(p, upc, smem, stream); break;
-        case 12: launch_stream_nw<GATE_UP, 12>(p, upc, smem, stream); break;
-        case 20: launch_stream_nw<GATE_UP, 20>(p, upc, smem, stream); break;
-        default: launch_stream_nw<GATE_UP, 16>(p, upc, smem, stream); break;
+        case 4: launch_stream_nw<GATE_UP, TASK4, 4>(p, upc, smem, stream); break;
+        case 8: launch_stream_nw<GATE_UP, TASK4, 8>(p, upc, smem, stream); break;
+        default: launch_stream_nw<GATE_UP, TASK4, kStreamWarps>(p, upc, smem, stream); break;
     }
 }
 
-// The streaming kernels need more dynamic shared memory than the default limit. The attribute
-// belongs to the function on one device, so it is set once per device that calls in.
+template <int NW>
+int set_stream_attr(int lim) {
+    const void* fns[] = {
+        reinterpret_cast<const void*>(k_stream<true, NW, 4>),        reinterpret_cast<const void*>(k_stream<false, NW, 4>),
+        reinterpret_cast<const void*>(k_stream<true, NW, 5>),        reinterpret_cast<const void*>(k_stream<false, NW, 5>),
+        reinterpret_cast<const void*>(k_stream<true, NW, 0>),        reinterpret_cast<const void*>(k_stream<false, NW, 0>),
+        reinterpret_cast<const void*>(k_stream<true, NW, 2, true>),  reinterpret_cast<const void*>(k_stream<false, NW, 2, true>),
+        reinterpret_cast<const void*>(k_stream<true, NW, 1, true>),  reinterpret_cast<const void*>(k_stream<false, NW, 1, true>)};
+    for (const void* f : fns) FRX_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+    return FRX_OK;
+}
+
 int set_smem_attr() {
     static std::mutex mu;
     static bool done[64] = {};
@@ -1079,23 +1083,10 @@ int set_smem_attr() {
     std::lock_guard<std::mutex> lk(mu);
     if (dev >= 0 && dev < 64 && done[dev]) return FRX_OK;
     const int lim = max_smem_optin() - 2048;   // dynamic part only: the kernels also hold a little static shared memory
+    if (int rc = set_stream_attr<4>(lim)) return rc;
+    if (int rc = set_stream_attr<8>(lim)) return rc;
+    if (int rc = set_stream_attr<kStreamWarps>(lim)) return rc;
     const void* fns[] = {
-        reinterpret_cast<const void*>(k_stream<true, 4, 4>), reinterpret_cast<const void*>(k_stream<true, 4, 5>),   reinterpret_cast<const void*>(k_stream<true, 4, 0>),
-        reinterpret_cast<const void*>(k_stream<false, 4, 4>), reinterpret_cast<const void*>(k_stream<false, 4, 5>),  reinterpret_cast<const void*>(k_stream<false, 4, 0>),
-        reinterpret_cast<const void*>(k_stream<true, 8, 4>), reinterpret_cast<const void*>(k_stream<true, 8, 5>),   reinterpret_cast<const void*>(k_stream<true, 8, 0>),
-        reinterpret_cast<const void*>(k_stream<false, 8, 4>), reinterpret_cast<const void*>(k_stream<false, 8, 5>),  reinterpret_cast<const void*>(k_stream<false, 8, 0>),
-        reinterpret_cast<const void*>(k_stream<true, 12, 4>), reinterpret_cast<const void*>(k_stream<true, 12, 5>),  reinterpret_cast<const void*>(k_stream<true, 12, 0>),
-        reinterpret_cast<const void*>(k_stream<false, 12, 4>), reinterpret_cast<const void*>(k_stream<false, 12, 5>), reinterpret_cast<const void*>(k_stream<false, 12, 0>),
-        reinterpret_cast<const void*>(k_stream<true, 16, 4>), reinterpret_cast<const void*>(k_stream<true, 16, 5>),  reinterpret_cast<const void*>(k_stream<true, 16, 0>),
-        reinterpret_cast<const void*>(k_stream<false, 16, 4>), reinterpret_cast<const void*>(k_stream<false, 16, 5>), reinterpret_cast<const void*>(k_stream<false, 16, 0>),
-        reinterpret_cast<const void*>(k_stream<true, 20, 4>), reinterpret_cast<const void*>(k_stream<true, 20, 5>),  reinterpret_cast<const void*>(k_stream<true, 20, 0>),
-        reinterpret_cast<const void*>(k_stream<false, 20, 4>), reinterpret_cast<const void*>(k_stream<false, 20, 5>), reinterpret_cast<const void*>(k_stream<false, 20, 0>),
-        reinterpret_cast<const void*>(k_stream<true, 4, 2, true>), reinterpret_cast<const void*>(k_stream<true, 4, 1, true>),   reinterpret_cast<const void*>(k_stream<true, 4, 0, true>),
-        reinterpret_cast<const void*>(k_stream<false, 4, 2, true>), reinterpret_cast<const void*>(k_stream<false, 4, 1, true>),  reinterpret_cast<const void*>(k_stream<false, 4, 0, true>),
-        reinterpret_cast<const void*>(k_stream<true, 8, 2, true>), reinterpret_cast<const void*>(k_stream<true, 8, 1, true>),   reinterpret_cast<const void*>(k_stream<true, 8, 0, true>),
-        reinterpret_cast<const void*>(k_stream<false, 8, 2, true>), reinterpret_cast<const void*>(k_stream<false, 8, 1, true>),  reinterpret_cast<const void*>(k_stream<false, 8, 0, true>),
-        reinterpret_cast<const void*>(k_stream<true, 16, 2, true>), reinterpret_cast<const void*>(k_stream<true, 16, 1, true>),  reinterpret_cast<const void*>(k_stream<true, 16, 0, true>),
-        reinterpret_cast<const void*>(k_stream<false, 16, 2, true>), reinterpret_cast<const void*>(k_stream<false, 16, 1, true>), reinterpret_cast<const void*>(k_stream<false, 16, 0, true>),
         reinterpret_cast<const void*>(k_ffn<4>), reinterpret_cast<const void*>(k_ffn<8>), reinterpret_cast<const void*>(k_ffn<16>)};
     for (const void* f : fns) FRX_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
     // the head kernel's grouping tables: 12 bytes per expert, 4 per slot, 52 per item (at most 4096 experts, 64 x 32 slots, 2064 items)
@@ -1148,9 +1139,9 @@ void launch_ffn(StreamParams p, const ActBufs& xb, const ActBufs& hb, size_t h_r
     p.aa = xb.a;
     p.ac = xb.c;
     if (task4_gu)
-        FRX_LAUNCH(kKGateUp, stream, launch_stream4<true>(p, cfg.nw_gu, p.n / kUnitK / cfg.cpt_gu, cfg.smem_gu, stream));
+        FRX_LAUNCH(kKGateUp, stream, launch_stream<true, true>(p, cfg.nw_gu, p.n / kUnitK / cfg.cpt_gu, cfg.smem_gu, stream));
     else
-        FRX_LAUNCH(kKGateUp, stream, launch_stream<true>(p, cfg.nw_gu, p.n / kUnitK / cfg.cpt_gu, cfg.smem_gu, stream));
+        FRX_LAUNCH(kKGateUp, stream, launch_stream<true, false>(p, cfg.nw_gu, p.n / kUnitK / cfg.cpt_gu, cfg.smem_gu, stream));
     // decode with items of at most four tokens: down makes the hidden rows itself, from gu
     p.from_gu = fold_quant && g_narrow && task4_dn && !p.row_list && !p.block64 ? 1 : 0;
     const size_t nblk = h_rows * (p.ff / kQ8);
@@ -1164,9 +1155,9 @@ void launch_ffn(StreamParams p, const ActBufs& xb, const ActBufs& hb, size_t h_r
     p.aa = hb.a;
     p.ac = hb.c;
     if (task4_dn)
-        FRX_LAUNCH(kKDown, stream, launch_stream4<false>(p, cfg.nw_dn, p.ff / kUnitK / cfg.cpt_dn, cfg.smem_dn, stream));
+        FRX_LAUNCH(kKDown, stream, launch_stream<false, true>(p, cfg.nw_dn, p.ff / kUnitK / cfg.cpt_dn, cfg.smem_dn, stream));
     else
-        FRX_LAUNCH(kKDown, stream, launch_stream<false>(p, cfg.nw_dn, p.ff / kUnitK, cfg.smem_dn, stream));
+        FRX_LAUNCH(kKDown, stream, launch_stream<false, false>(p, cfg.nw_dn, p.ff / kUnitK, cfg.smem_dn, stream));
 }
 
 // Which calls take the two-kernel form (frx_small.cuh): at most this many tokens, and at most five rounds of its first
@@ -1308,7 +1299,7 @@ int decode_steps(const void* experts, size_t stride, int E, int e_lo, int e_hi, 
         return launch_small(p, scfg, stream);
     }
     // with items cut at four tokens either streaming kernel may take tasks of four row groups
-    const bool task4_gu = g_narrow && (g_task4 & 1), task4_dn = g_narrow && (g_task4 & 2);
+    const bool task4_gu = g_narrow && (g_task4 & 1), task4_dn = g_narrow && (g_task4 & 2) && (ff / kUnitK % 2 == 0 || T <= kTask4OddTokens);
     StreamCfg cfg;
     if (int rc = stream_cfg(n, ff, cfg, L.max_items, false)) return rc;   // max_items: the most items a chunk of tokens can make
     if (task4_gu || task4_dn) {
@@ -1782,7 +1773,7 @@ int frx_debug_set_gate_up_chunks(int chunks) {
 }
 int frx_debug_set_consumer_warps(int nw) {
     if (nw != 8 && nw != 12 && nw != 16 && nw != 20) return FRX_ERR_ARG;
-    g_nw = nw;
+    g_nw = nw == 8 ? 8 : kStreamWarps;
     return FRX_OK;
 }
 int frx_debug_set_small_launch_limits(int four_warps, int eight_warps) {

@@ -62,7 +62,7 @@ const char* frx_profile_class_name(int cls);
 
 /* Tuning knobs for measurements and tests; no counterpart in the reference. Process-wide and not
  * thread-safe: set them before any compute call, not while calls are in flight.
- * frx_debug_set_consumer_warps: warps per block of the streaming expert kernel (8, 12, 16 or 20; default 16).
+ * frx_debug_set_consumer_warps: 8: blocks of the streaming expert kernel have 8 warps; 12, 16 or 20 (default): 12 that multiply and 4 that build.
  * frx_debug_set_gate_up_chunks: the number of K slices a gate/up task is fetched in (0: chosen by shape).
  * frx_debug_set_narrow_items: 1 (default) lets work items of at most four tokens take the narrow
  * form of the inner product (two row groups share one MMA accumulator, half the float work per row);

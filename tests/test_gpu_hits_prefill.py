@@ -109,3 +109,21 @@ def test_grouping_edges(port, T, E, K):
     for s in sorted({0, T * K - 1, *rng.integers(0, T * K, size=24).tolist()}):
         t, k = divmod(s, K)
         assert rel_max(got[s], port.expert_ffn(planar[ids[t, k] % len(planar)], n, ff, xq[t], xd[t])) < 1e-5
+
+
+@pytest.mark.parametrize("n,ff", [(512, 256), (384, 640), (2560, 128)])
+def test_warps_that_only_build_items_give_the_same_bits(port, n, ff):
+    # the large block of the streaming kernels leaves the item buffers to four warps of its own; here a block goes
+    # through more than twice as many items as it has buffers, against blocks whose warps do both
+    from flashrt_b200.lib import check, lib
+    T, E, K = 900, 256, 6                # 21 tokens per expert: about 900 items of up to eight
+    ex = Experts(port, n, ff, E, shared=False, direct=True)
+    x = cuda(synth.activations(T, n))
+    ids = cuda(np.argsort(synth.zipf_logits(T, E), axis=1)[:, :K].astype(np.int32))
+    got = moe.moe_q2.run(ex.base, ex.stride, E, n, ff, x, ids)
+    try:
+        check(lib.frx_debug_set_consumer_warps(8))
+        want = moe.moe_q2.run(ex.base, ex.stride, E, n, ff, x, ids)
+    finally:
+        check(lib.frx_debug_set_consumer_warps(12))
+    assert torch.equal(got, want)
