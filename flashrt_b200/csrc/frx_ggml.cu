@@ -9,8 +9,8 @@
 // (third_party/ggml/src/ggml-cuda/vecdotq.cuh:728-771): per 32-value chunk an exact integer sum
 // of (q - 1) * a, scaled as d2 * d8 * sumi in float; chunks are added in float.
 //
-// One kernel serves every entry. A block takes one work item (an expert and up to NT activation
-// rows) and a run of weight rows. The rows are contiguous in memory, so a tile of them is staged
+// One kernel serves the gemv entries. A block takes one job (an expert and an activation row) and a
+// run of weight rows. The rows are contiguous in memory, so a tile of them is staged
 // in shared memory by one 1-D bulk (TMA) copy; a lane owns a pair of neighbouring blocks (36 bytes,
 // nine conflict-free 32-bit shared-memory loads) and the activations are kept in shared memory
 // transposed so that crumb p of a weight word lines up with one int8x4 word: 16 dp4a per block and
@@ -38,6 +38,8 @@ inline size_t act_row_bytes(int64_t ncols) { return size_t(padded_cols(ncols) / 
 // which uses the fast exponential).
 __global__ void __launch_bounds__(256) k_q8_1(const float* __restrict__ x, const float* __restrict__ u, int64_t ncols, int64_t padded,
                                               uint8_t* __restrict__ y) {
+    pdl_wait();
+    pdl_trigger();
     const int64_t i0 = int64_t(blockDim.x) * blockIdx.x + threadIdx.x, t = blockIdx.y;
     if (i0 >= padded) return;   // padded is a multiple of the block
     float xi = 0.0f;
@@ -78,16 +80,16 @@ struct DotArgs {
 struct DotSmem {
     uint32_t at, d8, sa, w, bar, abort, total;
 };
-__host__ __device__ inline DotSmem dot_smem(int nt, int ncols, int tile_bytes, bool gate) {
+__host__ __device__ inline DotSmem dot_smem(int ncols, int tile_bytes, bool gate) {
     DotSmem s{};
     const uint32_t nch = uint32_t(ncols / kQ8);
     uint32_t off = 0;
     s.at = off;
-    off += uint32_t(nt) * uint32_t(ncols);
+    off += uint32_t(ncols);
     s.d8 = off;
-    off += uint32_t(nt) * nch * 4;
+    off += nch * 4;
     s.sa = off;
-    off += uint32_t(nt) * nch * 4;
+    off += nch * 4;
     off = (off + 127u) & ~127u;
     s.w = off;
     off += uint32_t(tile_bytes) * (gate ? 2u : 1u);
@@ -132,55 +134,57 @@ __device__ __forceinline__ int chunk_sum(uint32_t w0, uint32_t w1, const uint4& 
     return s - suma;
 }
 
-template <int NT, bool GATE>
+// Bound with one token (eight jobs): latency, of the chain ids -> weights -> product; so a block asks for its first tile as
+// soon as it knows its expert and prepares the activations meanwhile, and its launch overlaps the kernel in front. One
+// token through 8 experts of 2560 x 640 (routing, two quantizations, two products, combine): 43.5 -> 31 us.
+template <bool GATE>
 __global__ void __launch_bounds__(kDotThreads) k_ggml_dot(const DotArgs a) {
     extern __shared__ __align__(128) uint8_t smem[];
     const int nb = a.ncols / kQK, np = nb / 2, nch = a.ncols / kQ8;
     const uint32_t row_bytes = uint32_t(nb) * kBlockBytes;
     const uint32_t tile_bytes = uint32_t(a.rows_per_tile) * row_bytes;
-    const DotSmem sm = dot_smem(NT, a.ncols, int(tile_bytes), GATE);
+    const DotSmem sm = dot_smem(a.ncols, int(tile_bytes), GATE);
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + sm.bar);
     volatile int* abort = reinterpret_cast<volatile int*>(smem + sm.abort);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-
-    // ---- this block's work item
-    __shared__ int s_act_rows[NT];
-    int e = 0, m = 1;
-    int act_rows[NT], dst_rows[NT];
-    {
-        const int j = blockIdx.x;
-        e = a.ids ? a.ids[j] : 0;
-#pragma unroll
-        for (int q = 0; q < NT; ++q) {
-            dst_rows[q] = j;
-            act_rows[q] = j / a.act_div;
-        }
-    }
     if (tid == 0) {
         mbar_init(bar, 1);
         *abort = 0;
         mbar_fence_init();
-#pragma unroll
-        for (int j = 0; j < NT; ++j) s_act_rows[j] = act_rows[j];
     }
-    __syncthreads();
+    pdl_wait();
+    pdl_trigger();
+    const int job = blockIdx.x, e = a.ids ? a.ids[job] : 0;
+    const uint8_t* wsrc = a.w + size_t(e) * a.expert_stride;
+    const uint8_t* gsrc = GATE ? a.gate + size_t(e) * a.expert_stride : nullptr;
+    uint8_t* wt = smem + sm.w;
+    uint8_t* gt = wt + tile_bytes;
+    const int n_tiles = (a.nrows + a.rows_per_tile - 1) / a.rows_per_tile;
+    auto by_tma = [&](int tile) { return a.tma && (tile + 1) * a.rows_per_tile <= a.nrows; };
+    auto fetch = [&](int tile) {   // thread 0: a whole tile by bulk copies
+        const size_t at = size_t(tile) * tile_bytes;
+        mbar_expect_tx(bar, tile_bytes * (GATE ? 2u : 1u));
+        bulk_g2s(wt, wsrc + at, tile_bytes, bar);
+        if (GATE) bulk_g2s(gt, gsrc + at, tile_bytes, bar);
+    };
+    if (tid == 0 && by_tma(blockIdx.y)) fetch(blockIdx.y);
 
     // ---- activations: codes transposed per 16 values (word p of a group = values p, 4 + p, 8 + p,
     // 12 + p), chunk scales, chunk code sums
     uint32_t* at = reinterpret_cast<uint32_t*>(smem + sm.at);
     float* d8 = reinterpret_cast<float*>(smem + sm.d8);
     int* sa = reinterpret_cast<int*>(smem + sm.sa);
-    for (int idx = tid; idx < m * nch; idx += kDotThreads) {
-        const int j = idx / nch, c = idx % nch;
-        const uint32_t* blk = reinterpret_cast<const uint32_t*>(a.xq + size_t(s_act_rows[j]) * a.act_row + size_t(c) * kQ81Bytes);
+    const uint8_t* act = a.xq + size_t(job / a.act_div) * a.act_row;
+    for (int c = tid; c < nch; c += kDotThreads) {
+        const uint32_t* blk = reinterpret_cast<const uint32_t*>(act + size_t(c) * kQ81Bytes);
         uint32_t v[9];
 #pragma unroll
         for (int i = 0; i < 9; ++i) v[i] = blk[i];
-        d8[j * nch + c] = __half2float(__ushort_as_half(uint16_t(v[0] & 0xffffu)));
+        d8[c] = __half2float(__ushort_as_half(uint16_t(v[0] & 0xffffu)));
         int s = 0;
 #pragma unroll
         for (int i = 1; i < 9; ++i) s = __dp4a(int(v[i]), 0x01010101, s);
-        sa[j * nch + c] = s;
+        sa[c] = s;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const uint32_t u0 = v[1 + 4 * h], u1 = v[2 + 4 * h], u2 = v[3 + 4 * h], u3 = v[4 + 4 * h];
@@ -191,7 +195,7 @@ __global__ void __launch_bounds__(kDotThreads) k_ggml_dot(const DotArgs a) {
             o.y = __byte_perm(lo01, lo23, 0x7632);
             o.z = __byte_perm(hi01, hi23, 0x5410);
             o.w = __byte_perm(hi01, hi23, 0x7632);
-            reinterpret_cast<uint4*>(at + size_t(j) * (a.ncols / 4))[c * 2 + h] = o;
+            reinterpret_cast<uint4*>(at)[c * 2 + h] = o;
         }
     }
     __syncthreads();
@@ -200,25 +204,19 @@ __global__ void __launch_bounds__(kDotThreads) k_ggml_dot(const DotArgs a) {
     const int rpp = (np < 32 && 32 % np == 0) ? 32 / np : 1;   // rows per pass of a warp
     const int width = 32 / rpp;                                // lanes per row
     const int lane_row = lane / width, lane_p = lane % width;
-    const uint8_t* wsrc = a.w + size_t(e) * a.expert_stride;
-    const uint8_t* gsrc = GATE ? a.gate + size_t(e) * a.expert_stride : nullptr;
-    uint8_t* wt = smem + sm.w;
-    uint8_t* gt = wt + tile_bytes;
-    const int n_tiles = (a.nrows + a.rows_per_tile - 1) / a.rows_per_tile;
     uint32_t phase = 0;
     for (int tile = blockIdx.y; tile < n_tiles; tile += gridDim.y) {
         const int r0 = tile * a.rows_per_tile, rows = min(a.rows_per_tile, a.nrows - r0);
-        const uint32_t bytes = uint32_t(rows) * row_bytes;
-        __syncthreads();   // everyone is done with the previous tile
-        if (a.tma && rows == a.rows_per_tile) {
-            if (tid == 0) {
-                mbar_expect_tx(bar, bytes * (GATE ? 2u : 1u));
-                bulk_g2s(wt, wsrc + size_t(r0) * row_bytes, bytes, bar);
-                if (GATE) bulk_g2s(gt, gsrc + size_t(r0) * row_bytes, bytes, bar);
+        if (by_tma(tile)) {
+            if (tile != int(blockIdx.y)) {
+                __syncthreads();   // everyone is done with the previous tile
+                if (tid == 0) fetch(tile);
             }
             mbar_wait_bounded(bar, phase, abort, a.wait_ns);
             phase ^= 1u;
         } else {
+            const uint32_t bytes = uint32_t(rows) * row_bytes;
+            __syncthreads();
             const uint32_t* s0 = reinterpret_cast<const uint32_t*>(wsrc + size_t(r0) * row_bytes);
             for (uint32_t i = tid; i < bytes / 4; i += kDotThreads) reinterpret_cast<uint32_t*>(wt)[i] = s0[i];
             if (GATE) {
@@ -230,46 +228,29 @@ __global__ void __launch_bounds__(kDotThreads) k_ggml_dot(const DotArgs a) {
         for (int rb = warp * rpp; rb < rows; rb += kDotWarps * rpp) {   // uniform for the warp: the sums below are shuffled
             const int rr = rb + lane_row;
             const bool live = rr < rows;
-            float acc[NT], gacc[NT];
-#pragma unroll
-            for (int j = 0; j < NT; ++j) acc[j] = gacc[j] = 0.0f;
+            float v = 0.0f, g = 0.0f;
             for (int pi = lane_p; live && pi < np; pi += width) {
                 float d0, d1, g0 = 0.0f, g1 = 0.0f;
                 uint32_t c[8], gc[8];
                 load_pair(wt + size_t(rr) * row_bytes + size_t(pi) * 36, d0, d1, c);
                 if (GATE) load_pair(gt + size_t(rr) * row_bytes + size_t(pi) * 36, g0, g1, gc);
+                const uint4* aj = reinterpret_cast<const uint4*>(at) + pi * 8;
 #pragma unroll
-                for (int j = 0; j < NT; ++j) {
-                    if (j < m) {
-                        const uint4* aj = reinterpret_cast<const uint4*>(at + size_t(j) * (a.ncols / 4)) + pi * 8;
-                        const float* dj = d8 + j * nch + pi * 4;
-                        const int* sj = sa + j * nch + pi * 4;
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {   // the four chunks of the pair
-                            const uint4 a0 = aj[2 * q], a1 = aj[2 * q + 1];
-                            const float dw = q < 2 ? d0 : d1;
-                            const int s = chunk_sum(c[2 * q], c[2 * q + 1], a0, a1, sj[q]);
-                            acc[j] = __fadd_rn(acc[j], __fmul_rn(__fmul_rn(dw, dj[q]), float(s)));   // d2 * d8 * sumi
-                            if (GATE) {
-                                const float dg = q < 2 ? g0 : g1;
-                                const int sg = chunk_sum(gc[2 * q], gc[2 * q + 1], a0, a1, sj[q]);
-                                gacc[j] = __fadd_rn(gacc[j], __fmul_rn(__fmul_rn(dg, dj[q]), float(sg)));
-                            }
-                        }
-                    }
+                for (int q = 0; q < 4; ++q) {   // the four chunks of the pair
+                    const uint4 a0 = aj[2 * q], a1 = aj[2 * q + 1];
+                    const float dx = d8[pi * 4 + q];
+                    const int sx = sa[pi * 4 + q];
+                    v = __fadd_rn(v, __fmul_rn(__fmul_rn(q < 2 ? d0 : d1, dx), float(chunk_sum(c[2 * q], c[2 * q + 1], a0, a1, sx))));   // d2 * d8 * sumi
+                    if (GATE) g = __fadd_rn(g, __fmul_rn(__fmul_rn(q < 2 ? g0 : g1, dx), float(chunk_sum(gc[2 * q], gc[2 * q + 1], a0, a1, sx))));
                 }
             }
-#pragma unroll
-            for (int j = 0; j < NT; ++j) {
-                float v = acc[j], g = gacc[j];
-                for (int o = width >> 1; o > 0; o >>= 1) {
-                    v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, o));
-                    if (GATE) g = __fadd_rn(g, __shfl_xor_sync(0xffffffffu, g, o));
-                }
-                if (j < m && lane_p == 0 && live) {
-                    if (GATE) v = __fmul_rn(__fdiv_rn(g, __fadd_rn(1.0f, expf(-g))), v);   // ggml unary.cuh:98-100
-                    a.dst[size_t(dst_rows[j]) * a.nrows + r0 + rr] = v;
-                }
+            for (int o = width >> 1; o > 0; o >>= 1) {
+                v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, o));
+                if (GATE) g = __fadd_rn(g, __shfl_xor_sync(0xffffffffu, g, o));
+            }
+            if (lane_p == 0 && live) {
+                if (GATE) v = __fmul_rn(__fdiv_rn(g, __fadd_rn(1.0f, expf(-g))), v);   // ggml unary.cuh:98-100
+                a.dst[size_t(job) * a.nrows + r0 + rr] = v;
             }
         }
     }
@@ -281,24 +262,23 @@ int dot_tile_rows(int ncols) {
     return kDotWarps * rpp * 2;   // two passes of every warp per tile: 18 KB of weights at the usual shapes
 }
 
-template <int NT, bool GATE>
+template <bool GATE>
 int launch_dot(DotArgs a, int grid_x, cudaStream_t stream) {
     a.rows_per_tile = dot_tile_rows(a.ncols);
     const uint32_t row_bytes = uint32_t(a.ncols / kQK) * kBlockBytes, tile_bytes = uint32_t(a.rows_per_tile) * row_bytes;
     a.tma = ((uintptr_t(a.w) | uintptr_t(a.gate) | a.expert_stride | tile_bytes) % 16 == 0) ? 1 : 0;
     a.wait_ns = wait_limit_ns();
-    const DotSmem sm = dot_smem(NT, a.ncols, int(tile_bytes), GATE);
+    const DotSmem sm = dot_smem(a.ncols, int(tile_bytes), GATE);
     if (int(sm.total) > max_smem_optin() - 1024) return fail(FRX_ERR_SHAPE, "ggml-layout product: ncols %d needs %u bytes of shared memory", a.ncols, sm.total);
     static std::mutex mu;
-    static unsigned set_mask[64] = {};
+    static bool set[64] = {};
     int dev = 0;
     FRX_CUDA(cudaGetDevice(&dev));
     {
         std::lock_guard<std::mutex> lk(mu);
-        const unsigned bit = 1u << ((NT > 1 ? 2 : 0) + (GATE ? 1 : 0));
-        if (dev >= 0 && dev < 64 && !(set_mask[dev] & bit)) {
-            FRX_CUDA(cudaFuncSetAttribute(k_ggml_dot<NT, GATE>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin() - 1024));   // less the static part
-            set_mask[dev] |= bit;
+        if (dev >= 0 && dev < 64 && !set[dev]) {
+            FRX_CUDA(cudaFuncSetAttribute(k_ggml_dot<GATE>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin() - 1024));
+            set[dev] = true;
         }
     }
     const int n_tiles = (a.nrows + a.rows_per_tile - 1) / a.rows_per_tile;
@@ -306,8 +286,7 @@ int launch_dot(DotArgs a, int grid_x, cudaStream_t stream) {
     const int sms = sm_count() > 0 ? sm_count() : 148;
     int gy = n_tiles;
     while (gy > 1 && (long long)grid_x * gy > 8LL * sms && gy % 2 == 0) gy /= 2;
-    k_ggml_dot<NT, GATE><<<dim3(unsigned(grid_x), unsigned(gy)), kDotThreads, sm.total, stream>>>(a);
-    FRX_CUDA(cudaGetLastError());
+    FRX_CUDA(launch_pdl(k_ggml_dot<GATE>, dim3(unsigned(grid_x), unsigned(gy)), dim3(kDotThreads), sm.total, stream, a));
     return FRX_OK;
 }
 
@@ -539,34 +518,35 @@ __global__ void __launch_bounds__(kRqThreads, 6) k_q8_0_to_q2_0(const uint8_t* _
 // ---- the grouped product (gemm::moe_run): int8 tensor cores
 // A block takes 128 weight rows and up to 64 of the slots of one expert and walks K in chunks of 128 (two
 // blocks of weights, 36 bytes per row) through a ring of shared-memory stages filled with cp.async: the
-// rows as they are in the file, the activations in the MMA's fragment order, their scales and the
-// accumulators' initial values per pair of slots. 8 warps, 32 rows x 32 slots each: a lane reads a
-// row's 36 bytes (at a stride of 48: conflict-free 16-byte loads shared by the four lanes of a quad),
+// rows as they are in the file, the activations in the MMA's fragment order, their scales per
+// pair of slots. A warp has 32 rows and all the slots, so a row is unpacked once: a lane
+// reads its row's nine words (conflict-free, shared by the four lanes of a quad),
 // shifts lane t's crumbs into place and masks them, which gives the A operand for a K order of
 // {t, 4 + t, 8 + t, 12 + t}; the quantizer writes the activation codes in that order.
-// Per 32 values the MMA starts at kMagicBits - sum(codes) and so ends at kMagicBits + sum((q - 1) * a), which
+// The codes are made signed (code - 1) while they are unpacked, which is cheaper than a sum of the activations per chunk
+// and column. The MMA of 32 values starts at kMagicBits and so ends at kMagicBits + sum((q - 1) * a), which
 // read as a float is kMagic plus the chunk's exact integer sum.
-// What bounds it: issue slots and the int8 MMA together (a 16 x 8 x 64 tile costs two MMAs and eight packed
-// fp32 operations). 1,000 tokens x 8 of 128 experts of 2560 x 640, three products: 11.8 ms before (the dp4a kernel below,
-// eight slots per pass over the weights), 0.5 ms now.
-constexpr int kGmRows = 128, kGmTok = 64, kGmK = 128, kGmStages = 4, kGmThreads = 256;
-constexpr int kGmWStride = 48;                               // bytes per row of a chunk: 36 used
-constexpr int kGmBytesW = kGmRows * kGmWStride;              // 6 KB
+// What bounds it: issue slots (a 16 x 8 x 64 tile costs two MMAs and eight packed fp32 operations of two slots) and what
+// shared memory delivers, about even. 1,000 tokens x 8 of 128 experts of 2560 x 640, per product: 157 us with two warps
+// side by side over the slots (each unpacking the rows, half of them idle behind a short item) and the copies' addresses
+// computed anew, 118 us now (0.24 ms less over the three products of a prompt).
+constexpr int kGmRows = 128, kGmTok = 64, kGmK = 128, kGmStages = 4, kGmThreads = 128;
+constexpr int kGmBytesW = kGmRows * 36;
 constexpr int kGmBytesB = kGmTok * kGmK;                     // [block][8 slots][lane] 16 bytes
 constexpr int kGmBytesA = 2 * (kGmTok / 2) * 16;             // [block][pair of slots] {a0, a0', a1, a1'}
-constexpr int kGmBytesC = 2 * (kGmTok / 2) * 32;             // [block][pair][half] {c, c', c, c'}
-constexpr int kGmStage = kGmBytesW + kGmBytesB + kGmBytesA + kGmBytesC;
+constexpr int kGmStage = kGmBytesW + kGmBytesB + kGmBytesA;
 constexpr int kGmSmem = kGmStages * kGmStage;
 
 // Workspace form of the activations: per row int8 codes in fragment order (word (t * 4 + 2 s + h) of a 64-block
-// holds elements 32 s + 16 h + {t, 4 + t, 8 + t, 12 + t}), the chunk scales d (through fp16, as Q8_1 stores them),
-// and kMagicBits - sum(codes). Quantization is quantize.cu's: d = amax / 127, q = roundf(x / d).
+// holds elements 32 s + 16 h + {t, 4 + t, 8 + t, 12 + t}) and the chunk scales d (through fp16, as Q8_1 stores them).
+// Quantization is quantize.cu's: d = amax / 127, q = roundf(x / d).
 struct GmAct {
     int8_t* q;     // [rows][ncols]
     float* d;      // [rows][ncols / 32]
-    int32_t* c;    // [rows][ncols / 32]
 };
 __global__ void __launch_bounds__(256) k_gm_quant(const float* __restrict__ x, int ncols, size_t n_quads, GmAct a) {
+    pdl_wait();
+    pdl_trigger();
     const size_t quad = size_t(blockIdx.x) * 256 + threadIdx.x;   // four consecutive values; eight lanes one chunk of 32
     if (quad >= n_quads) return;                                  // (a multiple of 32: warps are live as a whole)
     float hv[4];
@@ -581,22 +561,15 @@ __global__ void __launch_bounds__(256) k_gm_quant(const float* __restrict__ x, i
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
     const float d = __fdiv_rn(am, 127.0f);
-    int sum = 0;
     const int j = int(quad & 7), h = j >> 2, i = j & 3;           // elements 16 h + 4 i + t of the chunk, t = 0 .. 3
     const size_t chunk = quad >> 3;
     int8_t* blk = a.q + (chunk >> 1) * 64 + (chunk & 1) * 8 + h * 4 + i;
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
         const int code = am == 0.0f ? 0 : int(round_half_away(__fdiv_rn(hv[t], d)));
-        sum += code;
         blk[t * 16] = int8_t(code);
     }
-#pragma unroll
-    for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (j == 0) {
-        a.d[chunk] = __half2float(__float2half_rn(d));
-        a.c[chunk] = kMagicBits - sum;
-    }
+    if (j == 0) a.d[chunk] = __half2float(__float2half_rn(d));
 }
 
 struct GmArgs {
@@ -612,12 +585,25 @@ struct GmArgs {
     int E, K, x_per_slot;
 };
 
+// D = A * B + C, A and B signed bytes
+__device__ __forceinline__ void mma_s8s8_c4(uint64_t& lo, uint64_t& hi, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                            uint32_t b1, const int4& c) {
+    asm volatile(
+        "{\n\t.reg .b32 d0, d1, d2, d3;\n\t"
+        "mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {d0,d1,d2,d3}, {%2,%3,%4,%5}, {%6,%7}, {%8,%9,%10,%11};\n\t"
+        "mov.b64 %0, {d0,d1};\n\t"
+        "mov.b64 %1, {d2,d3};\n\t}"
+        : "=l"(lo), "=l"(hi)
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c.x), "r"(c.y), "r"(c.z), "r"(c.w));
+}
 __device__ __forceinline__ void gm_cp4(uint32_t dst, const void* src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory"); }
 __device__ __forceinline__ void gm_cp16(uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
 
-__global__ void __launch_bounds__(kGmThreads, 2) k_gm_mma(const GmArgs a) {
+__global__ void __launch_bounds__(kGmThreads, 3) k_gm_mma(const GmArgs a) {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ int s_slot[kGmTok], s_act[kGmTok];
+    pdl_wait();
+    pdl_trigger();
     const int item = blockIdx.x;
     if (item >= a.status[1]) return;
     int lo = 0, hi = a.E;   // the expert with item_off[e] <= item < item_off[e + 1]
@@ -625,7 +611,10 @@ __global__ void __launch_bounds__(kGmThreads, 2) k_gm_mma(const GmArgs a) {
         const int mid = (lo + hi) >> 1;
         if (a.item_off[mid] <= item) lo = mid; else hi = mid;
     }
-    const int e = lo, base = a.bounds[e] + (item - a.item_off[e]) * kGmTok, m = min(kGmTok, a.bounds[e + 1] - base);
+    // an expert's slots in equal items of whole columns of eight: a last item of a few slots would cost as much unpacking
+    const int e = lo, first = a.bounds[e], end = a.bounds[e + 1], parts = a.item_off[e + 1] - a.item_off[e];
+    const int per = ((end - first + parts - 1) / parts + 7) & ~7;
+    const int base = first + (item - a.item_off[e]) * per, m = min(per, end - base);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
     if (tid < kGmTok) {   // columns beyond m repeat the last slot and are not stored
         const int slot = a.perm[base + min(tid, m - 1)];
@@ -639,32 +628,39 @@ __global__ void __launch_bounds__(kGmThreads, 2) k_gm_mma(const GmArgs a) {
     const uint32_t s0 = smem_u32(smem);
     const int m8 = (m + 7) & ~7;   // slots whose activations are fetched
 
-    // this thread's copies of a chunk. Weights: 128 rows x 9 words, 4.5 per thread; codes: m8 x 8 vectors of 16 bytes
+    // This thread's copies of a chunk: nine words of the weights (word i of the tile's 128 x 9 by thread i % 128; rows beyond
+    // the matrix repeat its last one), 16 bytes of the codes of up to four slots, a scale and a sum of up to two.
+    // Where they start is found once.
     const int nch = a.ncols / kQ8;
+    uint32_t w_at[9];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+        const int idx = tid + i * kGmThreads, row = idx / 9, w = idx - row * 9;
+        w_at[i] = uint32_t(min(row, rows - 1)) * row_bytes + w * 4;
+    }
+    const int8_t* q_at[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) q_at[i] = a.act.q + size_t(s_act[(tid >> 3) + 16 * i]) * a.ncols + (tid & 7) * 16;   // vector v: block v >> 2, lane t = v & 3
+    size_t d_at[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) d_at[i] = size_t(s_act[(tid >> 2) + 32 * i]) * nch + (tid & 3);                       // one of the four chunks of 32
+    const uint32_t q_to = ((tid & 7) >> 2) * (kGmTok * 64) + (tid >> 6) * 512 + (((tid >> 3) & 7) * 4 + (tid & 3)) * 16;
+    const uint32_t d_to = ((tid & 2) >> 1) * (kGmTok / 2 * 16) + (tid >> 3) * 16 + (tid & 1) * 8 + ((tid >> 2) & 1) * 4;
     auto fetch = [&](int kc) {
         const uint32_t st = s0 + uint32_t(kc % kGmStages) * kGmStage;
+        const uint8_t* wk = wsrc + size_t(kc) * 36;
 #pragma unroll
-        for (int i = 0; i < 5; ++i) {
-            const int idx = tid + i * kGmThreads;
-            if (idx < kGmRows * 9) {
-                const int row = idx / 9, w = idx - row * 9;
-                gm_cp4(st + row * kGmWStride + w * 4, wsrc + size_t(min(row, rows - 1)) * row_bytes + size_t(kc) * 36 + w * 4);
-            }
-        }
+        for (int i = 0; i < 9; ++i) gm_cp4(st + (tid + i * kGmThreads) * 4, wk + w_at[i]);
         const uint32_t sb = st + kGmBytesW;
-        for (int idx = tid; idx < m8 * 8; idx += kGmThreads) {
-            const int tok = idx >> 3, v = idx & 7;   // vector v: block v >> 2, lane t = v & 3
-            gm_cp16(sb + (v >> 2) * (kGmTok * 64) + (tok >> 3) * 512 + ((tok & 7) * 4 + (v & 3)) * 16, a.act.q + size_t(s_act[tok]) * a.ncols + size_t(kc) * kGmK + v * 16);
-        }
-        const uint32_t sa = sb + kGmBytesB, sc = sa + kGmBytesA;
-        for (int idx = tid; idx < m8 * 4; idx += kGmThreads) {
-            const int tok = idx >> 2, ch = idx & 3, b = ch >> 1, h = ch & 1;   // chunk ch of the four of 128 values
-            const size_t at = size_t(s_act[tok]) * nch + size_t(kc) * 4 + ch;
-            const uint32_t pair = uint32_t(b * (kGmTok / 2) + (tok >> 1));
-            gm_cp4(sa + pair * 16 + h * 8 + (tok & 1) * 4, a.act.d + at);
-            gm_cp4(sc + pair * 32 + h * 16 + (tok & 1) * 4, a.act.c + at);
-            gm_cp4(sc + pair * 32 + h * 16 + 8 + (tok & 1) * 4, a.act.c + at);
-        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if ((tid >> 3) + 16 * i < m8) gm_cp16(sb + q_to + i * 1024, q_at[i] + size_t(kc) * kGmK);
+        const uint32_t sa = sb + kGmBytesB;
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            if ((tid >> 2) + 32 * i < m8) {
+                gm_cp4(sa + d_to + i * 256, a.act.d + d_at[i] + size_t(kc) * 4);
+            }
     };
     const int chunks = a.ncols / kGmK;
 #pragma unroll
@@ -672,75 +668,76 @@ __global__ void __launch_bounds__(kGmThreads, 2) k_gm_mma(const GmArgs a) {
         if (i < chunks) fetch(i);
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    const int wr = (warp & 3) * 32, wt = (warp >> 2) * 32;   // this warp's rows and slots of the tile
-    const int nt = min(4, (m - wt + 7) >> 3);                // live columns of eight slots
-    uint64_t acc[2][4][2];
+    const int wr = warp * 32;         // this warp's rows of the tile
+    const int nt = m8 >> 3;           // live columns of eight slots
+    uint64_t acc[2][8][2];
 #pragma unroll
     for (int r = 0; r < 2; ++r)
 #pragma unroll
-        for (int n = 0; n < 4; ++n) acc[r][n][0] = acc[r][n][1] = 0ull;
-    const uint64_t magic = pack2(kMagic, kMagic);
+        for (int n = 0; n < 8; ++n) acc[r][n][0] = acc[r][n][1] = 0ull;
+    // the accumulators' start in four registers that stay: as constants they would be loaded again for every MMA
+    const uint64_t magic = pack2(kMagic, kMagic), neg_magic = pack2(-kMagic, -kMagic);
+    int4 start;
+    asm volatile("mov.b32 %0, %4;\n\tmov.b32 %1, %4;\n\tmov.b32 %2, %4;\n\tmov.b32 %3, %4;" : "=r"(start.x), "=r"(start.y), "=r"(start.z), "=r"(start.w) : "r"(kMagicBits));
     for (int kc = 0; kc < chunks; ++kc) {
         asm volatile("cp.async.wait_group %0;" ::"n"(kGmStages - 2) : "memory");
         __syncthreads();   // everyone's share of this chunk has landed, and everyone is done with the chunk before
         if (kc + kGmStages - 1 < chunks) fetch(kc + kGmStages - 1);
         asm volatile("cp.async.commit_group;" ::: "memory");
-        if (nt <= 0) continue;
         const uint8_t* st = smem + (kc % kGmStages) * kGmStage;
-        const uint8_t* sw = st + (wr + g) * kGmWStride;
+        const uint32_t* sw = reinterpret_cast<const uint32_t*>(st) + (wr + g) * 9;
         uint32_t w[2][2][8];      // [group of 16 rows][row g / g + 8][word]: this lane's crumbs, lowest two bits of every byte
         uint64_t dw[2][2][2];     // [group][row][block]: the weight scale, twice
 #pragma unroll
         for (int r = 0; r < 2; ++r)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const uint8_t* p = sw + (r * 16 + h * 8) * kGmWStride;
-                const uint4 v0 = *reinterpret_cast<const uint4*>(p), v1 = *reinterpret_cast<const uint4*>(p + 16);
-                const uint32_t v2 = *reinterpret_cast<const uint32_t*>(p + 32);
-                const float d0 = __half2float(__ushort_as_half(uint16_t(v0.x & 0xffffu))), d1 = __half2float(__ushort_as_half(uint16_t(v1.x >> 16)));
+                uint32_t v[9];    // {d, 16 code bytes}, {d, 16 code bytes}
+#pragma unroll
+                for (int i = 0; i < 9; ++i) v[i] = sw[(r * 16 + h * 8) * 9 + i];
+                const float d0 = __half2float(__ushort_as_half(uint16_t(v[0] & 0xffffu))), d1 = __half2float(__ushort_as_half(uint16_t(v[4] >> 16)));
                 dw[r][h][0] = pack2(d0, d0);
                 dw[r][h][1] = pack2(d1, d1);
-                w[r][h][0] = __funnelshift_r(v0.x, v0.y, 16);
-                w[r][h][1] = __funnelshift_r(v0.y, v0.z, 16);
-                w[r][h][2] = __funnelshift_r(v0.z, v0.w, 16);
-                w[r][h][3] = __funnelshift_r(v0.w, v1.x, 16);
-                w[r][h][4] = v1.y;
-                w[r][h][5] = v1.z;
-                w[r][h][6] = v1.w;
-                w[r][h][7] = v2;
 #pragma unroll
-                for (int i = 0; i < 8; ++i) w[r][h][i] = (w[r][h][i] >> (2 * t4)) & 0x03030303u;
+                for (int i = 0; i < 4; ++i) {
+                    w[r][h][i] = __funnelshift_r(v[i], v[i + 1], 16);
+                    w[r][h][4 + i] = v[5 + i];
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) w[r][h][i] = (((w[r][h][i] >> (2 * t4)) & 0x03030303u) + 0x7f7f7f7fu) ^ 0x80808080u;   // code - 1 in every byte
             }
-        const uint8_t* sb = st + kGmBytesW + (wt >> 3) * 512 + lane * 16;
-        const uint8_t* sa = st + kGmBytesW + kGmBytesB + ((wt >> 1) + t4) * 16;
-        const uint8_t* sc = st + kGmBytesW + kGmBytesB + kGmBytesA + ((wt >> 1) + t4) * 32;
+        const uint8_t* sb = st + kGmBytesW + lane * 16;
+        const uint8_t* sa = st + kGmBytesW + kGmBytesB + t4 * 16;
 #pragma unroll
         for (int b = 0; b < 2; ++b)
 #pragma unroll
-            for (int n = 0; n < 4; ++n) {
-                if (n >= nt) break;
-                const uint4 bf = *reinterpret_cast<const uint4*>(sb + b * (kGmTok * 64) + n * 512);
-                const ulonglong2 d8 = *reinterpret_cast<const ulonglong2*>(sa + b * (kGmTok / 2 * 16) + n * 64);
-                const int4 c0 = *reinterpret_cast<const int4*>(sc + b * (kGmTok / 2 * 32) + n * 128), c1 = *reinterpret_cast<const int4*>(sc + b * (kGmTok / 2 * 32) + n * 128 + 16);
+            for (int np = 0; np < 8; np += 2) {   // two columns at a time, so that one's loads and products run beside the other's
+                if (np >= nt) break;               // (the second may be one that nothing fetched: it is not stored)
 #pragma unroll
-                for (int r = 0; r < 2; ++r) {
-                    uint64_t lo0, hi0, lo1, hi1;
-                    mma_u8s8_c4(lo0, hi0, w[r][0][4 * b], w[r][1][4 * b], w[r][0][4 * b + 1], w[r][1][4 * b + 1], bf.x, bf.y, c0);
-                    mma_u8s8_c4(lo1, hi1, w[r][0][4 * b + 2], w[r][1][4 * b + 2], w[r][0][4 * b + 3], w[r][1][4 * b + 3], bf.z, bf.w, c1);
-                    // acc += d2 * (d8[0] * sum0 + d8[1] * sum1)
-                    const uint64_t u_lo = fma2(d8.y, sub2(lo1, magic), mul2(d8.x, sub2(lo0, magic)));
-                    const uint64_t u_hi = fma2(d8.y, sub2(hi1, magic), mul2(d8.x, sub2(hi0, magic)));
-                    acc[r][n][0] = fma2(dw[r][0][b], u_lo, acc[r][n][0]);
-                    acc[r][n][1] = fma2(dw[r][1][b], u_hi, acc[r][n][1]);
+                for (int n = np; n < np + 2; ++n) {
+                    const uint4 bf = *reinterpret_cast<const uint4*>(sb + b * (kGmTok * 64) + n * 512);
+                    const ulonglong2 d8 = *reinterpret_cast<const ulonglong2*>(sa + b * (kGmTok / 2 * 16) + n * 64);
+                    const uint64_t md = mul2(d8.x, neg_magic);   // exact (two bits times eleven): d * sum in one rounding either way
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        uint64_t lo0, hi0, lo1, hi1;
+                        mma_s8s8_c4(lo0, hi0, w[r][0][4 * b], w[r][1][4 * b], w[r][0][4 * b + 1], w[r][1][4 * b + 1], bf.x, bf.y, start);
+                        mma_s8s8_c4(lo1, hi1, w[r][0][4 * b + 2], w[r][1][4 * b + 2], w[r][0][4 * b + 3], w[r][1][4 * b + 3], bf.z, bf.w, start);
+                        // acc += d2 * (d8[0] * sum0 + d8[1] * sum1)
+                        const uint64_t u_lo = fma2(d8.y, sub2(lo1, magic), fma2(lo0, d8.x, md));
+                        const uint64_t u_hi = fma2(d8.y, sub2(hi1, magic), fma2(hi0, d8.x, md));
+                        acc[r][n][0] = fma2(dw[r][0][b], u_lo, acc[r][n][0]);
+                        acc[r][n][1] = fma2(dw[r][1][b], u_hi, acc[r][n][1]);
+                    }
                 }
             }
     }
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
+    for (int n = 0; n < 8; ++n) {
         if (n >= nt) break;
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-            const int tok = wt + n * 8 + 2 * t4 + k;
+            const int tok = n * 8 + 2 * t4 + k;
             if (tok >= m) continue;
             float* o = a.dst + size_t(s_slot[tok]) * a.nrows + r0;
 #pragma unroll
@@ -758,7 +755,7 @@ __global__ void __launch_bounds__(kGmThreads, 2) k_gm_mma(const GmArgs a) {
 
 // ---- grouped plan in a workspace
 struct PlanLayout {
-    size_t status, chunk_cnt, bounds, item_off, perm, act_q, act_d, act_c, total;
+    size_t status, chunk_cnt, bounds, item_off, perm, act_q, act_d, total;
     int n_chunks, max_items;
 };
 PlanLayout plan_layout(int64_t ncols, int64_t rows, int E) {
@@ -778,13 +775,12 @@ PlanLayout plan_layout(int64_t ncols, int64_t rows, int E) {
     L.perm = take(size_t(rows) * 4);
     L.act_q = take(size_t(rows) * ncols);
     L.act_d = take(size_t(rows) * (ncols / kQ8) * 4);
-    L.act_c = take(size_t(rows) * (ncols / kQ8) * 4);
     L.total = off;
     return L;
 }
 constexpr int kPlanMaxExperts = 4096;
 GmAct plan_act(uint8_t* base, const PlanLayout& L) {
-    return GmAct{reinterpret_cast<int8_t*>(base + L.act_q), reinterpret_cast<float*>(base + L.act_d), reinterpret_cast<int32_t*>(base + L.act_c)};
+    return GmAct{reinterpret_cast<int8_t*>(base + L.act_q), reinterpret_cast<float*>(base + L.act_d)};
 }
 
 }  // namespace
@@ -809,7 +805,7 @@ int frx_gemv_quantize_q8_1(const float* x, int64_t ncols, int n_tok, void* xq, f
     if (n_tok == 0) return FRX_OK;
     if (!x || !xq || uintptr_t(xq) % 4) return fail(FRX_ERR_ARG, "gemv::quantize_q8_1: null or misaligned pointer");
     const int64_t padded = padded_cols(ncols);
-    FRX_LAUNCH(kKQuant, stream, k_q8_1<<<dim3(unsigned(padded / 256), unsigned(n_tok)), 256, 0, stream>>>(x, nullptr, ncols, padded, static_cast<uint8_t*>(xq)));
+    FRX_LAUNCH(kKQuant, stream, launch_pdl(k_q8_1, dim3(unsigned(padded / 256), unsigned(n_tok)), dim3(256), 0, stream, x, static_cast<const float*>(nullptr), ncols, padded, static_cast<uint8_t*>(xq)));
     FRX_CUDA(cudaGetLastError());
     return FRX_OK;
 }
@@ -819,7 +815,7 @@ int frx_gemv_swiglu_q8_1(const float* g, const float* u, int64_t ncols, int n_to
     if (n_tok == 0) return FRX_OK;
     if (!g || !u || !xq || uintptr_t(xq) % 4) return fail(FRX_ERR_ARG, "gemv::swiglu_q8_1: null or misaligned pointer");
     const int64_t padded = padded_cols(ncols);
-    FRX_LAUNCH(kKQuant, stream, k_q8_1<<<dim3(unsigned(padded / 256), unsigned(n_tok)), 256, 0, stream>>>(g, u, ncols, padded, static_cast<uint8_t*>(xq)));
+    FRX_LAUNCH(kKQuant, stream, launch_pdl(k_q8_1, dim3(unsigned(padded / 256), unsigned(n_tok)), dim3(256), 0, stream, g, u, ncols, padded, static_cast<uint8_t*>(xq)));
     FRX_CUDA(cudaGetLastError());
     return FRX_OK;
 }
@@ -844,9 +840,9 @@ int frx_gemv_moe_q(uint32_t ggml_type, const void* w, const void* gate, const vo
     a.n_jobs = n_tok * k;
     a.act_div = act_per_expert ? 1 : k;
     if (gate)
-        FRX_LAUNCH(kKGateUp, stream, { if (int rc = launch_dot<1, true>(a, a.n_jobs, stream)) return rc; });
+        FRX_LAUNCH(kKGateUp, stream, { if (int rc = launch_dot<true>(a, a.n_jobs, stream)) return rc; });
     else
-        FRX_LAUNCH(kKDown, stream, { if (int rc = launch_dot<1, false>(a, a.n_jobs, stream)) return rc; });
+        FRX_LAUNCH(kKDown, stream, { if (int rc = launch_dot<false>(a, a.n_jobs, stream)) return rc; });
     return FRX_OK;
 }
 
@@ -870,9 +866,9 @@ int frx_gemv_moe_q2_0(const void* w, const void* gate, const void* xq, const int
     a.n_jobs = n_ids;
     a.act_div = per_channel_act ? 1 : n_ids;   // one activation row for every channel, or one each
     if (gate)
-        FRX_LAUNCH(kKGateUp, stream, { if (int rc = launch_dot<1, true>(a, a.n_jobs, stream)) return rc; });
+        FRX_LAUNCH(kKGateUp, stream, { if (int rc = launch_dot<true>(a, a.n_jobs, stream)) return rc; });
     else
-        FRX_LAUNCH(kKDown, stream, { if (int rc = launch_dot<1, false>(a, a.n_jobs, stream)) return rc; });
+        FRX_LAUNCH(kKDown, stream, { if (int rc = launch_dot<false>(a, a.n_jobs, stream)) return rc; });
     return FRX_OK;
 }
 
@@ -891,7 +887,7 @@ int frx_gemv_matvec_q(uint32_t ggml_type, const void* W, const void* xq, float* 
     a.nrows = int(nrows);
     a.n_jobs = n_tok;
     a.act_div = 1;
-    FRX_LAUNCH(kKDown, stream, { if (int rc = launch_dot<1, false>(a, a.n_jobs, stream)) return rc; });
+    FRX_LAUNCH(kKDown, stream, { if (int rc = launch_dot<false>(a, a.n_jobs, stream)) return rc; });
     return FRX_OK;
 }
 
@@ -936,7 +932,7 @@ int frx_gemm_moe_prepare(frx_gemm_moe_plan* plan, uint32_t ggml_type, int n_expe
     const int S = int(rows), E = n_experts;
     // one row of codes per token, or per (token, expert) slot when every slot has its own activations
     const size_t n_quads = size_t(x_per_slot ? rows : T) * size_t(ncols / 4);
-    FRX_LAUNCH(kKQuant, stream, k_gm_quant<<<unsigned((n_quads + 255) / 256), 256, 0, stream>>>(x, int(ncols), n_quads, plan_act(base, L)));
+    FRX_LAUNCH(kKQuant, stream, launch_pdl(k_gm_quant, dim3(unsigned((n_quads + 255) / 256)), dim3(256), 0, stream, x, int(ncols), n_quads, plan_act(base, L)));
     FRX_LAUNCH(kKGroup, stream, launch_pdl(k_pf_hist, dim3(L.n_chunks), dim3(256), size_t(E) * 4, stream, ids, S, E, chunk_cnt, status, (const int32_t*)nullptr, 0));
     FRX_LAUNCH(kKGroup, stream, launch_pdl(k_pf_scan, dim3(1), dim3(1024), 0, stream, chunk_cnt, L.n_chunks, E, bounds, item_off, status, L.max_items, kGmTok, TokenBlocks{}));
     FRX_LAUNCH(kKGroup, stream, launch_pdl(k_pf_place, dim3(L.n_chunks), dim3(kChunkSlots), pf_place_smem(E), stream, ids, S, E, (const int*)chunk_cnt, (const int*)bounds, perm,
@@ -975,7 +971,7 @@ int frx_gemm_moe_run(const frx_gemm_moe_plan* plan, const void* W, int64_t exper
     a.K = plan->K;
     a.x_per_slot = plan->x_per_slot;
     const dim3 grid(unsigned(L.max_items), unsigned((nrows + kGmRows - 1) / kGmRows));
-    FRX_LAUNCH(kKDown, stream, k_gm_mma<<<grid, kGmThreads, kGmSmem, stream>>>(a));
+    FRX_LAUNCH(kKDown, stream, launch_pdl(k_gm_mma, grid, dim3(kGmThreads), size_t(kGmSmem), stream, a));
     FRX_CUDA(cudaGetLastError());
     return FRX_OK;
 }
