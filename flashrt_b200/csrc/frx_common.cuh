@@ -448,7 +448,9 @@ __device__ __forceinline__ float round_half_away(float v) {
 __device__ __forceinline__ float expf_cr(float x) {
     if (!(x == x)) return x;
     const double xd = double(fminf(fmaxf(x, -110.0f), 90.0f));   // beyond: 0 or inf as a float either way
-    const double kd = rint(xd * 1.4426950408889634);
+    // rounded to an integer by adding and subtracting 1.5 * 2^52, which leaves it in the low word too: the conversions
+    // (rint, double to int) run at a quarter of this rate or less
+    const double km = __dadd_rn(__dmul_rn(xd, 1.4426950408889634), 6755399441055744.0), kd = __dsub_rn(km, 6755399441055744.0);
     double r = fma(-kd, 0x1.62e42fee00000p-1, xd);
     r = fma(-kd, 0x1.a39ef35793c76p-33, r);
     double p = 1.0 / 6227020800.0;
@@ -465,7 +467,7 @@ __device__ __forceinline__ float expf_cr(float x) {
     p = fma(p, r, 0.5);
     p = fma(p, r, 1.0);
     p = fma(p, r, 1.0);
-    const double scale = __hiloint2double((__double2int_rn(kd) + 1023) << 20, 0);   // 2^k, k in [-159, 130]
+    const double scale = __hiloint2double((__double2loint(km) + 1023) << 20, 0);   // 2^k, k in [-159, 130]
     return __double2float_rn(p * scale);
 }
 

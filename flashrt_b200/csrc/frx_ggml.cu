@@ -529,7 +529,7 @@ __global__ void __launch_bounds__(kRqThreads, 6) k_q8_0_to_q2_0(const uint8_t* _
 // What bounds it: issue slots (a 16 x 8 x 64 tile costs two MMAs and eight packed fp32 operations of two slots) and what
 // shared memory delivers, about even. 1,000 tokens x 8 of 128 experts of 2560 x 640, per product: 157 us with two warps
 // side by side over the slots (each unpacking the rows, half of them idle behind a short item) and the copies' addresses
-// computed anew, 118 us now (0.24 ms less over the three products of a prompt).
+// computed anew, 118 us now.
 constexpr int kGmRows = 128, kGmTok = 64, kGmK = 128, kGmStages = 4, kGmThreads = 128;
 constexpr int kGmBytesW = kGmRows * 36;
 constexpr int kGmBytesB = kGmTok * kGmK;                     // [block][8 slots][lane] 16 bytes
