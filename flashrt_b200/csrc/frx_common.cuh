@@ -116,6 +116,14 @@ __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// its two halves, for work between them
+__device__ __forceinline__ void cluster_arrive_all() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait_all() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// a word of another block's shared memory, at this block's address for it (once that block is known to run)
+__device__ __forceinline__ void st_cluster(uint32_t addr, int rank, int v) {
+    asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, %1;\n\tst.shared::cluster.s32 [ra], %2;\n\t}" ::"r"(addr), "r"(rank), "r"(v) : "memory");
+}
+
 // Device-side error codes written to a workspace's status word.
 enum : int {
     kDevOk = 0,

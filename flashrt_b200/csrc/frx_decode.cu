@@ -91,6 +91,8 @@ Layout make_layout(int T, int K, int n, int ff) {
 // block b takes the tasks [ranges[b], ranges[b + 1]) (numbered item * tasks_per_expert + task),
 // boundaries placed so that every block gets the same weight, a task of a small item weighing 16
 // and one of a larger item `heavy`. dyn then has max_items more ints.
+// The three results (items, order, split) do not depend on each other; three blocks make one each.
+enum { kPartItems = 0, kPartSplit = 1, kPartOrder = 2, kGroupParts = 3 };
 struct DownSplit {
     int* ranges;            // [blocks + 1], or null: no split is written
     int blocks;             // blocks of the down kernel
@@ -101,8 +103,8 @@ struct DownSplit {
 __device__ __forceinline__ void group_block(unsigned long long* dyn, const int32_t* __restrict__ ids, int T, int K, int E, int e_lo,
                                             int e_hi, const uint8_t* __restrict__ experts, size_t stride,
                                             const uint8_t* __restrict__ shared, Item* __restrict__ items, int* __restrict__ status,
-                                            int32_t* __restrict__ order, int max_items, int tpi, bool zero_counters = false,
-                                            DownSplit split = DownSplit{nullptr, 0, 0, 16, 0}, int sh_lo = 0, int sh_hi = 1 << 30) {
+                                            int32_t* __restrict__ order, int max_items, int tpi, DownSplit split, int sh_lo, int sh_hi,
+                                            int part, bool have_ids) {
     // the shared expert is applied to tokens [sh_lo, sh_hi) (all of them unless the caller deals them among ranks)
     sh_lo = max(sh_lo, 0);
     sh_hi = max(min(sh_hi, T), sh_lo);
@@ -111,19 +113,39 @@ __device__ __forceinline__ void group_block(unsigned long long* dyn, const int32
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int32_t* sid = reinterpret_cast<int32_t*>(mask + E);   // the ids, read many times below
     int* wgt = sid + T * K;                                // with `split`: weight of a task of every item, then their running sums
-    if (tid == 0 && status[3] != kCookie) {   // first use of this workspace
+    if (part == kPartItems && tid == 0 && status[3] != kCookie) {   // first use of this workspace
         status[0] = kDevOk;
         status[2] = 0;
         status[3] = kCookie;
     }
+    if (part == kPartOrder) {
+        if (!have_ids) {
+            for (int s = tid; s < T * K; s += 1024) sid[s] = ids[s];
+            __syncthreads();
+        }
+        // Slots of a token by ascending expert id: slot s takes the place given by the number of the
+        // token's slots that come before it (smaller id, or the same id and a smaller k).
+        for (int s = tid; s < T * K; s += 1024) {
+            const int t = s / K, k = s - t * K, e = sid[s];
+            int rank = 0;
+            for (int j = 0; j < K; ++j) {
+                const int ej = sid[t * K + j];
+                rank += (ej < e || (ej == e && j < k)) ? 1 : 0;
+            }
+            order[t * K + rank] = (e < e_lo || e >= e_hi) ? -1 - s : s;   // slots of experts held elsewhere take no part in this rank's sum
+        }
+        return;
+    }
     for (int e = tid; e < E; e += 1024) mask[e] = 0ull;
     __syncthreads();
     for (int s = tid; s < T * K; s += 1024) {
-        const int e = ids[s];
-        sid[s] = e;
+        const int e = have_ids ? sid[s] : ids[s];
+        if (!have_ids) sid[s] = e;
         if (e < 0 || e >= E) {
-            status[0] = kDevBadExpertId;
-            status[2] = s;
+            if (part == kPartItems) {
+                status[0] = kDevBadExpertId;
+                status[2] = s;
+            }
         } else if (e >= e_lo && e < e_hi) {   // expert parallel: only the experts held here
             atomicOr(&mask[e], 1ull << (s / K));
         }
@@ -162,7 +184,7 @@ __device__ __forceinline__ void group_block(unsigned long long* dyn, const int32
     const int routed_items = warp_tot[31] & kCntMask, routed_weight = warp_tot[31] >> kCntBits;
     const int shared_items = shared ? (sh_hi - sh_lo + tpi - 1) / tpi : 0;
     if (routed_items + shared_items > max_items) {
-        if (tid == 0) {
+        if (part == kPartItems && tid == 0) {
             status[0] = kDevTooManyItems;
             status[1] = 0;
         }
@@ -192,6 +214,10 @@ __device__ __forceinline__ void group_block(unsigned long long* dyn, const int32
         const unsigned long long mk = mask[e];
         const int idx = __popcll(mk & ((1ull << t) - 1ull)), pc = __popcll(mk);
         const int j = idx / tpi, pos = idx - j * tpi, eb = ebase[e];
+        if (part == kPartSplit) {
+            if (pos == 0) wgt[(eb & kCntMask) + j] = (eb >> kCntBits) + j * weight_of(tpi);   // the expert's items in front are full
+            continue;
+        }
         Item* it = items_s + (eb & kCntMask) + j;
         it->slot[pos] = s;
         if (pos == 0) {
@@ -200,40 +226,29 @@ __device__ __forceinline__ void group_block(unsigned long long* dyn, const int32
             it->n_tok = m;
             it->expert = e;
             for (int z = m; z < kTokPerItem; ++z) it->slot[z] = 0;
-            if (split.ranges) wgt[(eb & kCntMask) + j] = (eb >> kCntBits) + j * weight_of(tpi);   // the expert's items in front are full
         }
     }
-    if (tid < shared_items) {
+    if (part == kPartSplit) {
+        if (tid < shared_items) wgt[routed_items + tid] = routed_weight + tid * weight_of(tpi);   // (all but the last shared item are full)
+    } else if (tid < shared_items) {
         Item it;
         it.blob = shared;
         it.expert = -1;
         const int t0 = sh_lo + tid * tpi, m = min(tpi, sh_hi - t0);
         it.n_tok = m;
         for (int j = 0; j < kTokPerItem; ++j) it.slot[j] = j < m ? T * K + t0 + j : 0;
-        if (split.ranges) wgt[routed_items + tid] = routed_weight + tid * weight_of(tpi);   // (all but the last shared item are full)
         items_s[routed_items + tid] = it;
     }
     __syncthreads();
-    for (int i = tid; i < (routed_items + shared_items) * int(sizeof(Item) / 16); i += 1024)
-        reinterpret_cast<uint4*>(items)[i] = reinterpret_cast<const uint4*>(items_s)[i];
-    if (tid == 0) status[1] = routed_items + shared_items;
-    if (zero_counters)
+    if (part == kPartItems) {
+        for (int i = tid; i < (routed_items + shared_items) * int(sizeof(Item) / 16); i += 1024)
+            reinterpret_cast<uint4*>(items)[i] = reinterpret_cast<const uint4*>(items_s)[i];
+        if (tid == 0) status[1] = routed_items + shared_items;
         for (int i = tid; i < routed_items + shared_items; i += 1024) status[kStatusWords + i] = 0;
-    // Slots of a token by ascending expert id: slot s takes the place given by the number of the
-    // token's slots that come before it (smaller id, or the same id and a smaller k).
-    for (int s = tid; s < T * K; s += 1024) {
-        const int t = s / K, k = s - t * K, e = sid[s];
-        int rank = 0;
-        for (int j = 0; j < K; ++j) {
-            const int ej = sid[t * K + j];
-            rank += (ej < e || (ej == e && j < k)) ? 1 : 0;
-        }
-        order[t * K + rank] = (e < e_lo || e >= e_hi) ? -1 - s : s;   // slots of experts held elsewhere take no part in this rank's sum
+        return;
     }
-    if (!split.ranges) return;
     // every boundary by bisection over the running weights
     const int n_items = routed_items + shared_items;
-    __syncthreads();
     if (tid <= split.blocks && n_items > 0) {
         const int tpe = split.tasks_per_expert;
         const int last_w = shared_items ? weight_of(min(tpi, sh_hi - sh_lo - (shared_items - 1) * tpi)) : 0;
@@ -260,11 +275,14 @@ __device__ __forceinline__ void group_block(unsigned long long* dyn, const int32
     }
 }
 
-// The head of a decode step, one launch of clusters of kHeadCluster blocks. Cluster 0 routes the
-// tokens (when given the router's logits; token t by warp t / kHeadCluster of block
-// t % kHeadCluster), meets at the cluster's hardware barrier, and its block 0 groups the tokens
-// into work items. All other blocks quantize x into the expert kernel's activation form; the two
-// halves do not depend on each other.
+// The head of a decode step, one launch of clusters of kHeadCluster blocks. In cluster 0 blocks kGroupParts and up route
+// the tokens (when given the router's logits), a warp each, and put the experts they choose straight into the shared
+// memory of blocks 0 .. kGroupParts - 1, which then make the work items, down's split and the order of summation (see
+// group_block); the weights follow while those work. All other blocks quantize x into the expert kernel's activation form;
+// the two halves do not depend on each other.
+// Bound: a chain of latencies. us from the end of the kernel in front to the last result, 16 / 64 tokens: 9.8 / 11.8 when
+// one block made all three from ids in global memory after the weights, 8.5 / 11.5 now (8 tokens of 512 / 256: 32.0 -> 30.0
+// us per layer).
 constexpr int kHeadCluster = 8;
 template <int V>   // router: logits per lane, E <= 32 * V; 0: no router
 __global__ void __launch_bounds__(1024) k_prologue(const float* __restrict__ logits, int32_t* __restrict__ ids, float* __restrict__ wts,
@@ -294,6 +312,7 @@ __global__ void __launch_bounds__(1024) k_prologue(const float* __restrict__ log
             touch_l2(xc);
         }
     }
+    if (V > 0 && blockIdx.x < kHeadCluster) cluster_sync_all();   // every block of the cluster runs: its shared memory may be written
     pdl_wait();
     pdl_trigger();
     if (stamps && blockIdx.x == 0 && threadIdx.x == 0) stamps[0] = global_ns();   // the kernels in front have ended
@@ -303,15 +322,44 @@ __global__ void __launch_bounds__(1024) k_prologue(const float* __restrict__ log
         for (size_t quad = qb * 1024 + threadIdx.x; quad < n_blocks * 8; quad += nqb * 1024) quant_frag_quad(x, n, quad, true, xq, xa, xc);
         return;
     }
-    const int rank = int(cluster_ctarank());   // cluster 0 is blocks 0 .. kHeadCluster - 1
-    if constexpr (V > 0) {
-        for (int t = warp * kHeadCluster + rank; t < T; t += 32 * kHeadCluster)
-            route_warp<V>(logits + size_t(t) * E, E, K, lane, ids + size_t(t) * K, wts + size_t(t) * K, nullptr, nullptr);
+    const int rank = blockIdx.x;   // cluster 0 is blocks 0 .. kHeadCluster - 1
+    if (rank >= kGroupParts) {
+        if constexpr (V > 0) {
+            static_assert(kMaxChunkTokens <= 32 * (kHeadCluster - kGroupParts), "a warp per token");
+            const int t = warp * (kHeadCluster - kGroupParts) + rank - kGroupParts;
+            const float* l = logits + size_t(t) * E;
+            const bool vec = t < T && route_vec<V>(l, E);
+            uint32_t key[V], my_key = 0;
+            int my_id = 0;
+            float m = 0.0f;
+            if (t < T) {
+                route_load<V>(l, E, lane, vec, key);
+                route_select<V>(key, vec, K, lane, my_key, my_id, m);
+                if (lane < K) {
+                    const uint32_t sid = smem_u32(dyn) + E * 8 + (t * K + lane) * 4;   // see group_block
+#pragma unroll
+                    for (int r = 0; r < kGroupParts; ++r) st_cluster(sid, r, my_id);
+                }
+                __syncwarp();
+            }
+            cluster_arrive_all();   // the ids are in place
+            if (t < T) {
+                route_load<V>(l, E, lane, vec, key);   // (again: the selection used them up)
+                const float w = route_weight(my_key, m, route_sum<V>(key, m), K, lane);
+                if (lane < K) {
+                    ids[size_t(t) * K + lane] = my_id;
+                    wts[size_t(t) * K + lane] = w;
+                }
+            }
+            __syncwarp();
+            cluster_wait_all();
+        }
+        return;
     }
-    if (stamps && blockIdx.x == 0 && threadIdx.x == 0) stamps[1] = global_ns();   // block 0's tokens are routed
-    cluster_sync_all();   // every block's ids are visible to block 0
-    if (stamps && blockIdx.x == 0 && threadIdx.x == 0) stamps[2] = global_ns();   // all tokens are routed
-    if (rank == 0) group_block(dyn, ids, T, K, E, e_lo, e_hi, experts, stride, shared, items, status, order, max_items, tpi, true, split, sh_lo, sh_hi);
+    if constexpr (V > 0) cluster_sync_all();   // the ids of all tokens are here
+    if (stamps && blockIdx.x == 0 && threadIdx.x == 0) stamps[1] = stamps[2] = global_ns();   // all tokens are routed
+    if (rank != kPartSplit || split.ranges)
+        group_block(dyn, ids, T, K, E, e_lo, e_hi, experts, stride, shared, items, status, order, max_items, tpi, split, sh_lo, sh_hi, rank, V > 0);
     if (stamps && blockIdx.x == 0) {
         __syncthreads();
         if (threadIdx.x == 0) stamps[3] = global_ns();   // the work items are written

@@ -25,12 +25,12 @@ __device__ __forceinline__ float key_value(uint32_t k) { return __uint_as_float(
 // holds experts 128 q + 4 L .. + 3 for q = 0 .. V / 4 - 1 (V / 4 vector loads, all in flight at
 // once); otherwise experts 32 i + L. Either way a lane's slots are in ascending expert order, which
 // the tie rule (lowest index wins) relies on.
-template <int V>   // logits per lane: E <= 32 * V
-__device__ __forceinline__ void route_warp(const float* __restrict__ l, int E, int K, int lane, int32_t* __restrict__ ids_t,
-                                           float* __restrict__ wts_t, uint32_t* counts, uint32_t* tail) {
-    const bool vec = (V % 4 == 0) && E == 32 * V && (reinterpret_cast<uintptr_t>(l) & 15) == 0;
-    auto slot_expert = [&](int i) { return vec ? 128 * (i >> 2) + 4 * lane + (i & 3) : 32 * i + lane; };
-    uint32_t key[V];
+// The expert of a lane's i-th logit: whole vectors when the row is aligned and full, else stride 32.
+template <int V>
+__device__ __forceinline__ bool route_vec(const float* l, int E) { return (V % 4 == 0) && E == 32 * V && (reinterpret_cast<uintptr_t>(l) & 15) == 0; }
+__device__ __forceinline__ int route_expert(bool vec, int lane, int i) { return vec ? 128 * (i >> 2) + 4 * lane + (i & 3) : 32 * i + lane; }
+template <int V>
+__device__ __forceinline__ void route_load(const float* __restrict__ l, int E, int lane, bool vec, uint32_t (&key)[V]) {
     if (vec) {
         float4 v[V / 4 > 0 ? V / 4 : 1];
 #pragma unroll
@@ -49,6 +49,25 @@ __device__ __forceinline__ void route_warp(const float* __restrict__ l, int E, i
             key[i] = e < E ? order_key(l[e] + 0.0f) : 0u;
         }
     }
+}
+
+// sum of exp(l - m) over the row, in double
+template <int V>
+__device__ __forceinline__ double route_sum(const uint32_t (&key)[V], float m) {
+    double part[4] = {0.0, 0.0, 0.0, 0.0};   // four running sums: the additions are slow and would otherwise form one chain
+#pragma unroll
+    for (int i = 0; i < V; ++i)
+        if (key[i] != 0u) part[i & 3] += double(expf(key_value(key[i]) - m));
+    double sum = (part[0] + part[1]) + (part[2] + part[3]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    return sum;
+}
+
+// Lane k gets the key and the expert of the k-th winner, all lanes the largest logit m. The keys of the winners become 0.
+template <int V>
+__device__ __forceinline__ void route_select(uint32_t (&key)[V], bool vec, int K, int lane, uint32_t& my_key, int& my_id, float& m) {
+    auto slot_expert = [&](int i) { return route_expert(vec, lane, i); };
     // every lane keeps its best and its second best key (with their experts): when its best is
     // taken, the second moves up without a rescan; the lane rescans only when it is hit again
     uint32_t best = 0, next = 0;
@@ -74,19 +93,10 @@ __device__ __forceinline__ void route_warp(const float* __restrict__ l, int E, i
     };
     rescan();
     bool next_valid = true;
-    const uint32_t kmax = __reduce_max_sync(0xffffffffu, best);
-    const float m = key_value(kmax);
-    double part[4] = {0.0, 0.0, 0.0, 0.0};   // four running sums: the additions are slow and would otherwise form one chain
-#pragma unroll
-    for (int i = 0; i < V; ++i)
-        if (key[i] != 0u) part[i & 3] += double(expf(key_value(key[i]) - m));
-    double sum = (part[0] + part[1]) + (part[2] + part[3]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-
+    m = key_value(__reduce_max_sync(0xffffffffu, best));
     // selection: K rounds on the integer keys only; lane k remembers the k-th winner
-    uint32_t my_key = 0;
-    int my_id = 0;
+    my_key = 0;
+    my_id = 0;
     for (int k = 0; k < K; ++k) {
         const uint32_t top = __reduce_max_sync(0xffffffffu, best);
         const int sel = __reduce_min_sync(0xffffffffu, best == top ? best_i : 0x7fffffff);
@@ -108,14 +118,34 @@ __device__ __forceinline__ void route_warp(const float* __restrict__ l, int E, i
             my_id = sel;
         }
     }
-    // probabilities of the winners, all lanes at once; their sum in selection order (lane order)
+}
+
+// probabilities of the winners, all lanes at once; their sum in selection order (lane order): lane k's weight
+__device__ __forceinline__ float route_weight(uint32_t my_key, float m, double sum, int K, int lane) {
     const float my_p = lane < K ? float(double(expf(key_value(my_key) - m)) / sum) : 0.0f;
     float wsum = 0.0f;
     for (int k = 0; k < K; ++k) wsum += __shfl_sync(0xffffffffu, my_p, k);
     wsum = fmaxf(wsum, 6.103515625e-5f);
+    return __fdiv_rn(my_p, wsum);
+}
+
+template <int V>   // logits per lane: E <= 32 * V
+__device__ __forceinline__ void route_warp(const float* __restrict__ l, int E, int K, int lane, int32_t* __restrict__ ids_t,
+                                           float* __restrict__ wts_t, uint32_t* counts, uint32_t* tail) {
+    const bool vec = route_vec<V>(l, E);
+    uint32_t key[V], my_key;
+    int my_id;
+    float m;
+    route_load<V>(l, E, lane, vec, key);
+    uint32_t top = 0;
+#pragma unroll
+    for (int i = 0; i < V; ++i) top = max(top, key[i]);
+    const double sum = route_sum<V>(key, key_value(__reduce_max_sync(0xffffffffu, top)));
+    route_select<V>(key, vec, K, lane, my_key, my_id, m);
+    const float w = route_weight(my_key, m, sum, K, lane);
     if (lane < K) {
         ids_t[lane] = my_id;
-        wts_t[lane] = __fdiv_rn(my_p, wsum);
+        wts_t[lane] = w;
         if (counts) atomicAdd(counts + my_id, 1u);
         if (tail) atomicAdd(tail + my_id, 1u);
     }
