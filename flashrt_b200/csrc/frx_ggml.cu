@@ -309,8 +309,9 @@ int check_dot_shape(const char* who, uint32_t type, int64_t ncols, int64_t nrows
 // units of 16384 above a sum of 8-bit magnitudes (both below 2^24 together), one half of the block at a time.
 // The bin follows from amax / |x|, good to 0.02 of a bin (the candidates are rounded to fp16: 2^-11 of 2.5 * 46 / 3 bins) and
 // settled by one exact comparison with the candidate it may just have missed.
-// What rounding remains (1.2e-6 X2 here, 66 * 2^-24 of the sum in the reference's order) decides nothing: candidates closer
-// to the best than that are summed again in the reference's order and compared as it does, about one block in a hundred.
+// What rounding remains (6 * 2^-24 X2 here: S1 rounds once, 2 S1 <= 4 X2 / d, then twice more; 66 * 2^-24 of the sum in the
+// reference's order) decides nothing: candidates closer to the best than twice that are summed again in the reference's
+// order and compared as it does.
 // Blocks whose candidates are not all normal fp16 numbers are summed so for all 24.
 //
 // In that sum a division is not needed: the values are d8 * q8 (exact, at most 18 significant bits), a candidate is an
@@ -321,18 +322,34 @@ int check_dot_shape(const char* who, uint32_t type, int64_t ncols, int64_t nrows
 // is exact. The codes of the chosen scale come from the same quotient enlarged by 2^-20, which takes it past a boundary
 // it lies on and past none that it does not.
 // Bound: issue slots, about 40 per value (six per value and candidate when each candidate was summed). 48 experts of
-// 2560 x 640 (236 M values): 1.35 ms with a sum per candidate, 0.65 ms so.
+// 2560 x 640 (236 M values): 1.35 ms with a sum per candidate, 0.51 ms so (0.62 with candidates divided one by one, wider bounds
+// and everything unrolled, which the instruction cache did not hold).
 constexpr int kRqThreads = 128, kRqCand = 24;
 constexpr float kRqCount = 16384.0f;   // a pass in a bin; the magnitudes of 32 values, twice each, stay below 8192
-constexpr uint32_t kRqRow = kRqThreads * 4;
+constexpr uint32_t kRqRow = kRqThreads * 4, kRqToBin = kRqCand * kRqRow;
+// candidate c is amax / div, div = 2.5f - 1.5f * float(c) / 23.0f, through fp16; and the correctly rounded 1 / div
+struct RqDiv {
+    float div[kRqCand], inv[kRqCand];
+    constexpr RqDiv() : div(), inv() {
+        for (int c = 0; c < kRqCand; ++c) {
+            div[c] = 2.5f - 1.5f * float(c) / 23.0f;
+            inv[c] = float(1.0 / double(div[c]));
+        }
+    }
+};
+__constant__ constexpr RqDiv kRqDiv;
 
 // the thread's own column of shared memory, by address (volatile: in program order)
+template <uint32_t OFF = 0>
 __device__ __forceinline__ float rq_load(uint32_t a) {
     float v;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+    asm volatile("ld.shared.f32 %0, [%1+%2];" : "=f"(v) : "r"(a), "n"(OFF));
     return v;
 }
-__device__ __forceinline__ void rq_store(uint32_t a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
+template <uint32_t OFF = 0>
+__device__ __forceinline__ void rq_store(uint32_t a, float v) {
+    asm volatile("st.shared.f32 [%0+%2], %1;" ::"r"(a), "f"(v), "n"(OFF) : "memory");
+}
 // word i (four values) of a block's half h: the 68 bytes are {d, 32 codes}, {d, 32 codes}
 __device__ __forceinline__ uint32_t rq_word(const uint32_t* w, int h, int i) { return h ? w[9 + i] : __funnelshift_r(w[i], w[i + 1], 16); }
 // value k of such a word as a float
@@ -360,8 +377,7 @@ __device__ __forceinline__ float rq_error(const uint32_t* w, float d_lo, float d
 __global__ void __launch_bounds__(kRqThreads, 6) k_q8_0_to_q2_0(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, size_t nblocks64) {
     __shared__ __align__(16) uint8_t in[kRqThreads * 68];
     __shared__ __align__(16) uint8_t out[kRqThreads * 18];
-    __shared__ float half_d[kRqCand * kRqThreads];        // [candidate][thread]: 0.5 d
-    __shared__ float bins[(kRqCand + 1) * kRqThreads];    // [candidates passed][thread]
+    __shared__ float half_d[(2 * kRqCand + 1) * kRqThreads];   // [candidate][thread]: 0.5 d; then the bins, [candidates passed][thread]
     const size_t b0 = size_t(blockIdx.x) * kRqThreads;
     const int tid = threadIdx.x, nb = int(min(size_t(kRqThreads), nblocks64 - b0));
     const uint8_t* s = src + b0 * 68;
@@ -394,23 +410,24 @@ __global__ void __launch_bounds__(kRqThreads, 6) k_q8_0_to_q2_0(const uint8_t* _
             sq[h] = q;
         }
         const float amax = fmaxf(fmaxf(0.0f, __fmul_rn(fabsf(d8[0]), mag[0])), __fmul_rn(fabsf(d8[1]), mag[1]));
-#pragma unroll
+        // the candidates. With 1 / div correctly rounded one residual makes amax * (1 / div) the correctly rounded quotient
+        // (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990), if nothing underflows.
+        const bool normal = amax >= 0x1p-12f && amax < 32768.0f && fabsf(d8[0]) < INFINITY && fabsf(d8[1]) < INFINITY;
+#pragma unroll 4
         for (int c = 0; c < kRqCand; ++c) {
-            // d = amax / (2.5f - 1.5f * float(c) / 23.0f), through fp16
-            const float div = __fsub_rn(2.5f, __fdiv_rn(__fmul_rn(1.5f, float(c)), 23.0f));
-            half_d[c * kRqThreads + tid] = 0.5f * __half2float(__float2half_rn(__fdiv_rn(amax, div)));
+            const float q = __fmul_rn(amax, kRqDiv.inv[c]), exact = __fmaf_rn(__fmaf_rn(-q, kRqDiv.div[c], amax), kRqDiv.inv[c], q);
+            half_d[c * kRqThreads + tid] = 0.5f * __half2float(__float2half_rn(normal ? exact : __fdiv_rn(amax, kRqDiv.div[c])));
         }
         uint32_t near_best = (1u << kRqCand) - 1;   // candidates that may have the smallest sum
-        if (amax >= 0x1p-12f && amax < 32768.0f && fabsf(d8[0]) < INFINITY && fabsf(d8[1]) < INFINITY) {
+        if (normal) {
             float first[kRqCand];   // suffix sums of the first half
-            const uint32_t cand0 = smem_u32(half_d) + tid * 4, bin0 = smem_u32(bins) + tid * 4;
-            const uint32_t base = cand0 - (0x4B000000u * kRqRow), to_bin = bin0 - cand0;
+            const uint32_t cand0 = smem_u32(half_d) + tid * 4, base = cand0 - (0x4B000000u * kRqRow);
             float best = 0.0f, x2 = 0.0f;
             float gain[kRqCand];    // d (2 S1 - d S2)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
 #pragma unroll
-                for (int c = 0; c <= kRqCand; ++c) rq_store(bin0 + c * kRqRow, 0.0f);
+                for (int c = 0; c <= kRqCand; ++c) rq_store<kRqToBin>(cand0 + c * kRqRow, 0.0f);
                 // candidates passed: floor((2.5 - amax / (2 |x|)) * 46 / 3 + 1); 0.03 less, so that the candidate to compare
                 // with is the next one, and rounded to nearest, so 0.5 less; in units of 23 for the clamp
                 const float c1 = __fdiv_rn(amax, -3.0f * fabsf(d8[h])), off = (2.5f * 46.0f / 3.0f + 0.47f) / 23.0f;
@@ -435,19 +452,19 @@ __global__ void __launch_bounds__(kRqThreads, 6) k_q8_0_to_q2_0(const uint8_t* _
                     }
 #pragma unroll
                     for (int k = 0; k < 8; ++k) {
-                        rq_store(a1[k] + to_bin, rq_load(a1[k] + to_bin) + one[k]);
-                        if (x[k] > 0.0f) rq_store(a3[k] + to_bin, rq_load(a3[k] + to_bin) + (one[k] + 2.0f * kRqCount));
+                        rq_store<kRqToBin>(a1[k], rq_load<kRqToBin>(a1[k]) + one[k]);
+                        if (x[k] > 0.0f) rq_store<kRqToBin>(a3[k], rq_load<kRqToBin>(a3[k]) + (one[k] + 2.0f * kRqCount));
                     }
                 }
                 float sum = 0.0f;
 #pragma unroll
                 for (int c = kRqCand - 1; c >= 0; --c) {
-                    sum += rq_load(bin0 + (c + 1) * kRqRow);   // exact: an integer below 2^24
+                    sum += rq_load<kRqToBin>(cand0 + (c + 1) * kRqRow);   // exact: an integer below 2^24
                     if (h == 0) {
                         first[c] = sum;
                     } else {
                         const float n0 = __fmaf_rn(first[c], 1.0f / kRqCount, kMagic) - kMagic, n1 = __fmaf_rn(sum, 1.0f / kRqCount, kMagic) - kMagic;
-                        const float s1 = __fmaf_rn(fabsf(d8[0]), __fmaf_rn(n0, -kRqCount, first[c]), fabsf(d8[1]) * __fmaf_rn(n1, -kRqCount, sum));
+                        const float s1 = __fmaf_rn(fabsf(d8[0]), __fmaf_rn(n0, -kRqCount, first[c]), fabsf(d8[1]) * __fmaf_rn(n1, -kRqCount, sum));   // (both products exact: 11 bits times 13)
                         const float d = 2.0f * rq_load(cand0 + c * kRqRow);
                         gain[c] = d * __fmaf_rn(-d, n0 + n1, 2.0f * s1);
                         best = fmaxf(best, gain[c]);
@@ -455,7 +472,7 @@ __global__ void __launch_bounds__(kRqThreads, 6) k_q8_0_to_q2_0(const uint8_t* _
                 }
                 x2 = __fmaf_rn(d8[h] * d8[h], float(sq[h]), x2);
             }
-            const float least = best - (3e-6f * x2 + 1e-5f * fmaxf(x2 - best, 0.0f));
+            const float least = best - (8e-7f * x2 + 8.2e-6f * fmaxf(x2 - best, 0.0f));
             near_best = 0;
 #pragma unroll
             for (int c = 0; c < kRqCand; ++c) near_best |= uint32_t(gain[c] >= least) << c;
@@ -480,9 +497,9 @@ __global__ void __launch_bounds__(kRqThreads, 6) k_q8_0_to_q2_0(const uint8_t* _
         o[0] = __half_as_ushort(__float2half_rn(best_d));
         if (best_d >= 0x1p-14f && best_d < INFINITY) {
             const float inv3 = __fdiv_rn(1.0f + 0x1p-20f, 3.0f * best_d);
-#pragma unroll
+#pragma unroll 2
             for (int k = 0; k < 8; ++k) {   // two bytes of four elements each
-                const float f = d8[k / 4] * inv3;
+                const float f = (k < 4 ? d8[0] : d8[1]) * inv3;
                 uint32_t v = 0;
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
@@ -498,7 +515,7 @@ __global__ void __launch_bounds__(kRqThreads, 6) k_q8_0_to_q2_0(const uint8_t* _
             for (int k = 0; k < 8; ++k) {
                 uint32_t v = 0;
                 for (int i = 0; i < 8; ++i) {
-                    const float xv = __fmul_rn(d8[k / 4], rq_value(rq_word(w, k / 4, (k % 4) * 2 + i / 4) ^ 0x80808080u, i % 4));
+                    const float xv = __fmul_rn(k < 4 ? d8[0] : d8[1], rq_value(rq_word(w, k / 4, (k % 4) * 2 + i / 4) ^ 0x80808080u, i % 4));
                     const int code = fin ? 1 + int(xv >= h1) + int(xv >= h3) - int(xv <= -h1) : 1;
                     v |= uint32_t(code) << (2 * i);
                 }
