@@ -12,14 +12,15 @@
 // after block.
 //
 // One block per SM works on tiles of 256 matrix rows x up to 48 tokens of one expert, in units of 128
-// weights of K. Warps: packed weights (bulk copies), activations and scales (bulk copies), two MMA
+// weights of K. Warps: packed weights (bulk copies), activations and scales (gathered), two MMA
 // issuers (one per row tile of 128), eight dequant warps (2-bit codes -> e4m3, written to tensor memory,
 // which spares shared memory the A operand's traffic: 48 KB per unit), sixteen epilogue warps. Tensor
 // memory: 384 columns of sums (two 64-blocks), 128 of weights. What bounds it: the fp32 pipe in
 // principle (four packed operations per two sums, 770 cycles per unit), in practice the issue slots
 // (5,400 warp instructions per unit, a packed operation taking two slots) and the hand-off of the two
 // sets of sums between the MMAs and the epilogue (about 600 cycles round trip). A unit takes 1,900
-// cycles. 16,384 tokens, 512 experts top-10, hidden 2048, width 512: gate/up 1,585 us, down 1,060 us; before, with
+// cycles. 16,384 tokens, 512 experts top-10, hidden 2048, width 512: gate/up 1,683 us, down 1,000 us (1,585 and 1,060
+// on activations that another kernel had gathered in 237); before, with
 // fp16 operands in shared memory, tiles of 128 x 128 and a hand-off per 64 weights: 2,520 and 1,620.
 #include "frx_umma.cuh"
 
