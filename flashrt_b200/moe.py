@@ -198,8 +198,8 @@ def moe_route_topk(logits: torch.Tensor, k: int, counts: torch.Tensor | None = N
     index) and weights float [T][k]."""
     _dev(logits, counts, tail_counts)
     T, E = logits.shape
-    ids = logits.new_empty((T, k), dtype=torch.int32)
-    wts = logits.new_empty((T, k), dtype=torch.float32)
+    ids = logits.new_empty(T, k, dtype=torch.int32)
+    wts = logits.new_empty(T, k, dtype=torch.float32)
     check(fast.route_topk(_raw_stream(stream), logits.data_ptr(), T, E, k, ids.data_ptr(), wts.data_ptr(), _addr(counts), _addr(tail_counts), tail_from))
     return ids, wts
 
@@ -212,8 +212,8 @@ def router_logits(w_router: torch.Tensor, w_gate: torch.Tensor | None, x: torch.
         raise FrxError(_l.ERR_ARG, "router_logits: bf16 weights and fp32 activations")
     T, n = x.shape
     E = w_router.shape[0]
-    logits = x.new_empty((T, E))
-    gate = x.new_empty((T,)) if w_gate is not None else None
+    logits = x.new_empty(T, E)
+    gate = x.new_empty(T) if w_gate is not None else None
     check(fast.router_logits(_raw_stream(stream), w_router.data_ptr(), _addr(w_gate), x.data_ptr(), T, E, n, logits.data_ptr(), _addr(gate)))
     return logits, gate
 
@@ -222,8 +222,8 @@ def quantize_q8(x: torch.Tensor, stream=None):
     """q2_0::quantize_q8 for every row of x [T][n]: codes int8 [T][n], scales float [T][n/32]."""
     _dev(x)
     T, n = x.shape
-    q = x.new_empty((T, n), dtype=torch.int8)
-    d = x.new_empty((T, n // Q8_BLOCK), dtype=torch.float32)
+    q = x.new_empty(T, n, dtype=torch.int8)
+    d = x.new_empty(T, n // Q8_BLOCK, dtype=torch.float32)
     check(fast.quantize_q8(_raw_stream(stream), x.data_ptr(), T, n, q.data_ptr(), d.data_ptr()))
     return q, d
 
@@ -416,7 +416,7 @@ def moe_combine(yh: torch.Tensor, w: torch.Tensor, hit_n: torch.Tensor | None, s
     _dev(yh, w, hit_n, shexp, gate, out)
     T, K, n = yh.shape
     if out is None:
-        out = yh.new_empty((T, n), dtype=torch.float32)
+        out = yh.new_empty(T, n, dtype=torch.float32)
     check(fast.moe_combine(out.data_ptr(), yh.data_ptr(), w.data_ptr(), _addr(hit_n), _addr(shexp), _addr(gate), n, K, T, _raw_stream(stream)))
     return out
 
@@ -479,7 +479,7 @@ class gemv:
     def quantize_q8_1(x: torch.Tensor, stream=None) -> torch.Tensor:
         _dev(x)
         n_tok, ncols = x.shape
-        xq = x.new_empty((gemv._q8_1_bytes(ncols, n_tok),), dtype=torch.uint8)
+        xq = x.new_empty(gemv._q8_1_bytes(ncols, n_tok), dtype=torch.uint8)
         check(fast.gemv_quantize_q8_1(x.data_ptr(), ncols, n_tok, xq.data_ptr(), _raw_stream(stream)))
         return xq
 
@@ -487,7 +487,7 @@ class gemv:
     def swiglu_q8_1(g: torch.Tensor, u: torch.Tensor, stream=None) -> torch.Tensor:
         _dev(g, u)
         n_tok, ncols = g.shape
-        xq = g.new_empty((gemv._q8_1_bytes(ncols, n_tok),), dtype=torch.uint8)
+        xq = g.new_empty(gemv._q8_1_bytes(ncols, n_tok), dtype=torch.uint8)
         check(fast.gemv_swiglu_q8_1(g.data_ptr(), u.data_ptr(), ncols, n_tok, xq.data_ptr(), _raw_stream(stream)))
         return xq
 
@@ -497,7 +497,7 @@ class gemv:
         """dst [n_tok][k][nrows] = W_{ids[t][j]} x (silu(G x) * (W x) with gate)."""
         _dev(w, gate, xq, ids)
         n_tok, k = ids.shape
-        dst = w.new_empty((n_tok, k, nrows), dtype=torch.float32)
+        dst = w.new_empty(n_tok, k, nrows, dtype=torch.float32)
         check(fast.gemv_moe_q(ggml_type, w.data_ptr(), _addr(gate), xq.data_ptr(), ids.data_ptr(), dst.data_ptr(), n_tok, k, ncols, nrows,
                               expert_stride_bytes, int(act_per_expert), _raw_stream(stream)))
         return dst
@@ -507,7 +507,7 @@ class gemv:
                  slot_stride_bytes: int, per_channel_act: bool, stream=None) -> torch.Tensor:
         _dev(w, gate, xq, ids)
         n_ids = ids.numel()
-        dst = w.new_empty((n_ids, nrows), dtype=torch.float32)
+        dst = w.new_empty(n_ids, nrows, dtype=torch.float32)
         check(fast.gemv_moe_q2_0(w.data_ptr(), _addr(gate), xq.data_ptr(), ids.data_ptr(), dst.data_ptr(), n_ids, ncols, nrows, slot_stride_bytes,
                                  int(per_channel_act), _raw_stream(stream)))
         return dst
@@ -516,8 +516,8 @@ class gemv:
     def matvec(ggml_type: int, W: torch.Tensor, x: torch.Tensor, nrows: int, stream=None) -> torch.Tensor:
         _dev(W, x)
         n_tok, ncols = x.shape
-        y = x.new_empty((n_tok, nrows), dtype=torch.float32)
-        scratch = x.new_empty((gemv._q8_1_bytes(ncols, n_tok),), dtype=torch.uint8)
+        y = x.new_empty(n_tok, nrows, dtype=torch.float32)
+        scratch = x.new_empty(gemv._q8_1_bytes(ncols, n_tok), dtype=torch.uint8)
         check(fast.gemv_matvec(ggml_type, W.data_ptr(), x.data_ptr(), y.data_ptr(), ncols, nrows, n_tok, scratch.data_ptr(), _raw_stream(stream)))
         return y
 
@@ -548,7 +548,7 @@ class gemm:
     @staticmethod
     def moe_run(plan: _GemmPlan, W: torch.Tensor, expert_stride_bytes: int, nrows: int, stream=None) -> torch.Tensor:
         _dev(W)
-        y = W.new_empty((plan.T, plan.K, nrows), dtype=torch.float32)
+        y = W.new_empty(plan.T, plan.K, nrows, dtype=torch.float32)
         check(fast.gemm_moe_run(C.addressof(plan), W.data_ptr(), expert_stride_bytes, y.data_ptr(), nrows, _raw_stream(stream)))
         return y
 
