@@ -433,25 +433,28 @@ __global__ void __maxnreg__(72) k_small_up(const SmallParams p) {
     // routing, so that their latency passes beside it
     const int cpr = p.n / 128, chunks = p.T * cpr;
     constexpr int kWarps = kUpThreads / 32, kAhead = 4;
-    const int w0 = p.T == 1 && VT > 0 ? 4 : 0, nw = kWarps - w0;   // (one token: the four warps that route it take no chunks)
+    // (one token: the four warps that route it take no chunks; while warp 0 groups alone it takes none)
+    const int w0 = p.T == 1 && VT > 0 ? 4 : p.T * p.K <= 32 ? 1 : 0, nw = kWarps - w0;
     const int c_first = warp >= w0 ? warp - w0 : chunks;
     float4 xv[kAhead];
     auto load_x = [&](int c0) {
 #pragma unroll
         for (int i = 0; i < kAhead; ++i) xv[i] = c0 + i * nw < chunks ? reinterpret_cast<const float4*>(p.x)[size_t(c0 + i * nw) * 32 + lane] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     };
-    auto quant_x = [&](int c0, const float4 (&v)[2]) {   // two chunks, nw apart, step by step together: each is one long dependent chain
-        float am[2], d[2], id[2];
-        int sum[2] = {0, 0};
-        uint32_t word[2] = {0u, 0u};
+    auto quant_x = [&](int c0, auto count) {   // chunks nw apart, step by step together: each is one long dependent chain
+        constexpr int N = decltype(count)::value;
+        const float4 (&v)[kAhead] = xv;
+        float am[N], d[N], id[N];
+        int sum[N] = {};
+        uint32_t word[N] = {};
 #pragma unroll
-        for (int k = 0; k < 2; ++k) am[k] = fmaxf(fmaxf(fabsf(v[k].x), fabsf(v[k].y)), fmaxf(fabsf(v[k].z), fabsf(v[k].w)));
+        for (int k = 0; k < N; ++k) am[k] = fmaxf(fmaxf(fabsf(v[k].x), fabsf(v[k].y)), fmaxf(fabsf(v[k].z), fabsf(v[k].w)));
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1)
 #pragma unroll
-            for (int k = 0; k < 2; ++k) am[k] = fmaxf(am[k], __shfl_xor_sync(0xffffffffu, am[k], o));
+            for (int k = 0; k < N; ++k) am[k] = fmaxf(am[k], __shfl_xor_sync(0xffffffffu, am[k], o));
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
+        for (int k = 0; k < N; ++k) {
             d[k] = __fdiv_rn(am[k], 127.0f);
             id[k] = d[k] != 0.0f ? __fdiv_rn(1.0f, d[k]) : 0.0f;
             const float hv[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
@@ -465,9 +468,9 @@ __global__ void __maxnreg__(72) k_small_up(const SmallParams p) {
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1)
 #pragma unroll
-            for (int k = 0; k < 2; ++k) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
+            for (int k = 0; k < N; ++k) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
+        for (int k = 0; k < N; ++k) {
             const int c = c0 + k * nw;
             if (c >= chunks) break;
             const int tok = c / cpr, q = (c - tok * cpr) * 32 + lane;   // quad of the row
@@ -491,9 +494,8 @@ __global__ void __maxnreg__(72) k_small_up(const SmallParams p) {
     small_plan<VT, kSmallGroups>(p, plan, reinterpret_cast<SmallRoute*>(smem + sm.terms), first, first, [&]() {
         for (int c0 = c_first; c0 < chunks; c0 += kAhead * nw) {
             if (c0 != c_first) load_x(c0);
-            const float4 a[2] = {xv[0], xv[1]}, b[2] = {xv[2], xv[3]};
-            quant_x(c0, a);
-            if (c0 + 2 * nw < chunks) quant_x(c0 + 2 * nw, b);
+            if (c0 + 2 * nw < chunks) quant_x(c0, std::integral_constant<int, kAhead>());
+            else quant_x(c0, std::integral_constant<int, 2>());
         }
     });
 
@@ -724,11 +726,7 @@ __global__ void __maxnreg__(72) k_small_down(const SmallParams p) {
         pdl_wait();
         mbar_spin(bar_h, 0u, abort, p.wait_ns);
         // ---------------- products: unit u of four items; lane (g, t4) finishes rows g, g + 8 of item t4
-        // (every warp walks all quads in order, so that it never waits for a later use of a slot than the next one)
-        int slot = 0, next = warp;   // next: this warp's next unit, counted over all quads
-        uint32_t phase = 0;
-        for (int q = 0; q < quads; ++q) {
-            mbar_spin(full + slot * 8, phase, abort, p.wait_ns);
+        auto quad = [&](int q, int slot, int next, int end) {   // units next, next + kDnProd, ... in front of `end`, counted over all quads
             const SmallItem& ib = plan.item[min(4 * q + (g >> 1), n_items - 1)];   // whose activations this lane brings
             const SmallItem& it = plan.item[min(4 * q + t4, n_items - 1)];         // whose rows it finishes
             const uint8_t* hb = smem + sm.hq + ib.slot[g & 1] * p.ff + t4 * 16;
@@ -737,7 +735,7 @@ __global__ void __maxnreg__(72) k_small_down(const SmallParams p) {
             const bool live = 4 * q + t4 < n_items, two = live && it.m > 1;
             float* o0 = terms + it.slot[0] * sm.tstride + g;
             float* o1 = terms + it.slot[1] * sm.tstride + g;
-            for (; next < (q + 1) * units; next += kDnProd) {
+            for (; next < end; next += kDnProd) {
                 const int u = next - q * units;
                 uint4 bf[2];
                 float4 v[2][2];
@@ -759,11 +757,27 @@ __global__ void __maxnreg__(72) k_small_down(const SmallParams p) {
                     }
                 });
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(empty + slot * 8);
-            if (++slot == p.ring) {
-                slot = 0;
-                phase ^= 1u;
+            return next;
+        };
+        int next = warp;
+        if (quads <= p.ring) {   // no slot is used twice: a warp goes from one of its units to the next
+            while (next < quads * units) {
+                const int q = next / units;
+                mbar_spin(full + q * 8, 0u, abort, p.wait_ns);
+                next = quad(q, q, next, (q + 1) * units);
+            }
+        } else {                 // every warp walks all quads in order, so that it never waits for a later use of a slot than the next one
+            int slot = 0;
+            uint32_t phase = 0;
+            for (int q = 0; q < quads; ++q) {
+                mbar_spin(full + slot * 8, phase, abort, p.wait_ns);
+                next = quad(q, slot, next, (q + 1) * units);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(empty + slot * 8);
+                if (++slot == p.ring) {
+                    slot = 0;
+                    phase ^= 1u;
+                }
             }
         }
     }
