@@ -1264,10 +1264,14 @@ int launch_small(SmallParams p, const SmallCfg& c, cudaStream_t stream) {
         }
     }
     p.wait_ns = wait_limit_ns();
+    // Two more warps for the quantization of x: with one token (126.5 -> 111.5 us for eight layers of 2048 / 512) and where the
+    // slots no longer fit one warp (6 tokens at 512 / 256: 22.5 -> 21.3 us per layer). With two or three tokens one warp groups
+    // meanwhile and they gain nothing (2560 / 640: 2 % slower).
+    const int up_threads = kUpThreads + (p.logits && (p.T == 1 || p.T * p.K > 32) ? kUpHelpers : 0);
     auto go = [&](auto k_up, auto k_down) {
         p.ring = kUpRing;
         p.tbufs = c.tbufs;
-        FRX_LAUNCH(kKGateUp, stream, launch_pdl(k_up, dim3(unsigned(sm_count())), dim3(kUpThreads), c.up, stream, p));
+        FRX_LAUNCH(kKGateUp, stream, launch_pdl(k_up, dim3(unsigned(sm_count())), dim3(unsigned(up_threads)), c.up, stream, p));
         p.ring = c.ring;
         FRX_LAUNCH(kKDown, stream, launch_pdl(k_down, dim3(unsigned(p.n / 16)), dim3(kDnThreads), c.down, stream, p));
     };

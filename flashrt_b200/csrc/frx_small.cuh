@@ -18,10 +18,12 @@
 constexpr int kSmallTok = 2;                          // tokens of an item
 constexpr int kSmallMaxT = 8, kSmallMaxSlots = 96;    // tokens, and routed slots
 constexpr int kUpProd = 8, kUpThreads = (kUpProd + 4 + 1) * 32;        // 8 warps of products, 4 of sums, 1 that fetches weights
+constexpr int kUpHelpers = 64;                        // threads that only quantize x: see launch_small
 constexpr int kUpBarThreads = (kUpProd + 4) * 32;
 constexpr int kDnProd = 12, kDnThreads = (kDnProd + 1) * 32;
 constexpr int kSmallGroups = 3;                       // tokens routed at a time, by four warps each
-// Registers: blocks of both kernels are to be resident side by side, 2 x 416 threads of at most 78. (16 warps of products and
+// Registers: blocks of both kernels are to be resident side by side, 480 + 416 threads of at most 72. (Two more warps of products
+// instead of the two that only quantize: 5 units of 16 on one scheduler instead of 4, 2 % slower at three tokens.) (16 warps of products and
 // 64 registers, with spills, were measured: 14.6 us per layer against 13.3 for one token, no gain for three.)
 
 struct SmallParams {
@@ -432,9 +434,10 @@ __global__ void __maxnreg__(72) k_small_up(const SmallParams p) {
     // x into Q8 fragments, 32 quads of four values (a chunk) per warp at a time; the first chunks are loaded before the
     // routing, so that their latency passes beside it
     const int cpr = p.n / 128, chunks = p.T * cpr;
-    constexpr int kWarps = kUpThreads / 32, kAhead = 4;
+    constexpr int kAhead = 4;
+    const int warps = int(blockDim.x >> 5);
     // (one token: the four warps that route it take no chunks; while warp 0 groups alone it takes none)
-    const int w0 = p.T == 1 && VT > 0 ? 4 : p.T * p.K <= 32 ? 1 : 0, nw = kWarps - w0;
+    const int w0 = p.T == 1 && VT > 0 ? 4 : p.T * p.K <= 32 ? 1 : 0, nw = warps - w0;
     const int c_first = warp >= w0 ? warp - w0 : chunks;
     float4 xv[kAhead];
     auto load_x = [&](int c0) {
@@ -601,7 +604,7 @@ __global__ void __maxnreg__(72) k_small_up(const SmallParams p) {
                 f[2 + s] = -(kMagic + float(s ? 16 * all : all));
             }
         }
-    } else if (lane == 0) {
+    } else if (warp == kUpProd + 4 && lane == 0) {
         // ---------------- the weights of a task: four consecutive row groups of its expert
         int slot = 0, item = item0, fb = fb0;
         uint32_t phase = 0;
