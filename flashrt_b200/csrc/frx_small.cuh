@@ -53,6 +53,32 @@ struct SmallParams {
     int tbufs;                    // k_small_up: buffers of terms (1 or 2)
 };
 
+// Loads of the routing inputs. k_small_down makes them before its wait, while the kernel in front still runs, and the same
+// addresses are rewritten from layer to layer and step to step: they are complete in the L2 by then (the kernel in front waited
+// for whatever wrote them before it let this one start), but this SM's L1 may still hold the lines that an earlier layer
+// read. So they bypass it. (A few hundred words per block, none read twice from here: eight layers of 2048 / 512 take one token
+// 111.3 us through the L1 and 110.8 past it, three tokens 200.7 and 201.1.)
+__device__ __forceinline__ float ld_l2(const float* p) {
+    float v;
+    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 ld_l2(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.cg.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ int32_t ld_l2(const int32_t* p) {
+    int32_t v;
+    asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ const uint8_t* ld_l2(const uint8_t* const* p) {
+    const uint8_t* v;
+    asm volatile("ld.global.cg.u64 %0, [%1];" : "=l"(v) : "l"(p));
+    return v;
+}
+
 // What every block works out for itself.
 struct SmallItem {
     const uint8_t* blob;
@@ -96,7 +122,7 @@ __device__ __forceinline__ void small_route(const SmallParams& p, SmallPlan& s, 
 #pragma unroll
             for (int q = 0; q < VT / 4; ++q) {
                 const bool in = e0 + 4 * q < p.E;
-                const float4 v = in ? *reinterpret_cast<const float4*>(l + e0 + 4 * q) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                const float4 v = in ? ld_l2(reinterpret_cast<const float4*>(l + e0 + 4 * q)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                 key[(4 * q) % VT] = in ? order_key(v.x + 0.0f) : 0u;
                 key[(4 * q + 1) % VT] = in ? order_key(v.y + 0.0f) : 0u;
                 key[(4 * q + 2) % VT] = in ? order_key(v.z + 0.0f) : 0u;
@@ -104,7 +130,7 @@ __device__ __forceinline__ void small_route(const SmallParams& p, SmallPlan& s, 
             }
         } else {
 #pragma unroll
-            for (int i = 0; i < VT; ++i) key[i] = e0 + i < p.E ? order_key(l[e0 + i] + 0.0f) : 0u;
+            for (int i = 0; i < VT; ++i) key[i] = e0 + i < p.E ? order_key(ld_l2(l + e0 + i) + 0.0f) : 0u;
         }
         uint32_t lm = key[0];
 #pragma unroll
@@ -179,7 +205,7 @@ __device__ __forceinline__ void small_plan(const SmallParams& p, SmallPlan& s, S
         if (tid < 4) s.ids[TK + tid] = -1;
     } else if (p.hit_ptr) {
         if (!one_warp) {   // an id for every pointer: the first slot that has it
-            for (int i = tid; i < TK; i += nt) s.ptr[i] = i % p.K < p.hit_n[i / p.K] ? p.hit_ptr[i] : nullptr;
+            for (int i = tid; i < TK; i += nt) s.ptr[i] = i % p.K < ld_l2(p.hit_n + i / p.K) ? ld_l2(p.hit_ptr + i) : nullptr;
             __syncthreads();
             for (int i = tid; i < TK + 4; i += nt) {
                 int id = -1;
@@ -192,9 +218,9 @@ __device__ __forceinline__ void small_plan(const SmallParams& p, SmallPlan& s, S
         }
     } else {
         for (int i = tid; i < TK + 4; i += nt) {
-            int e = i < TK ? p.ids[i] : -1;
+            int e = i < TK ? ld_l2(p.ids + i) : -1;
             if (i < TK) {
-                s.wts[i] = p.wts[i];
+                s.wts[i] = ld_l2(p.wts + i);
                 if (e < 0 || e >= p.E) {
                     if (report) {
                         p.status[0] = kDevBadExpertId;
@@ -237,7 +263,7 @@ __device__ __forceinline__ void small_plan(const SmallParams& p, SmallPlan& s, S
             int e = -1, cnt = 0, pos = 0;
             const uint8_t* ptr = nullptr;
             if (VT == 0 && p.hit_ptr) {   // an id for every pointer: the first slot that has it
-                if (lane < TK && lane % p.K < p.hit_n[lane / p.K]) ptr = p.hit_ptr[lane];
+                if (lane < TK && lane % p.K < ld_l2(p.hit_n + lane / p.K)) ptr = ld_l2(p.hit_ptr + lane);
 #pragma unroll 4
                 for (int j = TK - 1; j >= 0; --j)
                     if (__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(ptr), j) == reinterpret_cast<unsigned long long>(ptr) && ptr) e = j;
@@ -724,7 +750,7 @@ __global__ void __maxnreg__(72) k_small_down(const SmallParams p) {
                 const int slot = plan.ord[i];
                 list[i] = make_float2(plan.wts[slot], __int_as_float(plan.ids[slot] >= 0 ? slot : -1));
             }
-            if (tid < p.T && p.shared) list[TK + tid].x = p.gate_logit ? sigmoid_ref(p.gate_logit[tid]) : 1.0f;
+            if (tid < p.T && p.shared) list[TK + tid].x = p.gate_logit ? sigmoid_ref(ld_l2(p.gate_logit + tid)) : 1.0f;
         }
         pdl_wait();
         mbar_spin(bar_h, 0u, abort, p.wait_ns);

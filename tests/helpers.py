@@ -41,3 +41,20 @@ def rel_max(a: np.ndarray, b: np.ndarray) -> float:
 
 def cuda(a: np.ndarray) -> torch.Tensor:
     return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def launches_by_class(call) -> dict:
+    """What `call` launches through the library: {kernel class: launches}. Waits for it."""
+    from flashrt_b200.lib import check, lib
+    import ctypes as C
+    n = 9
+    ms, cnt = (C.c_float * n)(), (C.c_int * n)()
+    check(lib.frx_profile_begin())
+    try:
+        call()
+    finally:
+        check(lib.frx_profile_end(ms, cnt, n))
+    return {lib.frx_profile_class_name(i).decode(): cnt[i] for i in range(n) if cnt[i]}
+
+
+TWO_KERNELS = {"gate_up": 1, "down": 1}   # the decode layer for few tokens: every other form launches more
