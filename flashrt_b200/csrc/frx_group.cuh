@@ -129,10 +129,12 @@ __global__ void __launch_bounds__(1024) k_pf_scan(int* __restrict__ chunk_cnt, i
         bounds[e] = at_s;
         item_off[e] = at_i;
         if (blocks.meta && fits) {
-            const int nb = tb_count(c), units = (c + blocks.unit - 1) / blocks.unit;
-            for (int j = 0; j < nb; ++j) {
-                const int lo = units * j / nb * blocks.unit, hi = units * (j + 1) / nb * blocks.unit;
-                blocks.tb[at_t++] = make_int4(e, at_s + lo, min(hi, c) - lo, hi - lo);
+            // the first `more` blocks have a unit more than the others (units * j / nb would leave 32 bits from 1.3 million slots on)
+            const int nb = tb_count(c), units = (c + blocks.unit - 1) / blocks.unit, each = nb ? units / nb : 0, more = units - each * nb;
+            for (int j = 0, lo = 0; j < nb; ++j) {
+                const int width = (each + int(j < more)) * blocks.unit;
+                blocks.tb[at_t++] = make_int4(e, at_s + lo, min(width, c - lo), width);
+                lo += width;
             }
         }
         at_s += c;

@@ -127,3 +127,22 @@ def test_warps_that_only_build_items_give_the_same_bits(port, n, ff):
     finally:
         check(lib.frx_debug_set_consumer_warps(12))
     assert torch.equal(got, want)
+
+
+def test_prefill_with_more_slots_on_an_expert_than_a_square_root_of_int32(port):
+    # 1.4 million slots of one expert: 87,500 units of 16 in 29,167 token blocks, whose product is above 2^31
+    n, ff, T = 128, 128, 1_400_000
+    ex = Experts(port, n, ff, 1, shared=False)
+    rows = synth.activations(997, n)
+    x = cuda(rows).repeat(T // len(rows) + 1, 1)[:T]
+    ids = torch.zeros(T, 1, dtype=torch.int32, device="cuda")
+    ws = moe.workspace(moe.moe_q2.workspace_bytes(T, 1, n, ff, 1))
+    yd = moe.moe_q2.run(ex.base, ex.stride, 1, n, ff, x, ids, ws=ws, form="umma")
+    moe.workspace_status(ws)
+    xq, xd = port.quantize_q8(rows)
+    want = cuda(np.stack([port.expert_ffn(ex.planar[0], n, ff, q, d) for q, d in zip(xq, xd)]))
+    assert rel_max(yd[:len(rows)].cpu().numpy(), want.cpu().numpy()) < 1e-5
+    # the same token gives the same bits wherever it lies
+    whole = T // len(rows) * len(rows)
+    assert torch.equal(yd[:whole].view(-1, len(rows), n), yd[:len(rows)].expand(whole // len(rows), -1, -1))
+    assert torch.equal(yd[whole:], yd[:T - whole])
