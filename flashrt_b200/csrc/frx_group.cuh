@@ -129,10 +129,13 @@ __global__ void __launch_bounds__(1024) k_pf_scan(int* __restrict__ chunk_cnt, i
         bounds[e] = at_s;
         item_off[e] = at_i;
         if (blocks.meta && fits) {
-            // the first `more` blocks have a unit more than the others (units * j / nb would leave 32 bits from 1.3 million slots on)
+            // block j gets units * (j + 1) / nb - units * j / nb units, by running remainders: the products leave 32 bits from
+            // 1.3 million slots on
             const int nb = tb_count(c), units = (c + blocks.unit - 1) / blocks.unit, each = nb ? units / nb : 0, more = units - each * nb;
-            for (int j = 0, lo = 0; j < nb; ++j) {
-                const int width = (each + int(j < more)) * blocks.unit;
+            for (int j = 0, lo = 0, rest = 0; j < nb; ++j) {
+                rest += more;
+                const int width = (each + int(rest >= nb)) * blocks.unit;
+                if (rest >= nb) rest -= nb;
                 blocks.tb[at_t++] = make_int4(e, at_s + lo, min(width, c - lo), width);
                 lo += width;
             }
