@@ -166,8 +166,13 @@ __global__ void __launch_bounds__(256) k_pfu_quant_h(const float2* __restrict__ 
                                                      float* __restrict__ hd, int block64) {
     pdl_wait();
     pdl_trigger();
-    const size_t g = size_t(blockIdx.x) * 256 + threadIdx.x, blk = g >> 2;   // blk: the 32-block, over all rows
-    if (blk >= size_t(*n_rows) * (ff / kQ8)) return;                          // (ff is a multiple of 128: warps of 8 blocks are live as a whole)
+    const size_t g = size_t(blockIdx.x) * 256 + threadIdx.x, n_blk = size_t(*n_rows) * (ff / kQ8);
+    size_t blk = g >> 2;                       // the 32-block, over all rows
+    if ((g & ~size_t(31)) >> 2 >= n_blk) return;
+    // No exit inside a warp, the shuffles below need it whole: with rows of four blocks (ff = 128) an odd number of them
+    // ends in the middle of one. Lanes behind the end repeat the last 64-block and store nothing.
+    const bool live = blk < n_blk;
+    if (!live) blk = n_blk - 2 + (blk & 1);
     const int t = int(g & 3), s = int(blk & 1);
     const float4* src = reinterpret_cast<const float4*>(hf + blk * kQ8);
     float hv[8];
@@ -196,6 +201,7 @@ __global__ void __launch_bounds__(256) k_pfu_quant_h(const float2* __restrict__ 
         for (int i = 0; i < 4; ++i) code[i] = int(round_half_away(__fmul_rn(hv[4 * q + i], id)));
         split_codes(code, hi[q], lo[q]);
     }
+    if (!live) return;
     uint8_t* o = he + (blk >> 1) * 128 + piece_byte(0, t);
     *reinterpret_cast<uint2*>(o + piece_chunk(s, 0, t) * 16) = make_uint2(hi[0], hi[1]);
     *reinterpret_cast<uint2*>(o + piece_chunk(s, 1, t) * 16) = make_uint2(lo[0], lo[1]);

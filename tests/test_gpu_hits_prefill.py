@@ -146,3 +146,16 @@ def test_prefill_with_more_slots_on_an_expert_than_a_square_root_of_int32(port):
     whole = T // len(rows) * len(rows)
     assert torch.equal(yd[:whole].view(-1, len(rows), n), yd[:len(rows)].expand(whole // len(rows), -1, -1))
     assert torch.equal(yd[whole:], yd[:T - whole])
+
+
+@pytest.mark.parametrize("block64", [False, True])
+@pytest.mark.parametrize("S", [1, 3, 63, 64, 65, 4097])
+def test_hidden_quantizer_where_rows_end_inside_a_warp(port, S, block64):
+    # rows of four 32-blocks, eight to a warp: an odd number of rows leaves the last warp of the hidden-row quantizer half full
+    n, ff = 256, 128
+    ex = Experts(port, n, ff, 1, shared=False)
+    x, ids = cuda(synth.activations(S, n)), torch.zeros(S, 1, dtype=torch.int32, device="cuda")
+    ws = moe.workspace(moe.moe_q2.workspace_bytes(S, 1, n, ff, 1))
+    got, want = (moe.moe_q2.run_ex(ex.base, ex.stride, 1, n, ff, x, ids, block64=block64, ws=ws, form=f) for f in ("umma", "stream"))
+    moe.workspace_status(ws)
+    assert torch.equal(got, want)
