@@ -622,7 +622,7 @@ __global__ void __launch_bounds__(kGmThreads, 3) k_gm_mma(const GmArgs a) {
     pdl_wait();
     pdl_trigger();
     const int item = blockIdx.x;
-    if (item >= a.status[1]) return;
+    if (item >= a.status[1] || int(blockIdx.z * gridDim.y + blockIdx.y) * kGmRows >= a.nrows) return;
     int lo = 0, hi = a.E;   // the expert with item_off[e] <= item < item_off[e + 1]
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
@@ -639,14 +639,14 @@ __global__ void __launch_bounds__(kGmThreads, 3) k_gm_mma(const GmArgs a) {
         s_act[tid] = a.x_per_slot ? slot : slot / a.K;
     }
     __syncthreads();
-    const int r0 = blockIdx.y * kGmRows, rows = min(kGmRows, a.nrows - r0);
+    const int r0 = int(blockIdx.z * gridDim.y + blockIdx.y) * kGmRows, rows = min(kGmRows, a.nrows - r0);
     const uint32_t row_bytes = uint32_t(a.ncols / kQK) * kBlockBytes;
     const uint8_t* wsrc = a.w + size_t(e) * a.expert_stride + size_t(r0) * row_bytes;
     const uint32_t s0 = smem_u32(smem);
     const int m8 = (m + 7) & ~7;   // slots whose activations are fetched
 
     // This thread's copies of a chunk: nine words of the weights (word i of the tile's 128 x 9 by thread i % 128; rows beyond
-    // the matrix repeat its last one), 16 bytes of the codes of up to four slots, a scale and a sum of up to two.
+    // the matrix repeat its last one), 16 bytes of the codes of up to four slots, a scale of up to two.
     // Where they start is found once.
     const int nch = a.ncols / kQ8;
     uint32_t w_at[9];
@@ -987,7 +987,9 @@ int frx_gemm_moe_run(const frx_gemm_moe_plan* plan, const void* W, int64_t exper
     a.E = plan->n_experts;
     a.K = plan->K;
     a.x_per_slot = plan->x_per_slot;
-    const dim3 grid(unsigned(L.max_items), unsigned((nrows + kGmRows - 1) / kGmRows));
+    // (a grid has at most 65,535 blocks along y, and nrows may need twice as many tiles)
+    const unsigned tiles = unsigned((nrows + kGmRows - 1) / kGmRows), slices = (tiles + 65534) / 65535;
+    const dim3 grid(unsigned(L.max_items), (tiles + slices - 1) / slices, slices);
     FRX_LAUNCH(kKDown, stream, launch_pdl(k_gm_mma, grid, dim3(kGmThreads), size_t(kGmSmem), stream, a));
     FRX_CUDA(cudaGetLastError());
     return FRX_OK;

@@ -157,3 +157,19 @@ def test_grouped_products_at_tile_edges(port, ncols, nrows, T, K, E):
         want = port.moe_q2_0(wp.reshape(-1), None, xq[t0:t0 + 8].reshape(-1), ids[t0:t0 + 8], ncols, nrows, stride, False)
         # another order of at most 80 fp32 additions per row: 80 * 2^-24 of the terms' magnitude
         assert rel_l2(y[t0:t0 + 8], want) < 1e-5
+
+
+@pytest.mark.parametrize("nrows", [65535 * 128, 65535 * 128 + 1, 2 ** 24])
+def test_grouped_product_with_more_row_tiles_than_a_grid_dimension(port, nrows):
+    # the most rows that the entry accepts, against the one-token product; rows of one block pair repeat with a prime period
+    rng = np.random.default_rng(nrows)
+    some = cuda(synth.ggml_blocks(rng, 1009, 128).reshape(1009, -1))
+    w = some.repeat(nrows // 1009 + 1, 1)[:nrows].contiguous().view(-1)
+    x = rng.standard_normal((1, 128)).astype(np.float32)
+    ids = torch.zeros(1, 1, dtype=torch.int32, device="cuda")
+    ws = moe.workspace(moe.gemm.workspace_bytes(128, 1))
+    plan = moe.gemm.moe_prepare(Q2_0, 1, cuda(x), False, ids, 128, ws)
+    y = moe.gemm.moe_run(plan, w, nrows * 36, nrows).view(-1)
+    want = port.moe_q2_0(some.cpu().numpy().reshape(-1), None, port.quantize_q8_1(x).reshape(-1), np.zeros((1, 1), np.int32), 128, 1009, 1009 * 36, False)
+    assert rel_l2(y[:1009].cpu().numpy(), want.reshape(-1)) < 1e-5
+    assert torch.equal(y, y[:1009].repeat(nrows // 1009 + 1)[:nrows])
