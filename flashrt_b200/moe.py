@@ -36,6 +36,7 @@ def _stream(stream=None):
 
 
 def _addr(t: torch.Tensor | None):
+    """The address of t, or None: a tensor that must be there is refused by the library, with its own error."""
     return None if t is None else t.data_ptr()
 
 
@@ -272,7 +273,7 @@ def moe_decode(experts: int, stride: int, E: int, shared: int | None, n: int, ff
     if ws is None:
         ws = workspace(moe_decode_workspace_bytes(T, K, n, ff), x.device)
     wp, wb = _ws_span(ws)
-    check(fast.moe_decode(experts, stride, E, shared, n, ff, x.data_ptr(), ids.data_ptr(), wts.data_ptr(), _addr(gate_logit), T, K, out.data_ptr(),
+    check(fast.moe_decode(experts, stride, E, shared, n, ff, _addr(x), ids.data_ptr(), _addr(wts), _addr(gate_logit), T, K, out.data_ptr(),
                           _addr(yslot), wp, wb, _raw_stream(stream)))
     return out
 
@@ -283,7 +284,7 @@ def moe_decode_static(experts: int, stride: int, E: int, shared: int | None, n: 
     4 MiB scratch is used (frx_moe_decode_static). Calls on one device must not overlap."""
     _dev(x, ids, wts, gate_logit, out)
     T, K = ids.shape
-    check(fast.moe_decode_static(experts, stride, E, shared, n, ff, x.data_ptr(), ids.data_ptr(), wts.data_ptr(), _addr(gate_logit), T, K, out.data_ptr(),
+    check(fast.moe_decode_static(experts, stride, E, shared, n, ff, _addr(x), ids.data_ptr(), _addr(wts), _addr(gate_logit), T, K, _addr(out),
                                  _raw_stream(stream)))
     return out
 
@@ -299,7 +300,7 @@ def moe_layer(experts: int, stride: int, E: int, shared: int | None, n: int, ff:
     if ws is None:
         ws = workspace(moe_layer_workspace_bytes(T, K, n, ff), x.device)
     wp, wb = _ws_span(ws)
-    check(fast.moe_layer(experts, stride, E, shared, n, ff, x.data_ptr(), logits.data_ptr(), _addr(gate_logit), T, K, out.data_ptr(), _addr(ids_out),
+    check(fast.moe_layer(experts, stride, E, shared, n, ff, x.data_ptr(), _addr(logits), _addr(gate_logit), T, K, out.data_ptr(), _addr(ids_out),
                          _addr(wts_out), wp, wb, _raw_stream(stream)))
     return out
 
@@ -406,7 +407,7 @@ def moe_hits(hit_ptr: torch.Tensor, hit_n: torch.Tensor, K: int, x: torch.Tensor
     if scratch is None:
         scratch = workspace(moe_hits_scratch_bytes(K, n, ff, T), x.device)
     sp, sb = _ws_span(scratch)
-    check(fast.moe_hits(hit_ptr.data_ptr(), hit_n.data_ptr(), K, x.data_ptr(), n, ff, sp, sb, yh.data_ptr(), _raw_stream(stream), T))
+    check(fast.moe_hits(_addr(hit_ptr), _addr(hit_n), K, _addr(x), n, ff, sp, sb, _addr(yh), _raw_stream(stream), T))
     return yh
 
 
@@ -417,7 +418,7 @@ def moe_combine(yh: torch.Tensor, w: torch.Tensor, hit_n: torch.Tensor | None, s
     T, K, n = yh.shape
     if out is None:
         out = yh.new_empty(T, n, dtype=torch.float32)
-    check(fast.moe_combine(out.data_ptr(), yh.data_ptr(), w.data_ptr(), _addr(hit_n), _addr(shexp), _addr(gate), n, K, T, _raw_stream(stream)))
+    check(fast.moe_combine(out.data_ptr(), yh.data_ptr(), _addr(w), _addr(hit_n), _addr(shexp), _addr(gate), n, K, T, _raw_stream(stream)))
     return out
 
 
@@ -488,7 +489,7 @@ class gemv:
         _dev(g, u)
         n_tok, ncols = g.shape
         xq = g.new_empty(gemv._q8_1_bytes(ncols, n_tok), dtype=torch.uint8)
-        check(fast.gemv_swiglu_q8_1(g.data_ptr(), u.data_ptr(), ncols, n_tok, xq.data_ptr(), _raw_stream(stream)))
+        check(fast.gemv_swiglu_q8_1(g.data_ptr(), _addr(u), ncols, n_tok, xq.data_ptr(), _raw_stream(stream)))
         return xq
 
     @staticmethod
@@ -498,7 +499,7 @@ class gemv:
         _dev(w, gate, xq, ids)
         n_tok, k = ids.shape
         dst = w.new_empty(n_tok, k, nrows, dtype=torch.float32)
-        check(fast.gemv_moe_q(ggml_type, w.data_ptr(), _addr(gate), xq.data_ptr(), ids.data_ptr(), dst.data_ptr(), n_tok, k, ncols, nrows,
+        check(fast.gemv_moe_q(ggml_type, w.data_ptr(), _addr(gate), _addr(xq), ids.data_ptr(), dst.data_ptr(), n_tok, k, ncols, nrows,
                               expert_stride_bytes, int(act_per_expert), _raw_stream(stream)))
         return dst
 
@@ -508,7 +509,7 @@ class gemv:
         _dev(w, gate, xq, ids)
         n_ids = ids.numel()
         dst = w.new_empty(n_ids, nrows, dtype=torch.float32)
-        check(fast.gemv_moe_q2_0(w.data_ptr(), _addr(gate), xq.data_ptr(), ids.data_ptr(), dst.data_ptr(), n_ids, ncols, nrows, slot_stride_bytes,
+        check(fast.gemv_moe_q2_0(w.data_ptr(), _addr(gate), _addr(xq), ids.data_ptr(), dst.data_ptr(), n_ids, ncols, nrows, slot_stride_bytes,
                                  int(per_channel_act), _raw_stream(stream)))
         return dst
 
@@ -541,7 +542,7 @@ class gemm:
         T, K = ids.shape
         plan = _GemmPlan()
         wp, wb = _ws_span(ws)
-        check(fast.gemm_moe_prepare(C.addressof(plan), ggml_type, n_experts, x.data_ptr(), int(x_per_slot), ids.data_ptr(), T, K, ncols, wp, wb,
+        check(fast.gemm_moe_prepare(C.addressof(plan), ggml_type, n_experts, _addr(x), int(x_per_slot), ids.data_ptr(), T, K, ncols, wp, wb,
                                     _raw_stream(stream)))
         return plan
 
@@ -568,5 +569,5 @@ def chain_rmsnorm_unit(x: torch.Tensor, y: torch.Tensor, out: torch.Tensor | Non
     T, n = x.shape
     if out is None:
         out = torch.empty_like(x)
-    check(fast.chain_rmsnorm_unit(x.data_ptr(), y.data_ptr(), out.data_ptr(), T, n, _raw_stream(stream)))
+    check(fast.chain_rmsnorm_unit(x.data_ptr(), _addr(y), out.data_ptr(), T, n, _raw_stream(stream)))
     return out
