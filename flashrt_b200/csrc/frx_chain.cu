@@ -11,10 +11,30 @@
 namespace frx {
 namespace {
 
-// One block per token. Every thread loads its share of the row at once and leaves the squares in shared memory for the
-// one warp that adds them: the row then costs one trip to memory and n / 32 dependent additions, where one warp that
-// loaded as it added paid n / 128 trips. Verifying three tokens through eight layers
-// of 2048 elements: 223 -> 210 us per pass.
+// Two forms with the same order of additions (lane l of a warp adds the squares of elements l, l + 32, ... one after the
+// other, then the lanes are added), hence the same bits.
+//
+// A warp per token, which loads as it adds: n / 128 trips to memory, but 32 tokens at a time on an SM.
+__global__ void __launch_bounds__(32) k_chain_rmsnorm_warp(const float* __restrict__ x, const float* __restrict__ y, float* __restrict__ out, int n) {
+    pdl_wait();
+    pdl_trigger();
+    const int t = blockIdx.x, lane = threadIdx.x;
+    const float* xr = x + size_t(t) * n;
+    const float* yr = y + size_t(t) * n;
+    double ss = 0.0;
+    for (int i = lane; i < n; i += 32) {
+        const float r = __fadd_rn(xr[i], yr[i]);
+        ss = __dadd_rn(ss, __dmul_rn(double(r), double(r)));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss = __dadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, o));
+    const float inv = float(__ddiv_rn(1.0, __dsqrt_rn(__dadd_rn(__ddiv_rn(ss, double(n)), 1e-6))));
+    for (int i = lane; i < n; i += 32) out[size_t(t) * n + i] = __fmul_rn(__fadd_rn(xr[i], yr[i]), inv);
+}
+
+// A block per token. Every thread loads its share of the row at once and leaves the squares in shared memory for the
+// one warp that adds them: the row then costs one trip to memory and n / 32 dependent additions. Verifying three tokens
+// through eight layers of 2048 elements: 223 -> 210 us per pass with it.
 constexpr int kChainThreads = 512, kChainChunk = 4096;
 
 __global__ void __launch_bounds__(kChainThreads) k_chain_rmsnorm(const float* __restrict__ x, const float* __restrict__ y, float* __restrict__ out, int n) {
@@ -69,7 +89,16 @@ extern "C" int frx_chain_rmsnorm_unit(const float* x, const float* y, float* x_n
     if (T < 0 || n < 1) return fail(FRX_ERR_ARG, "frx_chain_rmsnorm_unit: T %d, n %d", T, n);
     if (T == 0) return FRX_OK;
     if (!x || !y || !x_next) return fail(FRX_ERR_ARG, "frx_chain_rmsnorm_unit: null pointer");
-    FRX_LAUNCH(kKCombine, stream, launch_pdl(k_chain_rmsnorm, dim3(unsigned(T)), dim3(kChainThreads), 0, stream, x, y, x_next, n));
+    // The block form is the faster one while its blocks (four to an SM) are all resident, and the longer the rows, the more
+    // trips it saves; beyond that the warp form has more tokens in flight, up to rows whose chunks of additions outweigh it.
+    // us, warp / block form, by row length: 512: 2.2 / 2.3 (1 token), 2.6 / 3.5 (512 tokens); 1024: 2.9 / 2.6 (1), 3.0 / 3.1
+    // (256), 3.2 / 3.9 (512); 2048: 4.2 / 3.2 (1), 4.7 / 4.7 (512), 5.2 / 6.5 (600), 17.3 / 28.7 (4,096); 4096: 8.0 / 6.4 (592),
+    // 17.1 / 25.5 (2,048); 8192: 11.9 / 7.6 (1), 29.9 / 24.2 (1,024), 109.5 / 91.3 (4,096).
+    const int per_sm = n >= 2048 ? 4 : n >= 1024 ? 2 : n >= 640 ? 1 : 0;
+    if (n >= 8192 || T <= per_sm * sm_count())
+        FRX_LAUNCH(kKCombine, stream, launch_pdl(k_chain_rmsnorm, dim3(unsigned(T)), dim3(kChainThreads), 0, stream, x, y, x_next, n));
+    else
+        FRX_LAUNCH(kKCombine, stream, launch_pdl(k_chain_rmsnorm_warp, dim3(unsigned(T)), dim3(32), 0, stream, x, y, x_next, n));
     FRX_CUDA(cudaGetLastError());
     return FRX_OK;
 }

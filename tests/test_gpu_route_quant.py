@@ -140,3 +140,17 @@ def test_chain_rmsnorm_order_of_additions(n):
         lanes = lanes + lanes[:, np.arange(32) ^ o]
     inv = (1.0 / np.sqrt(lanes[:, :1] / n + 1e-6)).astype(np.float32)
     assert np.array_equal(moe.chain_rmsnorm_unit(cuda(x), cuda(y)).cpu().numpy(), r * inv)
+
+
+@pytest.mark.parametrize("n,T", [(640, 149), (1024, 297), (2048, 593), (512, 2), (128, 4096)])
+def test_chain_rmsnorm_forms_give_the_same_bits(n, T):
+    # T is one token more than the block form takes at this length (none at 512 and 128): rows of the long call against calls
+    # of one token, which take the block form from 640 on
+    rng = np.random.default_rng(n)
+    x, y = cuda(rng.standard_normal((T, n), dtype=np.float32)), cuda(rng.standard_normal((T, n), dtype=np.float32))
+    got = moe.chain_rmsnorm_unit(x, y)
+    for t in {0, 1, T // 2, T - 1}:
+        assert torch.equal(moe.chain_rmsnorm_unit(x[t:t + 1].contiguous(), y[t:t + 1].contiguous())[0], got[t])
+    ref = (x + y).double()
+    ref = ref / (ref.square().mean(dim=1, keepdim=True) + 1e-6).sqrt()
+    assert float((got.double() - ref).abs().max() / ref.square().mean().sqrt()) < 1e-5   # rows of +-5: three roundings of 2^-24 each
