@@ -253,13 +253,15 @@ __global__ void __launch_bounds__(256) k_combine_partial(float* __restrict__ out
     }
 }
 
-// k_moe_combine / k_stream_combine semantics: k order, as the hit list gives it. V consecutive elements per thread (4
-// where rows and pointers are 16-byte aligned); the rows of eight slots are requested before the first addition.
-// Bound: HBM. 4,096 tokens x 10 rows of 2048: 99 us with one element per thread and one load in flight, 62 us now.
-template <int V>
+// k_moe_combine / k_stream_combine semantics: k order, as the hit list gives it. Two forms of the same additions.
+//
+// Four consecutive elements per thread, where rows and pointers are 16-byte aligned; the rows of eight slots are requested
+// before the first addition. Bound: HBM. 4,096 tokens x 10 rows of 2048: 99 us with one element per thread and one load in
+// flight, 62 us now.
 __global__ void __launch_bounds__(256) k_combine_hits(float* __restrict__ out, const float* __restrict__ yh,
                                                       const float* __restrict__ w, const int32_t* __restrict__ hit_n,
                                                       const float* __restrict__ shexp, const float* __restrict__ gate, int n, int K) {
+    constexpr int V = 4;
     pdl_wait();
     pdl_trigger();
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) * V;
@@ -295,4 +297,33 @@ __global__ void __launch_bounds__(256) k_combine_hits(float* __restrict__ out, c
 #pragma unroll
     for (int e = 0; e < V; ++e) o.v[e] = shexp ? __fadd_rn(acc[e], __fmul_rn(sh.v[e], g)) : acc[e];
     *reinterpret_cast<Vec*>(out + t * n + i) = o;
+}
+
+// One element per thread: whole groups of eight slots, and the rest one by one (bounds tests per load, as above, cost more than
+// the loads in flight save here: 4,096 tokens x 10 rows of 130 13.2 us with them, 7.2 without; of 2049 142 and 100).
+__global__ void __launch_bounds__(256) k_combine_hits_scalar(float* __restrict__ out, const float* __restrict__ yh,
+                                                             const float* __restrict__ w, const int32_t* __restrict__ hit_n,
+                                                             const float* __restrict__ shexp, const float* __restrict__ gate, int n, int K) {
+    pdl_wait();
+    pdl_trigger();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, t = blockIdx.y;
+    if (i >= n) return;
+    const int kn = hit_n ? hit_n[t] : K;
+    float acc = 0.0f;
+    const float* y = yh + size_t(t) * K * n + i;
+    const float* wt = w + size_t(t) * K;
+    int k = 0;
+    for (; k + kCombineBatch <= kn; k += kCombineBatch, y += size_t(kCombineBatch) * n) {
+        float v[kCombineBatch], c[kCombineBatch];
+#pragma unroll
+        for (int j = 0; j < kCombineBatch; ++j) v[j] = y[size_t(j) * n], c[j] = wt[k + j];
+#pragma unroll
+        for (int j = 0; j < kCombineBatch; ++j) acc = __fadd_rn(acc, __fmul_rn(c[j], v[j]));
+    }
+    for (; k < kn; ++k, y += n) acc = __fadd_rn(acc, __fmul_rn(wt[k], *y));
+    if (shexp) {
+        const float g = gate ? sigmoid_ref(gate[t]) : 1.0f;
+        acc = __fadd_rn(acc, __fmul_rn(shexp[size_t(t) * n + i], g));
+    }
+    out[size_t(t) * n + i] = acc;
 }

@@ -1782,9 +1782,9 @@ int frx_moe_combine(float* out, const float* yh, const float* w, const int32_t* 
     if (n < 1 || K < 1 || T < 0) return fail(FRX_ERR_ARG, "frx_moe_combine: n %d, K %d, T %d", n, K, T);
     if (T == 0) return FRX_OK;
     const bool vec = n % 4 == 0 && (uintptr_t(out) | uintptr_t(yh) | uintptr_t(shexp)) % 16 == 0;
-    const int per = vec ? 4 : 1, threads = n / per >= 256 ? 256 : 128;
+    const int per = vec ? 4 : 1, threads = std::min(256, ((n + per - 1) / per + 31) / 32 * 32);   // a row of up to 256 threads is one block of whole warps
     const dim3 grid((n + threads * per - 1) / (threads * per), T);
-    FRX_LAUNCH(kKCombine, stream, launch_pdl(vec ? k_combine_hits<4> : k_combine_hits<1>, grid, dim3(threads), 0, stream, out, yh, w, hit_n, shexp, gate, n, K));
+    FRX_LAUNCH(kKCombine, stream, launch_pdl(vec ? k_combine_hits : k_combine_hits_scalar, grid, dim3(threads), 0, stream, out, yh, w, hit_n, shexp, gate, n, K));
     FRX_CUDA(cudaGetLastError());
     return FRX_OK;
 }

@@ -502,3 +502,26 @@ def test_two_kernel_form_with_routing_rewritten_in_place(port, T, K):
             t.zero_()
         graph.replay()
         compare()
+
+
+@pytest.mark.parametrize("n,T,offset", [(1, 3, 0), (130, 252, 0), (2049, 17, 0), (512, 65, 1), (512, 65, 0), (1028, 40, 0)])
+@pytest.mark.parametrize("K", [1, 8, 9, 17])
+def test_combine_forms(n, T, offset, K):
+    # rows that can be read four elements at a time and rows that cannot (length, alignment), whole groups of eight slots and
+    # a rest: the additions are in k order in all of them, so the bits are the same
+    g = torch.Generator(device="cuda").manual_seed(n + K)
+    yh = torch.randn(T * K * n + offset, generator=g, device="cuda")[offset:].view(T, K, n)
+    w = torch.rand(T, K, generator=g, device="cuda")
+    hit_n = torch.randint(0, K + 1, (T,), dtype=torch.int32, generator=g, device="cuda")
+    sh, gate = torch.randn(T, n, generator=g, device="cuda"), torch.randn(T, generator=g, device="cuda")
+    sums = []
+    for counts in (None, hit_n):
+        acc = torch.zeros(T, n, device="cuda")
+        for k in range(K):
+            more = acc + w[:, k:k + 1] * yh[:, k]
+            acc = more if counts is None else torch.where((k < counts)[:, None], more, acc)
+        sums.append(acc)
+        assert torch.equal(moe.moe_combine(yh, w, counts, None, None), acc)
+    assert torch.equal(moe.moe_combine(yh, w, None, sh, None), sums[0] + sh)
+    out = moe.moe_combine(yh, w, hit_n, sh, gate)
+    assert torch.allclose(out, sums[1] + sh * torch.sigmoid(gate)[:, None], rtol=1e-6, atol=1e-6)   # (another exponential)
