@@ -999,10 +999,13 @@ struct StreamCfg {
 // blocks of 4 or 8 warps with deeper rings serve small batches better.
 // decode, when every item has at most four tokens: bit 0 = gate/up, bit 1 = down take tasks of four row groups
 // (k_stream's TASK4 form). Measured at batch 64: down gains from it, gate/up does not.
-// With an odd number of units (one to a chunk) down gains up to 16 tokens only (kTask4OddTokens): ff = 640 at 64 tokens 147.1
-// us per layer with it and 143.6 without, 384 / 640 at 16 tokens 41.7 and 43.8.
+// With an odd number of units (one to a chunk) from five on, down gains up to 16 tokens only (kTask4OddTokens): ff = 640 at 64
+// tokens 147.1 us per layer with it and 143.6 without, 384 / 640 at 16 tokens 41.7 and 43.8. With one or three units the pairs
+// of groups leave a task so short that the four-group form (and the quantizer inside it) always gains: us per layer with it /
+// without, 128 experts top-8, 24 / 64 tokens: 384 / 128 22.3 / 27.9 and 24.2 / 29.9; 2048 / 384 40.3 / 45.2 and 55.2 / 59.9; 512 experts
+// top-10, 64 tokens: 384 / 384 44.5 / 48.2, 2048 / 384 88.2 / 94.4.
 int g_task4 = 2;
-constexpr int kTask4OddTokens = 16;
+constexpr int kTask4OddTokens = 16, kTask4OddUnits = 3;
 int g_evict_first = 1;  // decode: the weight copies carry an evict-first L2 policy (see l2_policy_evict_first)
 int g_down_per_item = 256;   // weight of an item's buffer in down's split, in 1/16 of a task (measured best near 16 tasks: 102.4 us per layer against 103.5 with 0 and 106.5 with 1024)
 int g_down_heavy = 22;  // decode: weight of a down task of an item of three or four tokens when the tasks are shared out (16 = as one of a smaller item, 0 = even split by count)
@@ -1351,7 +1354,7 @@ int decode_steps(const void* experts, size_t stride, int E, int e_lo, int e_hi, 
         return launch_small(p, scfg, stream);
     }
     // with items cut at four tokens either streaming kernel may take tasks of four row groups
-    const bool task4_gu = g_narrow && (g_task4 & 1), task4_dn = g_narrow && (g_task4 & 2) && (ff / kUnitK % 2 == 0 || T <= kTask4OddTokens);
+    const bool task4_gu = g_narrow && (g_task4 & 1), task4_dn = g_narrow && (g_task4 & 2) && (ff / kUnitK % 2 == 0 || ff / kUnitK <= kTask4OddUnits || T <= kTask4OddTokens);
     StreamCfg cfg;
     if (int rc = stream_cfg(n, ff, cfg, L.max_items, false)) return rc;   // max_items: the most items a chunk of tokens can make
     if (task4_gu || task4_dn) {

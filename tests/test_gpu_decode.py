@@ -525,3 +525,26 @@ def test_combine_forms(n, T, offset, K):
     assert torch.equal(moe.moe_combine(yh, w, None, sh, None), sums[0] + sh)
     out = moe.moe_combine(yh, w, hit_n, sh, gate)
     assert torch.allclose(out, sums[1] + sh * torch.sigmoid(gate)[:, None], rtol=1e-6, atol=1e-6)   # (another exponential)
+
+
+@pytest.mark.parametrize("n,ff,T,four", [(256, 128, 17, True), (384, 384, 64, True), (128, 384, 70, True), (256, 640, 16, True), (256, 640, 17, False)])
+def test_down_task_forms_at_odd_unit_counts(port, n, ff, T, four):
+    # one or three units of K: four-group tasks (and no separate hidden-row quantizer) at any number of tokens, from five on
+    # up to 16 tokens; the pair form gives the same bits
+    from flashrt_b200.lib import check, lib
+    E, K = 40, 5
+    ex = Experts(port, n, ff, E, direct=True)
+    x = synth.activations(T, n)
+    ids, wts, _ = port.route(synth.router_logits(T, E), K)
+    gate = np.linspace(-1, 1, T).astype(np.float32)
+    got = []
+    classes = launches_by_class(lambda: got.append(run_decode(ex, x, ids, wts, gate)))
+    assert ("quant_q8" not in classes) == four, classes
+    try:
+        check(lib.frx_debug_set_four_group_tasks(0))
+        out, ys = run_decode(ex, x, ids, wts, gate)
+    finally:
+        check(lib.frx_debug_set_four_group_tasks(2))
+    assert np.array_equal(got[0][0], out) and np.array_equal(got[0][1], ys)
+    _, ref_ys, _ = port.moe_layer(ex.routed_planar(), ex.blob_bytes, ex.shared_planar, n, ff, x, ids, wts, gate, n_threads=8, want_slots=True)
+    assert max(rel_max(ys[s], ref_ys[s]) for s in range(T * K)) < 1e-5
