@@ -44,6 +44,7 @@ int cuda_fail(cudaError_t e, const char* what);
 
 int sm_count();
 int max_smem_optin();
+bool prefill_stream_fits(int n, int ff);   // whether the streaming kernels have room for their buffers at this shape
 
 // Optional per-kernel timing (frx_profile_begin / frx_profile_end): when switched on, every
 // launch made through FRX_LAUNCH is bracketed by two CUDA events on its own stream.

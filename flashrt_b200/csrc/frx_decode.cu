@@ -1448,6 +1448,12 @@ int decode_steps(const void* experts, size_t stride, int E, int e_lo, int e_hi, 
 }
 
 }  // namespace
+
+bool prefill_stream_fits(int n, int ff) {
+    StreamCfg cfg;
+    return stream_cfg(n, ff, cfg) == FRX_OK;
+}
+
 }  // namespace frx
 
 using namespace frx;

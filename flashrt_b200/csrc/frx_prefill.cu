@@ -27,6 +27,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 
+#include <algorithm>
 #include <mutex>
 
 namespace frx {
@@ -768,12 +769,29 @@ int set_pf_attr() {
 
 using namespace frx;
 
-// Which form: the tensor-memory form pays per unit of 256 rows x 128 weights whatever the number of tokens
-// in the tile, the streaming form reads an expert again for every eight tokens. Measured on B200
-// (us, uniform routing; hidden / width, experts; streaming against tensor memory): 2048 / 512, 512:
-// 16 tokens per expert 346 against 410, 24: 469 against 440, 32: 592 against 484, 128: 2098 against
-// 1419; 384 / 640, 128: 24: 87 against 92, 32: 101 against 97. With skewed routing they meet at 32.
+// Which form. The tensor-memory form pays per unit of 256 rows x 128 weights whatever the number of tokens in the tile, and its
+// tiles (token blocks x blocks of 256 rows) are whole SMs' work; the streaming form reads an expert again for every eight
+// tokens, but its tasks are small enough to fill the chip with any number of experts. So: 32 tokens per expert on average,
+// and the shorter of two estimates in microseconds on 148 SMs:
+//   tensor memory   units of K x 1.2 per tile and round of tiles over the SMs (at least one, on average half a round more than
+//                   full ones), for either product, and 4 more than the other form for its launches;
+//   streaming       0.02 + 0.26 (n ff / 2^20) per item of eight slots, of which an expert's last one is half full.
+// Measured (us, uniform routing, streaming / tensor memory; slots per expert at 2048 / 512): one expert 64: 32 / 47, 255: 37 / 55;
+// 4 experts 255: 60 / 64, 300: 65 / 64; 16 experts 96: 75 / 86, 200: 122 / 113; 32 experts 40: 72 / 68; 64 experts 32: 97 / 95,
+// 64: 153 / 140; 512 experts 24: 420 / 393, 32: 531 / 435. 512 / 256: 4 experts 255: 37 / 40, 16 experts 128: 45 / 42, 64 experts
+// 32: 45 / 42. 2560 / 640: one expert 96: 36 / 58, 64 experts 64: 218 / 194. Of 900 such points the estimate is off the faster
+// form by 0.7 % on average and 15 % at most; the mean number of tokens alone was off by 62 % (one expert).
+// With skewed routing the forms meet at the same mean.
 constexpr int kUmmaMinTokensPerExpert = 32;
+static bool umma_pays(long long slots, int E, int n, int ff) {
+    if (slots < (long long)kUmmaMinTokensPerExpert * E) return false;
+    const double sms = std::max(sm_count(), 1), blocks = double(slots) / kTileTok + 0.5 * E, items = double(slots) / kTokPerItem + 0.5 * E;
+    auto rounds = [&](int row_blocks) { return std::max(1.0, blocks * row_blocks / sms + 0.5); };
+    const int row_tiles = n / kTileRows;
+    const double umma = 1.2 * (rounds(2 * ff / (kRowTiles * kTileRows)) * (n / kUnitK) + rounds((row_tiles + 1) / 2) * (ff / kUnitK));
+    const double stream = items * (0.02 + 0.26 * double(n) * ff / (1 << 20)) * (148.0 / sms);
+    return umma + 4.0 < stream || !prefill_stream_fits(n, ff);
+}
 
 extern "C" {
 
@@ -784,6 +802,11 @@ int frx_moe_prefill_stream_ex(const void* experts, size_t stride, int E, int n, 
 int frx_moe_prefill_stream_q8_ep(const void* experts_local, size_t stride, int E_local, const int32_t* e_map, int E_all, int n, int ff,
                                  const int8_t* xq, const float* xd, const int32_t* ids, int T, int K, float* yd, void* ws, size_t ws_bytes,
                                  frx_stream_t stream);
+
+int frx_moe_prefill_form(int T, int K, int n, int ff, int E, int E_local) {
+    if (T < 1 || K < 1 || E < 1 || E_local < 1) return 1;
+    return umma_pays((long long)T * K * E_local / E, E_local, n, ff) ? 2 : 1;
+}
 
 size_t frx_moe_prefill_umma_workspace_bytes(int T, int K, int n, int ff, int E) {
     if (T < 1 || K < 1 || n < kUnitK || ff < kUnitK || E < 1) return 0;
@@ -875,12 +898,12 @@ int frx_moe_prefill_q8_ep(const void* experts_local, size_t stride, int E_local,
     if (!xq || !xd || !e_map) return fail(FRX_ERR_ARG, "frx_moe_prefill_q8_ep: null pointer");
     if (form < 0 || form > 2) return fail(FRX_ERR_ARG, "frx_moe_prefill_q8_ep: form %d", form);
     // the expected number of slots per local expert is T * K / E_all (the counts stay on the device)
-    const bool umma = form == 2 || (form == 0 && T > 0 && size_t(T) * K >= size_t(kUmmaMinTokensPerExpert) * size_t(E_all));
+    const bool umma = form == 2 || (form == 0 && frx_moe_prefill_form(T, K, n, ff, E_all, E_local) == 2);
     if (umma) return prefill_umma_impl(experts_local, stride, E_local, e_map, E_all, n, ff, nullptr, xq, xd, ids, T, K, yd, ws, ws_bytes, stream, 0, 0);
     return frx_moe_prefill_stream_q8_ep(experts_local, stride, E_local, e_map, E_all, n, ff, xq, xd, ids, T, K, yd, ws, ws_bytes, stream);
 }
 
-// ---- the public entry: both forms compute the same bits, see kUmmaMinTokensPerExpert
+// ---- the public entry: both forms compute the same bits, see umma_pays
 
 size_t frx_moe_prefill_workspace_bytes(int T, int K, int n, int ff, int E) {
     const size_t a = frx_moe_prefill_stream_workspace_bytes(T, K, n, ff, E), b = frx_moe_prefill_umma_workspace_bytes(T, K, n, ff, E);
@@ -895,7 +918,7 @@ int frx_moe_prefill(const void* experts, size_t stride, int E, int n, int ff, co
 
 int frx_moe_prefill_ex(const void* experts, size_t stride, int E, int n, int ff, const float* x, const int32_t* ids, int T, int K,
                        void* yd, void* ws, size_t ws_bytes, frx_stream_t stream, int block64, int yd_bf16) {
-    if (T > 0 && K > 0 && E > 0 && size_t(T) * K >= size_t(kUmmaMinTokensPerExpert) * E)
+    if (frx_moe_prefill_form(T, K, n, ff, E, E) == 2)
         return frx_moe_prefill_umma_ex(experts, stride, E, n, ff, x, ids, T, K, yd, ws, ws_bytes, stream, block64, yd_bf16);
     return frx_moe_prefill_stream_ex(experts, stride, E, n, ff, x, ids, T, K, yd, ws, ws_bytes, stream, block64, yd_bf16);
 }

@@ -393,9 +393,13 @@ int frx_moe_combine(float* out, const float* yh, const float* w, const int32_t* 
  * Two forms compute the same bits: frx_moe_prefill_umma runs the integer products on the tcgen05
  * tensor cores with accumulators in tensor memory, frx_moe_prefill_stream is the form the decode
  * path uses. frx_moe_prefill takes the tensor-memory form when experts receive 32 or more tokens
- * on average (T * K >= 32 * E) and the streaming form otherwise; the two are exported so each can
+ * on average (T * K >= 32 * E) and there are experts and rows enough to fill the GPU with its tiles, and the
+ * streaming form otherwise; the two are exported so each can
  * be called and measured on its own, with the same arguments and workspace size. */
 size_t frx_moe_prefill_workspace_bytes(int T, int K, int n, int ff, int E);
+/* The form that frx_moe_prefill (E_local = E) and frx_moe_prefill_q8_ep (E experts in all, E_local of them here) take for
+ * such a call: 1 the streaming form, 2 the tensor-memory form. */
+int frx_moe_prefill_form(int T, int K, int n, int ff, int E, int E_local);
 int frx_moe_prefill(const void* experts, size_t stride, int E, int n, int ff, const float* x, const int32_t* ids, int T,
                     int K, float* yd, void* ws, size_t ws_bytes, frx_stream_t stream);
 int frx_moe_prefill_umma(const void* experts, size_t stride, int E, int n, int ff, const float* x, const int32_t* ids, int T,

@@ -159,3 +159,18 @@ def test_hidden_quantizer_where_rows_end_inside_a_warp(port, S, block64):
     got, want = (moe.moe_q2.run_ex(ex.base, ex.stride, 1, n, ff, x, ids, block64=block64, ws=ws, form=f) for f in ("umma", "stream"))
     moe.workspace_status(ws)
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("n,ff,E,K,per_expert,umma", [(2048, 512, 1, 1, 64, False), (2560, 640, 2, 2, 200, False), (512, 256, 8, 4, 32, False), (512, 256, 64, 8, 31, False),
+                                                      (512, 256, 64, 8, 48, True), (2048, 512, 64, 8, 64, True), (384, 640, 16, 4, 300, True), (4096, 1024, 1, 1, 40, True)])
+def test_prefill_takes_the_form_that_fills_the_gpu(port, n, ff, E, K, per_expert, umma):
+    # few experts leave most SMs without a tile of the tensor-memory form; a shape that the streaming form has no room for takes
+    # the other one from 32 tokens per expert on
+    from flashrt_b200.lib import lib
+    T = per_expert * E // K
+    assert lib.frx_moe_prefill_form(T, K, n, ff, E, E) == (2 if umma else 1)
+    assert lib.frx_moe_prefill_form(4 * T, K, n, ff, 4 * E, E) == (2 if umma else 1)      # a quarter of the experts is here
+    ex = Experts(port, n, ff, E, shared=False, direct=True)
+    x, ids = cuda(synth.activations(T, n)), torch.randint(0, E, (T, K), dtype=torch.int32, device="cuda")
+    got = moe.moe_q2.run(ex.base, ex.stride, E, n, ff, x, ids)
+    assert torch.equal(got, moe.moe_q2.run(ex.base, ex.stride, E, n, ff, x, ids, form="umma" if umma else "stream"))
