@@ -153,7 +153,6 @@ __global__ void __launch_bounds__(kDotThreads) k_ggml_dot(const DotArgs a) {
         mbar_fence_init();
     }
     pdl_wait();
-    pdl_trigger();
     const int job = blockIdx.x, e = a.ids ? a.ids[job] : 0;
     const uint8_t* wsrc = a.w + size_t(e) * a.expert_stride;
     const uint8_t* gsrc = GATE ? a.gate + size_t(e) * a.expert_stride : nullptr;
@@ -254,6 +253,9 @@ __global__ void __launch_bounds__(kDotThreads) k_ggml_dot(const DotArgs a) {
             }
         }
     }
+    // The next kernel is let in as a block ends, not as it starts: blocks of it that wait beside this kernel's would share the SMs'
+    // slots unevenly (eight jobs of 4096 x 1024, 512 blocks: 17.6 us let in at the start, 12.8 at the end; one job 5.1, 5.0).
+    pdl_trigger();
 }
 
 int dot_tile_rows(int ncols) {
@@ -278,6 +280,11 @@ int launch_dot(DotArgs a, int grid_x, cudaStream_t stream) {
         std::lock_guard<std::mutex> lk(mu);
         if (dev >= 0 && dev < 64 && !set[dev]) {
             FRX_CUDA(cudaFuncSetAttribute(k_ggml_dot<GATE>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin() - 1024));
+            // The quantizer in front asks for the same split of the SM, though it uses no shared memory: an SM that runs it could not
+            // change its split, and this kernel's early blocks would crowd on the others (4 tokens x 4096 x 1024 with their
+            // quantization: 14.1 us, 9.0 so).
+            FRX_CUDA(cudaFuncSetAttribute(k_ggml_dot<GATE>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+            FRX_CUDA(cudaFuncSetAttribute(k_q8_1, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
             set[dev] = true;
         }
     }
