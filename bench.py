@@ -749,6 +749,15 @@ def bench_verify_stack(torch, moe, synth, dev, rank, world, L, layer, timeit, la
     return res
 
 
+def prefill_form(T, E_local, asked="auto"):
+    """The kernel form of T tokens of the benchmark's layer over E_local experts held here: what was asked for, or the library's choice."""
+    from flashrt_b200 import moe
+
+    if asked == "auto":
+        asked = "umma" if moe.lib.frx_moe_prefill_form(T, K, N_MODEL, FF, E, E_local) == 2 else "stream"
+    return {"umma": "tcgen05", "stream": "streaming"}[asked]
+
+
 def bench_prefill_extra(torch, dist, moe, synth, dev, rank, world, arena, e_lo, e_hi, keep, port, steps, layer_planar):
     """BASELINE configs[2] (one GPU: 4,096 tokens, Zipf routing) or configs[4] (several GPUs: 16,384
     tokens, uniform and Zipf routing, tokens and experts sharded, all-to-all dispatch and combine)
@@ -832,8 +841,8 @@ def bench_prefill_extra(torch, dist, moe, synth, dev, rank, world, arena, e_lo, 
                  "flops_per_step": flops, "tflops_step": round(flops / (ms * 1e-3) / 1e12, 1),
                  "tflops_expert_products_rank0": round(flops / world / max(gemm_ms, 1e-9) / 1e9, 1) if gemm_ms else None,
                  "frac_of_bf16_peak_step": round(flops / world / (ms * 1e-3) / 1e12 / peak_tf, 4), "peak_tflops": peak_tf,
-                 "form": ("tcgen05" if T * K >= 256 * E else "streaming") if world == 1
-                 else "streaming per chunk of 4 (slots per expert and chunk below 256); Q8 all-gather dispatch, fp32 reduce-scatter combine, "
+                 "form": prefill_form(T, E) if world == 1
+                 else f"{prefill_form(world * pipe.Tc, pipe.E_local)} per chunk of {pipe.chunks}; Q8 all-gather dispatch, fp32 reduce-scatter combine, "
                       + ("experts dealt round-robin by popularity" if routing == "zipf" else "contiguous expert ranges"),
                  "tokens_per_expert_rank0": {"mean": float(cnt.float().mean()), "max": int(cnt.max()), "min": int(cnt.min())}}
         if rank == 0 and port is not None and 0 in keep:
@@ -958,10 +967,10 @@ def run_prefill(args):
         print(json.dumps({
             "metric": "q2_0_moe_prefill_tokens_per_s", "value": T / (ms * 1e-3), "unit": "tokens/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "strong",
-            "dtype": "exact integer products (int8 / fp16 operands), fp32 scale and accumulate", "data": "synthetic",
+            "dtype": "exact integer products (int8 / e4m3 operands), fp32 scale and accumulate", "data": "synthetic",
             "config": {"workload": f"configs[{2 if world == 1 else 4}]: one Q2_0 MoE layer prefill, {T} tokens, hidden 2048, 512 experts top-10, "
                                    f"{'Zipf(1.1)' if args.routing == 'zipf' else 'uniform'} routing",
-                       "form": args.form, "parallelism": f"ep{world}", "l2": "453 MB of experts per step, larger than L2"},
+                       "form": prefill_form(T, E, args.form) if world == 1 else prefill_form(world * pipe.Tc, pipe.E_local), "parallelism": f"ep{world}", "l2": "453 MB of experts per step, larger than L2"},
             "clocks": clocks, "kernels": kernels,
             "roofline": {"bound": "tensor", "kernel": "expert product (gate/up + down), rank 0", "achieved": round(gemm_tf, 1), "peak": peak_tf,
                          "unit": "TFLOP/s", "frac": round(gemm_tf / peak_tf, 4), "flops_per_step": flops, "ms_gate_up": gu_ms,
