@@ -519,7 +519,7 @@ class gemv:
         n_tok, ncols = x.shape
         y = x.new_empty(n_tok, nrows, dtype=torch.float32)
         scratch = x.new_empty(gemv._q8_1_bytes(ncols, n_tok), dtype=torch.uint8)
-        check(fast.gemv_matvec(ggml_type, W.data_ptr(), x.data_ptr(), y.data_ptr(), ncols, nrows, n_tok, scratch.data_ptr(), _raw_stream(stream)))
+        check(fast.gemv_matvec(ggml_type, _addr(W), x.data_ptr(), y.data_ptr(), ncols, nrows, n_tok, scratch.data_ptr(), _raw_stream(stream)))
         return y
 
 

@@ -29,6 +29,7 @@ def test_missing_tensors_are_refused_by_the_library():
         lambda: moe.gemv.swiglu_q8_1(x, None),
         lambda: moe.gemv.moe_q(Q2_0, z, None, None, ids, n, 4, 576, False),
         lambda: moe.gemv.moe_q2_0(z, None, None, ids, n, 4, 576, False),
+        lambda: moe.gemv.matvec(Q2_0, None, x, 4),
         lambda: moe.gemm.moe_prepare(Q2_0, 4, None, False, ids, n, z),
         lambda: moe.chain_rmsnorm_unit(x, None, out=torch.empty_like(x)),
     ]
