@@ -10,6 +10,7 @@ import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libfrx.so")
+BINDING_PATH = os.path.join(HERE, "_frxpy.so")
 
 OK, ERR_ARG, ERR_SHAPE, ERR_WORKSPACE, ERR_CUDA, ERR_DEVICE = range(6)
 
@@ -22,9 +23,10 @@ class FrxError(RuntimeError):
         self.code = code
 
 
-if not os.path.exists(LIB_PATH):
-    raise ImportError(f"{LIB_PATH} is missing: build it with `python -m flashrt_b200.build` (needs nvcc); "
-                      "there is no CPU fallback")
+for _path in (LIB_PATH, BINDING_PATH):
+    if not os.path.exists(_path):
+        raise ImportError(f"{_path} is missing: build it with `python -m flashrt_b200.build` (needs nvcc); "
+                          "there is no CPU fallback")
 
 lib = C.CDLL(LIB_PATH)
 

@@ -99,3 +99,17 @@ def test_cpp_shim_compiles_against_the_header():
         r = subprocess.run([gxx, "-std=c++17", "-fsyntax-only", "-I" + os.path.join(ROOT, "include"), "-I" + cuda_inc, f.name],
                            capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
+
+
+@pytest.mark.parametrize("present", [(), ("libfrx.so",)])
+def test_import_without_built_files_says_what_to_build(tmp_path, present):
+    import subprocess
+    import sys
+    pkg = tmp_path / "flashrt_b200"
+    pkg.mkdir()
+    for name in ("__init__.py", "lib.py"):
+        (pkg / name).write_text(open(os.path.join(ROOT, "flashrt_b200", name)).read())
+    for name in present:
+        (pkg / name).symlink_to(os.path.join(ROOT, "flashrt_b200", name))
+    r = subprocess.run([sys.executable, "-c", "import flashrt_b200.lib"], cwd=tmp_path, capture_output=True, text=True)
+    assert r.returncode != 0 and "ImportError" in r.stderr and "flashrt_b200.build" in r.stderr, r.stderr
