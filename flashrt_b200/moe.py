@@ -23,12 +23,15 @@ def _ptr(t: torch.Tensor | None):
     return None if t is None else C.c_void_p(t.data_ptr())
 
 
-_current_raw_stream, _current_device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+# (absent from a torch built without CUDA, where this module can be imported all the same)
+_current_raw_stream, _current_device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
 
 
 def _raw_stream(stream=None) -> int:
     """The handle of `stream`, or of the current one (without making a Stream object of it)."""
-    return _current_raw_stream(_current_device()) if stream is None else stream.cuda_stream
+    if stream is not None:
+        return stream.cuda_stream
+    return _current_raw_stream(_current_device()) if _current_raw_stream else torch.cuda.current_stream().cuda_stream
 
 
 def _stream(stream=None):

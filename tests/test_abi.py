@@ -113,3 +113,16 @@ def test_import_without_built_files_says_what_to_build(tmp_path, present):
         (pkg / name).symlink_to(os.path.join(ROOT, "flashrt_b200", name))
     r = subprocess.run([sys.executable, "-c", "import flashrt_b200.lib"], cwd=tmp_path, capture_output=True, text=True)
     assert r.returncode != 0 and "ImportError" in r.stderr and "flashrt_b200.build" in r.stderr, r.stderr
+
+
+def test_import_with_a_torch_without_cuda():
+    # such a build of torch lacks the private functions behind the current stream; sizes and loaders need no stream
+    import subprocess
+    import sys
+    code = ("import torch\n"
+            "for f in ('_cuda_getCurrentRawStream', '_cuda_getDevice'):\n"
+            "    if hasattr(torch._C, f): delattr(torch._C, f)\n"
+            "from flashrt_b200 import moe\n"
+            "assert moe.expert_bytes(2048, 512) == 884736\n")
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
