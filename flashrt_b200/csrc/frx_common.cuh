@@ -101,16 +101,6 @@ inline cudaError_t launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 
     cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ uint32_t cluster_id_x() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%clusterid.x;" : "=r"(r));
-    return r;
-}
 // Hardware barrier over all threads of the cluster; writes made before it (global memory
 // included) are visible to the cluster's threads after it.
 __device__ __forceinline__ void cluster_sync_all() {
@@ -331,18 +321,8 @@ __device__ __forceinline__ void named_bar_sync(int id, int threads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-// D (16x8 s32) += A (16x32 u8, row) * B (32x8 s8, col)
-__device__ __forceinline__ void mma_u8s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                         uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-// D (16x8 s32) = A * B + C with every element of C equal to `c`; the results come back packed in
-// pairs: lo = {D[g][2t], D[g][2t+1]}, hi = the same columns of row g + 8.
-// The same with the accumulator input given as four registers (a quad loaded from shared memory).
+// D (16x8 s32) = A (16x32 u8, row) * B (32x8 s8, col) + C, with C given as four registers (a quad loaded from shared
+// memory); the results come back packed in pairs: lo = {D[g][2t], D[g][2t+1]}, hi = the same columns of row g + 8.
 __device__ __forceinline__ void mma_u8s8_c4(uint64_t& lo, uint64_t& hi, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                             uint32_t b1, const int4& c) {
     asm volatile(
@@ -395,17 +375,6 @@ __device__ __forceinline__ void lds128_if(uint4& v, uint32_t addr, bool on) {   
         "@q ld.shared.v4.u32 {%0,%1,%2,%3}, [%5];\n\t}"
         : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
         : "r"(uint32_t(on)), "r"(addr));
-}
-
-__device__ __forceinline__ void mma_u8s8_bias(uint64_t& lo, uint64_t& hi, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                              uint32_t b0, uint32_t b1, int c) {
-    asm volatile(
-        "{\n\t.reg .b32 d0, d1, d2, d3;\n\t"
-        "mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {d0,d1,d2,d3}, {%2,%3,%4,%5}, {%6,%7}, {%8,%8,%8,%8};\n\t"
-        "mov.b64 %0, {d0,d1};\n\t"
-        "mov.b64 %1, {d2,d3};\n\t}"
-        : "=l"(lo), "=l"(hi)
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c));
 }
 
 // Packed fp32 pairs (sm_100 f32x2 arithmetic): each half is an IEEE round-to-nearest operation,

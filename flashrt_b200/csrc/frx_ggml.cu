@@ -74,7 +74,7 @@ struct DotArgs {
     unsigned long long wait_ns;
     // job j has expert ids[j] (0 without ids), activation row j / act_div, output row j
     const int32_t* ids;
-    int n_jobs, act_div;
+    int act_div;
 };
 
 struct DotSmem {
@@ -861,12 +861,11 @@ int frx_gemv_moe_q(uint32_t ggml_type, const void* w, const void* gate, const vo
     a.ncols = int(ncols);
     a.nrows = int(nrows);
     a.ids = ids;
-    a.n_jobs = n_tok * k;
     a.act_div = act_per_expert ? 1 : k;
     if (gate)
-        FRX_LAUNCH(kKGateUp, stream, { if (int rc = launch_dot<true>(a, a.n_jobs, stream)) return rc; });
+        FRX_LAUNCH(kKGateUp, stream, { if (int rc = launch_dot<true>(a, n_tok * k, stream)) return rc; });
     else
-        FRX_LAUNCH(kKDown, stream, { if (int rc = launch_dot<false>(a, a.n_jobs, stream)) return rc; });
+        FRX_LAUNCH(kKDown, stream, { if (int rc = launch_dot<false>(a, n_tok * k, stream)) return rc; });
     return FRX_OK;
 }
 
@@ -887,12 +886,11 @@ int frx_gemv_moe_q2_0(const void* w, const void* gate, const void* xq, const int
     a.ncols = int(ncols);
     a.nrows = int(nrows);
     a.ids = ids;
-    a.n_jobs = n_ids;
     a.act_div = per_channel_act ? 1 : n_ids;   // one activation row for every channel, or one each
     if (gate)
-        FRX_LAUNCH(kKGateUp, stream, { if (int rc = launch_dot<true>(a, a.n_jobs, stream)) return rc; });
+        FRX_LAUNCH(kKGateUp, stream, { if (int rc = launch_dot<true>(a, n_ids, stream)) return rc; });
     else
-        FRX_LAUNCH(kKDown, stream, { if (int rc = launch_dot<false>(a, a.n_jobs, stream)) return rc; });
+        FRX_LAUNCH(kKDown, stream, { if (int rc = launch_dot<false>(a, n_ids, stream)) return rc; });
     return FRX_OK;
 }
 
@@ -909,9 +907,8 @@ int frx_gemv_matvec_q(uint32_t ggml_type, const void* W, const void* xq, float* 
     a.dst = y;
     a.ncols = int(ncols);
     a.nrows = int(nrows);
-    a.n_jobs = n_tok;
     a.act_div = 1;
-    FRX_LAUNCH(kKDown, stream, { if (int rc = launch_dot<false>(a, a.n_jobs, stream)) return rc; });
+    FRX_LAUNCH(kKDown, stream, { if (int rc = launch_dot<false>(a, n_tok, stream)) return rc; });
     return FRX_OK;
 }
 
