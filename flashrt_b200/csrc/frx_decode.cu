@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(1024) k_prologue(const float* __restrict__ log
             float m = 0.0f;
             if (t < T) {
                 route_load<V>(l, E, lane, vec, key);
-                route_select<V>(key, vec, K, lane, my_key, my_id, m);
+                route_select<V>(key, vec, K, lane, my_key, my_id, m, [](float) {});
                 if (lane < K) {
                     const uint32_t sid = smem_u32(dyn) + E * 8 + (t * K + lane) * 4;   // see group_block
 #pragma unroll

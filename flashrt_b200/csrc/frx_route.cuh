@@ -64,9 +64,10 @@ __device__ __forceinline__ double route_sum(const uint32_t (&key)[V], float m) {
     return sum;
 }
 
-// Lane k gets the key and the expert of the k-th winner, all lanes the largest logit m. The keys of the winners become 0.
-template <int V>
-__device__ __forceinline__ void route_select(uint32_t (&key)[V], bool vec, int K, int lane, uint32_t& my_key, int& my_id, float& m) {
+// Lane k gets the key and the expert of the k-th winner, all lanes the largest logit m. The keys of the winners become 0;
+// `whole` is called with m before that.
+template <int V, class Whole>
+__device__ __forceinline__ void route_select(uint32_t (&key)[V], bool vec, int K, int lane, uint32_t& my_key, int& my_id, float& m, Whole whole) {
     auto slot_expert = [&](int i) { return route_expert(vec, lane, i); };
     // every lane keeps its best and its second best key (with their experts): when its best is
     // taken, the second moves up without a rescan; the lane rescans only when it is hit again
@@ -94,6 +95,7 @@ __device__ __forceinline__ void route_select(uint32_t (&key)[V], bool vec, int K
     rescan();
     bool next_valid = true;
     m = key_value(__reduce_max_sync(0xffffffffu, best));
+    whole(m);
     // selection: K rounds on the integer keys only; lane k remembers the k-th winner
     my_key = 0;
     my_id = 0;
@@ -136,12 +138,9 @@ __device__ __forceinline__ void route_warp(const float* __restrict__ l, int E, i
     uint32_t key[V], my_key;
     int my_id;
     float m;
+    double sum;
     route_load<V>(l, E, lane, vec, key);
-    uint32_t top = 0;
-#pragma unroll
-    for (int i = 0; i < V; ++i) top = max(top, key[i]);
-    const double sum = route_sum<V>(key, key_value(__reduce_max_sync(0xffffffffu, top)));
-    route_select<V>(key, vec, K, lane, my_key, my_id, m);
+    route_select<V>(key, vec, K, lane, my_key, my_id, m, [&](float largest) { sum = route_sum<V>(key, largest); });
     const float w = route_weight(my_key, m, sum, K, lane);
     if (lane < K) {
         ids_t[lane] = my_id;
