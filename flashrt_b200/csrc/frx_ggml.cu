@@ -36,10 +36,11 @@ inline size_t act_row_bytes(int64_t ncols) { return size_t(padded_cols(ncols) / 
 // d = amax / 127, q = amax == 0 ? 0 : roundf(x / d); the block keeps half(d), half(sum of the inputs).
 // With `u`, the input is silu(g) * u first (gemv::swiglu_q8_1, kernels/cuda/ggml_gemv.cu:98-107,
 // which uses the fast exponential).
+// `early` lets the next kernel's blocks in at once: see launch_q8_1.
 __global__ void __launch_bounds__(256) k_q8_1(const float* __restrict__ x, const float* __restrict__ u, int64_t ncols, int64_t padded,
-                                              uint8_t* __restrict__ y) {
+                                              uint8_t* __restrict__ y, int early) {
     pdl_wait();
-    pdl_trigger();
+    if (early) pdl_trigger();
     const int64_t i0 = int64_t(blockDim.x) * blockIdx.x + threadIdx.x, t = blockIdx.y;
     if (i0 >= padded) return;   // padded is a multiple of the block
     float xi = 0.0f;
@@ -807,6 +808,14 @@ GmAct plan_act(uint8_t* base, const PlanLayout& L) {
     return GmAct{reinterpret_cast<int8_t*>(base + L.act_q), reinterpret_cast<float*>(base + L.act_d)};
 }
 
+// The next kernel's blocks are let in early only while the whole grid is resident (eight blocks of 256 threads per SM): in a longer
+// one they would wait in places that this kernel's own blocks need.
+cudaError_t launch_q8_1(const float* x, const float* u, int64_t ncols, int n_tok, void* xq, cudaStream_t stream) {
+    const int64_t padded = padded_cols(ncols), blocks = padded / 256 * n_tok;
+    return launch_pdl(k_q8_1, dim3(unsigned(padded / 256), unsigned(n_tok)), dim3(256), 0, stream, x, u, ncols, padded, static_cast<uint8_t*>(xq),
+                      int(blocks <= 8 * sm_count()));
+}
+
 }  // namespace
 }  // namespace frx
 
@@ -828,8 +837,7 @@ int frx_gemv_quantize_q8_1(const float* x, int64_t ncols, int n_tok, void* xq, f
     if (ncols < 1 || n_tok < 0) return fail(FRX_ERR_SHAPE, "gemv::quantize_q8_1: ncols %lld, n_tok %d", (long long)ncols, n_tok);
     if (n_tok == 0) return FRX_OK;
     if (!x || !xq || uintptr_t(xq) % 4) return fail(FRX_ERR_ARG, "gemv::quantize_q8_1: null or misaligned pointer");
-    const int64_t padded = padded_cols(ncols);
-    FRX_LAUNCH(kKQuant, stream, launch_pdl(k_q8_1, dim3(unsigned(padded / 256), unsigned(n_tok)), dim3(256), 0, stream, x, static_cast<const float*>(nullptr), ncols, padded, static_cast<uint8_t*>(xq)));
+    FRX_LAUNCH(kKQuant, stream, launch_q8_1(x, nullptr, ncols, n_tok, xq, stream));
     FRX_CUDA(cudaGetLastError());
     return FRX_OK;
 }
@@ -838,8 +846,7 @@ int frx_gemv_swiglu_q8_1(const float* g, const float* u, int64_t ncols, int n_to
     if (ncols < 1 || n_tok < 0) return fail(FRX_ERR_SHAPE, "gemv::swiglu_q8_1: ncols %lld, n_tok %d", (long long)ncols, n_tok);
     if (n_tok == 0) return FRX_OK;
     if (!g || !u || !xq || uintptr_t(xq) % 4) return fail(FRX_ERR_ARG, "gemv::swiglu_q8_1: null or misaligned pointer");
-    const int64_t padded = padded_cols(ncols);
-    FRX_LAUNCH(kKQuant, stream, launch_pdl(k_q8_1, dim3(unsigned(padded / 256), unsigned(n_tok)), dim3(256), 0, stream, g, u, ncols, padded, static_cast<uint8_t*>(xq)));
+    FRX_LAUNCH(kKQuant, stream, launch_q8_1(g, u, ncols, n_tok, xq, stream));
     FRX_CUDA(cudaGetLastError());
     return FRX_OK;
 }
