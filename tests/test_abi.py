@@ -49,6 +49,15 @@ def test_sizes(L):
     assert L.lib.frx_ep_buffer_bytes(0, 2048) == 0
 
 
+def test_q8_1_sizes_of_the_python_layer(L):
+    # gemv sizes its activation buffers without a call into the library; both say the same
+    from flashrt_b200.moe import gemv
+    for ncols in [1, 31, 32, 33, 480, 511, 512, 513, 640, 1024, 2560, 4095, 4096, 4097, 1 << 20]:
+        for n_tok in (0, 1, 2, 37, 1000):
+            assert gemv._q8_1_bytes(ncols, n_tok) == L.lib.frx_gemv_q8_1_bytes(ncols, n_tok), (ncols, n_tok)
+    assert gemv._q8_1_bytes(2560, 3) == 3 * 5 * 576
+
+
 def test_bad_arguments_are_rejected_with_a_message(L):
     one = C.c_void_p(256)   # never dereferenced: validation fails first
     assert L.lib.frx_q2_repack(None, 4, 256, one, None) == L.ERR_ARG

@@ -381,7 +381,8 @@ def test_stream_stamps_are_written_and_ordered(port):
 
 
 @pytest.mark.parametrize("n,ff,E,K,T,shared", [(128, 128, 1, 1, 1, True), (2048, 512, 48, 10, 4, True), (2560, 640, 40, 10, 3, False),
-                                               (384, 640, 130, 32, 1, True), (512, 256, 600, 12, 6, True), (256, 128, 33, 16, 2, False)])
+                                               (384, 640, 130, 32, 1, True), (512, 256, 600, 12, 6, True), (256, 128, 33, 16, 2, False),
+                                               (512, 256, 128, 8, 7, True), (256, 128, 40, 12, 8, True)])
 def test_two_kernel_form_gives_the_same_bits(port, n, ff, E, K, T, shared):
     # few tokens: routing, grouping and sums by every block; against the other form, which the oracle pins, at one and two
     # warps' worth of slots, one to eight logits per thread, ties in the router, and every unit count of the shapes in use
@@ -394,7 +395,7 @@ def test_two_kernel_form_gives_the_same_bits(port, n, ff, E, K, T, shared):
     x, gate = cuda(synth.activations(T, n)), cuda(np.linspace(-2, 2, T).astype(np.float32))
     for lg in (synth.router_logits(T, E), synth.tie_heavy_logits(T, E), np.zeros((T, E), np.float32)):
         got = []
-        for tokens in (0, 6):
+        for tokens in (0, 8):
             try:
                 check(lib.frx_debug_set_small_tokens(tokens))
                 ids, wts = torch.empty(T, K, dtype=torch.int32, device="cuda"), torch.empty(T, K, device="cuda")
@@ -405,6 +406,9 @@ def test_two_kernel_form_gives_the_same_bits(port, n, ff, E, K, T, shared):
                 out2 = moe.moe_decode(*args, ids, wts, gate, yslot=yslot, ws=ws)      # the given routing
                 moe.workspace_status(ws)
                 got.append((out, out2, ids, wts, yslot))
+                if tokens:   # the second arm is the two-kernel form indeed, with a router and with a given routing
+                    assert launches_by_class(lambda: moe.moe_layer(*args, cuda(lg), gate, K, ws=ws)) == TWO_KERNELS
+                    assert launches_by_class(lambda: moe.moe_decode(*args, ids, wts, gate, ws=ws)) == TWO_KERNELS
             finally:
                 check(lib.frx_debug_set_small_tokens(6))
         assert torch.equal(got[0][2], got[1][2]), "ids"
@@ -415,7 +419,22 @@ def test_two_kernel_form_gives_the_same_bits(port, n, ff, E, K, T, shared):
             assert torch.allclose(a, b, rtol=1e-5, atol=1e-5 * float(a.abs().max()))
 
 
-@pytest.mark.parametrize("T,K", [(1, 3), (2, 10), (4, 10), (5, 9)])
+@pytest.mark.parametrize("n,ff,T,K", [(128, 1408, 4, 3), (2048, 2048, 1, 4), (3968, 128, 2, 5), (1152, 4096, 2, 1)])
+def test_few_tokens_of_wide_experts(port, n, ff, T, K):
+    # widths whose tiles do not fit the other form's shared memory: the two-kernel form takes them, against the oracle
+    E = 6
+    ex = Experts(port, n, ff, E, direct=True)
+    x = synth.activations(T, n)
+    ids, wts, _ = port.route(synth.router_logits(T, E), K)
+    gate = np.linspace(-1, 1, T).astype(np.float32)
+    got = []
+    assert launches_by_class(lambda: got.append(run_decode(ex, x, ids, wts, gate))) == TWO_KERNELS
+    ref, ref_ys, _ = port.moe_layer(ex.routed_planar(), ex.blob_bytes, ex.shared_planar, n, ff, x, ids, wts, gate, n_threads=8, want_slots=True)
+    assert max(rel_max(got[0][1][s], ref_ys[s]) for s in range(T * K)) < 1e-5
+    assert rel_max(got[0][0], ref) < 1e-5
+
+
+@pytest.mark.parametrize("T,K", [(1, 3), (2, 10), (4, 10), (5, 9), (7, 10), (8, 11)])
 def test_two_kernel_hits_give_the_same_bits(port, T, K):
     from flashrt_b200.lib import check, lib
     n, ff = 512, 256
@@ -424,7 +443,7 @@ def test_two_kernel_hits_give_the_same_bits(port, T, K):
     ptrs = torch.tensor((ex.base + rng.integers(0, 16, size=T * K).astype(np.int64) * ex.stride), dtype=torch.int64, device="cuda")
     hit_n = cuda(rng.integers(0, K + 1, size=T).astype(np.int32))
     x, got = cuda(synth.activations(T, n)), []
-    for tokens in (0, 6):
+    for tokens in (0, 8):
         try:
             check(lib.frx_debug_set_small_tokens(tokens))
             yh = torch.full((T, K, n), 7.0, device="cuda")
@@ -432,6 +451,8 @@ def test_two_kernel_hits_give_the_same_bits(port, T, K):
             moe.moe_hits(ptrs, hit_n, K, x, n, ff, yh, scratch=scratch, T=T)
             moe.workspace_status(scratch)
             got.append(yh)
+            if tokens:
+                assert launches_by_class(lambda: moe.moe_hits(ptrs, hit_n, K, x, n, ff, torch.empty_like(yh), scratch=scratch, T=T)) == TWO_KERNELS
         finally:
             check(lib.frx_debug_set_small_tokens(6))
     assert torch.equal(got[0], got[1])
