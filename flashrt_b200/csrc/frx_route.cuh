@@ -128,7 +128,7 @@ __device__ __forceinline__ float route_weight(uint32_t my_key, float m, double s
     float wsum = 0.0f;
     for (int k = 0; k < K; ++k) wsum += __shfl_sync(0xffffffffu, my_p, k);
     wsum = fmaxf(wsum, 6.103515625e-5f);
-    return __fdiv_rn(my_p, wsum);
+    return lane < K ? __fdiv_rn(my_p, wsum) : 0.0f;   // (a quotient of 0 takes the division's slow path)
 }
 
 template <int V>   // logits per lane: E <= 32 * V
