@@ -36,6 +36,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         return LIB
     nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
     cmd = [nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
+           "-Xfatbin", "-compress-all",   # (nvcc compresses device code of its own accord only above some size)
            "-I" + os.path.join(ROOT, "include"), "-I" + os.path.join(HERE, "csrc"),
            "-shared", "-Xcompiler", "-fPIC", "-o", LIB] + sources()
     if verbose:

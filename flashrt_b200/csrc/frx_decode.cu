@@ -981,7 +981,7 @@ __global__ void __launch_bounds__(kChunkSlots) k_pf_place_items(const int32_t* _
 // ---------------------------------------------------------------------------------------------
 
 int g_nw = kStreamWarps;   // warps of k_stream that multiply (8 or kStreamWarps)
-int g_small4 = 0, g_small8 = 8;   // launches of at most this many tasks per SM take blocks of 4 / 8 warps with deeper rings (measured at 1 to 3 tokens: 8 warps 26.9 us per layer, 4 warps 27.7, 16 warps 28.9)
+int g_small8 = 8;   // launches of at most this many tasks per SM take blocks of 8 warps with deeper rings (measured at 1 to 3 tokens, before those had a form of their own: 8 warps 26.9 us per layer, 4 warps 27.7, 16 warps 28.9)
 int g_narrow = 1; // items of at most kNarrowTok tokens take the narrow form of the inner product
 int g_gu_chunks = 0;   // chunks per gate/up task (0: by shape)
 
@@ -1029,13 +1029,12 @@ int stream_cfg(int n, int ff, StreamCfg& c, long long max_items = 0, bool task4 
         cpt = chunks;
         const uint32_t chunk = task_bytes / uint32_t(cpt);
         int first = g_nw;
-        if (max_tasks > 0 && max_tasks <= (long long)g_small4 * sms) first = 4;
-        else if (max_tasks > 0 && max_tasks <= (long long)g_small8 * sms) first = 8;
+        if (max_tasks > 0 && max_tasks <= (long long)g_small8 * sms) first = 8;
         const int prefs[2] = {first, 8};
         for (int k = 0; k < 2; ++k) {
             nw = prefs[k];
             for (nbuf = kMaxItemBufs; nbuf >= 2; --nbuf)
-                for (rpw = nw <= 4 ? 8 : 4; rpw >= 2; --rpw) {
+                for (rpw = 4; rpw >= 2; --rpw) {
                     bytes = smem_plan(kdim, chunk, nw * rpw, nbuf).total;
                     if (int(bytes) <= budget) return true;
                 }
@@ -1108,7 +1107,6 @@ void launch_stream_nw(const StreamParams& p, int upc, uint32_t smem, cudaStream_
 template <bool GATE_UP, bool TASK4>
 void launch_stream(const StreamParams& p, int nw, int upc, uint32_t smem, cudaStream_t stream) {
     switch (nw) {
-        case 4: launch_stream_nw<GATE_UP, TASK4, 4>(p, upc, smem, stream); break;
         case 8: launch_stream_nw<GATE_UP, TASK4, 8>(p, upc, smem, stream); break;
         default: launch_stream_nw<GATE_UP, TASK4, kStreamWarps>(p, upc, smem, stream); break;
     }
@@ -1134,7 +1132,6 @@ int set_smem_attr() {
     std::lock_guard<std::mutex> lk(mu);
     if (dev >= 0 && dev < 64 && done[dev]) return FRX_OK;
     const int lim = max_smem_optin() - 2048;   // dynamic part only: the kernels also hold a little static shared memory
-    if (int rc = set_stream_attr<4>(lim)) return rc;
     if (int rc = set_stream_attr<8>(lim)) return rc;
     if (int rc = set_stream_attr<kStreamWarps>(lim)) return rc;
     const void* fns[] = {
@@ -1853,7 +1850,6 @@ int frx_debug_set_consumer_warps(int nw) {
 }
 int frx_debug_set_small_launch_limits(int four_warps, int eight_warps) {
     if (four_warps < 0 || eight_warps < four_warps) return FRX_ERR_ARG;
-    g_small4 = four_warps;
     g_small8 = eight_warps;
     return FRX_OK;
 }
