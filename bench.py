@@ -699,7 +699,7 @@ def bench_verify_stack(torch, moe, synth, dev, rank, world, L, layer, timeit, la
     """the expert stack walked by a speculative-verify window of three tokens
     (1 + 2 drafts), the layers chained by x_next = rmsnorm_unit(x + y) in fp32, router logits
     pre-generated per layer; expert parallel when launched on several GPUs. The step is bound by
-    48 x (five dependent kernels + the exchange), not by HBM: the fraction says how far."""
+    48 x (two dependent kernels and the join; on several GPUs five and the exchange), not by HBM: the fraction says how far."""
     T3 = 3
     ls_, gs_ = logits[:, :T3].contiguous(), gate[:, :T3].contiguous()
     xs = torch.empty(L + 1, T3, N_MODEL, device=dev)       # xs[l]: the input of layer l
@@ -721,7 +721,7 @@ def bench_verify_stack(torch, moe, synth, dev, rank, world, L, layer, timeit, la
     res = {"workload": f"configs[3]: {L} chained layers, {T3} tokens per step, 512 experts top-10 + shared, ep{world}",
            "value": round(T3 / (t * 1e-3), 1), "unit": "tokens/s", "ms_per_step": round(t, 4), "us_per_layer": round(t * 1e3 / L, 2),
            "algorithmic_bytes_per_step": int(step_bytes), "hbm_frac_of_peak": round(step_bytes / world / (t * 1e-3) / 1e9 / peak, 4),
-           "note": "latency-limited: a layer is five dependent kernels (plus the exchange on several GPUs) over about 10 MB of weights"}
+           "note": "latency-limited: a layer is two dependent kernels and the join (on several GPUs five and the exchange) over about 10 MB of weights"}
     if rank == 0 and port is not None:
         # Parity. The oracle needs only the experts the window uses: each layer's blobs are regenerated
         # on the device and the used ones copied out. Two figures: every layer's output against the
@@ -990,7 +990,7 @@ def main():
     ap.add_argument("--no-graph", action="store_true")
     ap.add_argument("--no-cpu", action="store_true")
     ap.add_argument("--no-extras", action="store_true", help="headline only: skip the decode_batches, prefill and verify_stack keys")
-    ap.add_argument("--nw", type=int, default=0, help="tuning: consumer warps of the streaming kernel (8, 12, 16, 20)")
+    ap.add_argument("--nw", type=int, default=0, help="tuning: warps of the streaming kernel that multiply (8 or 12)")
     ap.add_argument("--fused", type=int, default=None, help="tuning: 0 runs the decode FFN as three kernels instead of one")
     ap.add_argument("--deal-shared", type=int, default=1, help="expert parallel: 1 deals the shared expert's tokens among the ranks, 0 leaves them all to rank 0")
     ap.add_argument("--down-weight", type=int, default=None, help="tuning: weight (in 1/16) of a down task of a 3-4 token item in the split over blocks; 0 = even split")

@@ -12,7 +12,8 @@
 //                 rows of every item, so the weighted sum over a token's experts needs no other block.
 // Both split K over warps: the terms d * (a0 * S0 + a1 * S1) of a row's blocks are independent, only their sum
 // has an order. The terms go through shared memory and one thread per (row, token) adds them in block
-// order, so the results are the same bits as those of k_stream. Four row groups (up) or four items (down)
+// order, so a slot's row is the same bits as that of k_stream. (Routing weights may differ from k_route_topk's in their last
+// bit: the double-precision softmax sum is added in another order.) Four row groups (up) or four items (down)
 // are chained into one accumulator as in units_mma_n2.
 
 constexpr int kSmallTok = 2;                          // tokens of an item

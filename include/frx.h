@@ -62,7 +62,8 @@ const char* frx_profile_class_name(int cls);
 
 /* Tuning knobs for measurements and tests; no counterpart in the reference. Process-wide and not
  * thread-safe: set them before any compute call, not while calls are in flight.
- * frx_debug_set_consumer_warps: 8: blocks of the streaming expert kernel have 8 warps; 12, 16 or 20 (default): 12 that multiply and 4 that build.
+ * frx_debug_set_consumer_warps: 8: blocks of the streaming expert kernel have 8 warps that multiply and build item buffers;
+ * 12 (default), and 16 or 20 likewise: 12 that multiply and 4 that build.
  * frx_debug_set_gate_up_chunks: the number of K slices a gate/up task is fetched in (0: chosen by shape).
  * frx_debug_set_narrow_items: 1 (default) lets work items of at most four tokens take the narrow
  * form of the inner product (two row groups share one MMA accumulator, half the float work per row);
@@ -103,10 +104,11 @@ int frx_debug_set_down_item_weight(int sixteenths);
  * streaming kernels (three-kernel form) writes four globaltimer stamps per block there, gate/up's blocks first,
  * then down's: [0] block started, [1] the kernels in front have ended, [2] first item buffer built, [3] block
  * finished; and block 0 of the layer's first kernel four more behind them: [0] the kernels in front have ended,
- * [1] its own tokens routed, [2] all tokens routed, [3] work items written. NULL (default) switches it off. */
+ * [1] and [2] all tokens routed, [3] work items written. NULL (default) switches it off. */
 int frx_debug_set_stream_stamps(void* device_buffer);
 /* Calls of at most `tokens` tokens (0 .. 8, default 6; 0: never) may take the two-kernel form of the decode layer
- * and of frx_moe_hits, where it is the faster one. Same bits either way. */
+ * and of frx_moe_hits, where it is the faster one. Same ids and per-slot rows bit for bit; routing weights may differ in their
+ * last bit (the softmax sum is added in another order, in double), and the layer's output with them. */
 int frx_debug_set_small_tokens(int tokens);
 int frx_debug_set_ffn_buffers(int gate_up, int down);
 int frx_debug_set_wait_limit_ns(unsigned long long ns);
