@@ -391,6 +391,8 @@ __global__ void __launch_bounds__(kRqThreads, 6) k_q8_0_to_q2_0(const uint8_t* _
     const uint8_t* s = src + b0 * 68;
     if (nb == kRqThreads && uintptr_t(s) % 16 == 0) {
         for (int i = tid; i < kRqThreads * 68 / 16; i += kRqThreads) reinterpret_cast<uint4*>(in)[i] = reinterpret_cast<const uint4*>(s)[i];
+    } else if (uintptr_t(s) % 4 == 0) {   // the last blocks of a call, and sources that are not aligned to vectors
+        for (int i = tid; i < nb * 17; i += kRqThreads) reinterpret_cast<uint32_t*>(in)[i] = reinterpret_cast<const uint32_t*>(s)[i];
     } else {
         for (int i = tid; i < nb * 68; i += kRqThreads) in[i] = s[i];
     }
@@ -535,6 +537,8 @@ __global__ void __launch_bounds__(kRqThreads, 6) k_q8_0_to_q2_0(const uint8_t* _
     uint8_t* d = dst + b0 * 18;
     if (nb == kRqThreads && uintptr_t(d) % 16 == 0) {
         for (int i = tid; i < kRqThreads * 18 / 16; i += kRqThreads) reinterpret_cast<uint4*>(d)[i] = reinterpret_cast<const uint4*>(out)[i];
+    } else if (uintptr_t(d) % 2 == 0) {
+        for (int i = tid; i < nb * 9; i += kRqThreads) reinterpret_cast<uint16_t*>(d)[i] = reinterpret_cast<const uint16_t*>(out)[i];
     } else {
         for (int i = tid; i < nb * 18; i += kRqThreads) d[i] = out[i];
     }

@@ -130,6 +130,15 @@ def test_requantizer_bit_exact(port):
     assert not diff.any(), f"{int(diff.sum())} of {diff.size} blocks differ, first at {int(np.argmax(diff))}"
 
 
+@pytest.mark.parametrize("n,offset", [(1, 0), (100, 0), (127, 4), (129, 0), (301, 4), (301, 1), (256, 2)])
+def test_requantizer_copies(port, n, offset):
+    # whole and partial blocks of threads, sources aligned to vectors, words and bytes
+    src = q8_0_edge_blocks(n, seed=n)[:n * 68]
+    buf = torch.zeros(src.size + offset, dtype=torch.uint8, device="cuda")
+    buf[offset:] = cuda(src)
+    assert np.array_equal(moe.convert_q8_0_to_q2_0(buf[offset:]).cpu().numpy(), port.convert_q8_0_to_q2_0(src))
+
+
 def test_unsupported_type_and_shapes_are_rejected():
     z = torch.zeros(4096, dtype=torch.uint8, device="cuda")
     ids = torch.zeros(1, 1, dtype=torch.int32, device="cuda")
