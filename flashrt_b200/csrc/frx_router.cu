@@ -6,7 +6,7 @@
 // additions differs from the reference's (and from one GPU generation's launch shape to another in
 // the reference itself), so parity is to a tolerance, against a float64 sum.
 //
-// One block works on tiles of 8 rows x 16 tokens or 16 rows x 16, 24 or 40. Each of its 8 warps takes an eighth of K and
+// One block works on tiles of 8 rows x 16 or 64 tokens or 16 rows x 16, 24 or 40. Each of its 8 warps takes an eighth of K and
 // walks it in pieces of 32: the piece of x (fp32) and of W (bf16) go through the warp's own shared memory (cp.async),
 // a lane accumulates 4 rows x TJ tokens, and at the end the eight partial tiles are added in warp order (fixed, so results
 // are reproducible and do not depend on the tile).
@@ -31,8 +31,9 @@ struct RtShape {
     static constexpr int piece = tok * kRtPad * 4 + rows * kRtPiece * 2;   // x (fp32, padded rows), W (bf16)
     static constexpr int warp = depth * piece;
     static constexpr int smem = kRtWarps * warp;
+    static constexpr int red = tok + 1;   // row of partial sums: odd, the sums are read across rows
     static_assert(rows % 8 == 0 && tok % 4 == 0, "the copies take 8 rows of W and 4 tokens at a time");
-    static_assert(kRtWarps * rows * tok * 4 <= smem, "the reduction buffer reuses the pieces' shared memory");
+    static_assert(kRtWarps * rows * red * 4 <= smem, "the reduction buffer reuses the pieces' shared memory");
 };
 
 __device__ __forceinline__ float bf16_lo(uint32_t u) { return __uint_as_float(u << 16); }
@@ -131,14 +132,14 @@ __global__ void __launch_bounds__(kRtWarps * 32, 2) k_router_logits(const uint16
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int j = 0; j < TJ; ++j) red[(warp * Sh::rows + ry + RY * i) * Sh::tok + tx + Sh::tx * j] = acc[i][j];
+            for (int j = 0; j < TJ; ++j) red[(warp * Sh::rows + ry + RY * i) * Sh::red + tx + Sh::tx * j] = acc[i][j];
         __syncthreads();
         for (int o = threadIdx.x; o < Sh::rows * Sh::tok; o += kRtWarps * 32) {
             const int row = o % Sh::rows, tok = o / Sh::rows, rr = r0 + row, t = t0 + tok;   // (rows of a token are neighbours in the output)
-            const float* pr = red + row * Sh::tok + tok;
+            const float* pr = red + row * Sh::red + tok;
             float sum = pr[0];
 #pragma unroll
-            for (int w = 1; w < kRtWarps; ++w) sum += pr[w * Sh::rows * Sh::tok];
+            for (int w = 1; w < kRtWarps; ++w) sum += pr[w * Sh::rows * Sh::red];
             if (t < T) {
                 if (rr < E) logits[size_t(t) * E + rr] = sum;
                 else if (rr < rows_total && gate_logit) gate_logit[t] = sum;
@@ -191,9 +192,15 @@ extern "C" int frx_router_logits(frx_stream_t stream, const void* w_router, cons
     const int rows = E + (w_gate ? 1 : 0), sms = sm_count();
     // few tokens: small tiles, as long as no SM gets a second one
     if (router_tiles<2, 1>(rows, T) <= sms) return launch_router<2, 1>(wr, wg, x, T, E, n, logits, gate_logit, stream);
-    // else the tile for which the busiest SM finishes first: a tile costs about TJ + 1 (measured at 37 to 1024 tokens)
-    auto cost = [&](int tiles, int tj) { return (tiles + sms - 1) / sms * (tj + 1); };
-    const int c2 = cost(router_tiles<4, 2>(rows, T), 2), c3 = cost(router_tiles<4, 3>(rows, T), 3), c5 = cost(router_tiles<4, 5>(rows, T), 5);
+    // up to eight rows leave half of a tile of 16 empty: eight rows x 64 tokens (8 experts, 16,384 tokens of 1024: 27.3 us in tiles of
+    // 16 rows, 16.7 so; 4,096 tokens of 256: 3.8 and 3.6)
+    if (rows <= 8) return launch_router<2, 4>(wr, wg, x, T, E, n, logits, gate_logit, stream);
+    // else the tile for which the busiest SM finishes first: one of 16 rows costs about TJ + 1 (measured at 37 to 1024 tokens), one of
+    // 8 x 64 about 6.5; the latter comes out ahead at 17 to 24 rows (16 experts and the gate, 6,000 tokens of 1024: 17.9 us in tiles
+    // of 16 rows, 16.7 so)
+    auto cost = [&](int tiles, int each) { return (tiles + sms - 1) / sms * each; };
+    const int c2 = cost(router_tiles<4, 2>(rows, T), 6), c3 = cost(router_tiles<4, 3>(rows, T), 8), c5 = cost(router_tiles<4, 5>(rows, T), 12);
+    if (cost(router_tiles<2, 4>(rows, T), 13) < std::min({c2, c3, c5})) return launch_router<2, 4>(wr, wg, x, T, E, n, logits, gate_logit, stream);
     if (c2 <= c3 && c2 <= c5) return launch_router<4, 2>(wr, wg, x, T, E, n, logits, gate_logit, stream);
     if (c3 <= c5) return launch_router<4, 3>(wr, wg, x, T, E, n, logits, gate_logit, stream);
     return launch_router<4, 5>(wr, wg, x, T, E, n, logits, gate_logit, stream);

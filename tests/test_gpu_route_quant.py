@@ -111,7 +111,8 @@ def test_router_projection(T, E, n, gate):
     assert np.array_equal(ids.cpu().numpy(), top)
 
 
-@pytest.mark.parametrize("T,E", [(15, 512), (16, 40), (17, 512), (33, 512), (40, 15), (41, 512), (64, 512), (137, 511), (293, 512), (321, 16)])
+@pytest.mark.parametrize("T,E", [(15, 512), (16, 40), (17, 512), (33, 512), (40, 15), (41, 512), (64, 512), (137, 511), (293, 512), (321, 16),
+                                 (2369, 7), (2433, 3), (9473, 7), (2400, 8), (6001, 16)])
 def test_router_projection_same_bits_for_any_tile(T, E):
     # every tile adds in the same order (eight slices of n one after the other), so a token's logits do not
     # depend on how many tokens the call has; tails of rows and tokens included
