@@ -817,7 +817,7 @@ GmAct plan_act(uint8_t* base, const PlanLayout& L) {
 cudaError_t launch_q8_1(const float* x, const float* u, int64_t ncols, int n_tok, void* xq, cudaStream_t stream) {
     const int64_t padded = padded_cols(ncols), blocks = padded / 256 * n_tok;
     return launch_pdl(k_q8_1, dim3(unsigned(padded / 256), unsigned(n_tok)), dim3(256), 0, stream, x, u, ncols, padded, static_cast<uint8_t*>(xq),
-                      int(blocks <= 8 * sm_count()));
+                      int(blocks <= 512 || blocks <= 8 * sm_count()));   // (64 SMs are there in any case: one token's call does not ask for the number)
 }
 
 }  // namespace
