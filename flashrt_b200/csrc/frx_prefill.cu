@@ -159,10 +159,25 @@ __global__ void __launch_bounds__(256) k_pfu_expand_q8(const int8_t* __restrict_
     *reinterpret_cast<uint32_t*>(blk + piece_chunk(s, 1, t) * 16 + piece_byte(q, t)) = lo;
 }
 
+// silu(g) * u with the fast exponential and reciprocal, within kSwigluErr of swiglu_ref for g >= -80: ex2 and rcp are good to 2^-22 and
+// 2^-23 (PTX ISA), -g log2 e rounds by at most 2^-24 of 116, which the exponential makes 2^-17.6, three more roundings.
+constexpr float kSwigluErr = 0x1p-16f;
+__device__ __forceinline__ float swiglu_fast(float g, float u) {
+    float e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(g * -1.44269504f));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+    return g * r * u;
+}
+
 // Q8 of the hidden rows (in the grouped order, the first *n_rows of them) into e4m3 pieces and block scales, like
 // k_pfu_quant_x. A thread owns the eight values of element group t of a 32-block (4 t .. + 3 and 16 + 4 t .. + 3), four
-// neighbouring lanes one 32-block: silu(gate x) * up x is formed here (eight independent exponentials
-// per thread hide their latency), the block maximum comes from two shuffles, each piece is one 8-byte store.
+// neighbouring lanes one 32-block: silu(gate x) * up x is formed here, the block maximum comes from two shuffles, each piece is
+// one 8-byte store.
+//
+// The codes are those of swiglu_ref, but only two kinds of values need it: those that may be a block's largest (it sets the scale), and
+// those whose code could round the other way. All values are formed fast; the ones in question, in a few rounds of at most one per lane
+// (between one and two for a warp's 256 values), once more exactly. Bound: HBM (10 bytes a value, 130 us at 163,840 rows of 512) and issue:
+// 179 us there, 254 with the double-precision exponential for every value.
 __global__ void __launch_bounds__(256) k_pfu_quant_h(const float2* __restrict__ hf, int ff, const int* __restrict__ n_rows, uint8_t* __restrict__ he,
                                                      float* __restrict__ hd, int block64) {
     pdl_wait();
@@ -178,30 +193,68 @@ __global__ void __launch_bounds__(256) k_pfu_quant_h(const float2* __restrict__ 
     const float4* src = reinterpret_cast<const float4*>(hf + blk * kQ8);
     float hv[8];
     float am = 0.0f;
+    uint32_t ask = 0;   // values to be formed exactly
 #pragma unroll
     for (int q = 0; q < 2; ++q)
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const float4 gu = src[q * 8 + t * 2 + i];   // (gate, up) of two hidden values
-            hv[q * 4 + 2 * i] = swiglu_ref(gu.x, gu.y);
-            hv[q * 4 + 2 * i + 1] = swiglu_ref(gu.z, gu.w);
+            hv[q * 4 + 2 * i] = swiglu_fast(gu.x, gu.y);
+            hv[q * 4 + 2 * i + 1] = swiglu_fast(gu.z, gu.w);
+            ask |= uint32_t(!(gu.x >= -80.0f)) << (q * 4 + 2 * i) | uint32_t(!(gu.z >= -80.0f)) << (q * 4 + 2 * i + 1);
         }
+    auto block_max = [&](float v) {
+        v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
+        v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
+        if (block64) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 4));   // eight lanes hold one 64-value scale block
+        return v;
+    };
+    auto exact = [&](int i) {
+        const float2 gu = hf[blk * kQ8 + (i >> 2) * 16 + t * 4 + (i & 3)];
+        return swiglu_ref(gu.x, gu.y);
+    };
 #pragma unroll
     for (int i = 0; i < 8; ++i) am = fmaxf(am, fabsf(hv[i]));
-    am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 1));
-    am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 2));
-    if (block64) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 4));   // eight lanes hold one 64-value scale block
+    am = block_max(am);
+    // (no number, none at all, and so large or small that an intermediate of the fast form may leave the range of floats: everything exactly)
+    if (!(am > 1e-25f && am < 1e25f)) ask = 0xffu;
+    const float lim = am * (1.0f - 4.0f * kSwigluErr);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ask |= uint32_t(!(fabsf(hv[i]) < lim)) << i;
+    am = 0.0f;
+    while (__any_sync(0xffffffffu, ask != 0)) {
+        if (ask) {
+            const int i = __ffs(ask) - 1;
+            ask &= ask - 1;
+            const float v = exact(i);
+            am = fmaxf(am, fabsf(v));
+#pragma unroll
+            for (int k = 0; k < 8; ++k) hv[k] = k == i ? v : hv[k];
+        }
+    }
+    am = block_max(am);
     // quant/q2_0/q2_0.cpp:101-113: d = amax / 127, id = 1 / d, q = roundf(v * id), d through fp16
     const float d = __fdiv_rn(am, 127.0f);
     const float id = d != 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
+    int code[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float c = __fmul_rn(hv[i], id), m = c + kMagic;   // |c| <= 127 and a bit
+        code[i] = __float_as_int(m) - kMagicBits;
+        ask |= uint32_t(!(fabsf(c - (m - kMagic)) < 0.5f - 2.0f * kSwigluErr * fabsf(c))) << i;
+    }
+    while (__any_sync(0xffffffffu, ask != 0)) {
+        if (ask) {
+            const int i = __ffs(ask) - 1;
+            ask &= ask - 1;
+            const int c = int(round_half_away(__fmul_rn(exact(i), id)));
+#pragma unroll
+            for (int k = 0; k < 8; ++k) code[k] = k == i ? c : code[k];
+        }
+    }
     uint32_t hi[2], lo[2];
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-        int code[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) code[i] = int(round_half_away(__fmul_rn(hv[4 * q + i], id)));
-        split_codes(code, hi[q], lo[q]);
-    }
+    for (int q = 0; q < 2; ++q) split_codes(*reinterpret_cast<const int(*)[4]>(code + 4 * q), hi[q], lo[q]);
     if (!live) return;
     uint8_t* o = he + (blk >> 1) * 128 + piece_byte(0, t);
     *reinterpret_cast<uint2*>(o + piece_chunk(s, 0, t) * 16) = make_uint2(hi[0], hi[1]);

@@ -161,6 +161,31 @@ def test_hidden_quantizer_where_rows_end_inside_a_warp(port, S, block64):
     assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("block64", [False, True])
+@pytest.mark.parametrize("spread", [0.02, 8.0, 6e4, "special"])
+def test_hidden_quantizer_over_the_range_of_the_swiglu(port, spread, block64):
+    # gate values from a few units (where codes lie next to rounding boundaries) to beyond the exponential's range, products beyond that of
+    # floats, rows of zeros, infinite and missing numbers: the codes are those of the exact SwiGLU, to the bit
+    n, ff, E, S = 256, 384, 2, 333
+    rng = np.random.default_rng(11)
+    planar = np.zeros((E, moe.expert_bytes(n, ff)), np.uint8)
+    off = 0
+    for rows, cols in ((ff, n), (ff, n), (n, ff)):
+        nblk = rows * cols // 64
+        planar[:, off:off + nblk * 16] = rng.integers(0, 256, (E, nblk * 16))
+        scale = rng.normal(0, 0.02 if spread == "special" or cols == ff else spread, (E, nblk)).clip(-6e4, 6e4).astype(np.float16)
+        if spread == "special" and cols == n:
+            scale[:, rng.integers(0, nblk, 40)] = rng.choice(np.array([np.inf, -np.inf, np.nan, 6e4, 6e-8], np.float16), 40)
+            scale[0, :nblk // 4] = 0
+        planar[:, off + nblk * 16:off + nblk * 18] = scale.view(np.uint8)
+        off += nblk * 18
+    tiled = moe.tile_experts(cuda(planar.reshape(-1)), n, ff, E)
+    x = synth.activations(S, n) * rng.choice(np.array([1e-30, 1e-3, 1.0, 3e4], np.float32), (S, 1))
+    ids = cuda(rng.integers(0, E, (S, 1)).astype(np.int32))
+    got, want = (moe.moe_q2.run_ex(tiled.data_ptr(), moe.expert_stride(n, ff), E, n, ff, cuda(x), ids, block64=block64, form=f) for f in ("umma", "stream"))
+    assert torch.allclose(got, want, rtol=0, atol=0, equal_nan=True)
+
+
 @pytest.mark.parametrize("n,ff,E,K,per_expert,umma", [(2048, 512, 1, 1, 64, False), (2560, 640, 2, 2, 200, False), (512, 256, 8, 4, 32, False), (512, 256, 64, 8, 31, False),
                                                       (512, 256, 64, 8, 48, True), (2048, 512, 64, 8, 64, True), (384, 640, 16, 4, 300, True), (4096, 1024, 1, 1, 40, True)])
 def test_prefill_takes_the_form_that_fills_the_gpu(port, n, ff, E, K, per_expert, umma):
