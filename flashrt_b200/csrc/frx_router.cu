@@ -6,171 +6,171 @@
 // additions differs from the reference's (and from one GPU generation's launch shape to another in
 // the reference itself), so parity is to a tolerance, against a float64 sum.
 //
-// One block works on tiles of 8 rows x 16 or 64 tokens or 16 rows x 16, 24 or 40. Each of its 8 warps takes an eighth of K and
-// walks it in pieces of 32: the piece of x (fp32) and of W (bf16) go through the warp's own shared memory (cp.async),
-// a lane accumulates 4 rows x TJ tokens, and at the end the eight partial tiles are added in warp order (fixed, so results
-// are reproducible and do not depend on the tile).
-// Bound: the latency of a chain of pieces for few tokens (hence four in flight in the small tile); with more, what a
-// shared-memory load delivers (128 bytes a clock: 24 clocks of loads and 16 of multiply-adds per 4 x 4 x 4) and the last
-// wave. Rows of x are padded so that no two tokens of a quarter-warp share a bank.
-// 513 rows of 2560, us: 17 tokens 16.6 -> 7.2, 37 tokens 17.2 -> 9.4, 293 tokens 49 -> 30, 1024 tokens 126 -> 89 (before: one
-// tile of 8 x 64 for any number of tokens, one piece in flight).
+// The products run on the tensor cores without losing a bit: an fp32 value is the sum of three bf16 values of eight significant
+// bits each (cut off, not rounded; of an activation below 2^-110 what is below 2^-133 is lost), so W x = W hi + W mid + W lo, every
+// product exact in fp32. Three chained MMAs of 16 K start at
+// zero and their result is added to a running fp32 sum, so what is rounded is 16 K at a time.
+//
+// A block works on a tile of 16 MT rows x 8 NT tokens; each of its 8 warps takes an eighth of K and walks it 32 at a time, straight from
+// global memory into the MMA's registers: a lane takes eight neighbouring K of a row (one 16-byte load) and of a token (two), which is
+// another order of K inside the 32, the same for both operands. At the end the eight partial tiles are added in warp order
+// (fixed, so results are reproducible and do not depend on the tile).
+// Bound: the latency of a step (a load from the L2, the split, chains of three MMAs) with two pieces in flight, and for many tokens what the
+// L2 delivers (all blocks together read x once per row tile and W once per token tile: 63 MB at 293 tokens in tiles of 48 x 32, 200 MB in
+// tiles of 16 x 8). 513 rows of 2560, us: 1 token 6.1 ->
+// 3.8, 37 tokens 9.2 -> 5.4, 293 tokens 29.5 -> 16.8, 1024 tokens 87 -> 45 (before: multiply-adds from shared memory). Error against float64,
+// relative 2-norm: 1.1e-7, 3.2e-7 before (320 additions in a row).
 #include "frx_common.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <mutex>
 
 namespace frx {
 namespace {
 
-constexpr int kRtWarps = 8, kRtPiece = 32, kRtPad = 36;   // 36: rows stay 16-byte aligned, no bank conflicts
-// RY lanes along the rows (4 rows each), 32 / RY along the tokens (TJ tokens each)
-template <int RY, int TJ>
-struct RtShape {
-    static constexpr int tx = 32 / RY, rows = 4 * RY, tok = tx * TJ, depth = TJ == 1 ? 4 : 2;
-    static constexpr int piece = tok * kRtPad * 4 + rows * kRtPiece * 2;   // x (fp32, padded rows), W (bf16)
-    static constexpr int warp = depth * piece;
-    static constexpr int smem = kRtWarps * warp;
-    static constexpr int red = tok + 1;   // row of partial sums: odd, the sums are read across rows
-    static_assert(rows % 8 == 0 && tok % 4 == 0, "the copies take 8 rows of W and 4 tokens at a time");
-    static_assert(kRtWarps * rows * red * 4 <= smem, "the reduction buffer reuses the pieces' shared memory");
-};
+constexpr int kRtWarps = 8, kRtPiece = 32;
 
-__device__ __forceinline__ float bf16_lo(uint32_t u) { return __uint_as_float(u << 16); }
-__device__ __forceinline__ float bf16_hi(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
-// 16 bytes global -> shared without passing through registers; src_bytes = 0 writes zeros
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t src_bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
+// D = A * B + D, bf16 operands, fp32 sums
+__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// The three bf16 pieces of two values, packed. (An infinity is its own first piece; what is left of a number that is none is none.)
+__device__ __forceinline__ void split_pair(float a, float b, uint32_t (&p)[3]) {
+    const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
+    p[0] = __byte_perm(ua, ub, 0x7632);
+    const float ra = fabsf(a) == INFINITY ? 0.0f : a - __uint_as_float(ua & 0xffff0000u), rb = fabsf(b) == INFINITY ? 0.0f : b - __uint_as_float(ub & 0xffff0000u);
+    const uint32_t va = __float_as_uint(ra), vb = __float_as_uint(rb);
+    p[1] = __byte_perm(va, vb, 0x7632);
+    p[2] = __byte_perm(__float_as_uint(ra - __uint_as_float(va & 0xffff0000u)), __float_as_uint(rb - __uint_as_float(vb & 0xffff0000u)), 0x7632);
+}
 
 // rows: E router rows followed by the gate row when w_gate is given (row E). W rows are n bf16 each.
-template <int RY, int TJ>
-__global__ void __launch_bounds__(kRtWarps * 32, 2) k_router_logits(const uint16_t* __restrict__ w_router, const uint16_t* __restrict__ w_gate,
+template <int MT, int NT>
+__global__ void __launch_bounds__(kRtWarps * 32, MT * NT <= 4 ? 2 : 1) k_router_logits(const uint16_t* __restrict__ w_router, const uint16_t* __restrict__ w_gate,
                                                                   const float* __restrict__ x, int T, int E, int n,
                                                                   float* __restrict__ logits, float* __restrict__ gate_logit) {
-    using Sh = RtShape<RY, TJ>;
-    extern __shared__ __align__(16) uint8_t smem[];
+    constexpr int kRows = 16 * MT, kTok = 8 * NT, kRed = kRows + 1;   // partial sums are kept per token: [token][row], odd rows
+    extern __shared__ float red[];   // [warp][token][row]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+    const int rows_total = E + (w_gate ? 1 : 0), row_tiles = (rows_total + kRows - 1) / kRows;
+    const int r0 = int(blockIdx.x) % row_tiles * kRows, t0 = int(blockIdx.x) / row_tiles * kTok;
+    const int steps = n / (kRtWarps * kRtPiece);
+    const size_t k0 = size_t(warp) * steps * kRtPiece + t4 * 8;
+    const uint16_t* wp[MT][2];   // rows beyond the last repeat it, tokens likewise; neither is stored
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int r = min(r0 + 16 * i + 8 * h + g, rows_total - 1);
+            wp[i][h] = (r < E ? w_router + size_t(r) * n : w_gate) + k0;
+        }
+    const float* xp[NT];
+#pragma unroll
+    for (int j = 0; j < NT; ++j) xp[j] = x + size_t(min(t0 + 8 * j + g, T - 1)) * n + k0;
+    struct Piece {
+        uint4 w[MT][2];
+        float4 x[NT][2];
+    };
+    auto load = [&](Piece& p, int s) {
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) p.w[i][h] = __ldg(reinterpret_cast<const uint4*>(wp[i][h] + s * kRtPiece));
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) p.x[j][h] = *(reinterpret_cast<const float4*>(xp[j] + s * kRtPiece) + h);
+    };
+    float acc[MT][NT][4];
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc[i][j][k] = 0.0f;
+    auto multiply = [&](const Piece& p) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {   // the first and the second four of a lane's eight K
+            uint32_t b[NT][2][3];
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+                split_pair(p.x[j][h].x, p.x[j][h].y, b[j][0]);
+                split_pair(p.x[j][h].z, p.x[j][h].w, b[j][1]);
+            }
+#pragma unroll
+            for (int i = 0; i < MT; ++i) {
+                const uint32_t a0 = h ? p.w[i][0].z : p.w[i][0].x, a2 = h ? p.w[i][0].w : p.w[i][0].y, a1 = h ? p.w[i][1].z : p.w[i][1].x, a3 = h ? p.w[i][1].w : p.w[i][1].y;
+#pragma unroll
+                for (int j = 0; j < NT; ++j) {
+                    float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                    for (int k = 2; k >= 0; --k) mma_bf16(d, a0, a1, a2, a3, b[j][0][k], b[j][1][k]);   // the smallest first
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) acc[i][j][k] += d[k];
+                }
+            }
+        }
+    };
+    // W is a weight: its first piece may come in before the kernels in front have ended
+    Piece p[2];
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) touch_l2(wp[i][h]);
     pdl_wait();
     pdl_trigger();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t mine = smem_u32(smem) + warp * Sh::warp;
-    const int rows_total = E + (w_gate ? 1 : 0), row_tiles = (rows_total + Sh::rows - 1) / Sh::rows, tiles = row_tiles * ((T + Sh::tok - 1) / Sh::tok);
-    const int ry = lane / Sh::tx, tx = lane % Sh::tx;   // this lane's tile: rows ry + RY i, tokens tx + Sh::tx j (no bank conflicts)
-    const int kslice = n / kRtWarps, pieces = kslice / kRtPiece, kbase = warp * kslice;
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const int r0 = tile % row_tiles * Sh::rows, t0 = tile / row_tiles * Sh::tok;
-        const int wrow = lane >> 2, wk = (lane & 3) * 8;   // this lane's 8 weights of a piece, in rows wrow, wrow + 8, ...
-        const uint16_t* wsrc[Sh::rows / 8];
-        uint32_t wbytes[Sh::rows / 8];
+    load(p[0], 0);
+    for (int s = 0; s < steps; s += 2) {
+        if (s + 1 < steps) load(p[1], s + 1);
+        multiply(p[0]);
+        if (s + 2 < steps) load(p[0], s + 2);
+        if (s + 1 < steps) multiply(p[1]);
+    }
+    // the eight slices of K: partial tiles to shared memory, then a thread per (row, token) adds them in warp order
 #pragma unroll
-        for (int i = 0; i < Sh::rows / 8; ++i) {
-            const int r = r0 + wrow + 8 * i;
-            wsrc[i] = (r < E || !w_gate ? w_router + size_t(min(r, E - 1)) * n : w_gate) + kbase + wk;
-            wbytes[i] = r < rows_total ? 16u : 0u;
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) red[(warp * kTok + 8 * j + 2 * t4 + (k & 1)) * kRed + 16 * i + 8 * (k >> 1) + g] = acc[i][j][k];
+    __syncthreads();
+    for (int o = threadIdx.x; o < kRows * kTok; o += kRtWarps * 32) {
+        const int row = o % kRows, tok = o / kRows, rr = r0 + row, t = t0 + tok;   // (rows of a token are neighbours in the output)
+        const float* pr = red + tok * kRed + row;
+        float sum = pr[0];
+#pragma unroll
+        for (int w = 1; w < kRtWarps; ++w) sum += pr[w * kTok * kRed];
+        if (t < T) {
+            if (rr < E) logits[size_t(t) * E + rr] = sum;
+            else if (rr < rows_total && gate_logit) gate_logit[t] = sum;
         }
-        // the copy of one piece into its buffer: 8 float4 of x per token, 32 bf16 of W per row
-        auto fetch = [&](int piece) {
-            if (piece < pieces) {
-                const uint32_t buf = mine + (piece % Sh::depth) * Sh::piece;
-                const int k0 = kbase + piece * kRtPiece;
-#pragma unroll
-                for (int it = 0; it < Sh::tok / 4; ++it) {
-                    const int tok = it * 4 + (lane >> 3), k4 = lane & 7;
-                    const bool in = t0 + tok < T;
-                    cp_async16(buf + (tok * kRtPad + k4 * 4) * 4, x + size_t(in ? t0 + tok : 0) * n + k0 + k4 * 4, in ? 16u : 0u);
-                }
-#pragma unroll
-                for (int i = 0; i < Sh::rows / 8; ++i)
-                    cp_async16(buf + Sh::tok * kRtPad * 4 + ((wrow + 8 * i) * kRtPiece + wk) * 2, wsrc[i] + piece * kRtPiece, wbytes[i]);
-            }
-            cp_async_commit();
-        };
-        float acc[4][TJ];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < TJ; ++j) acc[i][j] = 0.0f;
-#pragma unroll
-        for (int i = 0; i < Sh::depth - 1; ++i) fetch(i);
-        for (int piece = 0; piece < pieces; ++piece) {
-            fetch(piece + Sh::depth - 1);
-            cp_async_wait<Sh::depth - 1>();
-            __syncwarp();
-            const uint8_t* buf = smem + warp * Sh::warp + (piece % Sh::depth) * Sh::piece;
-            const float* xs = reinterpret_cast<const float*>(buf);
-            const uint8_t* ws = buf + Sh::tok * kRtPad * 4;
-#pragma unroll
-            for (int k4 = 0; k4 < kRtPiece / 4; ++k4) {
-                float4 wv[4], xv[TJ];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const uint2 u = *reinterpret_cast<const uint2*>(ws + ((ry + RY * i) * kRtPiece + k4 * 4) * 2);
-                    wv[i] = make_float4(bf16_lo(u.x), bf16_hi(u.x), bf16_lo(u.y), bf16_hi(u.y));
-                }
-#pragma unroll
-                for (int j = 0; j < TJ; ++j) xv[j] = *reinterpret_cast<const float4*>(xs + (tx + Sh::tx * j) * kRtPad + k4 * 4);
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < TJ; ++j) {
-                        acc[i][j] = fmaf(wv[i].x, xv[j].x, acc[i][j]);
-                        acc[i][j] = fmaf(wv[i].y, xv[j].y, acc[i][j]);
-                        acc[i][j] = fmaf(wv[i].z, xv[j].z, acc[i][j]);
-                        acc[i][j] = fmaf(wv[i].w, xv[j].w, acc[i][j]);
-                    }
-            }
-            __syncwarp();   // the buffers are refilled by the next iteration
-        }
-        // the eight K-slices: partial tiles to shared memory (the pieces are no longer needed), then one
-        // thread per (row, token) adds them in warp order
-        cp_async_wait<0>();
-        __syncthreads();
-        float* red = reinterpret_cast<float*>(smem);   // [warp][row][token]
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < TJ; ++j) red[(warp * Sh::rows + ry + RY * i) * Sh::red + tx + Sh::tx * j] = acc[i][j];
-        __syncthreads();
-        for (int o = threadIdx.x; o < Sh::rows * Sh::tok; o += kRtWarps * 32) {
-            const int row = o % Sh::rows, tok = o / Sh::rows, rr = r0 + row, t = t0 + tok;   // (rows of a token are neighbours in the output)
-            const float* pr = red + row * Sh::red + tok;
-            float sum = pr[0];
-#pragma unroll
-            for (int w = 1; w < kRtWarps; ++w) sum += pr[w * Sh::rows * Sh::red];
-            if (t < T) {
-                if (rr < E) logits[size_t(t) * E + rr] = sum;
-                else if (rr < rows_total && gate_logit) gate_logit[t] = sum;
-            }
-        }
-        __syncthreads();
     }
 }
 
-template <int RY, int TJ>
-int router_tiles(int rows, int T) {
-    return (rows + RtShape<RY, TJ>::rows - 1) / RtShape<RY, TJ>::rows * ((T + RtShape<RY, TJ>::tok - 1) / RtShape<RY, TJ>::tok);
+template <int MT, int NT>
+constexpr int router_smem() { return kRtWarps * 8 * NT * (16 * MT + 1) * 4; }
+template <int MT, int NT>
+long long router_tiles(int rows, int T) {
+    return (long long)((rows + 16 * MT - 1) / (16 * MT)) * ((T + 8 * NT - 1) / (8 * NT));
 }
 
-template <int RY, int TJ>
+template <int MT, int NT>
 int launch_router(const uint16_t* w_router, const uint16_t* w_gate, const float* x, int T, int E, int n, float* logits, float* gate_logit, cudaStream_t stream) {
-    static std::once_flag once[64];
-    int dev = 0;
-    FRX_CUDA(cudaGetDevice(&dev));
-    cudaError_t attr = cudaSuccess;
-    if (dev >= 0 && dev < 64)
-        std::call_once(once[dev], [&] {
-            attr = cudaFuncSetAttribute(k_router_logits<RY, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, RtShape<RY, TJ>::smem);
-            // two blocks per SM: without this the SM is split for one
-            if (attr == cudaSuccess) attr = cudaFuncSetAttribute(k_router_logits<RY, TJ>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-        });
-    if (attr != cudaSuccess) return cuda_fail(attr, "frx_router_logits: cudaFuncSetAttribute");
-    const int tiles = router_tiles<RY, TJ>(E + (w_gate ? 1 : 0), T);
-    const int per_sm = std::max(1, (max_smem_optin() + 1024) / (RtShape<RY, TJ>::smem + 1024));
-    FRX_LAUNCH(kKRoute, stream, launch_pdl(k_router_logits<RY, TJ>, dim3(unsigned(std::min(tiles, per_sm * sm_count()))), dim3(kRtWarps * 32), size_t(RtShape<RY, TJ>::smem), stream,
-                                            w_router, w_gate, x, T, E, n, logits, gate_logit));
+    const long long tiles = router_tiles<MT, NT>(E + (w_gate ? 1 : 0), T);
+    if (tiles > 0x7fffffffLL) return fail(FRX_ERR_SHAPE, "frx_router_logits: %d rows x %d tokens", E, T);
+    if constexpr (router_smem<MT, NT>() > 48 * 1024) {
+        static std::once_flag once[64];
+        int dev = 0;
+        FRX_CUDA(cudaGetDevice(&dev));
+        cudaError_t attr = cudaSuccess;
+        if (dev >= 0 && dev < 64) std::call_once(once[dev], [&] { attr = cudaFuncSetAttribute(k_router_logits<MT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, router_smem<MT, NT>()); });
+        if (attr != cudaSuccess) return cuda_fail(attr, "frx_router_logits: cudaFuncSetAttribute");
+    }
+    FRX_LAUNCH(kKRoute, stream, launch_pdl(k_router_logits<MT, NT>, dim3(unsigned(tiles)), dim3(kRtWarps * 32), size_t(router_smem<MT, NT>()), stream, w_router, w_gate, x, T, E, n, logits, gate_logit));
     FRX_CUDA(cudaGetLastError());
     return FRX_OK;
 }
@@ -189,19 +189,20 @@ extern "C" int frx_router_logits(frx_stream_t stream, const void* w_router, cons
     if (T == 0) return FRX_OK;
     const auto* wr = static_cast<const uint16_t*>(w_router);
     const auto* wg = static_cast<const uint16_t*>(w_gate);
-    const int rows = E + (w_gate ? 1 : 0), sms = sm_count();
-    // few tokens: small tiles, as long as no SM gets a second one
-    if (router_tiles<2, 1>(rows, T) <= sms) return launch_router<2, 1>(wr, wg, x, T, E, n, logits, gate_logit, stream);
-    // up to eight rows leave half of a tile of 16 empty: eight rows x 64 tokens (8 experts, 16,384 tokens of 1024: 27.3 us in tiles of
-    // 16 rows, 16.7 so; 4,096 tokens of 256: 3.8 and 3.6)
-    if (rows <= 8) return launch_router<2, 4>(wr, wg, x, T, E, n, logits, gate_logit, stream);
-    // else the tile for which the busiest SM finishes first: one of 16 rows costs about TJ + 1 (measured at 37 to 1024 tokens), one of
-    // 8 x 64 about 6.5; the latter comes out ahead at 17 to 24 rows (16 experts and the gate, 6,000 tokens of 1024: 17.9 us in tiles
-    // of 16 rows, 16.7 so)
-    auto cost = [&](int tiles, int each) { return (tiles + sms - 1) / sms * each; };
-    const int c2 = cost(router_tiles<4, 2>(rows, T), 6), c3 = cost(router_tiles<4, 3>(rows, T), 8), c5 = cost(router_tiles<4, 5>(rows, T), 12);
-    if (cost(router_tiles<2, 4>(rows, T), 13) < std::min({c2, c3, c5})) return launch_router<2, 4>(wr, wg, x, T, E, n, logits, gate_logit, stream);
-    if (c2 <= c3 && c2 <= c5) return launch_router<4, 2>(wr, wg, x, T, E, n, logits, gate_logit, stream);
-    if (c3 <= c5) return launch_router<4, 3>(wr, wg, x, T, E, n, logits, gate_logit, stream);
-    return launch_router<4, 5>(wr, wg, x, T, E, n, logits, gate_logit, stream);
+    // The tile by an estimate in microseconds for every one: steps of K, and waves of a tile per SM (two of the two small ones share an SM,
+    // which their figures contain). Fitted to 128, 256 and 512 rows of 512, 2048 and 2560 at 1 to 1024 tokens, where the one that it picks is
+    // at most a tenth slower than the best.
+    const int rows = E + (w_gate ? 1 : 0);
+    const double s = n / (kRtWarps * kRtPiece), sms = std::max(sm_count(), 1);
+    auto waves = [&](long long tiles) { return std::ceil(double(tiles) / sms); };
+    const double c11 = 0.5 + 0.08 * s + (0.37 + 0.22 * s) * waves(router_tiles<1, 1>(rows, T)), c22 = 0.82 + 0.14 * s + (0.61 + 0.47 * s) * waves(router_tiles<2, 2>(rows, T)),
+                 c32 = (1.8 + 0.73 * s) * waves(router_tiles<3, 2>(rows, T)), c34 = (2.7 + 1.3 * s) * waves(router_tiles<3, 4>(rows, T));
+    // up to 16 rows have no second row tile to share the tokens with: long tiles once there are many (7 rows and the gate, 16,384 tokens of 256:
+    // 12.2 us in tiles of 16 x 8, 7.0 so; 9,000 tokens of 2560: 19.8)
+    if (rows <= 16 && router_tiles<1, 1>(rows, T) > 2 * sms) return launch_router<1, 4>(wr, wg, x, T, E, n, logits, gate_logit, stream);
+    const double least = std::min({c11, c22, c32, c34});
+    if (least == c11) return launch_router<1, 1>(wr, wg, x, T, E, n, logits, gate_logit, stream);
+    if (least == c22) return launch_router<2, 2>(wr, wg, x, T, E, n, logits, gate_logit, stream);
+    if (least == c32) return launch_router<3, 2>(wr, wg, x, T, E, n, logits, gate_logit, stream);
+    return launch_router<3, 4>(wr, wg, x, T, E, n, logits, gate_logit, stream);
 }

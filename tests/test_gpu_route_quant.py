@@ -127,6 +127,28 @@ def test_router_projection_same_bits_for_any_tile(T, E):
         assert torch.equal(one[0], logits[t]) and torch.equal(g1[0], gate[t])
 
 
+@pytest.mark.parametrize("T,E,n", [(1, 1, 256), (9, 15, 512), (33, 17, 256), (130, 511, 2560), (300, 513, 2048), (600, 512, 768), (2500, 7, 256), (9480, 15, 256)])
+def test_router_projection_keeps_every_bit_of_the_activations(T, E, n):
+    # activations with full 24-bit mantissas over the exponent range (the kernel multiplies them in three pieces of eight bits): rows from
+    # 1e-36 to 1e30, an infinity and a missing number; every tile shape, tails of rows and tokens. The pieces and products are exact, so
+    # what is left is the rounding of fp32 sums: n / 16 additions, bounded by n / 16 * 2^-24 of the sum of magnitudes; and of an activation
+    # what is below bf16's smallest subnormal number, 2^-133
+    g = torch.Generator(device="cuda").manual_seed(n + T)
+    w = torch.randn(E, n, generator=g, device="cuda").to(torch.bfloat16)
+    wg = torch.randn(n, generator=g, device="cuda").to(torch.bfloat16)
+    x = torch.randn(T, n, generator=g, device="cuda") * torch.tensor([1.0, 1e-36, 1e30, 1e-20], device="cuda")[torch.arange(T, device="cuda") % 4][:, None]
+    if T > 8:
+        x[T - 1, n // 3], x[T - 2, n - 1], x[T - 3, 0] = float("inf"), float("-inf"), float("nan")
+    logits, gate = moe.router_logits(w, wg, x)
+    ref, mag = x.double() @ torch.cat([w, wg[None]]).double().T, x.double().abs() @ torch.cat([w, wg[None]]).double().abs().T
+    got = torch.cat([logits, gate.view(T, 1)], dim=1).double()
+    lost = torch.cat([w, wg[None]]).double().abs().sum(dim=1) * 2.0 ** -133
+    bound = mag * (n / 16 * 2.0 ** -24) + lost[None] + 1e-43
+    fin = torch.isfinite(ref)
+    assert torch.equal(torch.isnan(got), torch.isnan(ref)) and torch.equal(got[~fin & ~torch.isnan(ref)], ref[~fin & ~torch.isnan(ref)])
+    assert bool(((got - ref).abs()[fin] <= bound[fin]).all())
+
+
 @pytest.mark.parametrize("n", [1, 31, 33, 512, 2048, 4095, 4096, 4097, 9000])
 def test_chain_rmsnorm_order_of_additions(n):
     rng = np.random.default_rng(n)
