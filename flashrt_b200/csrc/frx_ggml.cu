@@ -329,7 +329,7 @@ int check_dot_shape(const char* who, uint32_t type, int64_t ncols, int64_t nrows
 // [-1, 2] in the same instruction, rounded by a magic addition; x - q d rounds once in a fused multiply-add because q d
 // is exact. The codes of the chosen scale come from the same quotient enlarged by 2^-20, which takes it past a boundary
 // it lies on and past none that it does not.
-// Bound: issue slots, about 40 per value (six per value and candidate when each candidate was summed). 48 experts of
+// Bound: issue slots, about 63 per value (six per value and candidate when each candidate was summed). 48 experts of
 // 2560 x 640 (236 M values): 1.35 ms with a sum per candidate, 0.51 ms so (0.62 with candidates divided one by one, wider bounds
 // and everything unrolled, which the instruction cache did not hold).
 constexpr int kRqThreads = 128, kRqCand = 24;
