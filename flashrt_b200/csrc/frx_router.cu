@@ -38,14 +38,51 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// The three bf16 pieces of two values, packed. (An infinity is its own first piece; what is left of a number that is none is none.)
+// The three bf16 pieces of two values, packed. (What is left of an infinity is no number: see multiply_add.)
 __device__ __forceinline__ void split_pair(float a, float b, uint32_t (&p)[3]) {
     const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
     p[0] = __byte_perm(ua, ub, 0x7632);
-    const float ra = fabsf(a) == INFINITY ? 0.0f : a - __uint_as_float(ua & 0xffff0000u), rb = fabsf(b) == INFINITY ? 0.0f : b - __uint_as_float(ub & 0xffff0000u);
+    const float ra = a - __uint_as_float(ua & 0xffff0000u), rb = b - __uint_as_float(ub & 0xffff0000u);
     const uint32_t va = __float_as_uint(ra), vb = __float_as_uint(rb);
     p[1] = __byte_perm(va, vb, 0x7632);
     p[2] = __byte_perm(__float_as_uint(ra - __uint_as_float(va & 0xffff0000u)), __float_as_uint(rb - __uint_as_float(vb & 0xffff0000u)), 0x7632);
+}
+
+// One logit by fp32 multiply-adds in order, the eight slices of K each for itself and then one after the other: for a sum of
+// pieces that is not finite. An infinite weight times a piece that is zero is no number, where a multiply-add gives the infinity, and
+// 16 products together may leave the range of floats where one after the other does not. (Four slices side by side, and wide loads:
+// what takes the time is that every lane of a warp reads a row of its own. 300 tokens x 513 rows of 2560: 22 us more for one token
+// with an infinity, 80 for infinite weights in two rows, 330 if no logit is finite.)
+__device__ __noinline__ float multiply_add(const uint16_t* w, const float* x, int n) {
+    const int slice = n / kRtWarps;
+    float sum = 0.0f;
+    for (int s0 = 0; s0 < kRtWarps; s0 += 4) {
+        float acc[4] = {};
+        for (int k = 0; k < slice; k += 8) {
+            uint4 u[4];
+            float4 v[4][2];
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {
+                u[s] = __ldg(reinterpret_cast<const uint4*>(w + size_t(s0 + s) * slice + k));
+                v[s][0] = *reinterpret_cast<const float4*>(x + size_t(s0 + s) * slice + k);
+                v[s][1] = *reinterpret_cast<const float4*>(x + size_t(s0 + s) * slice + k + 4);
+            }
+            auto four = [](float& a, uint32_t lo, uint32_t hi, const float4& v) {
+                a = fmaf(__uint_as_float(lo << 16), v.x, a);
+                a = fmaf(__uint_as_float(lo & 0xffff0000u), v.y, a);
+                a = fmaf(__uint_as_float(hi << 16), v.z, a);
+                a = fmaf(__uint_as_float(hi & 0xffff0000u), v.w, a);
+            };
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {
+                four(acc[s], u[s].x, u[s].y, v[s][0]);
+                four(acc[s], u[s].z, u[s].w, v[s][1]);
+            }
+        }
+#pragma unroll
+        for (int s = 0; s < 4; ++s) sum = s0 + s ? sum + acc[s] : acc[s];
+    }
+    return sum;
 }
 
 // rows: E router rows followed by the gate row when w_gate is given (row E). W rows are n bf16 each.
@@ -144,9 +181,10 @@ __global__ void __launch_bounds__(kRtWarps * 32, MT * NT <= 4 ? 2 : 1) k_router_
         float sum = pr[0];
 #pragma unroll
         for (int w = 1; w < kRtWarps; ++w) sum += pr[w * kTok * kRed];
-        if (t < T) {
+        if (t < T && rr < rows_total) {
+            if (!(fabsf(sum) < INFINITY)) sum = multiply_add(rr < E ? w_router + size_t(rr) * n : w_gate, x + size_t(t) * n, n);
             if (rr < E) logits[size_t(t) * E + rr] = sum;
-            else if (rr < rows_total && gate_logit) gate_logit[t] = sum;
+            else gate_logit[t] = sum;
         }
     }
 }

@@ -149,6 +149,29 @@ def test_router_projection_keeps_every_bit_of_the_activations(T, E, n):
     assert bool(((got - ref).abs()[fin] <= bound[fin]).all())
 
 
+# tokens, experts and n that reach each of the five tiles on 148 SMs, with tails of rows and tokens (the gate is one row more)
+ROUTER_TILES = [(5, 99, 512), (501, 510, 512), (501, 130, 768), (301, 513, 2048), (2500, 7, 256)]
+
+
+@pytest.mark.parametrize("T,E,n", ROUTER_TILES)
+def test_router_projection_with_infinite_weights(T, E, n):
+    # activations of eight significant bits, as a bf16 residual stream has them: an infinite weight gives an infinite logit as in a
+    # multiply-add, a missing number or an infinity times zero a missing number, and no other logit changes
+    g = torch.Generator(device="cuda").manual_seed(T + E)
+    w = torch.randn(E + 1, n, generator=g, device="cuda").to(torch.bfloat16)
+    x = torch.randn(T, n, generator=g, device="cuda").to(torch.bfloat16).float()
+    x[T // 2, n // 4] = 0.0
+    x[T - 1, 3] = float("inf")
+    clean = torch.cat([a.reshape(T, -1) for a in moe.router_logits(w[:E].contiguous(), w[E], x)], dim=1)
+    w[1, n // 4], w[E - 1, n - 1], w[E - 2, 0], w[E, n // 2] = float("inf"), float("-inf"), float("nan"), float("-inf")
+    got = torch.cat([a.reshape(T, -1) for a in moe.router_logits(w[:E].contiguous(), w[E], x)], dim=1)
+    ref = x.double() @ w.double().T
+    fin = torch.isfinite(ref)
+    assert not fin[:, [1, E - 1, E - 2, E]].any() and torch.isinf(ref[:, 1]).sum() >= T - 2 and torch.isnan(ref[T // 2, 1])
+    assert torch.equal(torch.isnan(got), torch.isnan(ref)) and torch.equal(got[torch.isinf(ref)].double(), ref[torch.isinf(ref)])
+    assert torch.equal(got[fin], clean[fin])
+
+
 @pytest.mark.parametrize("n", [1, 31, 33, 512, 2048, 4095, 4096, 4097, 9000])
 def test_chain_rmsnorm_order_of_additions(n):
     rng = np.random.default_rng(n)
