@@ -7,9 +7,8 @@
 // the reference itself), so parity is to a tolerance, against a float64 sum.
 //
 // The products run on the tensor cores without losing a bit: an fp32 value is the sum of three bf16 values of eight significant
-// bits each (cut off, not rounded; of an activation below 2^-110 what is below 2^-133 is lost), so W x = W hi + W mid + W lo, every
-// product exact in fp32. Three chained MMAs of 16 K start at
-// zero and their result is added to a running fp32 sum, so what is rounded is 16 K at a time.
+// bits each (cut off, not rounded; multiply_add below has the exceptions), so W x = W hi + W mid + W lo, every product exact in fp32.
+// Three chained MMAs of 16 K start at zero and their result is added to a running fp32 sum, so what is rounded is 16 K at a time.
 //
 // A block works on a tile of 16 MT rows x 8 NT tokens; each of its 8 warps takes an eighth of K and walks it 32 at a time, straight from
 // global memory into the MMA's registers: a lane takes eight neighbouring K of a row (one 16-byte load) and of a token (two), which is
@@ -38,19 +37,23 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// The three bf16 pieces of two values, packed. (What is left of an infinity is no number: see multiply_add.)
-__device__ __forceinline__ void split_pair(float a, float b, uint32_t (&p)[3]) {
+// The three bf16 pieces of two values, packed. (What is left of an infinity is no number: see multiply_add.) `over` collects
+// the bits of the last remainders, whose lower halves are what the third piece has no place for.
+__device__ __forceinline__ void split_pair(float a, float b, uint32_t (&p)[3], uint32_t& over) {
     const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
     p[0] = __byte_perm(ua, ub, 0x7632);
     const float ra = a - __uint_as_float(ua & 0xffff0000u), rb = b - __uint_as_float(ub & 0xffff0000u);
     const uint32_t va = __float_as_uint(ra), vb = __float_as_uint(rb);
     p[1] = __byte_perm(va, vb, 0x7632);
-    p[2] = __byte_perm(__float_as_uint(ra - __uint_as_float(va & 0xffff0000u)), __float_as_uint(rb - __uint_as_float(vb & 0xffff0000u)), 0x7632);
+    const uint32_t la = __float_as_uint(ra - __uint_as_float(va & 0xffff0000u)), lb = __float_as_uint(rb - __uint_as_float(vb & 0xffff0000u));
+    p[2] = __byte_perm(la, lb, 0x7632);
+    over |= la | lb;
 }
 
-// One logit by fp32 multiply-adds in order, the eight slices of K each for itself and then one after the other: for a sum of
-// pieces that is not finite. An infinite weight times a piece that is zero is no number, where a multiply-add gives the infinity, and
-// 16 products together may leave the range of floats where one after the other does not. (Four slices side by side, and wide loads:
+// One logit by fp32 multiply-adds in order, the eight slices of K each for itself and then one after the other, for what three bf16
+// pieces cannot do. A sum that is not finite: an infinite weight times a piece that is zero is no number, where a multiply-add gives the
+// infinity, and 16 products together may leave the range of floats where one after the other does not. And a token with an activation
+// below 2^-110 whose third piece would need bits below 2^-133, bf16's smallest number. (Four slices side by side, and wide loads:
 // what takes the time is that every lane of a warp reads a row of its own. 300 tokens x 513 rows of 2560: 22 us more for one token
 // with an infinity, 80 for infinite weights in two rows, 330 if no logit is finite.)
 __device__ __noinline__ float multiply_add(const uint16_t* w, const float* x, int n) {
@@ -122,6 +125,7 @@ __global__ void __launch_bounds__(kRtWarps * 32, MT * NT <= 4 ? 2 : 1) k_router_
 #pragma unroll
             for (int h = 0; h < 2; ++h) p.x[j][h] = *(reinterpret_cast<const float4*>(xp[j] + s * kRtPiece) + h);
     };
+    uint32_t over[NT] = {};
     float acc[MT][NT][4];
 #pragma unroll
     for (int i = 0; i < MT; ++i)
@@ -135,8 +139,8 @@ __global__ void __launch_bounds__(kRtWarps * 32, MT * NT <= 4 ? 2 : 1) k_router_
             uint32_t b[NT][2][3];
 #pragma unroll
             for (int j = 0; j < NT; ++j) {
-                split_pair(p.x[j][h].x, p.x[j][h].y, b[j][0]);
-                split_pair(p.x[j][h].z, p.x[j][h].w, b[j][1]);
+                split_pair(p.x[j][h].x, p.x[j][h].y, b[j][0], over[j]);
+                split_pair(p.x[j][h].z, p.x[j][h].w, b[j][1], over[j]);
             }
 #pragma unroll
             for (int i = 0; i < MT; ++i) {
@@ -166,6 +170,17 @@ __global__ void __launch_bounds__(kRtWarps * 32, MT * NT <= 4 ? 2 : 1) k_router_
         multiply(p[0]);
         if (s + 2 < steps) load(p[0], s + 2);
         if (s + 1 < steps) multiply(p[1]);
+    }
+    // tokens with an activation that three pieces do not hold get no number, for multiply_add below
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+        const uint32_t lanes = __ballot_sync(0xffffffffu, over[j] & 0xffffu);   // four lanes a token
+        if (lanes)
+#pragma unroll
+            for (int i = 0; i < MT; ++i)
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (lanes >> 4 * (2 * t4 + (k & 1)) & 15u) acc[i][j][k] = NAN;
     }
     // the eight slices of K: partial tiles to shared memory, then a thread per (row, token) adds them in warp order
 #pragma unroll

@@ -172,6 +172,43 @@ def test_router_projection_with_infinite_weights(T, E, n):
     assert torch.equal(got[fin], clean[fin])
 
 
+@pytest.mark.parametrize("T,E,n", ROUTER_TILES)
+def test_router_projection_one_activation_comes_through_whole(T, E, n):
+    # a token with one activation, of 24 significant bits and any exponent down to the smallest subnormal number, and rows of one weight,
+    # +1 or -1, at a place of their own: the logit is that activation, to the bit, or zero
+    g = torch.Generator(device="cuda").manual_seed(T + n)
+    places = torch.randint(0, n, (T,), generator=g, device="cuda")
+    bits = torch.randint(0, 255 << 23, (T,), generator=g, device="cuda", dtype=torch.int32)   # all finite magnitudes
+    bits[::3] = torch.randint(1, 40 << 23, bits[::3].shape, generator=g, device="cuda", dtype=torch.int32)   # below 2^-87
+    bits[:3] = torch.tensor([1, (1 << 23) - 1, (255 << 23) - 1], device="cuda")
+    v = (bits | torch.randint(0, 2, (T,), generator=g, device="cuda", dtype=torch.int32) << 31).view(torch.float32)
+    x = torch.zeros(T, n, device="cuda").scatter_(1, places[:, None], v[:, None])
+    rows = torch.randint(0, n, (E + 1,), generator=g, device="cuda")
+    rows[::2] = places[torch.arange(0, E + 1, 2, device="cuda") % T]   # so that some meet
+    sign = torch.randint(0, 2, (E + 1,), generator=g, device="cuda").float() * 2 - 1
+    w = torch.zeros(E + 1, n, device="cuda").scatter_(1, rows[:, None], sign[:, None]).to(torch.bfloat16)
+    got = torch.cat([a.reshape(T, -1) for a in moe.router_logits(w[:E].contiguous(), w[E], x)], dim=1)
+    want = torch.where(places[:, None] == rows[None, :], v[:, None] * sign[None, :], torch.zeros((), device="cuda"))
+    assert (want != 0).sum() >= min(T, E) // 2 and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("exponent", [-109, -112, -118, -124, -130])
+@pytest.mark.parametrize("T,E,n", ROUTER_TILES)
+def test_router_projection_of_small_activations(T, E, n, exponent):
+    # below 2^-110 a third piece of eight bits would be below bf16's smallest number. fp32 products and sums in eight slices one after the
+    # other: n / 8 + 7 additions of at most 2^-24 of the magnitudes, or of half the smallest subnormal number
+    g = torch.Generator(device="cuda").manual_seed(T + E + exponent)
+    w = torch.randn(E + 1, n, generator=g, device="cuda").to(torch.bfloat16)
+    x = torch.randn(T, n, generator=g, device="cuda")
+    x[1::2] *= 2.0 ** exponent
+    x[0, 1:] *= 2.0 ** exponent   # small ones beside an ordinary one
+    got = torch.cat([a.reshape(T, -1) for a in moe.router_logits(w[:E].contiguous(), w[E], x)], dim=1).double()
+    ref, mag = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    assert ((got - ref).abs() <= (n // 8 + 7) * (mag * 2.0 ** -24 + 2.0 ** -150)).all()
+    small = (got - ref)[1::2].norm() / ref[1::2].norm()
+    assert small < 2e-6 + 2.0 ** (-148 - exponent)   # (three pieces alone: 2^(-135 - exponent) and more)
+
+
 @pytest.mark.parametrize("n", [1, 31, 33, 512, 2048, 4095, 4096, 4097, 9000])
 def test_chain_rmsnorm_order_of_additions(n):
     rng = np.random.default_rng(n)
