@@ -161,6 +161,8 @@ __global__ void __launch_bounds__(256) k_pfu_expand_q8(const int8_t* __restrict_
 
 // silu(g) * u with the fast exponential and reciprocal, within kSwigluErr of swiglu_ref for g >= -80: ex2 and rcp are good to 2^-22 and
 // 2^-23 (PTX ISA), -g log2 e rounds by at most 2^-24 of 116, which the exponential makes 2^-17.6, three more roundings.
+// silu(g) leaves the normal numbers only for |g| < 2^-125. There -g log2 e is flushed to zero or next to it, the exponential is 1, the
+// reciprocal of 2 is exact (as run, not as documented) and g / 2 is rounded alike in both forms, so that no u can bring a difference back.
 constexpr float kSwigluErr = 0x1p-16f;
 __device__ __forceinline__ float swiglu_fast(float g, float u) {
     float e, r;
@@ -216,7 +218,7 @@ __global__ void __launch_bounds__(256) k_pfu_quant_h(const float2* __restrict__ 
 #pragma unroll
     for (int i = 0; i < 8; ++i) am = fmaxf(am, fabsf(hv[i]));
     am = block_max(am);
-    // (no number, none at all, and so large or small that an intermediate of the fast form may leave the range of floats: everything exactly)
+    // (no number, none at all, and so large or small that a product of the fast form may have left the range of floats: everything exactly)
     if (!(am > 1e-25f && am < 1e25f)) ask = 0xffu;
     const float lim = am * (1.0f - 4.0f * kSwigluErr);
 #pragma unroll
@@ -871,6 +873,21 @@ int frx_moe_prefill_umma(const void* experts, size_t stride, int E, int n, int f
     return frx_moe_prefill_umma_ex(experts, stride, E, n, ff, x, ids, T, K, yd, ws, ws_bytes, stream, 0, 0);
 }
 
+static void quant_h(const float2* hf, const int* n_rows, int max_rows, int ff, uint8_t* he, float* hd, int block64, frx_stream_t stream) {
+    const size_t groups = size_t(max_rows) * size_t(ff / 8);
+    FRX_LAUNCH(kKQuant, stream, launch_pdl(k_pfu_quant_h, dim3(unsigned((groups + 255) / 256)), dim3(256), 0, stream, hf, ff, n_rows, he, hd, block64));
+}
+
+int frx_debug_quantize_hidden(const float* pairs, const int* n_rows, int max_rows, int ff, void* pieces, float* scales, int block64, frx_stream_t stream) {
+    if (!pairs || !n_rows || !pieces || !scales) return fail(FRX_ERR_ARG, "frx_debug_quantize_hidden: null pointer");
+    if (max_rows < 0 || max_rows > 1 << 20 || ff < kUnitK || ff % kUnitK || ff > 8192) return fail(FRX_ERR_SHAPE, "frx_debug_quantize_hidden: %d rows of %d", max_rows, ff);
+    if ((uintptr_t(pairs) | uintptr_t(pieces)) % 16 || uintptr_t(scales) % 4) return fail(FRX_ERR_ARG, "frx_debug_quantize_hidden: pairs and pieces must be 16-byte aligned");
+    if (max_rows == 0) return FRX_OK;
+    quant_h(reinterpret_cast<const float2*>(pairs), n_rows, max_rows, ff, static_cast<uint8_t*>(pieces), scales, block64, stream);
+    FRX_CUDA(cudaGetLastError());
+    return FRX_OK;
+}
+
 static int prefill_umma_impl(const void* experts, size_t stride, int E, const int32_t* e_map, int E_all, int n, int ff, const float* x,
                              const int8_t* xq_in, const float* xd_in, const int32_t* ids, int T, int K, void* yd, void* ws, size_t ws_bytes,
                              frx_stream_t stream, int block64, int yd_bf16) {
@@ -927,9 +944,7 @@ static int prefill_umma_impl(const void* experts, size_t stride, int E, const in
     p.act = xe;
     p.act_scale = xq_in ? xd_in : xd;
     FRX_LAUNCH(kKGateUp, stream, launch_pdl(k_pf_umma<true>, blocks, dim3(kThreads), pf_smem().total, stream, p));
-    const size_t groups = size_t(S) * size_t(ff / 8);
-    FRX_LAUNCH(kKQuant, stream, launch_pdl(k_pfu_quant_h, dim3(unsigned((groups + 255) / 256)), dim3(256), 0, stream, (const float2*)p.hf, ff, (const int*)(bounds + E), base + L.he,
-                                           reinterpret_cast<float*>(base + L.hd), block64));
+    quant_h(p.hf, bounds + E, S, ff, base + L.he, reinterpret_cast<float*>(base + L.hd), block64, stream);
     p.act = base + L.he;
     p.act_scale = reinterpret_cast<const float*>(base + L.hd);
     FRX_LAUNCH(kKDown, stream, launch_pdl(k_pf_umma<false>, blocks, dim3(kThreads), pf_smem().total, stream, p));

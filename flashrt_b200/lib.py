@@ -95,6 +95,7 @@ SIGNATURES = {
     "frx_debug_set_ffn_buffers": (_i, [_i, _i]),
     "frx_debug_set_small_tokens": (_i, [_i]),
     "frx_debug_set_wait_limit_ns": (_i, [C.c_ulonglong]),
+    "frx_debug_quantize_hidden": (_i, [_vp, _vp, _i, _i, _vp, _vp, _i, _vp]),
     "frx_moe_decode_static_status": (_i, [_vp]),
     "frx_moe_layer_ep_allreduce": (_i, [_vp, _sz, _i, _i, _i, _vp, _i, _i, _vp, _vp, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
     "frx_moe_layer_ep_allreduce_dealt": (_i, [_vp, _sz, _i, _i, _i, _vp, _i, _i, _i, _i, _vp, _vp, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),

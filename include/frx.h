@@ -112,6 +112,12 @@ int frx_debug_set_stream_stamps(void* device_buffer);
 int frx_debug_set_small_tokens(int tokens);
 int frx_debug_set_ffn_buffers(int gate_up, int down);
 int frx_debug_set_wait_limit_ns(unsigned long long ns);
+/* The hidden-row quantizer of the tensor-memory prefill form on its own: pairs [max_rows][ff][2] (gate x, up x), of which the first
+ * *n_rows rows (device, at most max_rows) are taken; pieces [rows][ff / 64][128 bytes] and scales [rows][ff / 32] as its down product
+ * reads them. The code of element 32 s + 16 q + 4 t + i of 64 is the sum of the e4m3 bytes 64 s + 32 p + 16 (t / 2) + 8 (t % 2) + 4 q + i
+ * for p = 0 and 1. ff a multiple of 128, pointers 16-byte aligned. */
+int frx_debug_quantize_hidden(const float* pairs, const int* n_rows, int max_rows, int ff, void* pieces, float* scales, int block64,
+                              frx_stream_t stream);
 
 /* ---- Q2_0 storage (quant/q2_0/q2_0.hpp:27-56, quant/q2_0/q2_0.cpp:43-71) ---- */
 

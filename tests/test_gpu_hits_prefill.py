@@ -161,11 +161,89 @@ def test_hidden_quantizer_where_rows_end_inside_a_warp(port, S, block64):
     assert torch.equal(got, want)
 
 
+def hidden_codes(pairs, block):
+    """The quantizer of hidden rows restated: fp32 silu(g) * u with a correctly rounded exponential, d = amax / 127, id = 1 / d,
+    codes to the nearest integer, halves away from zero; missing numbers have code 0 and no part in the maximum."""
+    f32 = np.float32
+    g, u = pairs[..., 0], pairs[..., 1]
+    with np.errstate(all="ignore"):
+        h = (g / (f32(1) + np.exp(-g.astype(np.float64)).astype(f32)) * u).reshape(len(g), -1, block)
+        d = np.fmax.reduce(np.abs(h), axis=-1, keepdims=True, initial=f32(0)) / f32(127)
+        c = h * np.where(d != 0, f32(1) / d, f32(0))
+        t = np.trunc(c)
+        code = np.nan_to_num(np.where(np.abs(c - t) >= 0.5, t + np.copysign(f32(1), c), t)).reshape(g.shape)
+        scale = np.repeat(d[..., 0].astype(np.float16).astype(f32), block // 32, axis=-1)
+    assert h.dtype == d.dtype == c.dtype == f32
+    return code, scale, np.broadcast_to(d, h.shape).reshape(g.shape)
+
+
+def hidden_rows(kind, R, ff, rng):
+    """(gate x, up x) pairs [R][ff][2]: the values that decide which of the quantizer's values are formed how."""
+    g, u = rng.normal(0, 3, (R, ff)), rng.normal(0, 1, (R, ff))
+    some = rng.random((R, ff)) < 0.3
+    sign = rng.choice([-1.0, 1.0], (R, ff))
+    if kind == "steep":                    # gates to beyond both ends of the exponential's range
+        g *= 40
+    elif kind == "rounding":               # codes next to, and on, the halves: silu(g) = g from 17 on
+        g, u = np.where(rng.random((R, ff)) < 0.1, 127.0, rng.integers(17, 127, (R, ff)) + 0.5), sign * (1 + rng.integers(-2, 3, (R, ff)) * 2.0 ** -23)
+    elif kind == "last of the exponential":
+        g, u = rng.uniform(-95, -70, (R, ff)), sign * 10 ** rng.uniform(8, 12, (R, ff))
+    elif kind == "tiny gates":             # silu(g) below the normal numbers, brought back by u
+        tiny = np.where(rng.random((R, ff)) < 0.5, rng.integers(1, 64, (R, ff)) * 2.0 ** -149, 10 ** rng.uniform(-44.5, -37, (R, ff)))
+        g, u = np.where(some, sign * tiny, g), np.where(some, 10 ** rng.uniform(13, 38, (R, ff)), u * 1e-6)
+    elif kind == "small":                  # block maxima around 1e-25 and down to where d is no normal number
+        g, u = g * 1e-13, u * 10 ** rng.uniform(-26, -11, (R, 1))
+    elif kind == "large":                  # around 1e25 and beyond the floats
+        g, u = np.abs(g) * 1e12, u * 10 ** rng.uniform(11, 27, (R, 1))
+    elif kind == "zeros":                  # whole blocks, whole rows, and blocks with a single value
+        g[:, :ff // 2] = 0
+        g[R // 2:] = sign[R // 2:] * 0.0
+        u[: R // 4, ff // 2:] = 0
+        g[R // 2:, 5::64] = 2.0
+    elif kind == "equal":                  # every value may be the largest
+        g[:], u = 3.0, sign
+    elif kind == "not finite":             # one in every third block
+        g = np.abs(g) + 0.1                # (an infinite up x times a positive gate)
+        for i, j in zip(*np.nonzero(rng.random((R, ff // 32)) < 0.33)):
+            (g if rng.random() < 0.5 else u)[i, 32 * j + rng.integers(32)] = rng.choice([np.inf, -np.inf, np.nan])
+    else:
+        assert kind == "ordinary"
+    return np.stack([g, u], axis=-1).astype(np.float32)
+
+
+@pytest.mark.parametrize("block", [32, 64])
+@pytest.mark.parametrize("kind", ["ordinary", "steep", "rounding", "last of the exponential", "tiny gates", "small", "large", "zeros", "equal", "not finite"])
+def test_hidden_quantizer_codes(kind, block):
+    from flashrt_b200.lib import check, lib
+    R, ff = 4001, 384
+    pairs = hidden_rows(kind, R, ff, np.random.default_rng(5))
+    pieces = torch.full((R + 3, ff // 64, 128), 0x55, dtype=torch.uint8, device="cuda")
+    scales = torch.full((R + 3, ff // 32), -7.0, device="cuda")
+    x, n_rows = cuda(np.concatenate([pairs, pairs[:3]])), torch.tensor([R], dtype=torch.int32, device="cuda")
+    check(lib.frx_debug_quantize_hidden(x.data_ptr(), n_rows.data_ptr(), R + 3, ff, pieces.data_ptr(), scales.data_ptr(), int(block == 64),
+                                        torch.cuda.current_stream().cuda_stream))
+    assert (pieces[R:] == 0x55).all() and (scales[R:] == -7).all()   # rows that are not there
+    # bytes [s][piece][t / 2][t % 2][q][i] -> elements [s][q][t][i]
+    b = pieces[:R].cpu().view(torch.float8_e4m3fn).float().view(R, ff // 64, 2, 2, 2, 2, 2, 4).sum(dim=3)
+    got = b.permute(0, 1, 2, 5, 3, 4, 6).reshape(R, ff).numpy()
+    want, scale, d = hidden_codes(pairs, block)
+    assert np.array_equal(scales[:R].cpu().numpy(), scale)
+    sure = d >= 2.0 ** -126   # below, 1 / d may be none, and the scale is 0 as fp16
+    assert sure.any() and np.array_equal(got[sure], want[sure])
+    if kind not in ("not finite", "large"):
+        assert (np.abs(want[sure]).max(initial=0) == 127) and (kind == "zeros" or (want[sure] != 0).mean() > 0.1)
+    if kind in ("ordinary", "steep", "rounding"):   # an exponential that is off by 2^-18 would show
+        off = pairs.copy()
+        off[..., 1] *= np.random.default_rng(6).choice(np.float32([1 - 2.0 ** -18, 1 + 2.0 ** -18]), off.shape[:2])
+        assert (hidden_codes(off, block)[0] != want).sum() > 10
+
+
 @pytest.mark.parametrize("block64", [False, True])
 @pytest.mark.parametrize("spread", [0.02, 8.0, 6e4, "special"])
 def test_hidden_quantizer_over_the_range_of_the_swiglu(port, spread, block64):
-    # gate values from a few units (where codes lie next to rounding boundaries) to beyond the exponential's range, products beyond that of
-    # floats, rows of zeros, infinite and missing numbers: the codes are those of the exact SwiGLU, to the bit
+    # the whole product against the form that computes the exact SwiGLU for every value, gate values from a few units to beyond the
+    # exponential's range. Scales pass through fp16, so rows of large values come out as missing numbers and rows of small ones as zeros
+    # (all of them in "special"): what this shows for those is that they do so in both forms. test_hidden_quantizer_codes has the codes.
     n, ff, E, S = 256, 384, 2, 333
     rng = np.random.default_rng(11)
     planar = np.zeros((E, moe.expert_bytes(n, ff)), np.uint8)
