@@ -209,6 +209,31 @@ def test_router_projection_of_small_activations(T, E, n, exponent):
     assert small < 2e-6 + 2.0 ** (-148 - exponent)   # (three pieces alone: 2^(-135 - exponent) and more)
 
 
+@pytest.mark.parametrize("T,E,n", [(1, 64, 512), (37, 512, 2048), (293, 130, 2560), (2500, 7, 256)])
+def test_router_projection_of_activations_that_are_rewritten_in_place(T, E, n):
+    # the kernel in front writes x, lets the projection start early, and the next step writes the same addresses again; directly and replayed
+    g = torch.Generator(device="cuda").manual_seed(T)
+    w = torch.randn(E, n, generator=g, device="cuda").to(torch.bfloat16)
+    src = torch.randn(12, T, n, generator=g, device="cuda")
+    zero, x = torch.zeros(T, n, device="cuda"), torch.empty(T, n, device="cuda")
+    want = [moe.router_logits(w, w[0], moe.chain_rmsnorm_unit(s, zero)) for s in src]
+    torch.cuda.synchronize()
+
+    def steps():
+        return [moe.router_logits(w, w[0], moe.chain_rmsnorm_unit(s, zero, out=x)) for s in src]
+
+    for _ in range(3):
+        got = steps()
+        assert all(torch.equal(a, b) for p, q in zip(got, want) for a, b in zip(p, q))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = steps()
+    src.copy_(src.flip(0))
+    for _ in range(2):
+        graph.replay()
+    assert all(torch.equal(a, b) for p, q in zip(got, reversed(want)) for a, b in zip(p, q))
+
+
 @pytest.mark.parametrize("n", [1, 31, 33, 512, 2048, 4095, 4096, 4097, 9000])
 def test_chain_rmsnorm_order_of_additions(n):
     rng = np.random.default_rng(n)
