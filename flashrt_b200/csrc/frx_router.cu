@@ -96,7 +96,10 @@ template <int MT, int NT>
 __global__ void __launch_bounds__(kRtWarps * 32, MT * NT <= 4 ? 2 : 1) k_router_logits(const uint16_t* __restrict__ w_router, const uint16_t* __restrict__ w_gate,
                                                                   const float* x, int T, int E, int n,
                                                                   float* __restrict__ logits, float* __restrict__ gate_logit) {
-    constexpr int kRows = 16 * MT, kTok = 8 * NT, kRed = kRows + 1;   // partial sums are kept per token: [token][row], odd rows
+    // Partial sums are kept per token: [token][row]. With rows of 4 more than a multiple of 16, the four tokens x eight rows that a warp
+    // stores at a time fall into 32 banks (odd rows put up to four in one; 513 rows of 512, 293 tokens 5.7 -> 5.2 us, 8,192
+    // tokens 97 -> 91; of 2560 16.6 -> 16.5).
+    constexpr int kRows = 16 * MT, kTok = 8 * NT, kRed = kRows + 4;
     extern __shared__ float red[];   // [warp][token][row]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
     const int rows_total = E + (w_gate ? 1 : 0), row_tiles = (rows_total + kRows - 1) / kRows;
@@ -208,7 +211,7 @@ __global__ void __launch_bounds__(kRtWarps * 32, MT * NT <= 4 ? 2 : 1) k_router_
 }
 
 template <int MT, int NT>
-constexpr int router_smem() { return kRtWarps * 8 * NT * (16 * MT + 1) * 4; }
+constexpr int router_smem() { return kRtWarps * 8 * NT * (16 * MT + 4) * 4; }
 template <int MT, int NT>
 long long router_tiles(int rows, int T) {
     return (long long)((rows + 16 * MT - 1) / (16 * MT)) * ((T + 8 * NT - 1) / (8 * NT));
