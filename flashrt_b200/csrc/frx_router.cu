@@ -249,6 +249,22 @@ int launch_router(const uint16_t* w_router, const uint16_t* w_gate, const float*
     return FRX_OK;
 }
 
+// The tile for `rows` rows (the gate's among them), as 10 MT + NT.
+int router_tile(int rows, int T, int n, int sm_number) {
+    // The tile by an estimate in microseconds for every one: steps of K, and waves of a tile per SM (two of the two small ones share an SM,
+    // which their figures contain). Fitted to 128, 256 and 512 rows of 512, 2048 and 2560 at 1 to 1024 tokens. Of 932 points with 8 to
+    // 2048 rows of 256 to 7168 and 1 to 8192 tokens the one that it picks is 0.9 % slower than the best on average and 14 % at most.
+    const double s = n / (kRtWarps * kRtPiece), sms = std::max(sm_number, 1);
+    auto waves = [&](long long tiles) { return std::ceil(double(tiles) / sms); };
+    const double c11 = 0.5 + 0.08 * s + (0.37 + 0.22 * s) * waves(router_tiles<1, 1>(rows, T)), c22 = 0.82 + 0.14 * s + (0.61 + 0.47 * s) * waves(router_tiles<2, 2>(rows, T)),
+                 c32 = (1.8 + 0.73 * s) * waves(router_tiles<3, 2>(rows, T)), c34 = (2.7 + 1.3 * s) * waves(router_tiles<3, 4>(rows, T));
+    // up to 16 rows have no second row tile to share the tokens with: long tiles once there are many (7 rows and the gate, 16,384 tokens of 256:
+    // 12.2 us in tiles of 16 x 8, 7.0 so; 9,000 tokens of 2560: 19.8)
+    if (rows <= 16 && router_tiles<1, 1>(rows, T) > 2 * sms) return 14;
+    const double least = std::min({c11, c22, c32, c34});
+    return least == c11 ? 11 : least == c22 ? 22 : least == c32 ? 32 : 34;
+}
+
 }  // namespace
 }  // namespace frx
 
@@ -263,20 +279,17 @@ extern "C" int frx_router_logits(frx_stream_t stream, const void* w_router, cons
     if (T == 0) return FRX_OK;
     const auto* wr = static_cast<const uint16_t*>(w_router);
     const auto* wg = static_cast<const uint16_t*>(w_gate);
-    // The tile by an estimate in microseconds for every one: steps of K, and waves of a tile per SM (two of the two small ones share an SM,
-    // which their figures contain). Fitted to 128, 256 and 512 rows of 512, 2048 and 2560 at 1 to 1024 tokens, where the one that it picks is
-    // at most a tenth slower than the best.
-    const int rows = E + (w_gate ? 1 : 0);
-    const double s = n / (kRtWarps * kRtPiece), sms = std::max(sm_count(), 1);
-    auto waves = [&](long long tiles) { return std::ceil(double(tiles) / sms); };
-    const double c11 = 0.5 + 0.08 * s + (0.37 + 0.22 * s) * waves(router_tiles<1, 1>(rows, T)), c22 = 0.82 + 0.14 * s + (0.61 + 0.47 * s) * waves(router_tiles<2, 2>(rows, T)),
-                 c32 = (1.8 + 0.73 * s) * waves(router_tiles<3, 2>(rows, T)), c34 = (2.7 + 1.3 * s) * waves(router_tiles<3, 4>(rows, T));
-    // up to 16 rows have no second row tile to share the tokens with: long tiles once there are many (7 rows and the gate, 16,384 tokens of 256:
-    // 12.2 us in tiles of 16 x 8, 7.0 so; 9,000 tokens of 2560: 19.8)
-    if (rows <= 16 && router_tiles<1, 1>(rows, T) > 2 * sms) return launch_router<1, 4>(wr, wg, x, T, E, n, logits, gate_logit, stream);
-    const double least = std::min({c11, c22, c32, c34});
-    if (least == c11) return launch_router<1, 1>(wr, wg, x, T, E, n, logits, gate_logit, stream);
-    if (least == c22) return launch_router<2, 2>(wr, wg, x, T, E, n, logits, gate_logit, stream);
-    if (least == c32) return launch_router<3, 2>(wr, wg, x, T, E, n, logits, gate_logit, stream);
-    return launch_router<3, 4>(wr, wg, x, T, E, n, logits, gate_logit, stream);
+    switch (router_tile(E + (w_gate ? 1 : 0), T, n, sm_count())) {
+        case 11: return launch_router<1, 1>(wr, wg, x, T, E, n, logits, gate_logit, stream);
+        case 14: return launch_router<1, 4>(wr, wg, x, T, E, n, logits, gate_logit, stream);
+        case 22: return launch_router<2, 2>(wr, wg, x, T, E, n, logits, gate_logit, stream);
+        case 32: return launch_router<3, 2>(wr, wg, x, T, E, n, logits, gate_logit, stream);
+        default: return launch_router<3, 4>(wr, wg, x, T, E, n, logits, gate_logit, stream);
+    }
+}
+
+extern "C" int frx_router_logits_tile(int T, int rows, int n, int sms) {
+    if (T < 1 || rows < 1 || n < 256 || n % 256 || sms < 0) return 0;
+    const int tile = router_tile(rows, T, n, sms ? sms : sm_count());
+    return tile / 10 * 16 * 100 + tile % 10 * 8;
 }

@@ -72,6 +72,7 @@ SIGNATURES = {
     "frx_gguf_tensor": (_i, [_vp, C.c_char_p, _vp, _vp, _vp, _vp, _vp]),
     "frx_arena_load_gguf": (_i, [_vp, _vp, _i, _i, _i, _i, _i, _vp, _vp, _vp]),
     "frx_router_logits": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _vp, _vp]),
+    "frx_router_logits_tile": (_i, [_i, _i, _i, _i]),
     "frx_moe_layer_ep": (_i, [_vp, _sz, _i, _i, _i, _vp, _i, _i, _vp, _vp, _vp, _i, _i, _vp, _vp, _vp, _vp, _sz, _vp]),
     "frx_ep_buffer_bytes": (_sz, [_i, _i]),
     "frx_ep_flags_offset": (_sz, [_i, _i]),

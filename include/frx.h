@@ -274,6 +274,9 @@ int frx_arena_load_gguf(frx_arena* a, const frx_gguf* g, int layer0, int n_layer
  * frx_moe_layer takes. n a multiple of 256 (as in the reference), pointers 16-byte aligned. */
 int frx_router_logits(frx_stream_t stream, const void* w_router, const void* w_gate, const float* x, int T, int E, int n,
                       float* logits, float* gate_logit);
+/* The tile that frx_router_logits takes for T tokens and `rows` rows (E, and one for the gate) of n on a device with `sms` SMs (0:
+ * this one): 100 * its rows + its tokens; 0 for a shape that it does not take. A token's logits are the same bits in every tile. */
+int frx_router_logits_tile(int T, int rows, int n, int sms);
 
 /* Router + layer in one call: logits [T][E] -> top-K -> frx_moe_decode. ids_out / wts_out [T][K]
  * (may be null) receive the routing. Workspace: frx_moe_layer_workspace_bytes. */
