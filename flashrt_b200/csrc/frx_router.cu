@@ -8,7 +8,9 @@
 //
 // The products run on the tensor cores without losing a bit: an fp32 value is the sum of three bf16 values of eight significant
 // bits each (cut off, not rounded; multiply_add below has the exceptions), so W x = W hi + W mid + W lo, every product exact in fp32.
-// Three chained MMAs of 16 K start at zero and their result is added to a running fp32 sum, so what is rounded is 16 K at a time.
+// Three chained MMAs of 16 K start at zero and their result is added to a running fp32 sum: exact products, and four sums per 16 K that may
+// round (an MMA in a way that PTX leaves open). Relative error against float64, 2-norm: 1.1e-7 for 2560 terms, 3.2e-7 with 320 multiply-adds
+// in a row.
 //
 // A block works on a tile of 16 MT rows x 8 NT tokens; each of its 8 warps takes an eighth of K and walks it 32 at a time, straight from
 // global memory into the MMA's registers: a lane takes eight neighbouring K of a row (one 16-byte load) and of a token (two), which is
@@ -16,9 +18,8 @@
 // (fixed, so results are reproducible and do not depend on the tile).
 // Bound: the latency of a step (a load from the L2, the split, chains of three MMAs) with two pieces in flight, and for many tokens what the
 // L2 delivers (all blocks together read x once per row tile and W once per token tile: 63 MB at 293 tokens in tiles of 48 x 32, 200 MB in
-// tiles of 16 x 8). 513 rows of 2560, us: 1 token 6.1 ->
-// 3.8, 37 tokens 9.2 -> 5.4, 293 tokens 29.5 -> 16.8, 1024 tokens 87 -> 45 (before: multiply-adds from shared memory). Error against float64,
-// relative 2-norm: 1.1e-7, 3.2e-7 before (320 additions in a row).
+// tiles of 16 x 8). 513 rows of 2560, us, against multiply-adds from shared memory: 1 token 6.1 -> 3.7, 37 tokens 9.1 -> 5.2, 293 tokens
+// 29.3 -> 15.8, 1024 tokens 87.5 -> 39.3.
 #include "frx_common.cuh"
 
 #include <algorithm>
