@@ -229,8 +229,8 @@ __global__ void __launch_bounds__(kRtWarps * 32, MT * NT <= 4 ? 2 : 1) k_router_
 template <int MT, int NT>
 constexpr int router_smem() { return kRtWarps * 8 * NT * (16 * MT + 4) * 4; }
 template <int MT, int NT>
-long long router_tiles(int rows, int T) {
-    return (long long)((rows + 16 * MT - 1) / (16 * MT)) * ((T + 8 * NT - 1) / (8 * NT));
+long long router_tiles(long long rows, long long T) {
+    return (rows + 16 * MT - 1) / (16 * MT) * ((T + 8 * NT - 1) / (8 * NT));
 }
 
 template <int MT, int NT>
